@@ -107,10 +107,22 @@ constexpr int CAMTAB = 56;  // doubles per camera table entry (CamTab)
 constexpr int CAMTAB32 = 40;  // floats per FP32 camera table entry: M, D, fx, sk, fy (the mixed Jacobian)
 constexpr int RES_TAB2F = 18;  // FP32 pairs per camera of the mixed projection: M, t, fx sk cx fy cy, a pad (16-byte rows)
 constexpr int TILE = 16;    // dense Cholesky tile size
-constexpr int SCHUR_CHUNK = 32;  // pair-list entries per off-diagonal Schur work unit (11/16-parameter cameras)
-constexpr int OFF_MIN_LEN = 8;   // 6-parameter cameras: fewest pair-list entries per off-diagonal chunk
+constexpr int SCHUR_CHUNK = 32;  // pair-list entries an off-diagonal unit stages at a time (11/16-parameter cameras, FP32)
 constexpr int MX_UNIT = 256;     // 6-parameter cameras, FP32 products: pair-list entries per warp unit
-constexpr int DIAG_CHUNK = 16;   // observations per diagonal Schur work unit (11/16-parameter cameras)
+constexpr int DIAG_CHUNK = 16;   // observations a diagonal unit stages at a time (11/16-parameter cameras, FP32)
+// Entries of an off-diagonal Schur unit and observations of a diagonal one
+// (FP64 products; both forms with 11/16-parameter cameras).  A unit writes one
+// partial block, which the reduction reads back, so units are as long as
+// leaves enough of them to fill the GPU's resident warps (cnp 6, a warp each)
+// or CTAs (cnp 11/16) several times over.  Multiples of 32: whole chunks of
+// the fixed-point products, and FP32 groups that do not depend on the length.
+inline int unit_len(long long n, long long units, int most)
+{
+    const long long len = ((n / units + 31) / 32) * 32;
+    return (int)(len < 32 ? 32 : len > most ? most : len);
+}
+inline int off_unit_len(int cnp, long long entries) { return unit_len(entries, cnp == 6 ? 8192 : 4096, cnp == 6 ? 256 : 512); }
+inline int diag_unit_len(int cnp, long long obs) { return unit_len(obs, cnp == 6 ? 4096 : 2048, 256); }
 constexpr int SD_THREADS = 128, SD_PER = 8;     // 6-parameter cameras: one CTA per unit, 8 observations a thread
 constexpr int DIAG_SUPER = SD_THREADS * SD_PER;  // observations per diagonal unit, 6-parameter cameras
 constexpr int CAM_CHUNK = 512;   // observations per camera-reduction work unit (11/16-parameter cameras)
@@ -194,26 +206,22 @@ struct DeviceProblem {
     int *pair_a = nullptr;     // entries: observation of camera k
     int *pair_b = nullptr;     // entries: observation of camera l
     long long n_pair_entries = 0;
-    // off-diagonal Schur work, two layouts whose partial slots are numbered in
-    // pair-list order (each pair's slots form one range):
-    // units of <= SCHUR_CHUNK entries of one pair, one slot each, longest
-    // first (FP32 products, and 11/16-parameter cameras);
+    // off-diagonal Schur work, units of one pair whose partial slots are
+    // numbered in pair-list order, longest first: of <= off_unit_len entries
+    // (FP64 products, and 11/16-parameter cameras in both forms);
     SchurUnit *off_units = nullptr;
     int n_off_units = 0;
     int *off_unit_start = nullptr;  // per pair: first unit (n_pairs + 1)
-    // 6-parameter cameras, FP64 products: the pair list cut into equal chunks
-    // (SchurUnit: first pair, first entry, entries, first slot), one per thread
-    // of one resident wave, a slot per pair a chunk touches
-    SchurUnit *off_chunks = nullptr;
-    int n_off_chunks = 0;
     // 6-parameter cameras, FP32 products: units of <= MX_UNIT entries of one
-    // pair, one warp and one slot each, longest first
+    // pair, one warp and one slot each
     SchurUnit *mx_units = nullptr;
     int n_mx_units = 0;
     int *mx_unit_start = nullptr;  // per pair: first unit (n_pairs + 1)
-    int n_off_chunk_slots = 0;
-    int *off_chunk_start = nullptr;  // per pair: first slot (n_pairs + 1)
-    int *pair_start = nullptr;       // per pair: first entry (n_pairs + 1)
+    // 6-parameter cameras, FP64 products: diagonal units of <= diag_unit_len
+    // observations of one camera (the FP32 products' are diag_units)
+    SchurUnit *fx_diag_units = nullptr;
+    int n_fx_diag_units = 0;
+    int *fx_diag_unit_start = nullptr;  // per camera (nc + 1)
     SchurUnit *diag_units = nullptr;  // per camera chunks of cam_obs
     int n_diag_units = 0;
     int *diag_unit_start = nullptr;   // per camera (nc + 1)
@@ -240,7 +248,9 @@ struct DeviceProblem {
     float *Vinv2f = nullptr;      // 12 per point: V^-1 as FP32 pairs hi + lo (the mixed form's Y)
     float *gb32 = nullptr;        // 3 per point: gb rounded to FP32 (the mixed form's ea sums)
     float *camtab32 = nullptr;    // CAMTAB32 per camera: the table's M, D, fx, sk, fy in FP32 (mixed J)
-    double *Y = nullptr;          // 18 per obs
+    double *Y = nullptr;          // 18 per obs; FP64 form: Y's limb rows (fx_words per obs), Y after psba_eval_reduced
+    int2 *Wq = nullptr;           // FP64 form: W's limb rows (fx_words per obs)
+    int2 *fx_ex = nullptr;        // FP64 form: per obs, the exponents of its Y and W limb rows
     double *schur_partial = nullptr;  // off-diagonal slots (off_partial_slots), then the diagonal units'
     double *S = nullptr;          // Np x Np (lower)
     double *Ssave = nullptr;      // copy of S (trust-region modified-Cholesky fallback, refinement), Nm3 x Nm3
@@ -260,7 +270,7 @@ struct DeviceProblem {
     int2 *chol_tasks = nullptr;   // helper tasks of the dense factor, in dependency order
     int chol_n_tasks = 0;
     int chol_grid_cap = 0;        // CTAs of the dense factor at most (0: one per SM)
-    long long wait_limit = DEFAULT_WAIT_LIMIT;  // polls per device-side wait (dense factor flags, Y copies)
+    long long wait_limit = DEFAULT_WAIT_LIMIT;  // polls per device-side wait (dense factor flags)
     double *chol_pre = nullptr;   // second-subdiagonal tiles before their solve (Np / TILE tiles)
     int *chol_flags = nullptr;    // one flag per dataflow task (value = epoch when done)
     int chol_n_flags = 0;
@@ -300,21 +310,19 @@ int residual_blocks(const DeviceProblem &d);
 
 // Damping trial: V^-1, Y, Schur complement, ea.
 void launch_vinv(const DeviceProblem &d, double mu, cudaStream_t s);
-void launch_yblocks(const DeviceProblem &d, cudaStream_t s);
-// Per-device kernel attributes (dynamic shared-memory opt-ins); call with the
-// device current before the first launch on it.
+void launch_yblocks(const DeviceProblem &d, cudaStream_t s);  // Y itself (FP64: for psba_eval_reduced)
 constexpr int MAX_DEVICES = 64;
-int prepare_device_kernels();
 void launch_schur(const DeviceProblem &d, double mu, cudaStream_t s);
 void launch_schur_off(const DeviceProblem &d, cudaStream_t s);
-// threads of one resident wave of the 6-parameter off-diagonal Schur kernel on this device
-int schur_off_wave_threads();
 // off-diagonal partial slots reserved ahead of the diagonal partials (the larger layout)
 inline size_t off_partial_slots(const DeviceProblem &d)
 {
-    size_t n = (size_t)(d.n_off_units > d.n_off_chunk_slots ? d.n_off_units : d.n_off_chunk_slots);
-    return n > (size_t)d.n_mx_units ? n : (size_t)d.n_mx_units;
+    return (size_t)(d.n_off_units > d.n_mx_units ? d.n_off_units : d.n_mx_units);
 }
+// FP64 form (psba_schurfx.cu): Y and W as limb rows, then all products of the
+// Schur complement in one or two launches
+void launch_limb_rows(const DeviceProblem &d, cudaStream_t s);
+void launch_schur_fx(const DeviceProblem &d, double *diag_partial, cudaStream_t s);
 void launch_schur_diag(const DeviceProblem &d, cudaStream_t s);
 void launch_schur_reduce(const DeviceProblem &d, double mu, cudaStream_t s);
 // Back-substitution: eb, dpb and partial sums for |dp|^2 and dp.(mu dp + g).

@@ -1055,14 +1055,10 @@ __device__ __forceinline__ void vinv_one(const R *Vi, R mu, R *out)
 // is kept in FP64: for a point seen from two nearby cameras V_i is nearly
 // singular, and an FP32 V_i + mu I (which drops mu) or an FP32 V^-1 moves the
 // LM fixed point by ~1e-2 of the cost.
-// Each damping trial starts here, so this launch also clears the status word
-// of the trial's bulk copies (status[2], set by k_yblocks_bulk when a wait
-// runs out), which nothing else resets.
 __global__ void k_vinv(int np, const double *__restrict__ V, double mu, double *__restrict__ Vinv,
-                       float *__restrict__ Vinv2f, int *__restrict__ status)
+                       float *__restrict__ Vinv2f)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) status[2] = 0;
     if (i >= np) return;
     double vi[6], out[6];
 #pragma unroll
@@ -1087,8 +1083,7 @@ void launch_vinv(const DeviceProblem &d, double mu, cudaStream_t s)
 {
     if (d.np == 0) return;
     k_vinv<<<ceil_div(d.np, 128), 128, 0, s>>>(d.np, d.V, mu, d.Vinv,
-                                               d.prec == PSBA_PREC_MIXED && d.cnp == 6 ? d.Vinv2f : nullptr,
-                                               d.status);
+                                               d.prec == PSBA_PREC_MIXED && d.cnp == 6 ? d.Vinv2f : nullptr);
     note_launch(1);
 }
 
@@ -1102,7 +1097,7 @@ void launch_vinv(const DeviceProblem &d, double mu, cudaStream_t s)
 // accuracy of an FP64 product: a V^-1 rounded to FP32 instead breaks it for
 // points seen from nearby cameras (V nearly singular, V^-1 with large entries
 // of both signs), which sent LM to minima ~3% higher.  The FP64 form is
-// k_yblocks_bulk.
+// k_limb_rows.
 __global__ void __launch_bounds__(256) k_yblocks(int no, const int *__restrict__ obs_pt,
                                                  const float *__restrict__ W, const float *__restrict__ Vinv2f,
                                                  float *__restrict__ Y)
@@ -1152,142 +1147,11 @@ __global__ void __launch_bounds__(256) k_yblocks(int no, const int *__restrict__
     for (int k = lane; k < 9 * nrow; k += 32) dst[k] = b[k];
 }
 
-// Bulk asynchronous copies between global and shared memory (the copy
-// engine of the SM, no registers in flight): a global -> shared copy signals
-// an mbarrier with its byte count; a shared -> global copy is a bulk group.
-// Addresses and sizes are multiples of 16 bytes.
-__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(unsigned long long *bar)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, unsigned bytes, unsigned long long *bar)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
-// waits for phase 0 of the barrier, at most `limit` polls; false if it ran out
-__device__ __forceinline__ bool mbar_wait0(unsigned long long *bar, long long limit)
-{
-    for (long long it = 0; it < limit; ++it) {
-        unsigned done;
-        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0; selp.u32 %0, 1, 0, p; }"
-                     : "=r"(done)
-                     : "r"(smem_u32(bar))
-                     : "memory");
-        if (done) return true;
-    }
-    return false;
-}
-__device__ __forceinline__ void bulk_s2g(void *dst, const void *src, unsigned bytes)
-{
-    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)),
-                 "r"(bytes)
-                 : "memory");
-    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-}
-
-// Y = W V^-1 (FP64) for YB_ROWS consecutive observations per CTA: their W
-// rows (contiguous, 144 bytes each) come into shared memory by one bulk copy,
-// each thread forms its row of Y there (16-byte shared loads at a 144-byte
-// stride: no bank conflicts), and one bulk copy writes the CTA's Y rows
-// back (the products of compute_Yblks.cl:26-37).  A copy that does not
-// complete within poll_limit polls sets status[2] (the trial then reports
-// the wait budget exhausted); the CTA then waits for the copy to land in
-// its shared memory (at most YB_DRAIN_LIMIT polls: a bulk copy of 37 KB from
-// this GPU's own memory completes in microseconds) before it leaves.  Should
-// the drain wait also run out, the CTA leaves with the copy possibly still
-// in flight; that needs a copy stalled for the whole drain budget, which no
-// test provokes.
-constexpr int YB_ROWS = 256;
-constexpr long long YB_DRAIN_LIMIT = 1LL << 22;
-
-__global__ void __launch_bounds__(YB_ROWS) k_yblocks_bulk(int no, const int *__restrict__ obs_pt,
-                                                          const double *__restrict__ W,
-                                                          const double *__restrict__ Vinv, double *__restrict__ Y,
-                                                          int *__restrict__ status, long long poll_limit)
-{
-    extern __shared__ __align__(16) double yb_sm[];  // W rows, then Y rows
-    __shared__ __align__(8) unsigned long long bar;
-    double *sw = yb_sm, *sy = yb_sm + YB_ROWS * 18;
-    const int o0 = blockIdx.x * YB_ROWS, rows = min(YB_ROWS, no - o0), t = threadIdx.x;
-    const unsigned bytes = (unsigned)rows * 18u * 8u;
-    if (t == 0) mbar_init(&bar);
-    __syncthreads();
-    if (t == 0) bulk_g2s(sw, W + 18 * (size_t)o0, bytes, &bar);
-    double s00 = 0, s01 = 0, s02 = 0, s11 = 0, s12 = 0, s22 = 0;
-    if (t < rows) {  // the point's V^-1 while the rows arrive
-        const double *vi = Vinv + 6 * (size_t)__ldg(obs_pt + o0 + t);
-        s00 = __ldg(vi); s01 = __ldg(vi + 1); s02 = __ldg(vi + 2);
-        s11 = __ldg(vi + 3); s12 = __ldg(vi + 4); s22 = __ldg(vi + 5);
-    }
-    if (!mbar_wait0(&bar, poll_limit)) {
-        if (t == 0) atomicExch(status + 2, 2);
-        mbar_wait0(&bar, YB_DRAIN_LIMIT);  // the copy may still land in this CTA's memory
-        return;
-    }
-    if (t < rows) {
-        const double2 *w2 = reinterpret_cast<const double2 *>(sw + 18 * t);
-        double w[18], y[18];
-#pragma unroll
-        for (int e = 0; e < 9; ++e) {
-            const double2 v = w2[e];
-            w[2 * e] = v.x;
-            w[2 * e + 1] = v.y;
-        }
-#pragma unroll
-        for (int r = 0; r < 6; ++r) {
-            const double w0 = w[3 * r], w1 = w[3 * r + 1], w2v = w[3 * r + 2];
-            y[3 * r + 0] = w0 * s00 + w1 * s01 + w2v * s02;
-            y[3 * r + 1] = w0 * s01 + w1 * s11 + w2v * s12;
-            y[3 * r + 2] = w0 * s02 + w1 * s12 + w2v * s22;
-        }
-        double2 *y2 = reinterpret_cast<double2 *>(sy + 18 * t);
-#pragma unroll
-        for (int e = 0; e < 9; ++e) y2[e] = make_double2(y[2 * e], y[2 * e + 1]);
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the rows, visible to the bulk copy
-    __syncthreads();
-    if (t == 0) bulk_s2g(Y + 18 * (size_t)o0, sy, bytes);
-}
-
-// The bulk Y kernel's dynamic shared memory (73,728 B) is above the default
-// 48 KB limit; the opt-in is a per-device attribute, so it is set once for
-// every device a handle is created on, with that device current.
-int prepare_device_kernels()
-{
-    static std::mutex mu;
-    static bool done[MAX_DEVICES] = {};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return set_error(std::string("cudaGetDevice: ") + cudaGetErrorString(e)), PSBA_ERR_CUDA;
-    if (dev < 0 || dev >= MAX_DEVICES) return set_error("device index out of range"), PSBA_ERR_ARG;
-    std::lock_guard<std::mutex> lk(mu);
-    if (done[dev]) return PSBA_OK;
-    e = cudaFuncSetAttribute(k_yblocks_bulk, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(2 * YB_ROWS * 18 * sizeof(double)));
-    if (e != cudaSuccess)
-        return set_error(std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e)), PSBA_ERR_CUDA;
-    done[dev] = true;
-    return PSBA_OK;
-}
-
 void launch_yblocks(const DeviceProblem &d, cudaStream_t s)
 {
-    if (d.cnp != 6) return launch_yblocks_v(d, s);
     if (d.no == 0) return;
-    if (d.prec == PSBA_PREC_FP64) {
-        const int smem = (int)(2 * YB_ROWS * 18 * sizeof(double));
-        k_yblocks_bulk<<<ceil_div(d.no, YB_ROWS), YB_ROWS, smem, s>>>(d.no, d.obs_pt, d.W, d.Vinv, d.Y, d.status,
-                                                                      d.wait_limit);
-    } else
-        k_yblocks<<<ceil_div(d.no, 256), 256, 0, s>>>(d.no, d.obs_pt, (const float *)d.W, d.Vinv2f, (float *)d.Y);
+    if (d.cnp != 6 || d.prec == PSBA_PREC_FP64) return launch_yblocks_v(d, s);
+    k_yblocks<<<ceil_div(d.no, 256), 256, 0, s>>>(d.no, d.obs_pt, (const float *)d.W, d.Vinv2f, (float *)d.Y);
     note_launch(1);
 }
 
@@ -1299,93 +1163,9 @@ void launch_yblocks(const DeviceProblem &d, cudaStream_t s)
 // observations, the 21 lower entries plus the 6 ea sums.  The slots are then
 // summed in order (k_schur_reduce).
 //
-// FP64 products (6-parameter cameras): the pair list cut into equal chunks,
-// one per thread of one resident wave, so that every SM issues the same
-// number of FP64 multiply-adds; a thread writes its sums to the next slot
-// whenever its chunk passes into the next pair.
-template <typename R>
-__device__ __forceinline__ void off_products(const R *y, const R *w, R *acc)
-{
-#pragma unroll
-    for (int r = 0; r < 6; ++r)
-#pragma unroll
-        for (int c = 0; c < 6; ++c) {
-            R s = acc[r * 6 + c];
-            s = fma(y[3 * r], w[3 * c], s);
-            s = fma(y[3 * r + 1], w[3 * c + 1], s);
-            s = fma(y[3 * r + 2], w[3 * c + 2], s);
-            acc[r * 6 + c] = s;
-        }
-}
-
-template <typename R>
-__device__ __forceinline__ void schur_off_chunk(int uid, int n_chunks, const SchurUnit *__restrict__ chunks,
-                                                const int *__restrict__ pair_start, const int *__restrict__ pa,
-                                                const int *__restrict__ pb, const R *__restrict__ Y,
-                                                const R *__restrict__ W, double *__restrict__ partial)
-{
-    if (uid >= n_chunks) return;
-    const SchurUnit u = chunks[uid];
-    int q = u.slot, slot = u.out;
-    int next = __ldg(pair_start + q + 1);  // first entry of the next pair
-    const int end = u.begin + u.count;
-    double acc[36];
-#pragma unroll
-    for (int e = 0; e < 36; ++e) acc[e] = 0.0;
-    static_assert(is_fp64<R>(), "FP64 products; FP32 products take the unit kernel");
-    for (int t = u.begin; t < end; ++t) {
-        if (t == next) {
-            double *p = partial + (size_t)slot * 36;
-#pragma unroll
-            for (int e = 0; e < 36; ++e) {
-                p[e] = acc[e];
-                acc[e] = 0.0;
-            }
-            ++slot;
-            ++q;
-            next = __ldg(pair_start + q + 1);
-        }
-        const int a = __ldg(pa + t), b = __ldg(pb + t);
-        R w[18], y[18];
-        ldn<R, 18>(W + 18 * (size_t)b, w);
-        ldn<R, 18>(Y + 18 * (size_t)a, y);
-        off_products<R>(y, w, acc);
-    }
-    double *p = partial + (size_t)slot * 36;
-#pragma unroll
-    for (int e = 0; e < 36; ++e) p[e] = acc[e];
-}
-
-
+// FP64 products run in block fixed point (psba_schurfx.cu); these are the FP32
+// products of the mixed form.
 constexpr int DIAG_NV = 27;  // 21 lower entries + 6 ea sums
-
-// The 21 lower entries of Y W^T into acc (R); the 6 sums of Y gb into eacc
-// in FP64 from the exact products in both forms: ea = ga - sum Y gb cancels
-// near the optimum, where the step is set by it.
-template <typename R>
-__device__ __forceinline__ void diag_products(const R *y, const R *w, double g0, double g1, double g2, R *acc,
-                                              double *eacc)
-{
-    int v = 0;
-#pragma unroll
-    for (int r = 0; r < 6; ++r)
-#pragma unroll
-        for (int c = 0; c <= r; ++c, ++v) {
-            R s = acc[v];
-            s = fma(y[3 * r], w[3 * c], s);
-            s = fma(y[3 * r + 1], w[3 * c + 1], s);
-            s = fma(y[3 * r + 2], w[3 * c + 2], s);
-            acc[v] = s;
-        }
-#pragma unroll
-    for (int r = 0; r < 6; ++r) {
-        double s = eacc[r];
-        s = fma((double)y[3 * r], g0, s);
-        s = fma((double)y[3 * r + 1], g1, s);
-        s = fma((double)y[3 * r + 2], g2, s);
-        eacc[r] = s;
-    }
-}
 
 // The mixed form's diagonal products: the 21 block sums and the 6 ea sums
 // (y . gb) of one observation, all in FP32.
@@ -1415,142 +1195,72 @@ __device__ __forceinline__ void diag_products_f32(const float *y, const float *w
 
 // Diagonal blocks U_k - sum Y W^T (lower 21) and the ea sums (6): one CTA of
 // SD_THREADS per unit of <= DIAG_SUPER observations of one camera, SD_PER
-// consecutive observations per thread (FP64: accumulated directly; mixed:
-// FP32 products over the thread's observations, then one FP64 addition).
-// The CTA then sums its threads' partials in a fixed order (each output by
-// four threads over 32 partials each, then the four) and writes one partial
-// per unit, so a camera has only a handful for k_schur_reduce.  In the mixed
-// form the unit's observation and point indices are first gathered into
-// shared memory (sidx, 2 DIAG_SUPER ints) by the whole CTA, so a thread's
+// consecutive observations per thread: FP32 products over the thread's
+// observations, then FP64.  The CTA then sums its threads' partials in a fixed
+// order and writes one partial per unit, so a camera has only a handful for
+// k_schur_reduce.  The unit's observation and point indices are first gathered
+// into shared memory (sidx, 2 DIAG_SUPER ints) by the whole CTA, so a thread's
 // walk waits for one L2 round trip per observation instead of three.
-// The mixed form's CTA reduction is narrower (two xor-shuffle levels first,
-// then 32 partials per output in shared memory): its shared buffer is also
-// the off-diagonal warps' index buffer, and a smaller one leaves the L1 more
-// room for the rows those warps gather.
+// The CTA reduction is narrow (two xor-shuffle levels first, then 32
+// partials per output in shared memory): its shared buffer is also the
+// off-diagonal warps' index buffer, and a smaller one leaves the L1 more room
+// for the rows those warps gather.
 constexpr int SD_RED_MX = SD_THREADS / 4;
 
-template <typename R>
 __device__ __forceinline__ void schur_diag_cta(const SchurUnit u, const int *__restrict__ cam_obs,
-                                               const int *__restrict__ obs_pt, const R *__restrict__ Y,
-                                               const R *__restrict__ W, const R *__restrict__ gb,
-                                               double *__restrict__ partial, double *red_buf,
-                                               int *sidx = nullptr)
+                                               const int *__restrict__ obs_pt, const float *__restrict__ Y,
+                                               const float *__restrict__ W, const float *__restrict__ gb,
+                                               double *__restrict__ partial, double *red_buf, int *sidx)
 {
     static_assert(SD_THREADS == 128 && DIAG_NV * 4 <= SD_THREADS, "four summing threads per output");
+    static_assert(SD_PER <= FLUSH, "one FP32 flush per thread");
     const int t = threadIdx.x;
-    double acc[DIAG_NV];
-#pragma unroll
-    for (int e = 0; e < DIAG_NV; ++e) acc[e] = 0.0;
     const int o1 = min(u.count, (t + 1) * SD_PER);
-    if constexpr (is_fp64<R>()) {
-        for (int o = t * SD_PER; o < o1; ++o) {
-            const int a = __ldg(cam_obs + u.begin + o);
-            const int i = __ldg(obs_pt + a);
-            R w[18], y[18];
-            ldn<R, 18>(W + 18 * (size_t)a, w);
-            ldn<R, 18>(Y + 18 * (size_t)a, y);
-            const double g0 = __ldg(gb + 3 * (size_t)i), g1 = __ldg(gb + 3 * (size_t)i + 1),
-                         g2 = __ldg(gb + 3 * (size_t)i + 2);
-            diag_products<R>(y, w, g0, g1, g2, acc, acc + 21);
-        }
-    } else {
-        static_assert(SD_PER <= FLUSH, "one FP32 flush per thread");
-        for (int k = t; k < u.count; k += SD_THREADS) {
-            const int a = __ldg(cam_obs + u.begin + k);
-            sidx[k] = a;
-            sidx[DIAG_SUPER + k] = __ldg(obs_pt + a);
-        }
-        __syncthreads();
-        // the block and the ea sums alike: FP32 products summed over the
-        // thread's observations (gb rounded to FP32 once per point), then FP64
-        float part[DIAG_NV];
-#pragma unroll
-        for (int e = 0; e < DIAG_NV; ++e) part[e] = 0.0f;
-#pragma unroll 2
-        for (int o = t * SD_PER; o < o1; ++o) {
-            const int a = sidx[o];
-            const int i = sidx[DIAG_SUPER + o];
-            float w[18], y[18];
-            ldn<float, 18>(W + 18 * (size_t)a, w);
-            ldn<float, 18>(Y + 18 * (size_t)a, y);
-            const float g0 = __ldg(gb + 3 * (size_t)i), g1 = __ldg(gb + 3 * (size_t)i + 1),
-                        g2 = __ldg(gb + 3 * (size_t)i + 2);
-            diag_products_f32(y, w, g0, g1, g2, part);
-        }
-        __syncthreads();  // the walk's indices are read: red may overlay them
-#pragma unroll
-        for (int e = 0; e < DIAG_NV; ++e) acc[e] = (double)part[e];
+    for (int k = t; k < u.count; k += SD_THREADS) {
+        const int a = __ldg(cam_obs + u.begin + k);
+        sidx[k] = a;
+        sidx[DIAG_SUPER + k] = __ldg(obs_pt + a);
     }
-    // fixed-order CTA sum: each output by four threads over W partials
-    // each, then the four (W = 32: one per thread; mixed form, W = 8 per
-    // warp after two xor levels over lanes l, l + 8, l + 16, l + 24)
-    constexpr int NP = is_fp64<R>() ? SD_THREADS : SD_RED_MX;
-    double(*red)[NP + 1] = reinterpret_cast<double(*)[NP + 1]>(red_buf);
-    if constexpr (is_fp64<R>()) {
+    __syncthreads();
+    // the block and the ea sums alike: FP32 products summed over the
+    // thread's observations (gb rounded to FP32 once per point), then FP64
+    float part[DIAG_NV];
 #pragma unroll
-        for (int e = 0; e < DIAG_NV; ++e) red[e][t] = acc[e];
-    } else {
-        const int lane = t & 31;
+    for (int e = 0; e < DIAG_NV; ++e) part[e] = 0.0f;
+#pragma unroll 2
+    for (int o = t * SD_PER; o < o1; ++o) {
+        const int a = sidx[o];
+        const int i = sidx[DIAG_SUPER + o];
+        float w[18], y[18];
+        ldn<float, 18>(W + 18 * (size_t)a, w);
+        ldn<float, 18>(Y + 18 * (size_t)a, y);
+        const float g0 = __ldg(gb + 3 * (size_t)i), g1 = __ldg(gb + 3 * (size_t)i + 1),
+                    g2 = __ldg(gb + 3 * (size_t)i + 2);
+        diag_products_f32(y, w, g0, g1, g2, part);
+    }
+    __syncthreads();  // the walk's indices are read: red may overlay them
+    // fixed-order CTA sum: two xor levels over lanes l, l + 8, l + 16, l + 24,
+    // then each output by four threads over 8 partials each, then the four
+    double(*red)[SD_RED_MX + 1] = reinterpret_cast<double(*)[SD_RED_MX + 1]>(red_buf);
+    const int lane = t & 31;
 #pragma unroll
-        for (int e = 0; e < DIAG_NV; ++e) {
-            double x = acc[e];
-            x += __shfl_xor_sync(0xffffffffu, x, 16);
-            x += __shfl_xor_sync(0xffffffffu, x, 8);
-            if (lane < 8) red[e][(t >> 5) * 8 + lane] = x;
-        }
+    for (int e = 0; e < DIAG_NV; ++e) {
+        double x = (double)part[e];
+        x += __shfl_xor_sync(0xffffffffu, x, 16);
+        x += __shfl_xor_sync(0xffffffffu, x, 8);
+        if (lane < 8) red[e][(t >> 5) * 8 + lane] = x;
     }
     __syncthreads();
     double s = 0.0;
     const int v = t >> 2, g = t & 3;
     if (v < DIAG_NV) {
 #pragma unroll 8
-        for (int q = 0; q < NP / 4; ++q) s += red[v][g * (NP / 4) + q];
+        for (int q = 0; q < SD_RED_MX / 4; ++q) s += red[v][g * (SD_RED_MX / 4) + q];
     }
     __syncthreads();
     if (v < DIAG_NV) red[v][g] = s;
     __syncthreads();
     if (t < DIAG_NV) partial[(size_t)u.out * DIAG_NV + t] = (red[t][0] + red[t][1]) + (red[t][2] + red[t][3]);
-}
-
-
-// FP64 products, 6-parameter cameras: the off-diagonal chunks (blocks below
-// off_ctas, 128 threads each) and the diagonal units (the rest) in one
-// launch.  Blocks are handed out in index order, so the off-diagonal chunks
-// fill one resident wave and the diagonal units run in its tail.
-__global__ void __launch_bounds__(128) k_schur(int n_chunks, int off_ctas, const SchurUnit *__restrict__ chunks,
-                                               const int *__restrict__ pair_start, const int *__restrict__ pa,
-                                               const int *__restrict__ pb, const SchurUnit *__restrict__ diag_units,
-                                               const int *__restrict__ cam_obs, const int *__restrict__ obs_pt,
-                                               const double *__restrict__ Y, const double *__restrict__ W,
-                                               const double *__restrict__ gb, double *__restrict__ off_partial,
-                                               double *__restrict__ diag_partial)
-{
-    static_assert(SD_THREADS == 128, "one block size for both parts");
-    __shared__ double red[DIAG_NV][SD_THREADS + 1];
-    if ((int)blockIdx.x < off_ctas)
-        schur_off_chunk<double>(blockIdx.x * 128 + threadIdx.x, n_chunks, chunks, pair_start, pa, pb, Y, W,
-                                off_partial);
-    else
-        schur_diag_cta<double>(diag_units[blockIdx.x - off_ctas], cam_obs, obs_pt, Y, W, gb, diag_partial, &red[0][0]);
-}
-
-int schur_off_wave_threads()
-{
-    // one resident wave of k_schur, per device (the serving lanes' threads
-    // ask at the same time)
-    static std::mutex mu;
-    static int threads[MAX_DEVICES] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= MAX_DEVICES) dev = 0;
-    std::lock_guard<std::mutex> lk(mu);
-    if (threads[dev] == 0) {
-        int sms = 0, per_sm = 0;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_schur, 128, 0);
-        threads[dev] = std::max(1, sms) * std::max(1, per_sm) * 128;
-    }
-    return threads[dev];
 }
 
 // FP32 products, 6-parameter cameras: one warp per unit of <= MX_UNIT
@@ -1721,7 +1431,7 @@ __global__ void __launch_bounds__(128, PSBA_SF32_MINB) k_schur_f32(int n_units, 
     static_assert(IDX_WORDS >= 2 * DIAG_SUPER, "the index buffer holds a diagonal unit's indices");
     __shared__ __align__(16) int buf[RED_WORDS > OFF_WORDS ? RED_WORDS : OFF_WORDS];
     if ((int)blockIdx.x < n_diag) {
-        schur_diag_cta<float>(diag_units[blockIdx.x], cam_obs, obs_pt, Y, W, gb32, diag_partial,
+        schur_diag_cta(diag_units[blockIdx.x], cam_obs, obs_pt, Y, W, gb32, diag_partial,
                               reinterpret_cast<double *>(buf), buf);
     } else {
         const int uid = (blockIdx.x - n_diag) * 4 + (threadIdx.x >> 5);
@@ -1782,31 +1492,22 @@ __global__ void k_pad_identity(int N, int Np, double *S, double *rhs)
 
 void launch_schur_off(const DeviceProblem &d, cudaStream_t s)
 {
+    double *diag_partial = d.schur_partial + off_partial_slots(d) * d.cnp * d.cnp;
+    if (d.prec == PSBA_PREC_FP64) return launch_schur_fx(d, diag_partial, s);  // the diagonal units too
     if (d.cnp != 6) return launch_schur_off_v(d, s);
-    if (d.prec == PSBA_PREC_FP64) {
-        // the diagonal units ride in the same launch (k_schur)
-        const int off_ctas = ceil_div(d.n_off_chunks, 128);
-        if (off_ctas + d.n_diag_units == 0) return;
-        k_schur<<<off_ctas + d.n_diag_units, 128, 0, s>>>(
-            d.n_off_chunks, off_ctas, d.off_chunks, d.pair_start, d.pair_a, d.pair_b, d.diag_units, d.cam_obs,
-            d.obs_pt, d.Y, d.W, d.g + d.N, d.schur_partial, d.schur_partial + off_partial_slots(d) * 36);
-        note_launch(1);
-        return;
-    }
     const int off_ctas = ceil_div(d.n_mx_units, 4);
     if (off_ctas + d.n_diag_units == 0) return;
     k_schur_f32<<<off_ctas + d.n_diag_units, 128, 0, s>>>(
         d.n_mx_units, d.n_diag_units, d.mx_units, d.pair_a, d.pair_b, d.diag_units, d.cam_obs, d.obs_pt,
-        (const float *)d.Y, (const float *)d.W, d.gb32, d.schur_partial,
-        d.schur_partial + off_partial_slots(d) * 36);
+        (const float *)d.Y, (const float *)d.W, d.gb32, d.schur_partial, diag_partial);
     note_launch(1);
 }
 
 void launch_schur_diag(const DeviceProblem &d, cudaStream_t s)
 {
-    // 6-parameter cameras: the diagonal units run in the off-diagonal launch
-    // (k_schur, k_schur_f32)
-    if (d.cnp != 6) launch_schur_diag_v(d, s);
+    // the diagonal units run with the off-diagonal ones, but for the mixed
+    // form's 11/16-parameter cameras
+    if (d.cnp != 6 && d.prec != PSBA_PREC_FP64) launch_schur_diag_v(d, s);
 }
 
 void launch_schur_reduce(const DeviceProblem &d, double mu, cudaStream_t s)
@@ -1823,10 +1524,12 @@ void launch_schur_reduce(const DeviceProblem &d, double mu, cudaStream_t s)
     double *off_partial = d.schur_partial;
     double *diag_partial = d.schur_partial + off_partial_slots(d) * 36;
     const int total = d.n_pairs * 36 + d.nc * DIAG_NV;
-    const int *off_start = d.prec == PSBA_PREC_FP64 ? d.off_chunk_start : d.mx_unit_start;
+    const bool f64 = d.prec == PSBA_PREC_FP64;
+    const int *off_start = f64 ? d.off_unit_start : d.mx_unit_start;
     k_schur_reduce<<<ceil_div(total, 128), 128, 0, s>>>(d.n_pairs, d.nc, d.Np, d.pair_kl,
                                                           off_start, off_partial,
-                                                          d.diag_unit_start, diag_partial, d.U, d.g,
+                                                          f64 ? d.fx_diag_unit_start : d.diag_unit_start,
+                                                          diag_partial, d.U, d.g,
                                                           mu, d.S, d.rhs);
     note_launch(1);
     if (d.Np > d.N) {
@@ -1873,7 +1576,7 @@ __device__ void finish_trial_block(int ncp, int nblocks, const double *__restric
     if (threadIdx.x == 0) {
         out->dp_L2 = r0[0];
         out->rho_den = r1[0];
-        out->chol_status = status[0] != 0 ? status[0] : (status[2] != 0 ? 2 : 0);  // [2]: a bulk copy's wait
+        out->chol_status = status[0];
     }
 }
 

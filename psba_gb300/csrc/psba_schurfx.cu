@@ -1,0 +1,532 @@
+// The FP64 Schur complement's products in block fixed point (psba_fixed.h):
+// S's off-diagonal blocks sum_i Y_ik W_il^T and the diagonal blocks with ea's
+// sums Y gb (compute_S.cl:39-77, compute_ea.cl:21-36).
+//
+// k_limb_rows forms Y = W V^-1 (compute_Yblks.cl:26-37) and cuts each
+// observation's Y and W rows into limbs, relative to the observation's own
+// largest value after the camera's row weights (fx_weight).  The sums then
+// need one more shift per pair entry, of its W row, to the largest
+// eY + eW among the 32 entries taken together: a point close to one camera has a W
+// row there 10^4 times the others' and Y rows as much smaller, and only what
+// lies 57 bits below the largest product is lost.  Cutting both rows at every
+// use instead (a point is in about six pairs per observation) cost 1,560
+// instructions per warp and 32 entries, twice the products' own.
+#include "psba_fixed.h"
+#include "psba_internal.h"
+
+namespace psba {
+
+namespace {
+
+inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
+
+constexpr int FX_CHUNK = 32;  // entries aligned to one exponent at a time
+
+// ---------------------------------------------------------------------------
+// Y and the limb rows.  A CTA takes LR_THREADS / TPO consecutive observations
+// (their W rows are contiguous), TPO threads each, TR rows a thread; rows go
+// through shared memory so that global loads and stores are coalesced.
+// Bound by the FP64 pipe (9 multiply-adds a row) and the ~25 integer
+// instructions that cut a value.
+constexpr int LR_THREADS = 128;
+
+template <int CNP>
+__global__ void __launch_bounds__(LR_THREADS) k_limb_rows(int no, const int *__restrict__ obs_pt,
+                                                          const int *__restrict__ obs_cam,
+                                                          const double *__restrict__ W,
+                                                          const double *__restrict__ Vinv,
+                                                          const double *__restrict__ U, int2 *__restrict__ Yq,
+                                                          int2 *__restrict__ Wq, int2 *__restrict__ ex)
+{
+    constexpr int RP = fx_rows(CNP), TPO = CNP == 6 ? 2 : 4, TR = RP / TPO, OB = LR_THREADS / TPO, WORDS = 3 * RP;
+    __shared__ __align__(16) double sw[OB * 3 * CNP];
+    __shared__ __align__(16) int2 sq[2][OB * WORDS];
+    const int o0 = blockIdx.x * OB, n = min(OB, no - o0), tid = threadIdx.x;
+    for (int e = tid; e < n * 3 * CNP; e += LR_THREADS) sw[e] = __ldg(W + 3 * CNP * (size_t)o0 + e);
+    const int t = tid / TPO, q = tid % TPO, o = o0 + min(t, n - 1);
+    const double *vi = Vinv + 6 * (size_t)__ldg(obs_pt + o);
+    const double *u = U + CNP * CNP * (size_t)__ldg(obs_cam + o);
+    const double s00 = __ldg(vi), s01 = __ldg(vi + 1), s02 = __ldg(vi + 2), s11 = __ldg(vi + 3), s12 = __ldg(vi + 4),
+                 s22 = __ldg(vi + 5);
+    int rho[TR];
+#pragma unroll
+    for (int a = 0; a < TR; ++a) {
+        const int r = q * TR + a;
+        rho[a] = r < CNP ? fx_weight(__ldg(u + (CNP + 1) * r)) : 0;
+    }
+    __syncthreads();
+    double w[TR][3], y[TR][3];
+    int ew = -4096, ey = -4096, bw = 0, by = 0;
+#pragma unroll
+    for (int a = 0; a < TR; ++a) {
+        const int r = q * TR + a;
+        if (r >= CNP) {
+#pragma unroll
+            for (int j = 0; j < 3; ++j) w[a][j] = y[a][j] = 0.0;
+            continue;
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j) w[a][j] = sw[min(t, n - 1) * 3 * CNP + 3 * r + j];
+        y[a][0] = w[a][0] * s00 + w[a][1] * s01 + w[a][2] * s02;
+        y[a][1] = w[a][0] * s01 + w[a][1] * s11 + w[a][2] * s12;
+        y[a][2] = w[a][0] * s02 + w[a][1] * s12 + w[a][2] * s22;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            ew = max(ew, fx_exp(w[a][j]) - rho[a]);
+            ey = max(ey, fx_exp(y[a][j]) - rho[a]);
+            bw |= fx_nonfinite(w[a][j]);
+            by |= fx_nonfinite(y[a][j]);
+        }
+    }
+#pragma unroll
+    for (int x = 1; x < TPO; x *= 2) {
+        ew = max(ew, __shfl_xor_sync(0xffffffffu, ew, x));
+        ey = max(ey, __shfl_xor_sync(0xffffffffu, ey, x));
+        bw |= __shfl_xor_sync(0xffffffffu, bw, x);
+        by |= __shfl_xor_sync(0xffffffffu, by, x);
+    }
+#pragma unroll
+    for (int a = 0; a < TR; ++a)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const int at = t * WORDS + j * RP + q * TR + a;
+            sq[0][at] = fx_limbs(y[a][j], ey + rho[a] - fx_exp(y[a][j]));
+            sq[1][at] = fx_limbs(w[a][j], ew + rho[a] - fx_exp(w[a][j]));
+        }
+    if (q == 0 && t < n) ex[o] = make_int2(by ? FX_NAN : ey, bw ? FX_NAN : ew);
+    __syncthreads();
+    int4 *yd = reinterpret_cast<int4 *>(Yq + WORDS * (size_t)o0), *wd = reinterpret_cast<int4 *>(Wq + WORDS * (size_t)o0);
+    const int4 *ys = reinterpret_cast<const int4 *>(sq[0]), *ws = reinterpret_cast<const int4 *>(sq[1]);
+    for (int e = tid; e < n * WORDS / 2; e += LR_THREADS) {
+        yd[e] = ys[e];
+        wd[e] = ws[e];
+    }
+}
+
+// What the product kernels read.
+struct FxArgs {
+    const int *pa, *pb;    // pair entries: observation of camera k, of camera l
+    const int *cam_obs;    // observations by camera
+    const int *obs_pt;
+    const int2 *Yq, *Wq, *ex;
+    const double *W, *Vinv;  // for entries with an infinity or a NaN
+    const double *U, *gb;
+    const int *pair_kl;
+    double *off_partial, *diag_partial;
+};
+
+// One output of a chunk that holds an infinity or a NaN, in plain FP64:
+// sum_t Y_t[r] . (W_t[c], or gb for column CNP), Y formed as in k_limb_rows.
+template <int CNP>
+__device__ __noinline__ double fx_plain(const FxArgs &g, const int *pa, const int *pb, int n, int r, int c, double acc)
+{
+    for (int t = 0; t < n; ++t) {
+        const int a = pa[t], i = g.obs_pt[a];
+        const double *w = g.W + 3 * CNP * (size_t)a + 3 * r, *s = g.Vinv + 6 * (size_t)i;
+        const double *x = c < CNP ? g.W + 3 * CNP * (size_t)pb[t] + 3 * c : g.gb + 3 * (size_t)i;
+        acc = fma(w[0] * s[0] + w[1] * s[1] + w[2] * s[2], x[0], acc);
+        acc = fma(w[0] * s[1] + w[1] * s[3] + w[2] * s[4], x[1], acc);
+        acc = fma(w[0] * s[2] + w[1] * s[4] + w[2] * s[5], x[2], acc);
+    }
+    return acc;
+}
+
+// The (r, c) of output v: row-major blocks, or (DIAG) the lower triangle, then ea as column CNP
+template <int CNP, bool DIAG>
+__device__ __forceinline__ void out_rc(int v, int &r, int &c)
+{
+    constexpr int NL = CNP * (CNP + 1) / 2;
+    if (!DIAG) {
+        r = v / CNP;
+        c = v % CNP;
+    } else if (v >= NL) {
+        r = v - NL;
+        c = CNP;
+    } else {
+        r = 0;
+        c = v;
+        while (c > r) c -= ++r;
+    }
+}
+template <int CNP, bool DIAG>
+__host__ __device__ constexpr int n_out()
+{
+    return DIAG ? CNP * (CNP + 1) / 2 + CNP : CNP * CNP;
+}
+
+// The exponent that output (r, c) of a unit adds to its chunks'
+template <int CNP, bool DIAG>
+__device__ __forceinline__ int out_weight(const FxArgs &g, int slot, int r, int c)
+{
+    const int k = DIAG ? slot : g.pair_kl[2 * slot], l = DIAG ? slot : g.pair_kl[2 * slot + 1];
+    int e = fx_weight(g.U[CNP * CNP * (size_t)k + (CNP + 1) * r]);
+    if (c < CNP) e += fx_weight(g.U[CNP * CNP * (size_t)l + (CNP + 1) * c]);
+    return e;
+}
+
+// N neighbouring limb words, as 16-byte loads where N is even
+template <int N>
+__device__ __forceinline__ void ld_limbs(const int2 *p, int2 *out)
+{
+    if constexpr (N % 2 == 0) {
+#pragma unroll
+        for (int k = 0; k < N; k += 2) {
+            const int4 v = *reinterpret_cast<const int4 *>(p + k);
+            out[k] = make_int2(v.x, v.y);
+            out[k + 1] = make_int2(v.z, v.w);
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < N; ++k) out[k] = p[k];
+    }
+}
+
+// A TR x TC tile of entry t's products
+template <int TR, int TC, int RP, int CP>
+__device__ __forceinline__ void fx_tile(const int2 *y, const int2 *w, long long (&hh)[TR][TC], long long (&hl)[TR][TC])
+{
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        int2 a[TR], b[TC];
+        ld_limbs<TR>(y + j * RP, a);
+        ld_limbs<TC>(w + j * CP, b);
+#pragma unroll
+        for (int p = 0; p < TR; ++p)
+#pragma unroll
+            for (int q = 0; q < TC; ++q) fx_mad(a[p], b[q], hh[p][q], hl[p][q]);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// 6-parameter cameras: a warp per unit, no block barriers.  Per 32 entries:
+// the entries' rows come into the warp's shared memory by 16-byte
+// asynchronous copies (the next chunk's are under way during the sums' end);
+// lane t moves entry t's W row (and gb, DIAG) to the chunk's exponent; lane
+// 4 g + q takes entries g, g + 8, g + 16, g + 24 and quadrant q of the block in
+// two 64-bit integers per output; the eight lane groups' totals meet in
+// shared memory, and a lane per output adds them to its FP64 sum.
+constexpr int F6_WARPS = 4;
+
+template <bool DIAG>
+__device__ void fx6_unit(const FxArgs &g, const SchurUnit u, int2 *sy, int2 *sw)
+{
+    constexpr int CNP = 6, TC = DIAG ? 4 : 3, CP = 2 * TC;  // columns: 6, or 6 + gb + a pad
+    constexpr int SY = 18, SW = DIAG ? 26 : 18;             // words from entry to entry: no bank conflicts
+    constexpr int NV = n_out<CNP, DIAG>(), PER = (NV + 31) / 32;
+    const int lane = threadIdx.x & 31, q = lane & 3, r0 = 3 * (q >> 1), c0 = TC * (q & 1);
+    long long *st = reinterpret_cast<long long *>(sy);  // the totals, over the rows that are read
+    static_assert(8 * 6 * CP <= FX_CHUNK * SY, "the totals fit");
+    double acc[PER];
+    int at[PER], we[PER];
+#pragma unroll
+    for (int p = 0; p < PER; ++p) {
+        acc[p] = 0.0;
+        at[p] = -1;
+        we[p] = 0;
+        const int v = lane + 32 * p;
+        if (v < NV) {
+            int r, c;
+            out_rc<CNP, DIAG>(v, r, c);
+            at[p] = r * CP + c;
+            we[p] = out_weight<CNP, DIAG>(g, u.slot, r, c);
+        }
+    }
+    const int *pa = DIAG ? g.cam_obs + u.begin : g.pa + u.begin, *pb = DIAG ? pa : g.pb + u.begin;
+    // entry lane of a chunk: its observations, and its exponents
+    int a = 0, b = 0, ey = 0, ew = 0;
+    auto indices = [&](int t0) {
+        const int t = min(t0 + lane, u.count - 1);
+        a = __ldg(pa + t);
+        b = DIAG ? a : __ldg(pb + t);
+    };
+    auto fetch = [&]() {
+        const int2 xa = __ldg(g.ex + a);
+        ey = xa.x;
+        ew = DIAG ? xa.y : __ldg(&g.ex[b].y);
+#pragma unroll
+        for (int m = 0; m < 9; ++m) {  // piece p of 9 x 32: row p / 9, 16 bytes p % 9
+            const int p = lane + 32 * m, r = p / 9, part = p - 9 * r;
+            const int ra = __shfl_sync(0xffffffffu, a, r), rb = __shfl_sync(0xffffffffu, b, r);
+            const int wd = DIAG ? (part / 3) * CP + 2 * (part % 3) : 2 * part;
+            cp_async16(sy + r * SY + 2 * part, g.Yq + 18 * (size_t)ra + 2 * part);
+            cp_async16(sw + r * SW + wd, g.Wq + 18 * (size_t)rb + 2 * part);
+        }
+    };
+    indices(0);
+    fetch();
+    for (int t0 = 0; t0 < u.count; t0 += FX_CHUNK) {
+        const int n = min(FX_CHUNK, u.count - t0);
+        const int e = lane < n ? ey + ew : -(1 << 20);
+        const int E = __reduce_max_sync(0xffffffffu, e);
+        bool bad = E >= FX_NAN / 2;
+        int Eg = 0;
+        double gv[3] = {0.0, 0.0, 0.0};
+        if (DIAG) {
+            const double *gp = g.gb + 3 * (size_t)__ldg(g.obs_pt + a);
+            int eg = -(1 << 20), nf = 0;
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                gv[j] = __ldg(gp + j);
+                eg = max(eg, fx_exp(gv[j]));
+                nf |= fx_nonfinite(gv[j]);
+            }
+            Eg = __reduce_max_sync(0xffffffffu, lane < n ? ey + eg : -(1 << 20));
+            bad |= __any_sync(0xffffffffu, nf);
+        }
+        const int eyt = ey;
+        cp_async_wait();
+        __syncwarp();
+        if (!bad) {
+            // entry lane's W row, d bits down
+            if (lane < n) {
+                const int d = E - e;
+                int4 *row = reinterpret_cast<int4 *>(sw + lane * SW);
+#pragma unroll
+                for (int m = 0; m < 9; ++m) {
+                    int4 &x = row[DIAG ? (m / 3) * (CP / 2) + m % 3 : m];
+                    const int2 s0 = fx_shift(make_int2(x.x, x.y), d), s1 = fx_shift(make_int2(x.z, x.w), d);
+                    x = make_int4(s0.x, s0.y, s1.x, s1.y);
+                }
+                if (DIAG)
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) {
+                        const int2 s = fx_limbs(gv[j], Eg - eyt - fx_exp(gv[j]));
+                        row[j * (CP / 2) + 3] = make_int4(s.x, s.y, 0, 0);
+                    }
+            }
+            __syncwarp();
+            long long hh[3][TC], hl[3][TC];
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int j = 0; j < TC; ++j) hh[i][j] = hl[i][j] = 0;
+#pragma unroll
+            for (int m = 0; m < FX_CHUNK / 8; ++m) {
+                const int t = (lane >> 2) + 8 * m;
+                if (t < n) fx_tile<3, TC, 6, CP>(sy + t * SY + r0, sw + t * SW + c0, hh, hl);
+            }
+            __syncwarp();  // the rows are read
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int j = 0; j < TC; ++j)
+                    st[(lane >> 2) * 6 * CP + (r0 + i) * CP + c0 + j] = fx_total(hh[i][j], hl[i][j]);
+            __syncwarp();
+#pragma unroll
+            for (int p = 0; p < PER; ++p) {
+                if (at[p] < 0) continue;
+                long long T = 0;
+#pragma unroll
+                for (int s = 0; s < 8; ++s) T += st[s * 6 * CP + at[p]];
+                acc[p] = fx_add(acc[p], T, we[p] + (DIAG && at[p] % CP == CNP ? Eg : E));
+            }
+        } else {
+#pragma unroll
+            for (int p = 0; p < PER; ++p)
+                if (at[p] >= 0) acc[p] = fx_plain<CNP>(g, pa + t0, pb + t0, n, at[p] / CP, at[p] % CP, acc[p]);
+        }
+        __syncwarp();
+        if (t0 + FX_CHUNK < u.count) {
+            indices(t0 + FX_CHUNK);
+            fetch();
+        }
+    }
+    double *out = (DIAG ? g.diag_partial : g.off_partial) + (size_t)u.out * NV;
+#pragma unroll
+    for (int p = 0; p < PER; ++p)
+        if (at[p] >= 0) out[lane + 32 * p] = acc[p];
+}
+
+// The diagonal units' blocks first (more work per entry), then the pairs'.
+__global__ void __launch_bounds__(32 * F6_WARPS, 4) k_schur_fx6(FxArgs g, int n_diag, const SchurUnit *__restrict__ diag,
+                                                             int n_off, const SchurUnit *__restrict__ off)
+{
+    __shared__ __align__(16) int2 sy[F6_WARPS][FX_CHUNK * 18], sw[F6_WARPS][FX_CHUNK * 26];
+    const int warp = threadIdx.x >> 5, diag_ctas = (n_diag + F6_WARPS - 1) / F6_WARPS;
+    if ((int)blockIdx.x < diag_ctas) {
+        const int uid = blockIdx.x * F6_WARPS + warp;
+        if (uid < n_diag) fx6_unit<true>(g, diag[uid], sy[warp], sw[warp]);
+    } else {
+        const int uid = (blockIdx.x - diag_ctas) * F6_WARPS + warp;
+        if (uid < n_off) fx6_unit<false>(g, off[uid], sy[warp], sw[warp]);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// 11- and 16-parameter cameras: a CTA of four warps per unit, the same steps;
+// half-warps take the entries in turn, 4 x 4 threads with a TR x TC tile each.
+constexpr int FV_THREADS = 128;
+
+template <int CNP, bool DIAG>
+__global__ void __launch_bounds__(FV_THREADS) k_schur_fxv(FxArgs g, const SchurUnit *__restrict__ units)
+{
+    constexpr int RP = fx_rows(CNP), TR = RP / 4, TC = DIAG && CNP == 16 ? 5 : TR, CP = 4 * TC;
+    constexpr int SY = 3 * RP + 2, SW = 3 * CP + 2, NW = FV_THREADS / 32;
+    constexpr int NV = n_out<CNP, DIAG>(), PER = (NV + FV_THREADS - 1) / FV_THREADS;
+    constexpr int PIECES = 3 * RP / 2;  // 16-byte pieces of a row
+    __shared__ __align__(16) int2 sy[FX_CHUNK * SY], sw[FX_CHUNK * SW];
+    __shared__ long long st[NW][RP * CP];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const SchurUnit u = units[blockIdx.x];
+    const int *pa = DIAG ? g.cam_obs + u.begin : g.pa + u.begin, *pb = DIAG ? pa : g.pb + u.begin;
+    for (int e = tid; e < FX_CHUNK * SW; e += FV_THREADS) sw[e] = make_int2(0, 0);  // the padding columns
+    double acc[PER];
+    int at[PER], we[PER];
+#pragma unroll
+    for (int p = 0; p < PER; ++p) {
+        acc[p] = 0.0;
+        at[p] = -1;
+        we[p] = 0;
+        const int v = tid + FV_THREADS * p;
+        if (v < NV) {
+            int r, c;
+            out_rc<CNP, DIAG>(v, r, c);
+            at[p] = r * CP + c;
+            we[p] = out_weight<CNP, DIAG>(g, u.slot, r, c);
+        }
+    }
+    int ey = 0, e = 0, pt = 0;
+    auto fetch = [&](int t0) {
+        const int n = min(FX_CHUNK, u.count - t0);
+        for (int p = tid; p < n * PIECES; p += FV_THREADS) {
+            const int t = p / PIECES, part = p % PIECES;
+            const int wd = (part / (RP / 2)) * CP + 2 * (part % (RP / 2));
+            cp_async16(sy + t * SY + 2 * part, g.Yq + 3 * RP * (size_t)__ldg(pa + t0 + t) + 2 * part);
+            cp_async16(sw + t * SW + wd, g.Wq + 3 * RP * (size_t)__ldg(pb + t0 + t) + 2 * part);
+        }
+        e = -(1 << 20);
+        if (lane < n) {  // every warp: entry lane's exponents
+            const int a = __ldg(pa + t0 + lane);
+            const int2 xa = __ldg(g.ex + a);
+            ey = xa.x;
+            e = ey + (DIAG ? xa.y : __ldg(&g.ex[__ldg(pb + t0 + lane)].y));
+            if (DIAG) pt = __ldg(g.obs_pt + a);
+        }
+    };
+    __syncthreads();
+    fetch(0);
+    for (int t0 = 0; t0 < u.count; t0 += FX_CHUNK) {
+        const int n = min(FX_CHUNK, u.count - t0);
+        const int E = __reduce_max_sync(0xffffffffu, e);
+        const int d = E - e;
+        bool bad = E >= FX_NAN / 2;  // the same in every warp
+        int Eg = 0;
+        double gv[3] = {0.0, 0.0, 0.0};
+        if (DIAG) {
+            int eg = -(1 << 20), nf = 0;
+            if (lane < n)
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    gv[j] = __ldg(g.gb + 3 * (size_t)pt + j);
+                    eg = max(eg, fx_exp(gv[j]));
+                    nf |= fx_nonfinite(gv[j]);
+                }
+            Eg = __reduce_max_sync(0xffffffffu, lane < n ? ey + eg : -(1 << 20));
+            bad |= __any_sync(0xffffffffu, nf);
+        }
+        const int eyt = ey;
+        cp_async_wait();
+        __syncthreads();
+        if (!bad) {
+            if (lane < n) {
+                // entry lane's W row, d bits down; the warps share out the row
+#pragma unroll
+                for (int m = 0; m < (PIECES + NW - 1) / NW; ++m) {
+                    const int part = warp + NW * m;
+                    if (part < PIECES) {
+                        int4 &x = *reinterpret_cast<int4 *>(sw + lane * SW + (part / (RP / 2)) * CP + 2 * (part % (RP / 2)));
+                        const int2 s0 = fx_shift(make_int2(x.x, x.y), d), s1 = fx_shift(make_int2(x.z, x.w), d);
+                        x = make_int4(s0.x, s0.y, s1.x, s1.y);
+                    }
+                }
+            }
+            if (DIAG) {
+                if (CNP < RP) __syncthreads();  // gb takes the place of the padding column that the shift has rewritten
+                if (lane < n && warp < 3)
+                    sw[lane * SW + warp * CP + CNP] = fx_limbs(gv[warp], Eg - eyt - fx_exp(gv[warp]));
+            }
+        }
+        __syncthreads();
+        if (!bad) {
+            const int l = tid & 15, r0 = (l >> 2) * TR, c0 = (l & 3) * TC;
+            long long hh[TR][TC], hl[TR][TC];
+#pragma unroll
+            for (int i = 0; i < TR; ++i)
+#pragma unroll
+                for (int j = 0; j < TC; ++j) hh[i][j] = hl[i][j] = 0;
+            for (int t = tid >> 4; t < n; t += FV_THREADS / 16)
+                fx_tile<TR, TC, RP, CP>(sy + t * SY + r0, sw + t * SW + c0, hh, hl);
+#pragma unroll
+            for (int i = 0; i < TR; ++i)
+#pragma unroll
+                for (int j = 0; j < TC; ++j) {
+                    long long T = fx_total(hh[i][j], hl[i][j]);
+                    T += __shfl_xor_sync(0xffffffffu, T, 16);
+                    if (lane < 16) st[warp][(r0 + i) * CP + c0 + j] = T;
+                }
+        }
+        __syncthreads();
+        if (t0 + FX_CHUNK < u.count) fetch(t0 + FX_CHUNK);
+#pragma unroll
+        for (int p = 0; p < PER; ++p) {
+            if (at[p] < 0) continue;
+            const int r = at[p] / CP, c = at[p] % CP;
+            if (bad) {
+                acc[p] = fx_plain<CNP>(g, pa + t0, pb + t0, n, r, c, acc[p]);
+                continue;
+            }
+            long long T = 0;
+#pragma unroll
+            for (int w = 0; w < NW; ++w) T += st[w][at[p]];
+            acc[p] = fx_add(acc[p], T, we[p] + (DIAG && c == CNP ? Eg : E));
+        }
+    }
+    double *out = (DIAG ? g.diag_partial : g.off_partial) + (size_t)u.out * NV;
+#pragma unroll
+    for (int p = 0; p < PER; ++p)
+        if (at[p] >= 0) out[tid + FV_THREADS * p] = acc[p];
+}
+
+template <int CNP>
+void limb_rows_t(const DeviceProblem &d, cudaStream_t s)
+{
+    constexpr int OB = LR_THREADS / (CNP == 6 ? 2 : 4);
+    k_limb_rows<CNP><<<ceil_div(d.no, OB), LR_THREADS, 0, s>>>(d.no, d.obs_pt, d.obs_cam, d.W, d.Vinv, d.U,
+                                                               reinterpret_cast<int2 *>(d.Y), d.Wq, d.fx_ex);
+}
+
+}  // namespace
+
+void launch_limb_rows(const DeviceProblem &d, cudaStream_t s)
+{
+    if (d.no == 0) return;
+    if (d.cnp == 6) limb_rows_t<6>(d, s);
+    else if (d.cnp == 11) limb_rows_t<11>(d, s);
+    else limb_rows_t<16>(d, s);
+    note_launch(1);
+}
+
+void launch_schur_fx(const DeviceProblem &d, double *diag_partial, cudaStream_t s)
+{
+    FxArgs g{d.pair_a, d.pair_b, d.cam_obs, d.obs_pt, reinterpret_cast<const int2 *>(d.Y), d.Wq, d.fx_ex, d.W, d.Vinv,
+             d.U, d.g + d.N, d.pair_kl, d.schur_partial, diag_partial};
+    if (d.cnp == 6) {
+        const int ctas = ceil_div(d.n_fx_diag_units, F6_WARPS) + ceil_div(d.n_off_units, F6_WARPS);
+        if (ctas == 0) return;
+        k_schur_fx6<<<ctas, 32 * F6_WARPS, 0, s>>>(g, d.n_fx_diag_units, d.fx_diag_units, d.n_off_units, d.off_units);
+        note_launch(1);
+        return;
+    }
+    if (d.n_diag_units > 0) {
+        if (d.cnp == 11) k_schur_fxv<11, true><<<d.n_diag_units, FV_THREADS, 0, s>>>(g, d.diag_units);
+        else k_schur_fxv<16, true><<<d.n_diag_units, FV_THREADS, 0, s>>>(g, d.diag_units);
+        note_launch(1);
+    }
+    if (d.n_off_units > 0) {
+        if (d.cnp == 11) k_schur_fxv<11, false><<<d.n_off_units, FV_THREADS, 0, s>>>(g, d.off_units);
+        else k_schur_fxv<16, false><<<d.n_off_units, FV_THREADS, 0, s>>>(g, d.off_units);
+        note_launch(1);
+    }
+}
+
+}  // namespace psba

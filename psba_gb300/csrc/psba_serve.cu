@@ -43,6 +43,7 @@
 #include <vector>
 
 #include "psba_batch_internal.h"
+#include "psba_fixed.h"
 
 using namespace psba;
 using namespace psba::batch;
@@ -329,7 +330,7 @@ void worker_main(psba_server *s)
 
 // Device bytes of a request on the single-problem engine (an upper estimate
 // of what psba_create allocates): per observation e, A, B, W, Y, J x
-// buffers and indices; per point V, V^-1, g, dp and trust-region vectors;
+// buffers, limb rows and indices; per point V, V^-1, g, dp and trust-region vectors;
 // the camera-pair entries and their Schur partials; S, its copy and the
 // dense-solve work arrays; 16 MB of slack for the small tables.
 size_t large_bytes(const psba_problem_desc &p, int cnp)
@@ -341,15 +342,12 @@ size_t large_bytes(const psba_problem_desc &p, int cnp)
         entries += (b - a) * (b - a - 1) / 2;
     }
     const size_t N = c * nc, Np = (N + TILE - 1) / TILE * TILE;
-    // off-diagonal partial slots: 6-parameter cameras, one per chunk plus one
-    // per pair boundary inside a chunk; otherwise one per unit
-    const size_t off_units = c == 6 ? std::min(entries / OFF_MIN_LEN + 1, (size_t)schur_off_wave_threads())
-                                    : entries / SCHUR_CHUNK;
-    const size_t per_obs = 2 + 2 * c + 6 + 2 * 3 * c + 3 * 2 + 3 + 4;
+    // Schur units of at least 32 entries or observations, and one more per pair and camera
+    const size_t off_units = entries / 32 + nc * (nc - 1) / 2, diag_units = no / 32 + nc;
+    const size_t per_obs = 2 + 2 * c + 6 + 3 * c + 2 * (size_t)fx_words(cnp) + 1 + 3 * 2 + 3 + 4;
     const size_t per_pt = 3 * 3 + 6 * 2 + 9 + 3 * 6;
     const size_t doubles = no * per_obs + np * per_pt + N * 8 + nc * (c * c + 2 * CAMTAB) + 3 * Np * Np +
-                           Np * TILE + (off_units + nc * 8) * c * c +
-                           (no / (c == 6 ? DIAG_SUPER : DIAG_CHUNK) + nc) * (c * (c + 1) / 2 + c);  // diagonal-unit partials
+                           Np * TILE + (off_units + nc * 8) * c * c + diag_units * (c * (c + 1) / 2 + c);
     // index-build scratch: counts and offsets per (pair-list segment, camera)
     const size_t segs = no / (size_t)pair_segment_len(p.n_cams, p.n_obs) + nc;
     return doubles * sizeof(double) + entries * 2 * sizeof(int) + segs * nc * 2 * sizeof(int) + ((size_t)16 << 20);

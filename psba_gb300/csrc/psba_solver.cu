@@ -15,6 +15,7 @@
 #include <mutex>
 #include <vector>
 
+#include "psba_fixed.h"
 #include "psba_internal.h"
 
 namespace psba {
@@ -333,7 +334,8 @@ void enqueue_reduced(psba_handle *h, double mu)
     }
     {
         StageScope sc(h, ST_Y);
-        launch_yblocks(d, h->stream);
+        if (d.prec == PSBA_PREC_FP64) launch_limb_rows(d, h->stream);
+        else launch_yblocks(d, h->stream);
     }
     {
         StageScope sc(h, ST_SCHUR_OFF);
@@ -947,56 +949,26 @@ int create_impl(const psba_problem_desc *p, psba_handle *h)
                      d.pt_start, d_off, d.pair_a, d.pair_b, h->stream);
     TRY(check_launch());
     // Schur work units; execution order longest first
-    std::vector<SchurUnit> off_units, off_chunks, diag_units, mx_units;
-    std::vector<int> off_start(n_pairs + 1, 0), chunk_start(n_pairs + 1, 0), diag_start(nc + 1, 0),
-        mx_start(n_pairs + 1, 0);
-    off_units.reserve((size_t)(n_entries / SCHUR_CHUNK) + (size_t)n_pairs);
-    for (int q = 0; q < n_pairs; ++q) {
-        for (long long b = pair_start[q]; b < pair_start[q + 1]; b += SCHUR_CHUNK) {
-            const int cnt = (int)std::min<long long>(SCHUR_CHUNK, pair_start[q + 1] - b);
-            off_units.push_back({q, (int)b, cnt, (int)off_units.size()});
+    std::vector<SchurUnit> off_units, diag_units, fx_diag_units, mx_units;
+    std::vector<int> off_start, diag_start, fx_diag_start, mx_start;
+    // units of at most len of the ranges start[q] .. start[q + 1], numbered in order
+    auto cut_units = [](const auto &start, int len, std::vector<SchurUnit> &units, std::vector<int> &first) {
+        const int n = (int)start.size() - 1;
+        first.assign((size_t)n + 1, 0);
+        units.reserve((size_t)(start[n] / len) + (size_t)n);
+        for (int q = 0; q < n; ++q) {
+            for (long long b = start[q]; b < start[q + 1]; b += len)
+                units.push_back({q, (int)b, (int)std::min<long long>(len, start[q + 1] - b), (int)units.size()});
+            first[q + 1] = (int)units.size();
         }
-        off_start[q + 1] = (int)off_units.size();
-    }
-    int n_chunk_slots = 0;
+    };
+    const int off_len = off_unit_len(d.cnp, n_entries), fx_diag_len = diag_unit_len(d.cnp, no);
+    const int dchunk = d.cnp == 6 ? DIAG_SUPER : fx_diag_len;
+    cut_units(pair_start, off_len, off_units, off_start);
+    cut_units(cam_start, dchunk, diag_units, diag_start);
     if (d.cnp == 6) {
-        // the pair list in equal chunks, one per thread of one resident wave,
-        // so every SM gets the same number of products; a chunk writes one
-        // slot per pair it touches, slots numbered in list order
-        const long long G = std::max(1, schur_off_wave_threads());
-        const long long len = std::max<long long>(OFF_MIN_LEN, (n_entries + G - 1) / G);
-        off_chunks.reserve((size_t)(n_entries / len) + 1);
-        int q = 0;
-        for (long long b = 0; b < n_entries; b += len) {
-            const long long e = std::min(n_entries, b + len);
-            while (pair_start[q + 1] <= b) ++q;
-            off_chunks.push_back({q, (int)b, (int)(e - b), n_chunk_slots});
-            for (long long sb = b, qq = q;; ++qq) {
-                if (sb == pair_start[qq]) chunk_start[qq] = n_chunk_slots;
-                ++n_chunk_slots;
-                const long long se = std::min(e, pair_start[qq + 1]);
-                if (se == e) break;
-                sb = se;
-            }
-        }
-        chunk_start[n_pairs] = n_chunk_slots;
-        // FP32 products: units of <= MX_UNIT entries of one pair, one warp each
-        mx_units.reserve((size_t)(n_entries / MX_UNIT) + (size_t)n_pairs);
-        for (int q = 0; q < n_pairs; ++q) {
-            for (long long b = pair_start[q]; b < pair_start[q + 1]; b += MX_UNIT) {
-                const int cnt = (int)std::min<long long>(MX_UNIT, pair_start[q + 1] - b);
-                mx_units.push_back({q, (int)b, cnt, (int)mx_units.size()});
-            }
-            mx_start[q + 1] = (int)mx_units.size();
-        }
-    }
-    const int dchunk = d.cnp == 6 ? DIAG_SUPER : DIAG_CHUNK;
-    for (int j = 0; j < nc; ++j) {
-        for (int b = cam_start[j]; b < cam_start[j + 1]; b += dchunk) {
-            const int cnt = std::min(dchunk, cam_start[j + 1] - b);
-            diag_units.push_back({j, b, cnt, (int)diag_units.size()});
-        }
-        diag_start[j + 1] = (int)diag_units.size();
+        cut_units(pair_start, MX_UNIT, mx_units, mx_start);  // FP32 products
+        cut_units(cam_start, fx_diag_len, fx_diag_units, fx_diag_start);
     }
     // stable order by count, descending (a counting sort: counts are 1..maxc)
     auto sort_by_count = [](std::vector<SchurUnit> &u, int maxc) {
@@ -1007,9 +979,10 @@ int create_impl(const psba_problem_desc *p, psba_handle *h)
         for (const SchurUnit &x : u) out[start[maxc - x.count]++] = x;
         u.swap(out);
     };
-    sort_by_count(off_units, SCHUR_CHUNK);
+    sort_by_count(off_units, off_len);
     sort_by_count(mx_units, MX_UNIT);
     sort_by_count(diag_units, dchunk);
+    sort_by_count(fx_diag_units, fx_diag_len);
     std::vector<CamUnit> cam_units;
     std::vector<int> cam_unit_start(nc + 1, 0);
     for (int j = 0; j < nc; ++j) {
@@ -1021,10 +994,9 @@ int create_impl(const psba_problem_desc *p, psba_handle *h)
     d.n_pairs = n_pairs;
     d.n_pair_entries = n_entries;
     d.n_off_units = (int)off_units.size();
-    d.n_off_chunks = (int)off_chunks.size();
-    d.n_off_chunk_slots = n_chunk_slots;
     d.n_mx_units = (int)mx_units.size();
     d.n_diag_units = (int)diag_units.size();
+    d.n_fx_diag_units = (int)fx_diag_units.size();
     d.n_cam_units = (int)cam_units.size();
 
     // ---- device memory
@@ -1036,9 +1008,8 @@ int create_impl(const psba_problem_desc *p, psba_handle *h)
     TRY(dalloc(h, &d.off_units, off_units.size()));
     TRY(dalloc(h, &d.off_unit_start, (size_t)n_pairs + 1));
     if (d.cnp == 6) {
-        TRY(dalloc(h, &d.pair_start, (size_t)n_pairs + 1));
-        TRY(dalloc(h, &d.off_chunk_start, (size_t)n_pairs + 1));
-        TRY(dalloc(h, &d.off_chunks, off_chunks.size()));
+        TRY(dalloc(h, &d.fx_diag_units, fx_diag_units.size()));
+        TRY(dalloc(h, &d.fx_diag_unit_start, (size_t)nc + 1));
         TRY(dalloc(h, &d.mx_units, mx_units.size()));
         TRY(dalloc(h, &d.mx_unit_start, (size_t)n_pairs + 1));
     }
@@ -1068,8 +1039,11 @@ int create_impl(const psba_problem_desc *p, psba_handle *h)
     TRY(dalloc(h, &d.Vinv, 6 * (size_t)np));
     TRY(dalloc(h, &d.Vinv2f, 12 * (size_t)np));
     TRY(dalloc(h, &d.gb32, 3 * (size_t)np));
-    TRY(dalloc(h, &d.Y, 3 * cnp * (size_t)no));
-    TRY(dalloc(h, &d.schur_partial, cnp * cnp * off_partial_slots(d) + diag_nv * diag_units.size()));
+    TRY(dalloc(h, &d.Y, (size_t)fx_words(d.cnp) * (size_t)no));
+    TRY(dalloc(h, &d.Wq, (size_t)fx_words(d.cnp) * (size_t)no));
+    TRY(dalloc(h, &d.fx_ex, (size_t)no));
+    TRY(dalloc(h, &d.schur_partial,
+               cnp * cnp * off_partial_slots(d) + diag_nv * std::max(diag_units.size(), fx_diag_units.size())));
     TRY(dalloc(h, &d.S, (size_t)d.Np * d.Np));
     d.Nm3 = d.N % 3 == 0 ? d.Np : ((d.Np + 2) / 3) * 3;
     TRY(dalloc(h, &d.Ssave, (size_t)d.Nm3 * d.Nm3));
@@ -1142,10 +1116,8 @@ int create_impl(const psba_problem_desc *p, psba_handle *h)
     TRY(upload(h, d.off_units, off_units.data(), off_units.size()));
     TRY(upload(h, d.off_unit_start, off_start.data(), off_start.size()));
     if (d.cnp == 6) {
-        const std::vector<int> ps(pair_start.begin(), pair_start.end());
-        TRY(upload(h, d.pair_start, ps.data(), ps.size()));
-        TRY(upload(h, d.off_chunk_start, chunk_start.data(), chunk_start.size()));
-        TRY(upload(h, d.off_chunks, off_chunks.data(), off_chunks.size()));
+        TRY(upload(h, d.fx_diag_units, fx_diag_units.data(), fx_diag_units.size()));
+        TRY(upload(h, d.fx_diag_unit_start, fx_diag_start.data(), fx_diag_start.size()));
         TRY(upload(h, d.mx_units, mx_units.data(), mx_units.size()));
         TRY(upload(h, d.mx_unit_start, mx_start.data(), mx_start.size()));
     }
@@ -1262,13 +1234,6 @@ int psba_create(const psba_problem_desc *desc, psba_handle **out)
     psba_handle *h = new (std::nothrow) psba_handle();
     if (!h) return set_error("host allocation failed"), PSBA_ERR_NOMEM;
     keep_pool_memory();
-    {
-        const int r = prepare_device_kernels();
-        if (r != PSBA_OK) {
-            destroy_impl(h);
-            return r;
-        }
-    }
     cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreate(&h->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&h->ev1);
@@ -1458,6 +1423,10 @@ int psba_eval_reduced(psba_handle *h, double mu, double *Vinv, double *Y, double
     h->last_mu = mu;
     TRY(check_launch());
     const size_t no = (size_t)d.no, np = (size_t)d.np;
+    if (Y && d.prec == PSBA_PREC_FP64) {  // in the place of its limb rows
+        launch_yblocks(d, h->stream);
+        TRY(check_launch());
+    }
     TRY(copy_out(h, Y, d.Y, 3 * (size_t)d.cnp * no));
     if (Vinv && np) {
         const int prec = d.prec;

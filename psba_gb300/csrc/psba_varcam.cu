@@ -321,7 +321,8 @@ __global__ void k_camera_finish_v(int nc, const int *__restrict__ unit_start, co
     if (r == c) uvdiag[CNP * (size_t)j + r] = sum;
 }
 
-// Y = W V^-1 per observation (V^-1 FP64, products FP64, stored in R).
+// Y = W V^-1 per observation (V^-1 FP64, products FP64, stored in R).  The FP64
+// solves take Y from k_limb_rows; the FP64 instances serve psba_eval_reduced.
 template <typename R, int CNP>
 __global__ void __launch_bounds__(256) k_yblocks_v(int no, const int *__restrict__ obs_pt, const R *__restrict__ W,
                                                    const double *__restrict__ Vinv, R *__restrict__ Y)
@@ -341,107 +342,124 @@ __global__ void __launch_bounds__(256) k_yblocks_v(int no, const int *__restrict
     }
 }
 
-// Off-diagonal Schur blocks: one CTA per unit of <= SCHUR_CHUNK common
-// points of a camera pair (k > l); the unit's Y_a and W_b rows are staged in
-// shared memory; thread t owns entries t, t + 128, ... of the cnp x cnp block.
-template <typename R, int CNP>
+// FP32 off-diagonal Schur blocks (the mixed form): one CTA per unit of
+// common points of a camera pair (k > l), SCHUR_CHUNK at a time: their Y_a and
+// W_b rows are staged in shared memory; thread t owns entries t, t + 128, ...
+// of the cnp x cnp block, FP32 sums of VFLUSH entries added in FP64.
+template <int CNP>
 __global__ void __launch_bounds__(VC_THREADS) k_schur_off_v(const SchurUnit *__restrict__ units,
                                                             const int *__restrict__ pa, const int *__restrict__ pb,
-                                                            const R *__restrict__ Y, const R *__restrict__ W,
+                                                            const float *__restrict__ Y, const float *__restrict__ W,
                                                             double *__restrict__ partial)
 {
     constexpr int NE = CNP * CNP, PER = (NE + VC_THREADS - 1) / VC_THREADS;
-    __shared__ R sy[SCHUR_CHUNK][3 * CNP], sw[SCHUR_CHUNK][3 * CNP];
+    __shared__ float sy[SCHUR_CHUNK][3 * CNP], sw[SCHUR_CHUNK][3 * CNP];
     const SchurUnit u = units[blockIdx.x];
-    for (int e = threadIdx.x; e < u.count * 3 * CNP; e += VC_THREADS) {
-        const int t = e / (3 * CNP), k = e % (3 * CNP);
-        sy[t][k] = Y[3 * CNP * (size_t)pa[u.begin + t] + k];
-        sw[t][k] = W[3 * CNP * (size_t)pb[u.begin + t] + k];
-    }
-    __syncthreads();
+    double acc[PER];
 #pragma unroll
-    for (int q = 0; q < PER; ++q) {
-        const int v = threadIdx.x + q * VC_THREADS;
-        if (v >= NE) continue;
-        const int r = v / CNP, c = v % CNP;
-        double acc = 0.0;
-        if constexpr (sizeof(R) == 8) {
-            for (int t = 0; t < u.count; ++t) {
-                acc = fma((double)sy[t][3 * r], (double)sw[t][3 * c], acc);
-                acc = fma((double)sy[t][3 * r + 1], (double)sw[t][3 * c + 1], acc);
-                acc = fma((double)sy[t][3 * r + 2], (double)sw[t][3 * c + 2], acc);
-            }
-        } else {
-            for (int f0 = 0; f0 < u.count; f0 += VFLUSH) {
-                R part = (R)0;
-                const int f1 = min(u.count, f0 + VFLUSH);
+    for (int q = 0; q < PER; ++q) acc[q] = 0.0;
+    for (int t0 = 0; t0 < u.count; t0 += SCHUR_CHUNK) {
+        const int n = min(SCHUR_CHUNK, u.count - t0);
+        __syncthreads();
+        for (int e = threadIdx.x; e < n * 3 * CNP; e += VC_THREADS) {
+            const int t = e / (3 * CNP), k = e % (3 * CNP);
+            sy[t][k] = Y[3 * CNP * (size_t)pa[u.begin + t0 + t] + k];
+            sw[t][k] = W[3 * CNP * (size_t)pb[u.begin + t0 + t] + k];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+            const int v = threadIdx.x + q * VC_THREADS;
+            if (v >= NE) continue;
+            const int r = v / CNP, c = v % CNP;
+            for (int f0 = 0; f0 < n; f0 += VFLUSH) {
+                float part = 0.0f;
+                const int f1 = min(n, f0 + VFLUSH);
                 for (int t = f0; t < f1; ++t) {
                     part = fma(sy[t][3 * r], sw[t][3 * c], part);
                     part = fma(sy[t][3 * r + 1], sw[t][3 * c + 1], part);
                     part = fma(sy[t][3 * r + 2], sw[t][3 * c + 2], part);
                 }
-                acc += (double)part;
+                acc[q] += (double)part;
             }
         }
-        partial[(size_t)u.out * NE + v] = acc;
+    }
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+        const int v = threadIdx.x + q * VC_THREADS;
+        if (v < NE) partial[(size_t)u.out * NE + v] = acc[q];
     }
 }
 
-// Diagonal Schur blocks and ea: one CTA per unit of <= DIAG_CHUNK
-// observations of a camera; lower-triangle entries of sum Y W^T and the
+// FP32 diagonal Schur blocks and ea: one CTA per unit of observations of a
+// camera, DIAG_CHUNK at a time; lower-triangle entries of sum Y W^T and the
 // cnp sums of Y gb.
-template <typename R, int CNP>
+template <int CNP>
 __global__ void __launch_bounds__(VC_THREADS) k_schur_diag_v(const SchurUnit *__restrict__ units,
                                                              const int *__restrict__ cam_obs,
                                                              const int *__restrict__ obs_pt,
-                                                             const R *__restrict__ Y, const R *__restrict__ W,
+                                                             const float *__restrict__ Y, const float *__restrict__ W,
                                                              const double *__restrict__ gb,
                                                              double *__restrict__ partial)
 {
     constexpr int NV = diag_nv<CNP>(), NL = CNP * (CNP + 1) / 2, PER = (NV + VC_THREADS - 1) / VC_THREADS;
-    __shared__ R sy[DIAG_CHUNK][3 * CNP], sw[DIAG_CHUNK][3 * CNP];
+    __shared__ float sy[DIAG_CHUNK][3 * CNP], sw[DIAG_CHUNK][3 * CNP];
     __shared__ double sg[DIAG_CHUNK][3];
     const SchurUnit u = units[blockIdx.x];
-    for (int e = threadIdx.x; e < u.count * 3 * CNP; e += VC_THREADS) {
-        const int t = e / (3 * CNP), k = e % (3 * CNP);
-        const int o = cam_obs[u.begin + t];
-        sy[t][k] = Y[3 * CNP * (size_t)o + k];
-        sw[t][k] = W[3 * CNP * (size_t)o + k];
+    double acc[PER];
+    int er[PER], ec[PER];
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+        acc[q] = 0.0;
+        er[q] = ec[q] = 0;
+        const int v = threadIdx.x + q * VC_THREADS;
+        if (v < NL) lower_rc(v, er[q], ec[q]);
     }
-    for (int e = threadIdx.x; e < u.count * 3; e += VC_THREADS) {
-        const int t = e / 3, k = e % 3;
-        sg[t][k] = gb[3 * (size_t)obs_pt[cam_obs[u.begin + t]] + k];
+    for (int t0 = 0; t0 < u.count; t0 += DIAG_CHUNK) {
+        const int n = min(DIAG_CHUNK, u.count - t0);
+        __syncthreads();
+        for (int e = threadIdx.x; e < n * 3 * CNP; e += VC_THREADS) {
+            const int t = e / (3 * CNP), k = e % (3 * CNP);
+            const int o = cam_obs[u.begin + t0 + t];
+            sy[t][k] = Y[3 * CNP * (size_t)o + k];
+            sw[t][k] = W[3 * CNP * (size_t)o + k];
+        }
+        for (int e = threadIdx.x; e < n * 3; e += VC_THREADS) {
+            const int t = e / 3, k = e % 3;
+            sg[t][k] = gb[3 * (size_t)obs_pt[cam_obs[u.begin + t0 + t]] + k];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+            const int v = threadIdx.x + q * VC_THREADS;
+            if (v >= NV) continue;
+            if (v < NL) {
+                const int r = er[q], c = ec[q];
+                for (int f0 = 0; f0 < n; f0 += VFLUSH) {
+                    float part = 0.0f;
+                    const int f1 = min(n, f0 + VFLUSH);
+                    for (int t = f0; t < f1; ++t) {
+                        part = fma(sy[t][3 * r], sw[t][3 * c], part);
+                        part = fma(sy[t][3 * r + 1], sw[t][3 * c + 1], part);
+                        part = fma(sy[t][3 * r + 2], sw[t][3 * c + 2], part);
+                    }
+                    acc[q] += (double)part;
+                }
+            } else {
+                // ea sums: FP64 from the exact products (ea cancels near the optimum)
+                const int r = v - NL;
+                for (int t = 0; t < n; ++t) {
+                    acc[q] = fma((double)sy[t][3 * r], sg[t][0], acc[q]);
+                    acc[q] = fma((double)sy[t][3 * r + 1], sg[t][1], acc[q]);
+                    acc[q] = fma((double)sy[t][3 * r + 2], sg[t][2], acc[q]);
+                }
+            }
+        }
     }
-    __syncthreads();
 #pragma unroll
     for (int q = 0; q < PER; ++q) {
         const int v = threadIdx.x + q * VC_THREADS;
-        if (v >= NV) continue;
-        double acc = 0.0;
-        if (v < NL) {
-            int r, c;
-            lower_rc(v, r, c);
-            for (int f0 = 0; f0 < u.count; f0 += VFLUSH) {
-                R part = (R)0;
-                const int f1 = min(u.count, f0 + VFLUSH);
-                for (int t = f0; t < f1; ++t) {
-                    part = fma(sy[t][3 * r], sw[t][3 * c], part);
-                    part = fma(sy[t][3 * r + 1], sw[t][3 * c + 1], part);
-                    part = fma(sy[t][3 * r + 2], sw[t][3 * c + 2], part);
-                }
-                acc += (double)part;
-            }
-        } else {
-            // ea sums: FP64 from the exact products in both forms (ea cancels
-            // near the optimum)
-            const int r = v - NL;
-            for (int t = 0; t < u.count; ++t) {
-                acc = fma((double)sy[t][3 * r], sg[t][0], acc);
-                acc = fma((double)sy[t][3 * r + 1], sg[t][1], acc);
-                acc = fma((double)sy[t][3 * r + 2], sg[t][2], acc);
-            }
-        }
-        partial[(size_t)u.out * NV + v] = acc;
+        if (v < NV) partial[(size_t)u.out * NV + v] = acc[q];
     }
 }
 
@@ -582,22 +600,22 @@ void camera_t(const DeviceProblem &d, double coeff, cudaStream_t s)
     note_launch(1);
 }
 
-template <typename R, int CNP>
+template <int CNP>
 void schur_off_t(const DeviceProblem &d, cudaStream_t s)
 {
     if (d.n_off_units == 0) return;
-    k_schur_off_v<R, CNP><<<d.n_off_units, VC_THREADS, 0, s>>>(d.off_units, d.pair_a, d.pair_b, (const R *)d.Y,
-                                                               (const R *)d.W, d.schur_partial);
+    k_schur_off_v<CNP><<<d.n_off_units, VC_THREADS, 0, s>>>(d.off_units, d.pair_a, d.pair_b, (const float *)d.Y,
+                                                            (const float *)d.W, d.schur_partial);
     note_launch(1);
 }
 
-template <typename R, int CNP>
+template <int CNP>
 void schur_diag_t(const DeviceProblem &d, cudaStream_t s)
 {
     if (d.n_diag_units == 0) return;
-    double *diag_partial = d.schur_partial + (size_t)d.n_off_units * CNP * CNP;
-    k_schur_diag_v<R, CNP><<<d.n_diag_units, VC_THREADS, 0, s>>>(d.diag_units, d.cam_obs, d.obs_pt, (const R *)d.Y,
-                                                                 (const R *)d.W, d.g + d.N, diag_partial);
+    double *diag_partial = d.schur_partial + off_partial_slots(d) * CNP * CNP;
+    k_schur_diag_v<CNP><<<d.n_diag_units, VC_THREADS, 0, s>>>(d.diag_units, d.cam_obs, d.obs_pt, (const float *)d.Y,
+                                                              (const float *)d.W, d.g + d.N, diag_partial);
     note_launch(1);
 }
 
@@ -605,7 +623,7 @@ template <int CNP>
 void reduce_t(const DeviceProblem &d, double mu, cudaStream_t s)
 {
     double *off_partial = d.schur_partial;
-    double *diag_partial = d.schur_partial + (size_t)d.n_off_units * CNP * CNP;
+    double *diag_partial = d.schur_partial + off_partial_slots(d) * CNP * CNP;
     const long long total = (long long)d.n_pairs * CNP * CNP + (long long)d.nc * diag_nv<CNP>();
     k_schur_reduce_v<CNP><<<ceil_div(total, 128), 128, 0, s>>>(d.n_pairs, d.nc, d.Np, d.pair_kl, d.off_unit_start,
                                                                off_partial, d.diag_unit_start, diag_partial, d.U,
@@ -645,7 +663,9 @@ void launch_yblocks_v(const DeviceProblem &d, cudaStream_t s)
     if (d.no == 0) return;
     const bool f64 = d.prec == PSBA_PREC_FP64;
     const int nb = ceil_div(d.no, 256);
-    if (d.cnp == 11) {
+    if (d.cnp == 6) {
+        k_yblocks_v<double, 6><<<nb, 256, 0, s>>>(d.no, d.obs_pt, d.W, d.Vinv, d.Y);
+    } else if (d.cnp == 11) {
         if (f64) k_yblocks_v<double, 11><<<nb, 256, 0, s>>>(d.no, d.obs_pt, d.W, d.Vinv, d.Y);
         else k_yblocks_v<float, 11><<<nb, 256, 0, s>>>(d.no, d.obs_pt, (const float *)d.W, d.Vinv, (float *)d.Y);
     } else {
@@ -655,9 +675,17 @@ void launch_yblocks_v(const DeviceProblem &d, cudaStream_t s)
     note_launch(1);
 }
 
-void launch_schur_off_v(const DeviceProblem &d, cudaStream_t s) { VC_DISPATCH(schur_off_t, d, s); }
+void launch_schur_off_v(const DeviceProblem &d, cudaStream_t s)
+{
+    if (d.cnp == 11) schur_off_t<11>(d, s);
+    else schur_off_t<16>(d, s);
+}
 
-void launch_schur_diag_v(const DeviceProblem &d, cudaStream_t s) { VC_DISPATCH(schur_diag_t, d, s); }
+void launch_schur_diag_v(const DeviceProblem &d, cudaStream_t s)
+{
+    if (d.cnp == 11) schur_diag_t<11>(d, s);
+    else schur_diag_t<16>(d, s);
+}
 
 void launch_schur_reduce_v(const DeviceProblem &d, double mu, cudaStream_t s)
 {
