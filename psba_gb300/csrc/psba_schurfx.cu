@@ -205,7 +205,7 @@ __device__ __forceinline__ void fx_tile(const int2 *y, const int2 *w, long long 
 // 4 g + q takes entries g, g + 8, g + 16, g + 24 and quadrant q of the block in
 // two 64-bit integers per output; the eight lane groups' totals meet in
 // shared memory, and a lane per output adds them to its FP64 sum.
-constexpr int F6_WARPS = 4;
+constexpr int F6_WARPS = 4, F6_CTAS = 4;  // resident CTAs per SM: 188 / 173 / 185 us with 3 / 4 / 5 at 88 cameras
 
 template <bool DIAG>
 __device__ void fx6_unit(const FxArgs &g, const SchurUnit u, int2 *sy, int2 *sw)
@@ -232,41 +232,47 @@ __device__ void fx6_unit(const FxArgs &g, const SchurUnit u, int2 *sy, int2 *sw)
         }
     }
     const int *pa = DIAG ? g.cam_obs + u.begin : g.pa + u.begin, *pb = DIAG ? pa : g.pb + u.begin;
-    // entry lane of a chunk: its observations, and its exponents
-    int a = 0, b = 0, ey = 0, ew = 0;
+    // entry lane of a chunk: its observations, its exponents and (DIAG) its
+    // point; while a chunk is summed, the next one's
+    int an = 0, bn = 0, ey = 0, ew = 0, pt = 0;
     auto indices = [&](int t0) {
         const int t = min(t0 + lane, u.count - 1);
-        a = __ldg(pa + t);
-        b = DIAG ? a : __ldg(pb + t);
+        an = __ldg(pa + t);
+        bn = DIAG ? an : __ldg(pb + t);
     };
-    auto fetch = [&]() {
-        const int2 xa = __ldg(g.ex + a);
-        ey = xa.x;
-        ew = DIAG ? xa.y : __ldg(&g.ex[b].y);
+    auto exponents = [&](int &y, int &w, int &i) {
+        const int2 x = __ldg(g.ex + an);
+        y = x.x;
+        w = DIAG ? x.y : __ldg(&g.ex[bn].y);
+        if (DIAG) i = __ldg(g.obs_pt + an);
+    };
+    auto rows = [&]() {
 #pragma unroll
         for (int m = 0; m < 9; ++m) {  // piece p of 9 x 32: row p / 9, 16 bytes p % 9
             const int p = lane + 32 * m, r = p / 9, part = p - 9 * r;
-            const int ra = __shfl_sync(0xffffffffu, a, r), rb = __shfl_sync(0xffffffffu, b, r);
+            const int ra = __shfl_sync(0xffffffffu, an, r), rb = __shfl_sync(0xffffffffu, bn, r);
             const int wd = DIAG ? (part / 3) * CP + 2 * (part % 3) : 2 * part;
             cp_async16(sy + r * SY + 2 * part, g.Yq + 18 * (size_t)ra + 2 * part);
             cp_async16(sw + r * SW + wd, g.Wq + 18 * (size_t)rb + 2 * part);
         }
     };
     indices(0);
-    fetch();
+    exponents(ey, ew, pt);
+    rows();
     for (int t0 = 0; t0 < u.count; t0 += FX_CHUNK) {
         const int n = min(FX_CHUNK, u.count - t0);
+        const bool more = t0 + FX_CHUNK < u.count;
+        if (more) indices(t0 + FX_CHUNK);
         const int e = lane < n ? ey + ew : -(1 << 20);
         const int E = __reduce_max_sync(0xffffffffu, e);
         bool bad = E >= FX_NAN / 2;
         int Eg = 0;
         double gv[3] = {0.0, 0.0, 0.0};
         if (DIAG) {
-            const double *gp = g.gb + 3 * (size_t)__ldg(g.obs_pt + a);
             int eg = -(1 << 20), nf = 0;
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
-                gv[j] = __ldg(gp + j);
+                gv[j] = __ldg(g.gb + 3 * (size_t)pt + j);
                 eg = max(eg, fx_exp(gv[j]));
                 nf |= fx_nonfinite(gv[j]);
             }
@@ -276,6 +282,7 @@ __device__ void fx6_unit(const FxArgs &g, const SchurUnit u, int2 *sy, int2 *sw)
         const int eyt = ey;
         cp_async_wait();
         __syncwarp();
+        if (more) exponents(ey, ew, pt);
         if (!bad) {
             // entry lane's W row, d bits down
             if (lane < n) {
@@ -326,10 +333,7 @@ __device__ void fx6_unit(const FxArgs &g, const SchurUnit u, int2 *sy, int2 *sw)
                 if (at[p] >= 0) acc[p] = fx_plain<CNP>(g, pa + t0, pb + t0, n, at[p] / CP, at[p] % CP, acc[p]);
         }
         __syncwarp();
-        if (t0 + FX_CHUNK < u.count) {
-            indices(t0 + FX_CHUNK);
-            fetch();
-        }
+        if (more) rows();
     }
     double *out = (DIAG ? g.diag_partial : g.off_partial) + (size_t)u.out * NV;
 #pragma unroll
@@ -338,7 +342,7 @@ __device__ void fx6_unit(const FxArgs &g, const SchurUnit u, int2 *sy, int2 *sw)
 }
 
 // The diagonal units' blocks first (more work per entry), then the pairs'.
-__global__ void __launch_bounds__(32 * F6_WARPS, 4) k_schur_fx6(FxArgs g, int n_diag, const SchurUnit *__restrict__ diag,
+__global__ void __launch_bounds__(32 * F6_WARPS, F6_CTAS) k_schur_fx6(FxArgs g, int n_diag, const SchurUnit *__restrict__ diag,
                                                              int n_off, const SchurUnit *__restrict__ off)
 {
     __shared__ __align__(16) int2 sy[F6_WARPS][FX_CHUNK * 18], sw[F6_WARPS][FX_CHUNK * 26];
