@@ -122,10 +122,11 @@ inline int unit_len(long long n, long long units, int most)
     return (int)(len < 32 ? 32 : len > most ? most : len);
 }
 inline int off_unit_len(int cnp, long long entries) { return unit_len(entries, cnp == 6 ? 8192 : 4096, cnp == 6 ? 256 : 512); }
+// observations of a camera-block unit, 11/16-parameter cameras
+inline int cam_unit_len(long long obs) { return unit_len(obs, 2048, 256); }
 inline int diag_unit_len(int cnp, long long obs) { return unit_len(obs, cnp == 6 ? 4096 : 2048, 256); }
 constexpr int SD_THREADS = 128, SD_PER = 8;     // 6-parameter cameras: one CTA per unit, 8 observations a thread
 constexpr int DIAG_SUPER = SD_THREADS * SD_PER;  // observations per diagonal unit, 6-parameter cameras
-constexpr int CAM_CHUNK = 512;   // observations per camera-reduction work unit (11/16-parameter cameras)
 constexpr int CAM_PER = 8, CAM_SUPER = 128 * CAM_PER;  // 6-parameter cameras: 8 observations a thread, 128 threads
 // eb/dpb kernel: warps of up to EB_PPW points (in pt_order), three lanes per
 // point times m = eb_lanes_per_point(views), EB_WARPS warps a block
@@ -323,6 +324,8 @@ inline size_t off_partial_slots(const DeviceProblem &d)
 // Schur complement in one or two launches
 void launch_limb_rows(const DeviceProblem &d, cudaStream_t s);
 void launch_schur_fx(const DeviceProblem &d, double *diag_partial, cudaStream_t s);
+// 11/16-parameter cameras: the camera units' sums A^T A and A^T e
+void launch_camera_fx(const DeviceProblem &d, cudaStream_t s);
 void launch_schur_diag(const DeviceProblem &d, cudaStream_t s);
 void launch_schur_reduce(const DeviceProblem &d, double mu, cudaStream_t s);
 // Back-substitution: eb, dpb and partial sums for |dp|^2 and dp.(mu dp + g).
@@ -336,7 +339,6 @@ void launch_sum_partials(const double *partial, int n, double *dst, cudaStream_t
 // cameras, the last block summing the points' partials in index order
 void launch_param_norm(const DeviceProblem &d, int nred, double *partial, double *dst_cams, double *dst_pts,
                        cudaStream_t s);
-void launch_finish_trial(const DeviceProblem &d, double mu, cudaStream_t s);
 void launch_max_uvdiag(const DeviceProblem &d, double *dst, cudaStream_t s);
 void launch_dot(const double *x, const double *y, long long n, double *partial, int nblocks,
                 double *dst, cudaStream_t s);
@@ -383,7 +385,7 @@ void launch_yblocks_v(const DeviceProblem &d, cudaStream_t s);
 void launch_schur_off_v(const DeviceProblem &d, cudaStream_t s);
 void launch_schur_diag_v(const DeviceProblem &d, cudaStream_t s);
 void launch_schur_reduce_v(const DeviceProblem &d, double mu, cudaStream_t s);
-void launch_eb_dpb_v(const DeviceProblem &d, double mu, int nblocks, cudaStream_t s);
+void launch_wt_dpa(const DeviceProblem &d, double *out, cudaStream_t s);  // W^T dpa, 3 per observation
 void launch_jmultiply_v(const DeviceProblem &d, const double *x, double *out, cudaStream_t s);
 void launch_residual_dist(const DeviceProblem &d, const double *tab, const double *pts, const double *dpb,
                           double *ex_out, double *partial, int nblocks, cudaStream_t s);

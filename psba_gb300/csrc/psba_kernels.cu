@@ -8,6 +8,7 @@
 //   22); U 36 per camera; g = [ga (6C) | gb (3P)].
 // Every reduction runs in a fixed order (no floating-point atomics), so a
 // solve is bit-for-bit repeatable.
+#include <algorithm>
 #include <mutex>
 
 #include "psba_internal.h"
@@ -1766,11 +1767,83 @@ __global__ void __launch_bounds__(256) k_eb_dpb(int np, int ncp, const int2 *__r
 // k_eb_dpb blocks: EB_WARPS warps of the schedule each, at least np / EB_PPB
 // (the variable-intrinsics version uses one thread per point, and its
 // surplus blocks write zero partials)
+// 11/16-parameter cameras: eb = gb - sum_j W_ij^T dpa_j from the
+// observations' sums, dpb = V^-1 eb and the trial's step scalars, a thread per point.
+__global__ void __launch_bounds__(256) k_eb_finish(int np, int ncp, const int *__restrict__ pt_start,
+                                                   const double *__restrict__ wd, const double *__restrict__ Vinv,
+                                                   const double *__restrict__ g, double mu, double *__restrict__ dp,
+                                                   double *__restrict__ eb, double *__restrict__ partial,
+                                                   const int *__restrict__ status, int *__restrict__ ticket,
+                                                   TrialScalars *__restrict__ out)
+{
+    __shared__ double r0[8], r1[8];
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    double s_sq = 0.0, s_rho = 0.0;
+    if (i < np) {
+        double e0 = 0.0, e1 = 0.0, e2 = 0.0;
+        const int end = pt_start[i + 1];
+#pragma unroll 4
+        for (int o = pt_start[i]; o < end; ++o) {
+            e0 += wd[3 * (size_t)o];
+            e1 += wd[3 * (size_t)o + 1];
+            e2 += wd[3 * (size_t)o + 2];
+        }
+        const double *gb = g + ncp + 3 * (size_t)i;
+        e0 = gb[0] - e0;
+        e1 = gb[1] - e1;
+        e2 = gb[2] - e2;
+        eb[3 * (size_t)i] = e0;
+        eb[3 * (size_t)i + 1] = e1;
+        eb[3 * (size_t)i + 2] = e2;
+        const double *vi = Vinv + 6 * (size_t)i;
+        const double d0 = vi[0] * e0 + vi[1] * e1 + vi[2] * e2;
+        const double d1 = vi[1] * e0 + vi[3] * e1 + vi[4] * e2;
+        const double d2 = vi[2] * e0 + vi[4] * e1 + vi[5] * e2;
+        double *db = dp + ncp + 3 * (size_t)i;
+        db[0] = d0;
+        db[1] = d1;
+        db[2] = d2;
+        s_sq = d0 * d0 + d1 * d1 + d2 * d2;
+        s_rho = d0 * (mu * d0 + gb[0]) + d1 * (mu * d1 + gb[1]) + d2 * (mu * d2 + gb[2]);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        s_sq += __shfl_xor_sync(0xffffffffu, s_sq, off);
+        s_rho += __shfl_xor_sync(0xffffffffu, s_rho, off);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        r0[threadIdx.x >> 5] = s_sq;
+        r1[threadIdx.x >> 5] = s_rho;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double a = r0[0], b = r1[0];
+#pragma unroll
+        for (int w = 1; w < 8; ++w) {
+            a += r0[w];
+            b += r1[w];
+        }
+        partial[2 * blockIdx.x] = a;
+        partial[2 * blockIdx.x + 1] = b;
+    }
+    if (take_last_ticket(ticket)) {
+        finish_trial_block(ncp, gridDim.x, dp, g, mu, partial, status, out);
+        if (threadIdx.x == 0) *ticket = 0;
+    }
+}
+
 int eb_blocks(const DeviceProblem &d) { return d.n_eb_warps / EB_WARPS; }
 
 void launch_eb_dpb(const DeviceProblem &d, double mu, cudaStream_t s)
 {
-    if (d.cnp != 6) return launch_eb_dpb_v(d, mu, eb_blocks(d), s);
+    if (d.cnp != 6) {
+        double *wd = d.Y;  // the trial's Y has been used: 3 sums per observation in its place
+        launch_wt_dpa(d, wd, s);
+        k_eb_finish<<<std::max(1, ceil_div(d.np, 256)), 256, 0, s>>>(d.np, d.N, d.pt_start, wd, d.Vinv, d.g, mu, d.dp,
+                                                                     d.eb, d.red_partial, d.status, d.tickets, d.scal);
+        note_launch(1);
+        return;
+    }
     // the camera part of dp in shared memory when it fits: each observation
     // reads its camera's six values
     const int stage = (size_t)d.N * sizeof(double) <= 48 * 1024 ? 1 : 0;
@@ -1785,24 +1858,6 @@ void launch_eb_dpb(const DeviceProblem &d, double mu, cudaStream_t s)
                                                           d.red_partial, stage, d.status, d.tickets, d.scal,
                                                           d.dpa2f, d.pts, d.wt ? nullptr : d.x2f);
     note_launch(1);
-}
-
-// Sum the dpa part and the per-block partials of the back-substitution in a
-// fixed order; copy the Cholesky status.  One block (11/16-parameter
-// cameras; for 6-parameter cameras k_eb_dpb's last block does this).
-__global__ void k_finish_trial(int ncp, int nblocks, const double *__restrict__ dp,
-                               const double *__restrict__ g, double mu,
-                               const double *__restrict__ partial, const int *__restrict__ status,
-                               TrialScalars *__restrict__ out)
-{
-    finish_trial_block(ncp, nblocks, dp, g, mu, partial, status, out);
-}
-
-void launch_finish_trial(const DeviceProblem &d, double mu, cudaStream_t s)
-{
-    if (d.cnp == 6) return;  // k_eb_dpb's last block did it
-    k_finish_trial<<<1, 256, 0, s>>>(d.N, eb_blocks(d), d.dp, d.g, mu, d.red_partial, d.status,
-                                     d.scal); note_launch(1);
 }
 
 // Fixed-order sum of n partials into *dst (one block).

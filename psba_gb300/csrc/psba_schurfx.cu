@@ -181,12 +181,12 @@ __device__ __forceinline__ void ld_limbs(const int2 *p, int2 *out)
     }
 }
 
-// A TR x TC tile of entry t's products
-template <int TR, int TC, int RP, int CP>
+// A TR x TC tile of entry t's products, summed over the NJ inner columns
+template <int TR, int TC, int RP, int CP, int NJ = 3>
 __device__ __forceinline__ void fx_tile(const int2 *y, const int2 *w, long long (&hh)[TR][TC], long long (&hl)[TR][TC])
 {
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
+    for (int j = 0; j < NJ; ++j) {
         int2 a[TR], b[TC];
         ld_limbs<TR>(y + j * RP, a);
         ld_limbs<TC>(w + j * CP, b);
@@ -491,6 +491,124 @@ __global__ void __launch_bounds__(FV_THREADS) k_schur_fxv(FxArgs g, const SchurU
         if (at[p] >= 0) out[tid + FV_THREADS * p] = acc[p];
 }
 
+// ---------------------------------------------------------------------------
+// U_j = sum A^T A (upper triangle) and ga_j = sum A^T e of a camera unit,
+// 11/16-parameter cameras: a Gram matrix of the observations' two rows of
+// [A | e], 32 observations at a time, each column cut relative to its largest
+// value among them (U_cc holds that value's square, so nothing that counts
+// against sqrt(U_rr U_cc) is lost), e as column CNP.  In FP64 the sums were two
+// multiply-adds per output and observation on the FP64 pipe.
+template <int CNP>
+__global__ void __launch_bounds__(FV_THREADS) k_camera_fx(const CamUnit *__restrict__ units,
+                                                          const int *__restrict__ cam_obs,
+                                                          const double *__restrict__ A, const double *__restrict__ ex,
+                                                          double *__restrict__ partial)
+{
+    constexpr int RP = fx_rows(CNP), TR = RP / 4, NC = CNP + 1, TC = (NC + 3) / 4, CP = 4 * TC, NW = FV_THREADS / 32;
+    constexpr int ST = 2 * CP + 2;  // words from observation to observation
+    constexpr int NU = CNP * (CNP + 1) / 2, NV = NU + CNP, PER = (NV + FV_THREADS - 1) / FV_THREADS;
+    __shared__ __align__(16) long long sa[FX_CHUNK * ST];
+    __shared__ long long st[NW][RP * CP];
+    __shared__ int s_E[CP];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const CamUnit u = units[blockIdx.x];
+    for (int e = tid; e < FX_CHUNK * ST; e += FV_THREADS) sa[e] = 0;  // the padding columns
+    double acc[PER];
+    int at[PER];
+#pragma unroll
+    for (int p = 0; p < PER; ++p) {
+        acc[p] = 0.0;
+        at[p] = -1;
+        const int v = tid + FV_THREADS * p;
+        if (v < NU) {  // row-major upper triangle
+            int r = 0, c = v;
+            while (c >= CNP - r) c -= CNP - r++;
+            at[p] = r * CP + r + c;
+        } else if (v < NV) {
+            at[p] = (v - NU) * CP + CNP;
+        }
+    }
+    for (int t0 = 0; t0 < u.count; t0 += FX_CHUNK) {
+        const int n = min(FX_CHUNK, u.count - t0);
+        __syncthreads();  // the last chunk's limbs are read
+        for (int e = tid; e < n * 2 * NC; e += FV_THREADS) {
+            const int t = e / (2 * NC), k = e % (2 * NC), i = k / NC, c = k % NC;
+            const size_t o = __ldg(cam_obs + u.begin + t0 + t);
+            sa[t * ST + i * CP + c] = __double_as_longlong(c < CNP ? __ldg(A + 2 * CNP * o + i * CNP + c) : __ldg(ex + 2 * o + i));
+        }
+        __syncthreads();
+        // a warp per column, a lane per observation
+        int bad = 0, E[TC];
+        double x[TC][2];
+#pragma unroll
+        for (int q = 0; q < TC; ++q) {
+            const int c = warp + NW * q;
+            int e = 1;
+            x[q][0] = x[q][1] = 0.0;
+            if (c < NC && lane < n) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    x[q][i] = __longlong_as_double(sa[lane * ST + i * CP + c]);
+                    e = max(e, fx_exp(x[q][i]));
+                    bad |= fx_nonfinite(x[q][i]);
+                }
+            }
+            E[q] = __reduce_max_sync(0xffffffffu, e);
+            if (lane == 0) s_E[c] = E[q];
+        }
+        if (__syncthreads_or(bad)) {  // an infinity or a NaN: plain FP64 sums
+#pragma unroll
+            for (int p = 0; p < PER; ++p)
+                if (at[p] >= 0)
+                    for (int t = 0; t < n; ++t)
+#pragma unroll
+                        for (int i = 0; i < 2; ++i)
+                            acc[p] = fma(__longlong_as_double(sa[t * ST + i * CP + at[p] / CP]),
+                                         __longlong_as_double(sa[t * ST + i * CP + at[p] % CP]), acc[p]);
+            continue;
+        }
+#pragma unroll
+        for (int q = 0; q < TC; ++q) {
+            const int c = warp + NW * q;
+            if (c < NC && lane < n)
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+                    *reinterpret_cast<int2 *>(sa + lane * ST + i * CP + c) = fx_limbs(x[q][i], E[q] - fx_exp(x[q][i]));
+        }
+        __syncthreads();
+        const int l = tid & 15, r0 = (l >> 2) * TR, c0 = (l & 3) * TC;
+        long long hh[TR][TC], hl[TR][TC];
+#pragma unroll
+        for (int i = 0; i < TR; ++i)
+#pragma unroll
+            for (int j = 0; j < TC; ++j) hh[i][j] = hl[i][j] = 0;
+        for (int t = tid >> 4; t < n; t += FV_THREADS / 16) {
+            const int2 *row = reinterpret_cast<const int2 *>(sa) + t * ST;
+            fx_tile<TR, TC, CP, CP, 2>(row + r0, row + c0, hh, hl);
+        }
+#pragma unroll
+        for (int i = 0; i < TR; ++i)
+#pragma unroll
+            for (int j = 0; j < TC; ++j) {
+                long long T = fx_total(hh[i][j], hl[i][j]);
+                T += __shfl_xor_sync(0xffffffffu, T, 16);
+                if (lane < 16) st[warp][(r0 + i) * CP + c0 + j] = T;
+            }
+        __syncthreads();
+#pragma unroll
+        for (int p = 0; p < PER; ++p) {
+            if (at[p] < 0) continue;
+            long long T = 0;
+#pragma unroll
+            for (int w = 0; w < NW; ++w) T += st[w][at[p]];
+            acc[p] = fx_add(acc[p], T, s_E[at[p] / CP] + s_E[at[p] % CP]);
+        }
+    }
+#pragma unroll
+    for (int p = 0; p < PER; ++p)
+        if (at[p] >= 0) partial[(size_t)blockIdx.x * NV + tid + FV_THREADS * p] = acc[p];
+}
+
 template <int CNP>
 void limb_rows_t(const DeviceProblem &d, cudaStream_t s)
 {
@@ -507,6 +625,14 @@ void launch_limb_rows(const DeviceProblem &d, cudaStream_t s)
     if (d.cnp == 6) limb_rows_t<6>(d, s);
     else if (d.cnp == 11) limb_rows_t<11>(d, s);
     else limb_rows_t<16>(d, s);
+    note_launch(1);
+}
+
+void launch_camera_fx(const DeviceProblem &d, cudaStream_t s)
+{
+    if (d.n_cam_units == 0) return;
+    if (d.cnp == 11) k_camera_fx<11><<<d.n_cam_units, FV_THREADS, 0, s>>>(d.cam_units, d.cam_obs, d.A, d.ex, d.cam_partial);
+    else k_camera_fx<16><<<d.n_cam_units, FV_THREADS, 0, s>>>(d.cam_units, d.cam_obs, d.A, d.ex, d.cam_partial);
     note_launch(1);
 }
 

@@ -369,7 +369,6 @@ void enqueue_step(psba_handle *h, double mu)
     {
         StageScope sc(h, ST_EBDPB);
         launch_eb_dpb(d, mu, h->stream);
-        launch_finish_trial(d, mu, h->stream);
     }
 }
 
@@ -986,7 +985,7 @@ int create_impl(const psba_problem_desc *p, psba_handle *h)
     std::vector<CamUnit> cam_units;
     std::vector<int> cam_unit_start(nc + 1, 0);
     for (int j = 0; j < nc; ++j) {
-        const int cchunk = d.cnp == 6 ? CAM_SUPER : CAM_CHUNK;
+        const int cchunk = d.cnp == 6 ? CAM_SUPER : cam_unit_len(no);
         for (int b = cam_start[j]; b < cam_start[j + 1]; b += cchunk)
             cam_units.push_back({j, b, std::min(cchunk, cam_start[j + 1] - b), 0});
         cam_unit_start[j + 1] = (int)cam_units.size();

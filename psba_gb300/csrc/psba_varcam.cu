@@ -29,10 +29,13 @@ namespace {
 inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 constexpr int VC_THREADS = 128;
+constexpr int LV_THREADS = 64;  // observations per CTA of the kernels that stage whole rows
 constexpr int VFLUSH = 8;
 
 template <int CNP> __host__ __device__ constexpr int cam_nv() { return CNP * (CNP + 1) / 2 + CNP; }  // U upper + ga
 template <int CNP> __host__ __device__ constexpr int diag_nv() { return CNP * (CNP + 1) / 2 + CNP; } // S lower + ea
+
+template <int CNP> __host__ __device__ constexpr int cam_threads() { return (cam_nv<CNP>() + 31) / 32 * 32; }
 
 // (r, c) of the v-th entry of the upper triangle, row-major
 __host__ __device__ inline void upper_rc(int v, int n, int &r, int &c)
@@ -59,20 +62,37 @@ __host__ __device__ inline void lower_rc(int v, int &r, int &c)
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// Linearization: one thread per observation.  Projection and residual in
-// FP64; derivatives evaluated in R from the FP64 quantities.
-template <typename R, int CNP>
-__global__ void __launch_bounds__(256) k_linearize_v(int no, const int *__restrict__ obs_pt,
-                                                     const int *__restrict__ obs_cam,
-                                                     const double *__restrict__ meas,
-                                                     const double *__restrict__ pts,
-                                                     const double *__restrict__ tab, double coeff,
-                                                     const double *__restrict__ wt,
-                                                     R *__restrict__ ex, R *__restrict__ A,
-                                                     R *__restrict__ B, R *__restrict__ W)
+// The rows a CTA's threads have formed, one row of L values each, into the
+// contiguous rows of `dst`: through shared memory, so that the stores are
+// coalesced (a thread's own row at a stride of L touches a sector per store).
+template <typename R, int L>
+__device__ __forceinline__ void put_rows(R *dst, const R *row, int n, R *buf)
 {
-    const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= no) return;
+    constexpr int LS = L | 1;  // odd stride: no bank conflicts
+    __syncthreads();           // the last rows are read
+#pragma unroll
+    for (int k = 0; k < L; ++k) buf[threadIdx.x * LS + k] = row[k];
+    __syncthreads();
+    for (int e = threadIdx.x; e < n * L; e += LV_THREADS) dst[e] = buf[(e / L) * LS + e % L];
+}
+
+// Linearization: one thread per observation, LV_THREADS consecutive ones a
+// CTA.  Projection and residual in FP64; derivatives evaluated in R from the
+// FP64 quantities; W = A^T (coeff B) (coeff is 1 or 2 in the drivers: the
+// same bits as coeff (A^T B)).
+template <typename R, int CNP>
+__global__ void __launch_bounds__(LV_THREADS) k_linearize_v(int no, const int *__restrict__ obs_pt,
+                                                            const int *__restrict__ obs_cam,
+                                                            const double *__restrict__ meas,
+                                                            const double *__restrict__ pts,
+                                                            const double *__restrict__ tab, double coeff,
+                                                            const double *__restrict__ wt,
+                                                            R *__restrict__ ex, R *__restrict__ A,
+                                                            R *__restrict__ B, R *__restrict__ W)
+{
+    __shared__ R buf[LV_THREADS * ((3 * CNP) | 1)];
+    const int o0 = blockIdx.x * LV_THREADS, n = min(LV_THREADS, no - o0);
+    const int o = o0 + min((int)threadIdx.x, n - 1);  // spare threads repeat the last one
     const int i = obs_pt[o], j = obs_cam[o];
     const CamTab *T = reinterpret_cast<const CamTab *>(tab + (size_t)CAMTAB * j);
     const double X0 = pts[3 * i], X1 = pts[3 * i + 1], X2 = pts[3 * i + 2];
@@ -109,8 +129,10 @@ __global__ void __launch_bounds__(256) k_linearize_v(int no, const int *__restri
         e1 = wc * e1;
         e0 = t0;
     }
-    ex[2 * (size_t)o] = (R)e0;
-    ex[2 * (size_t)o + 1] = (R)e1;
+    if (threadIdx.x < n) {
+        ex[2 * (size_t)o] = (R)e0;
+        ex[2 * (size_t)o + 1] = (R)e1;
+    }
     // H = d(u,v)/dXc = P Dd N
     const R fx = (R)T->fx, sk = (R)T->sk, fy = (R)T->fy, izr = (R)iz, xr = (R)x, yr = (R)y;
     const R pd00 = fx * (R)Dd00 + sk * (R)Dd10, pd01 = fx * (R)Dd01 + sk * (R)Dd11;
@@ -168,19 +190,17 @@ __global__ void __launch_bounds__(256) k_linearize_v(int no, const int *__restri
             b[1][c] = rc * b1;
         }
     }
-    R *Ao = A + 2 * CNP * (size_t)o, *Bo = B + 6 * (size_t)o, *Wo = W + 3 * CNP * (size_t)o;
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-#pragma unroll
-        for (int c = 0; c < CNP; ++c) Ao[r * CNP + c] = a[r][c];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) Bo[r * 3 + c] = b[r][c];
-    }
+    put_rows<R, 2 * CNP>(A + 2 * CNP * (size_t)o0, &a[0][0], n, buf);
+    put_rows<R, 6>(B + 6 * (size_t)o0, &b[0][0], n, buf);
     const R cf = (R)coeff;
+    R w[3 * CNP];
 #pragma unroll
-    for (int r = 0; r < CNP; ++r)
+    for (int c = 0; c < 3; ++c) {
+        const R b0 = cf * b[0][c], b1 = cf * b[1][c];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) Wo[r * 3 + c] = cf * (a[0][r] * b[0][c] + a[1][r] * b[1][c]);
+        for (int r = 0; r < CNP; ++r) w[3 * r + c] = a[0][r] * b0 + a[1][r] * b1;
+    }
+    put_rows<R, 3 * CNP>(W + 3 * CNP * (size_t)o0, w, n, buf);
 }
 
 // Cost of one observation with distortion (cnp 16); the 6- and 11-parameter
@@ -238,64 +258,51 @@ __global__ void __launch_bounds__(256) k_residual_dist(int no, const int *__rest
 }
 
 // ---------------------------------------------------------------------------
-// U_j (upper triangle) and ga_j per camera unit: the unit's A rows and
-// residuals are staged in shared memory 32 observations at a time; thread t
-// owns entries t, t + 128, ... and sums them over the unit in order.
-template <typename R, int CNP>
-__global__ void __launch_bounds__(VC_THREADS) k_camera_partial_v(const CamUnit *__restrict__ units,
-                                                                 const int *__restrict__ cam_obs,
-                                                                 const R *__restrict__ A,
-                                                                 const R *__restrict__ ex,
-                                                                 double *__restrict__ partial)
+// U_j (upper triangle) and ga_j per camera unit, the mixed form (the FP64
+// form's are k_camera_fx): the unit's A rows and residuals are staged in shared
+// memory 32 observations at a time; thread t owns output t and sums it over
+// the unit in order, FP32 sums of VFLUSH observations added in FP64.  The ga
+// outputs are FP64 chains, two additions an observation, so units are short.
+template <int CNP>
+__global__ void __launch_bounds__(cam_threads<CNP>()) k_camera_partial_v(const CamUnit *__restrict__ units,
+                                                                         const int *__restrict__ cam_obs,
+                                                                         const float *__restrict__ A,
+                                                                         const float *__restrict__ ex,
+                                                                         double *__restrict__ partial)
 {
-    constexpr int NV = cam_nv<CNP>(), NU = CNP * (CNP + 1) / 2, PER = (NV + VC_THREADS - 1) / VC_THREADS;
+    constexpr int NV = cam_nv<CNP>(), NU = CNP * (CNP + 1) / 2, T = cam_threads<CNP>();
     constexpr int CH = 32;
-    __shared__ R sa[CH][2 * CNP];
-    __shared__ R se[CH][2];
+    __shared__ float sa[CH][2 * CNP];
+    __shared__ float se[CH][2];
     const CamUnit u = units[blockIdx.x];
-    double acc[PER];
-    int er[PER], ec[PER];
-#pragma unroll
-    for (int q = 0; q < PER; ++q) {
-        acc[q] = 0.0;
-        const int v = threadIdx.x + q * VC_THREADS;
-        er[q] = ec[q] = -1;
-        if (v < NU) upper_rc(v, CNP, er[q], ec[q]);
-        else if (v < NV) er[q] = v - NU;  // gradient row
-    }
+    const int v = threadIdx.x;
+    double acc = 0.0;
+    int r = 0, c = 0;
+    if (v < NU) upper_rc(v, CNP, r, c);
+    else r = v - NU;  // gradient row
     for (int t0 = 0; t0 < u.count; t0 += CH) {
         const int n = min(CH, u.count - t0);
         __syncthreads();
-        for (int e = threadIdx.x; e < n * 2 * CNP; e += VC_THREADS) {
+        for (int e = threadIdx.x; e < n * 2 * CNP; e += T) {
             const int t = e / (2 * CNP), k = e % (2 * CNP);
             sa[t][k] = A[2 * CNP * (size_t)cam_obs[u.begin + t0 + t] + k];
         }
-        for (int e = threadIdx.x; e < n * 2; e += VC_THREADS)
+        for (int e = threadIdx.x; e < n * 2; e += T)
             se[e / 2][e % 2] = ex[2 * (size_t)cam_obs[u.begin + t0 + e / 2] + e % 2];
         __syncthreads();
-#pragma unroll
-        for (int q = 0; q < PER; ++q) {
-            const int v = threadIdx.x + q * VC_THREADS;
-            if (v >= NV) continue;
-            const int r = er[q], c = ec[q];
-            if (v < NU) {
-                for (int f0 = 0; f0 < n; f0 += VFLUSH) {
-                    R part = (R)0;
-                    const int f1 = min(n, f0 + VFLUSH);
-                    for (int t = f0; t < f1; ++t) part = part + sa[t][r] * sa[t][c] + sa[t][CNP + r] * sa[t][CNP + c];
-                    acc[q] += (double)part;
-                }
-            } else {
-                for (int t = 0; t < n; ++t)
-                    acc[q] = acc[q] + (double)sa[t][r] * (double)se[t][0] + (double)sa[t][CNP + r] * (double)se[t][1];
+        if (v < NU) {
+            for (int f0 = 0; f0 < n; f0 += VFLUSH) {
+                float part = 0.0f;
+                const int f1 = min(n, f0 + VFLUSH);
+                for (int t = f0; t < f1; ++t) part = part + sa[t][r] * sa[t][c] + sa[t][CNP + r] * sa[t][CNP + c];
+                acc += (double)part;
             }
+        } else if (v < NV) {
+            for (int t = 0; t < n; ++t)
+                acc = acc + (double)sa[t][r] * (double)se[t][0] + (double)sa[t][CNP + r] * (double)se[t][1];
         }
     }
-#pragma unroll
-    for (int q = 0; q < PER; ++q) {
-        const int v = threadIdx.x + q * VC_THREADS;
-        if (v < NV) partial[(size_t)blockIdx.x * NV + v] = acc[q];
-    }
+    if (v < NV) partial[(size_t)blockIdx.x * NV + v] = acc;
 }
 
 template <int CNP>
@@ -497,64 +504,37 @@ __global__ void k_schur_reduce_v(int n_pairs, int nc, int Np, const int *__restr
     S[(size_t)(CNP * k + r) * Np + CNP * k + c] = (r == c ? uu + mu : uu) - sum;
 }
 
-// eb = gb - sum_j W_ij^T dpa_j, dpb = V^-1 eb, gain-ratio partials (as k_eb_dpb).
+// W_ij^T dpa_j per observation (three FP64 sums), for k_eb_finish: a CTA's
+// LV_THREADS rows of W come into shared memory coalesced, two threads take a
+// row (even and odd camera parameters).  A thread per point walking its rows
+// at a stride of 264 (384) bytes took 260 us at 52 cameras and 377k
+// observations; this and the finish take 62.
 template <typename R, int CNP>
-__global__ void __launch_bounds__(256) k_eb_dpb_v(int np, int ncp, const int *__restrict__ pt_start,
-                                                  const int *__restrict__ pt_order,
-                                                  const int *__restrict__ obs_cam, const R *__restrict__ W,
-                                                  const double *__restrict__ Vinv, const double *__restrict__ g,
-                                                  double mu, double *__restrict__ dp, double *__restrict__ eb,
-                                                  double *__restrict__ partial)
+__global__ void __launch_bounds__(2 * LV_THREADS) k_wt_dpa(int no, const int *__restrict__ obs_cam,
+                                                           const R *__restrict__ W, const double *__restrict__ dpa,
+                                                           double *__restrict__ out)
 {
-    __shared__ double r0[256], r1[256];
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    double s_sq = 0.0, s_rho = 0.0;
-    if (t < np) {
-        const int i = pt_order[t];
-        double e0 = 0, e1 = 0, e2 = 0;
-        for (int o = pt_start[i]; o < pt_start[i + 1]; ++o) {
-            const R *w = W + 3 * CNP * (size_t)o;
-            const double *da = dp + CNP * (size_t)obs_cam[o];
-#pragma unroll 4
-            for (int k = 0; k < CNP; ++k) {
-                const double dk = da[k];
-                e0 = e0 + (double)w[3 * k] * dk;
-                e1 = e1 + (double)w[3 * k + 1] * dk;
-                e2 = e2 + (double)w[3 * k + 2] * dk;
-            }
-        }
-        const double *gb = g + ncp + 3 * (size_t)i;
-        e0 = gb[0] - e0;
-        e1 = gb[1] - e1;
-        e2 = gb[2] - e2;
-        eb[3 * (size_t)i] = e0;
-        eb[3 * (size_t)i + 1] = e1;
-        eb[3 * (size_t)i + 2] = e2;
-        const double *vi = Vinv + 6 * (size_t)i;
-        const double d0 = vi[0] * e0 + vi[1] * e1 + vi[2] * e2;
-        const double d1 = vi[1] * e0 + vi[3] * e1 + vi[4] * e2;
-        const double d2 = vi[2] * e0 + vi[4] * e1 + vi[5] * e2;
-        double *db = dp + ncp + 3 * (size_t)i;
-        db[0] = d0;
-        db[1] = d1;
-        db[2] = d2;
-        s_sq = d0 * d0 + d1 * d1 + d2 * d2;
-        s_rho = d0 * (mu * d0 + gb[0]) + d1 * (mu * d1 + gb[1]) + d2 * (mu * d2 + gb[2]);
-    }
-    r0[threadIdx.x] = s_sq;
-    r1[threadIdx.x] = s_rho;
+    constexpr int L = 3 * CNP, LS = L | 1;
+    __shared__ R sw[LV_THREADS * LS];
+    const int o0 = blockIdx.x * LV_THREADS, n = min(LV_THREADS, no - o0), t = threadIdx.x >> 1, h = threadIdx.x & 1;
+    for (int e = threadIdx.x; e < n * L; e += 2 * LV_THREADS) sw[(e / L) * LS + e % L] = __ldg(W + L * (size_t)o0 + e);
+    const double *da = dpa + CNP * (size_t)__ldg(obs_cam + o0 + min(t, n - 1));
+    double d[(CNP + 1) / 2];
+#pragma unroll
+    for (int k = 0; k < (CNP + 1) / 2; ++k) d[k] = 2 * k + h < CNP ? __ldg(da + 2 * k + h) : 0.0;
     __syncthreads();
-    for (int st = 128; st > 0; st >>= 1) {
-        if (threadIdx.x < st) {
-            r0[threadIdx.x] += r0[threadIdx.x + st];
-            r1[threadIdx.x] += r1[threadIdx.x + st];
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        partial[2 * blockIdx.x] = r0[0];
-        partial[2 * blockIdx.x + 1] = r1[0];
-    }
+    double s[3] = {0.0, 0.0, 0.0};
+    const R *w = sw + min(t, n - 1) * LS;
+#pragma unroll
+    for (int k = 0; k < (CNP + 1) / 2; ++k)
+        if (2 * k + h < CNP)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) s[c] = fma((double)w[3 * (2 * k + h) + c], d[k], s[c]);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) s[c] += __shfl_xor_sync(0xffffffffu, s[c], 1);
+    if (t < n && h == 0)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) out[3 * (size_t)(o0 + t) + c] = s[c];
 }
 
 template <typename R, int CNP>
@@ -583,7 +563,7 @@ namespace {
 template <typename R, int CNP>
 void linearize_t(const DeviceProblem &d, double coeff, cudaStream_t s)
 {
-    k_linearize_v<R, CNP><<<ceil_div(d.no, 256), 256, 0, s>>>(d.no, d.obs_pt, d.obs_cam, d.meas, d.pts, d.camtab,
+    k_linearize_v<R, CNP><<<ceil_div(d.no, LV_THREADS), LV_THREADS, 0, s>>>(d.no, d.obs_pt, d.obs_cam, d.meas, d.pts, d.camtab,
                                                               coeff, d.wt, (R *)d.ex, (R *)d.A, (R *)d.B, (R *)d.W);
 }
 
@@ -591,9 +571,13 @@ template <typename R, int CNP>
 void camera_t(const DeviceProblem &d, double coeff, cudaStream_t s)
 {
     if (d.n_cam_units > 0) {
-        k_camera_partial_v<R, CNP><<<d.n_cam_units, VC_THREADS, 0, s>>>(d.cam_units, d.cam_obs, (const R *)d.A,
-                                                                        (const R *)d.ex, d.cam_partial);
-        note_launch(1);
+        if constexpr (sizeof(R) == 8) {
+            launch_camera_fx(d, s);
+        } else {
+            k_camera_partial_v<CNP><<<d.n_cam_units, cam_threads<CNP>(), 0, s>>>(
+                d.cam_units, d.cam_obs, (const float *)d.A, (const float *)d.ex, d.cam_partial);
+            note_launch(1);
+        }
     }
     k_camera_finish_v<CNP><<<ceil_div((long long)d.nc * cam_nv<CNP>(), 128), 128, 0, s>>>(
         d.nc, d.cam_unit_start, d.cam_partial, coeff, d.U, d.g, d.uvdiag);
@@ -693,15 +677,17 @@ void launch_schur_reduce_v(const DeviceProblem &d, double mu, cudaStream_t s)
     else reduce_t<16>(d, mu, s);
 }
 
-void launch_eb_dpb_v(const DeviceProblem &d, double mu, int nblocks, cudaStream_t s)
+void launch_wt_dpa(const DeviceProblem &d, double *out, cudaStream_t s)
 {
+    if (d.no == 0) return;
     const bool f64 = d.prec == PSBA_PREC_FP64;
+    const int nb = ceil_div(d.no, LV_THREADS), nt = 2 * LV_THREADS;
     if (d.cnp == 11) {
-        if (f64) k_eb_dpb_v<double, 11><<<nblocks, 256, 0, s>>>(d.np, d.N, d.pt_start, d.pt_order, d.obs_cam, d.W, d.Vinv, d.g, mu, d.dp, d.eb, d.red_partial);
-        else k_eb_dpb_v<float, 11><<<nblocks, 256, 0, s>>>(d.np, d.N, d.pt_start, d.pt_order, d.obs_cam, (const float *)d.W, d.Vinv, d.g, mu, d.dp, d.eb, d.red_partial);
+        if (f64) k_wt_dpa<double, 11><<<nb, nt, 0, s>>>(d.no, d.obs_cam, d.W, d.dp, out);
+        else k_wt_dpa<float, 11><<<nb, nt, 0, s>>>(d.no, d.obs_cam, (const float *)d.W, d.dp, out);
     } else {
-        if (f64) k_eb_dpb_v<double, 16><<<nblocks, 256, 0, s>>>(d.np, d.N, d.pt_start, d.pt_order, d.obs_cam, d.W, d.Vinv, d.g, mu, d.dp, d.eb, d.red_partial);
-        else k_eb_dpb_v<float, 16><<<nblocks, 256, 0, s>>>(d.np, d.N, d.pt_start, d.pt_order, d.obs_cam, (const float *)d.W, d.Vinv, d.g, mu, d.dp, d.eb, d.red_partial);
+        if (f64) k_wt_dpa<double, 16><<<nb, nt, 0, s>>>(d.no, d.obs_cam, d.W, d.dp, out);
+        else k_wt_dpa<float, 16><<<nb, nt, 0, s>>>(d.no, d.obs_cam, (const float *)d.W, d.dp, out);
     }
     note_launch(1);
 }
