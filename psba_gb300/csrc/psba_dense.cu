@@ -1418,84 +1418,114 @@ void launch_refine(const DeviceProblem &d, const double *Sc, int ld, const doubl
 // and every entry below is <= beta; otherwise their columns are redone one
 // at a time with d = max(|c|, delta) and the theta/beta bound.
 //
-// One cooperative launch over CM_CTAS CTAs (grid-wide barriers), right-
-// looking: step j factors the 3x3 diagonal block of the already updated
-// matrix (every CTA redundantly, the same arithmetic), writes the panel
-// below it (a 3x3 block per thread) and, after a grid barrier that also
-// combines the "entry above beta" flags, updates the trailing lower triangle
-// with the rank-3 product of the panel (rows dealt to CTAs, columns to
-// threads).  Each entry thus takes the same sequence of 3-term subtractions,
-// in the same block order, as the reference's left-looking sums, so the plain
-// path rounds as before; the column-at-a-time path subtracts the earlier
-// blocks in those 3-term groups and the block's own columns one at a time.
-// The work per step is spread over the GPU instead of one block of threads
-// (at N = 528: ~33 ms on one CTA, where a step had at most 175 threads busy).
+// One cooperative launch, right-looking, one grid barrier per block step.  Row i
+// belongs to CTA i mod G, which keeps its rows in shared memory from the first
+// step to the last (where they do not fit, in S itself).  Per step every CTA
+// reads the step's three columns (n x 3, published by the rows' owners) and
+// forms the whole panel in shared memory, with the 3x3 factor, the test against
+// beta and, where it fails, the column-at-a-time path, so nothing of the
+// step's decisions goes between CTAs; it then updates its own rows with the
+// rank-3 product and publishes their next three columns.  Each entry takes
+// the same sequence of 3-term subtractions, in the same block order, as the
+// reference's left-looking sums; the column-at-a-time path subtracts the
+// earlier blocks in those 3-term groups and the block's own columns one at a
+// time.
+//
+// Bound by a step's chain: the columns' L2 round trip, the 3x3 factor's
+// divisions and roots (a warp issues an FP64 instruction per 64 cycles, so
+// they are dealt to lanes, five rounds deep), the panel and the barrier.  At
+// N = 528: 33 ms on one CTA; 4.65 ms with four barriers a step, a one-thread 3x3
+// factor and the flags of all CTAs read by every thread; 1.83 ms with one
+// barrier and the rows in S (each thread's updates waited for one another's
+// loads); 1.35 ms with the rows resident.
 constexpr int CM_THREADS = 256;
 
 __device__ double cta_max(double v, double *red)
 {
     for (int off = 16; off > 0; off >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, off));
+    __syncthreads();  // the last result is read
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
     __syncthreads();
     double r = red[0];
     for (int w = 1; w < CM_THREADS / 32; ++w) r = fmax(r, red[w]);
-    __syncthreads();
     return r;
 }
 
-__device__ int cta_or(int v, int *red)
+// The 3x3 factor of the block t (row-major, lower read) and its inverse by one
+// warp: L 00 10 11 20 21 22 and Li row-major; false if a pivot is not
+// positive and finite or an entry not finite (cholmod_blk.cl:135-191).
+__device__ bool cm_block(const double *t, double *L, double *Li, int lane)
 {
-    v = __any_sync(0xffffffffu, v) ? 1 : 0;
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    int r = 0;
-    for (int w = 0; w < CM_THREADS / 32; ++w) r |= red[w];
-    __syncthreads();
-    return r;
+    const double t0 = t[0], t3 = t[3], t4 = t[4], t6 = t[6], t7 = t[7], t8 = t[8];
+    auto from = [](double v, int src) { return __shfl_sync(0xffffffffu, v, src); };
+    // round 1
+    const double q1 = (lane == 0 ? t3 * t3 : t3 * t6) / t0;
+    const double p1 = t4 - from(q1, 0), cross = t7 - from(q1, 1);
+    const double a1 = -t8 * t3 * t3, a2 = 2 * t7 * t3 * t6, a3 = -t4 * t6 * t6;
+    const double a4 = t0 * (t4 * t8 - t7 * t7), a5 = -t3 * t3 + t0 * t4;
+    // round 2
+    const double q2 = (lane == 0 ? a1 + a2 + a3 + a4 : t0) / a5;
+    const double p2 = from(q2, 0), w4 = from(q2, 1);
+    // round 3
+    const double root = sqrt(lane == 0 ? t0 : lane == 1 ? p1 : lane == 2 ? p2 : w4);
+    const double l0 = from(root, 0), l2 = from(root, 1), l5 = from(root, 2), l4 = from(root, 3) * cross;
+    // round 4
+    const double q4 = (lane == 0 ? t3 : lane == 1 ? t6 : 1.0) / (lane <= 2 ? l0 : lane == 3 ? l2 : l5);
+    const double l1 = from(q4, 0), l3 = from(q4, 1);
+    // round 5
+    const double q5 = (lane == 0 ? -l1 : lane == 1 ? l1 * l4 - l2 * l3 : -l4) /
+                      (lane == 0 ? l0 * l2 : lane == 1 ? l0 * l2 * l5 : l2 * l5);
+    const double i0 = from(q4, 2), i4 = from(q4, 3), i8 = from(q4, 4), i3 = from(q5, 0), i6 = from(q5, 1), i7 = from(q5, 2);
+    if (lane == 0) {
+        L[0] = l0; L[1] = l1; L[2] = l2; L[3] = l3; L[4] = l4; L[5] = l5;
+        Li[0] = i0; Li[1] = 0; Li[2] = 0;
+        Li[3] = i3; Li[4] = i4; Li[5] = 0;
+        Li[6] = i6; Li[7] = i7; Li[8] = i8;
+    }
+    return isfinite(t0) && t0 > 0 && isfinite(p1) && p1 > 0 && isfinite(p2) && p2 > 0 && isfinite(l1) && isfinite(l3) &&
+           isfinite(l4);
 }
 
-// work: diag (n), orig (3 n), C (n), then gmax[2 G] and gflag[G] (doubles)
-__global__ void __launch_bounds__(CM_THREADS) k_cholmod(double *S, int n, int ld, double *E, double *work)
+// work: diag (n), then gmax[2 G], then the published columns, twice 3 n.
+// resident: the CTA's rows in shared memory (rows x n doubles after the panel's
+// 3 n), else in S; panel_stride > 0: the panel does not fit either and is a
+// slice of `panel` per CTA.
+__global__ void __launch_bounds__(CM_THREADS) k_cholmod(double *S, int n, int ld, double *E, double *work, int resident,
+                                                        double *panel, size_t panel_stride)
 {
     cg::grid_group grid = cg::this_grid();
+    extern __shared__ double cm_sm[];
     __shared__ double dred[CM_THREADS / 32];
-    __shared__ int ired[CM_THREADS / 32];
-    __shared__ double sh_L[6], sh_Li[9], sh_lxx;
-    __shared__ int sh_fail;
-    const int G = gridDim.x, b = blockIdx.x, tid = threadIdx.x;
-    const long long gtid = (long long)b * CM_THREADS + tid, gsize = (long long)G * CM_THREADS;
-    double *diag = work, *orig = work + n, *C = work + 4 * n, *gmax = work + 5 * n, *gflag = gmax + 2 * G;
-    // a grid-wide OR / max through per-CTA slots (after a grid barrier every
-    // CTA reads them all, in the same order)
-    auto grid_or = [&](int v) {
-        v = cta_or(v, ired);
-        if (tid == 0) gflag[b] = v ? 1.0 : 0.0;
-        grid.sync();
-        int r = 0;
-        for (int q = 0; q < G; ++q) r |= gflag[q] != 0.0;
-        grid.sync();  // the slots are reused
-        return r;
-    };
-    auto grid_max = [&](double v, int slot) {
-        v = cta_max(v, dred);
-        if (tid == 0) gmax[2 * b + slot] = v;
-        grid.sync();
-        double r = 0.0;
-        for (int q = 0; q < G; ++q) r = fmax(r, gmax[2 * q + slot]);
-        return r;
-    };
+    __shared__ double sh_t[9], sh_L[6], sh_Li[9], sh_lxx;
+    __shared__ int sh_ok;
+    const int G = gridDim.x, b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    double *P = panel_stride ? panel + (size_t)b * panel_stride : cm_sm;  // row r of the step's panel at 3 r
+    double *diag = work, *gmax = work + n, *cols = gmax + 2 * G;
+    // this CTA's rows b, b + G, ...: row b + q G at R + q pitch
+    double *R = resident ? cm_sm + 3 * (size_t)n : S + (size_t)b * ld;
+    const size_t pitch = resident ? (size_t)n : (size_t)G * ld;
+    const int n_rows = b < n ? (n - b + G - 1) / G : 0;
     // xi = max |offdiag|, gamma = max |diag| over the symmetric matrix (lower read)
     double xi = 0.0, gam = 0.0;
-    for (long long e = gtid; e < (long long)n * n; e += gsize) {
-        const int r = (int)(e / n), k = (int)(e % n);
-        if (r == k) {
-            gam = fmax(gam, fabs(S[(size_t)r * ld + r]));
-        } else {
-            const int hi = r > k ? r : k, lo = r > k ? k : r;
-            xi = fmax(xi, fabs(S[(size_t)hi * ld + lo]));
+    for (int q = 0; q < n_rows; ++q) {
+        const int r = b + q * G;
+        for (int k = tid; k < n; k += CM_THREADS) {
+            double *s = S + (size_t)r * ld + k;
+            if (k > r) {
+                *s = 0.0;
+                continue;
+            }
+            const double v = *s;
+            if (resident) R[q * pitch + k] = v;
+            if (k < 3) __stcg(cols + 3 * (size_t)r + k, v);
+            if (k == r) {
+                gam = fmax(gam, fabs(v));
+                diag[r] = v;
+            } else {
+                xi = fmax(xi, fabs(v));
+            }
         }
     }
-    for (long long r = gtid; r < n; r += gsize) diag[r] = S[(size_t)r * ld + r];
     xi = cta_max(xi, dred);
     gam = cta_max(gam, dred);
     if (tid == 0) {
@@ -1505,148 +1535,135 @@ __global__ void __launch_bounds__(CM_THREADS) k_cholmod(double *S, int n, int ld
     grid.sync();
     xi = 0.0;
     gam = 0.0;
-    for (int q = 0; q < G; ++q) {
-        xi = fmax(xi, gmax[2 * q]);
-        gam = fmax(gam, gmax[2 * q + 1]);
+    for (int q = tid; q < G; q += CM_THREADS) {
+        xi = fmax(xi, __ldcg(gmax + 2 * q));
+        gam = fmax(gam, __ldcg(gmax + 2 * q + 1));
     }
-    grid.sync();
+    xi = cta_max(xi, dred);
+    gam = cta_max(gam, dred);
     const double delta = 1e-15 * fmax(xi + gam, 1.0);
     double beta = fmax(gam, 1e-15);
-    beta = fmax(beta, xi / sqrt((double)(n * n - 1)));
+    beta = fmax(beta, xi / sqrt((double)n * (double)n - 1.0));
     beta = sqrt(beta);
     const int nb = n / 3;
     for (int j = 0; j < nb; ++j) {
-        const int j3 = 3 * j;
-        // the diagonal block, already updated by the earlier steps
-        if (tid == 0) {
-            double Tm[9];
-            for (int q = 0; q < 9; ++q) {
-                const int u = q / 3, v = q % 3;
-                Tm[q] = v > u ? S[(size_t)(j3 + v) * ld + j3 + u] : S[(size_t)(j3 + u) * ld + j3 + v];
+        const int j3 = 3 * j, t0 = j3 + 3;
+        const double *in = cols + 3 * (size_t)n * (j & 1);
+        double *out = cols + 3 * (size_t)n * ((j + 1) & 1);
+        // the step's columns, updated by the earlier steps: the 3x3 block for
+        // warp 0, all of them into the panel
+        if (warp == 0) {
+            if (lane < 9) {
+                const int u = lane / 3, v = lane % 3;
+                sh_t[lane] = __ldcg(in + 3 * (size_t)(j3 + max(u, v)) + min(u, v));
             }
-            int fail = 0;
-            const double p0 = Tm[0];
-            const double p1 = Tm[4] - Tm[3] * Tm[3] / Tm[0];
-            const double t1 = -Tm[8] * Tm[3] * Tm[3], t2 = 2 * Tm[7] * Tm[3] * Tm[6],
-                         t3 = -Tm[4] * Tm[6] * Tm[6];
-            const double t4 = Tm[0] * (Tm[4] * Tm[8] - Tm[7] * Tm[7]),
-                         t5 = -Tm[3] * Tm[3] + Tm[0] * Tm[4];
-            const double p2 = (t1 + t2 + t3 + t4) / t5;
-            if (!isfinite(p0) || p0 <= 0 || !isfinite(p1) || p1 <= 0 || !isfinite(p2) || p2 <= 0) fail = 1;
-            if (!fail) {
-                double *L = sh_L;
-                L[0] = sqrt(p0);
-                L[1] = Tm[3] / sqrt(Tm[0]);
-                L[2] = sqrt(p1);
-                L[3] = Tm[6] / sqrt(Tm[0]);
-                L[4] = sqrt(Tm[0] / (Tm[0] * Tm[4] - Tm[3] * Tm[3])) * (Tm[7] - Tm[3] * Tm[6] / Tm[0]);
-                L[5] = sqrt(p2);
-                if (!isfinite(L[1]) || !isfinite(L[3]) || !isfinite(L[4])) fail = 1;
-                double *Li = sh_Li;
-                Li[0] = 1 / L[0]; Li[1] = 0; Li[2] = 0;
-                Li[3] = -L[1] / (L[0] * L[2]); Li[4] = 1 / L[2]; Li[5] = 0;
-                Li[6] = (L[1] * L[4] - L[2] * L[3]) / (L[0] * L[2] * L[5]);
-                Li[7] = -L[4] / (L[2] * L[5]); Li[8] = 1 / L[5];
-            }
-            sh_fail = fail;
+            __syncwarp();
+            const bool ok = cm_block(sh_t, sh_L, sh_Li, lane);
+            if (lane == 0) sh_ok = ok;
+        } else {
+            for (int e = 3 * t0 + tid - 32; e < 3 * n; e += CM_THREADS - 32) P[e] = __ldcg(in + e);
         }
         __syncthreads();
-        const int fail = sh_fail;  // the same in every CTA
-        // keep the column block (rows j3 .. n-1) for the column-at-a-time path
-        for (long long e = gtid; e < (long long)(n - j3) * 3; e += gsize) {
-            const int r = j3 + (int)(e / 3), v = (int)(e % 3);
-            orig[(size_t)r * 3 + v] = S[(size_t)r * ld + j3 + v];
+        int big = sh_ok ? 0 : 1;
+        if (!big) {
+            // L_ij = T_ij Li^T, tested before it is kept
+            const double i0 = sh_Li[0], i3 = sh_Li[3], i4 = sh_Li[4], i6 = sh_Li[6], i7 = sh_Li[7], i8 = sh_Li[8];
+            for (int r = t0 + tid; r < n; r += CM_THREADS) {
+                const double x0 = P[3 * (size_t)r], x1 = P[3 * (size_t)r + 1], x2 = P[3 * (size_t)r + 2];
+                if (x0 * i0 > beta || x0 * i3 + x1 * i4 > beta || x0 * i6 + x1 * i7 + x2 * i8 > beta) big = 1;
+            }
+            big = __syncthreads_or(big);
+            if (!big) {
+                for (int r = t0 + tid; r < n; r += CM_THREADS) {
+                    const double x0 = P[3 * (size_t)r], x1 = P[3 * (size_t)r + 1], x2 = P[3 * (size_t)r + 2];
+                    P[3 * (size_t)r] = x0 * i0;
+                    P[3 * (size_t)r + 1] = x0 * i3 + x1 * i4;
+                    P[3 * (size_t)r + 2] = x0 * i6 + x1 * i7 + x2 * i8;
+                }
+                if (tid == 0) {
+                    double *d = P + 3 * (size_t)j3;
+                    d[0] = sh_L[0]; d[1] = 0; d[2] = 0;
+                    d[3] = sh_L[1]; d[4] = sh_L[2]; d[5] = 0;
+                    d[6] = sh_L[3]; d[7] = sh_L[4]; d[8] = sh_L[5];
+                }
+            }
         }
-        grid.sync();
-        int redo = fail;
-        if (!fail) {
-            // the diagonal block, then the blocks below: L_ij = T_ij Li^T
-            if (gtid == 0) {
-                double *dd = S + (size_t)j3 * ld + j3;
-                dd[0] = sh_L[0]; dd[1] = 0; dd[2] = 0;
-                dd[ld] = sh_L[1]; dd[ld + 1] = sh_L[2]; dd[ld + 2] = 0;
-                dd[2 * ld] = sh_L[3]; dd[2 * ld + 1] = sh_L[4]; dd[2 * ld + 2] = sh_L[5];
-            }
-            int big = 0;
-            for (long long blk = j + 1 + gtid; blk < nb; blk += gsize) {
-                double Tij[9];
-                for (int q = 0; q < 9; ++q) Tij[q] = S[(size_t)(3 * blk + q / 3) * ld + j3 + q % 3];
-                for (int u = 0; u < 3; ++u)
-                    for (int v = 0; v < 3; ++v) {
-                        const double val = (Tij[u * 3] * sh_Li[v * 3] + Tij[u * 3 + 1] * sh_Li[v * 3 + 1] +
-                                            Tij[u * 3 + 2] * sh_Li[v * 3 + 2]);
-                        S[(size_t)(3 * blk + u) * ld + j3 + v] = val;
-                        S[(size_t)(j3 + v) * ld + 3 * blk + u] = 0.0;
-                        if (val > beta) big = 1;
-                    }
-            }
-            redo = grid_or(big);
-        }
-        if (redo) {
-            // restore the column block and redo its columns one at a time
-            for (long long e = gtid; e < (long long)(n - j3) * 3; e += gsize) {
-                const int r = j3 + (int)(e / 3), v = (int)(e % 3);
-                S[(size_t)r * ld + j3 + v] = orig[(size_t)r * 3 + v];
-            }
-            grid.sync();
+        if (big) {
+            // the block's columns one at a time, from the values read above
+            if (tid < 9) P[3 * (size_t)j3 + tid] = tid / 3 >= tid % 3 ? sh_t[tid] : 0.0;
+            __syncthreads();
             for (int col = 0; col < 3; ++col) {
                 const int x = j3 + col;
-                if (tid == 0) {  // every CTA, the same arithmetic
-                    double sum = S[(size_t)x * ld + x];
-                    for (int k = j3; k < x; ++k) {
-                        const double l = S[(size_t)x * ld + k];
-                        sum -= l * l;
-                    }
-                    sum = fabs(sum);
-                    sh_lxx = sqrt(fmax(sum, delta));
+                const double *px = P + 3 * (size_t)x;
+                if (tid == 0) {
+                    double sum = px[col];
+                    for (int k = 0; k < col; ++k) sum -= px[k] * px[k];
+                    sh_lxx = sqrt(fmax(fabs(sum), delta));
                 }
                 __syncthreads();
-                const double lxx = sh_lxx;
-                int big = 0;
-                for (long long i = x + 1 + gtid; i < n; i += gsize) {
-                    double c = S[(size_t)i * ld + x];
-                    for (int k = j3; k < x; ++k) c = c - (S[(size_t)i * ld + k] * S[(size_t)x * ld + k]);
-                    C[i] = c;
-                    const double l = c / lxx;
-                    S[(size_t)i * ld + x] = l;
-                    S[(size_t)x * ld + i] = 0.0;
-                    if (l > beta) big = 1;
+                double lxx = sh_lxx, th = 0.0;
+                int over = 0;
+                for (int r = x + 1 + tid; r < n; r += CM_THREADS) {
+                    double *pr = P + 3 * (size_t)r;
+                    double c = pr[col];
+                    for (int k = 0; k < col; ++k) c = c - (pr[k] * px[k]);
+                    pr[col] = c;
+                    th = fmax(th, fabs(c));
+                    if (c / lxx > beta) over = 1;
                 }
-                big = grid_or(big);  // also orders the column's writes before the next column
-                if (gtid == 0) S[(size_t)x * ld + x] = lxx;
-                if (big) {
-                    double th = 0.0;
-                    for (long long i = x + 1 + gtid; i < n; i += gsize) th = fmax(th, fabs(C[i]));
-                    th = grid_max(th, 0);
-                    const double nl = th / beta;
-                    if (gtid == 0) S[(size_t)x * ld + x] = nl;
-                    for (long long i = x + 1 + gtid; i < n; i += gsize) S[(size_t)i * ld + x] = C[i] / nl;
-                }
-                grid.sync();
+                if (__syncthreads_or(over)) lxx = cta_max(th, dred) / beta;
+                for (int r = x + 1 + tid; r < n; r += CM_THREADS) P[3 * (size_t)r + col] /= lxx;
+                if (tid == 0) P[3 * (size_t)x + col] = lxx;
+                __syncthreads();
             }
         }
-        // the trailing lower triangle: S_ic -= L_i,j3.. L_c,j3.. (rank 3),
-        // rows i dealt to CTAs, columns c to threads
-        const int t0 = j3 + 3;
-        for (int i = t0 + b; i < n; i += G) {
-            const double *Li_ = S + (size_t)i * ld + j3;
-            const double a0 = Li_[0], a1 = Li_[1], a2 = Li_[2];
+        __syncthreads();
+        // this CTA's rows from j3 on: their L (into S, and their copy), then
+        // the rank-3 update S_ic -= L_i,j3.. L_c,j3.., c <= i, a warp per row
+        // and pass of 32 columns; the next step's columns go out first
+        const int q0 = j3 > b ? (j3 - b + G - 1) / G : 0;
+        for (int e = tid; e < 3 * (n_rows - q0); e += CM_THREADS) {
+            const int q = q0 + e / 3, c = e % 3, r = b + q * G;
+            if (r - j3 < c) continue;
+            const double v = P[3 * (size_t)r + c];
+            S[(size_t)r * ld + j3 + c] = v;
+            if (resident) R[q * pitch + j3 + c] = v;
+        }
+        for (int q = q0; q < n_rows; ++q) {
+            const int i = b + q * G;
+            if (i < t0) continue;
+            const double a0 = P[3 * (size_t)i], a1 = P[3 * (size_t)i + 1], a2 = P[3 * (size_t)i + 2];
+            double *row = R + q * pitch;
             for (int c = t0 + tid; c <= i; c += CM_THREADS) {
-                const double *Lc = S + (size_t)c * ld + j3;
-                S[(size_t)i * ld + c] -= (a0 * Lc[0] + a1 * Lc[1] + a2 * Lc[2]);
+                const double v = row[c] - (a0 * P[3 * (size_t)c] + a1 * P[3 * (size_t)c + 1] + a2 * P[3 * (size_t)c + 2]);
+                row[c] = v;
+                if (c < t0 + 3) __stcg(out + 3 * (size_t)i + (c - t0), v);
             }
         }
         grid.sync();
     }
-    for (long long i = gtid; i < n; i += gsize) {
+    // E_i = sum_k L_ik^2 - A_ii, a warp per row
+    for (int q = warp; q < n_rows; q += CM_THREADS / 32) {
+        const int i = b + q * G;
         double sum = 0.0;
-        for (int k = 0; k <= i; ++k) sum += S[(size_t)i * ld + k] * S[(size_t)i * ld + k];
-        E[i] = sum - diag[i];
+        for (int k = lane; k <= i; k += 32) {
+            const double v = R[q * pitch + k];
+            sum = fma(v, v, sum);
+        }
+        for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+        if (lane == 0) E[i] = sum - diag[i];
     }
 }
 
+// Dynamic shared memory at most (the rest of a CTA's 227 KB holds the static part)
+constexpr size_t CM_SMEM = 218 * 1024;
+
 // doubles of work the modified Cholesky needs at size n
-size_t cholmod_work(int n) { return 5 * (size_t)n + 3 * (size_t)CM_MAX_CTAS + 8; }
+size_t cholmod_work(int n)
+{
+    const size_t panel = 3 * (size_t)n * sizeof(double) > CM_SMEM ? 3 * (size_t)n * CM_MAX_CTAS : 0;
+    return 7 * (size_t)n + 2 * (size_t)CM_MAX_CTAS + 8 + panel;
+}
 
 void launch_cholmod(double *S, int n, int ld, double *E, double *work, cudaStream_t s, int grid_cap)
 {
@@ -1658,8 +1675,22 @@ void launch_cholmod(double *S, int n, int ld, double *E, double *work, cudaStrea
     const int rows = (n + 7) / 8;  // no more CTAs than the trailing rows can use
     if (rows < G) G = rows;
     if (G < 1) G = 1;
-    void *args[] = {&S, &n, &ld, &E, &work};
-    cudaLaunchCooperativeKernel((const void *)k_cholmod, dim3(G), dim3(CM_THREADS), args, 0, s);
+    // the panel (24 bytes a row) and the CTA's rows: resident up to n of about
+    // 1,700 on 152 CTAs, the panel alone up to 9,300
+    size_t smem = 3 * (size_t)n * sizeof(double), stride = 0;
+    const size_t all = smem + (size_t)((n + G - 1) / G) * n * sizeof(double);
+    int resident = all <= CM_SMEM;
+    if (resident) {
+        smem = all;
+    } else if (smem > CM_SMEM) {
+        smem = 0;
+        stride = 3 * (size_t)n;
+    }
+    if (smem > 40 * 1024)  // above the default limit (an attribute of the kernel on this device; the same value always)
+        cudaFuncSetAttribute(k_cholmod, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CM_SMEM);
+    double *panel = work + 7 * (size_t)n + 2 * CM_MAX_CTAS + 8;
+    void *args[] = {&S, &n, &ld, &E, &work, &resident, &panel, &stride};
+    cudaLaunchCooperativeKernel((const void *)k_cholmod, dim3(G), dim3(CM_THREADS), args, smem, s);
     note_launch(1);
 }
 
