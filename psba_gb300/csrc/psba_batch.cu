@@ -23,10 +23,12 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
 #include "psba_batch_internal.h"
+#include "psba_fixed_schur.h"
 
 namespace psba {
 namespace batch {
@@ -308,146 +310,280 @@ __device__ void vinv3(const double *Vi, double mu, double *out)
     out[5] = -(-a12 * a12 + a11 * a22) / T;
 }
 
-template <typename R>
-__device__ void stage_vinv_y(const BatchProblem &p, const Arenas<R> &ar, double mu)
+// FP64 form: V^-1, and Y = W V^-1 and W as limb rows (psba_fixed.h).  W's take the
+// place of the Jacobian rows (12 + 6 doubles per observation) and the rows'
+// exponents that of the residuals: both have been summed, and the next
+// linearization writes them afresh.
+__device__ FxArgs fx_args(const BatchProblem &p, const Arenas<double> &ar)
+{
+    return FxArgs{ar.i + p.i_pair_a,
+                  ar.i + p.i_pair_b,
+                  ar.i + p.i_cam_obs,
+                  ar.i + p.i_obs_pt,
+                  reinterpret_cast<const int2 *>(ar.r + p.r_Y),
+                  reinterpret_cast<const int2 *>(ar.r + p.r_A),
+                  reinterpret_cast<const int2 *>(ar.r + p.r_ex),
+                  ar.r + p.r_W,
+                  ar.d + p.d_Vinv,
+                  ar.d + p.d_U,
+                  ar.d + p.d_g + p.N,
+                  ar.i + p.i_pair_kl,
+                  nullptr,
+                  nullptr};
+}
+
+__device__ void stage_vinv_y(const BatchProblem &p, const Arenas<double> &ar, double mu)
 {
     const double *V = ar.d + p.d_V;
     double *Vi = ar.d + p.d_Vinv;
     for (int i = threadIdx.x; i < p.np; i += blockDim.x) vinv3(V + 6 * (size_t)i, mu, Vi + 6 * (size_t)i);
     __syncthreads();
-    const int *opt = ar.i + p.i_obs_pt;
-    const R *W = ar.r + p.r_W;
-    R *Y = ar.r + p.r_Y;
+    const int *opt = ar.i + p.i_obs_pt, *ocam = ar.i + p.i_obs_cam;
+    const double *W = ar.r + p.r_W, *U = ar.d + p.d_U;
+    int4 *Yq = reinterpret_cast<int4 *>(ar.r + p.r_Y), *Wq = reinterpret_cast<int4 *>(ar.r + p.r_A);
+    int2 *ex = reinterpret_cast<int2 *>(ar.r + p.r_ex);
     for (int o = threadIdx.x; o < p.no; o += blockDim.x) {
-        const double *s = Vi + 6 * (size_t)opt[o];
-        const R *w = W + 18 * (size_t)o;
-        R *y = Y + 18 * (size_t)o;
-        for (int r = 0; r < 6; ++r) {
-            const double w0 = w[3 * r], w1 = w[3 * r + 1], w2 = w[3 * r + 2];
-            y[3 * r] = (R)(w0 * s[0] + w1 * s[1] + w2 * s[2]);
-            y[3 * r + 1] = (R)(w0 * s[1] + w1 * s[3] + w2 * s[4]);
-            y[3 * r + 2] = (R)(w0 * s[2] + w1 * s[4] + w2 * s[5]);
+        const double *s = Vi + 6 * (size_t)opt[o], *u = U + 36 * (size_t)ocam[o];
+        const double2 *w2 = reinterpret_cast<const double2 *>(W + 18 * (size_t)o);
+        double w[18], y[18];
+        int rho[6], ew = -4096, ey = -4096, bw = 0, by = 0;
+#pragma unroll
+        for (int e = 0; e < 9; ++e) {
+            const double2 v = w2[e];
+            w[2 * e] = v.x;
+            w[2 * e + 1] = v.y;
         }
+#pragma unroll
+        for (int r = 0; r < 6; ++r) {
+            rho[r] = fx_weight(u[7 * r]);
+            const double w0 = w[3 * r], w1 = w[3 * r + 1], w2v = w[3 * r + 2];
+            y[3 * r] = w0 * s[0] + w1 * s[1] + w2v * s[2];
+            y[3 * r + 1] = w0 * s[1] + w1 * s[3] + w2v * s[4];
+            y[3 * r + 2] = w0 * s[2] + w1 * s[4] + w2v * s[5];
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                ew = max(ew, fx_exp(w[3 * r + j]) - rho[r]);
+                ey = max(ey, fx_exp(y[3 * r + j]) - rho[r]);
+                bw |= fx_nonfinite(w[3 * r + j]);
+                by |= fx_nonfinite(y[3 * r + j]);
+            }
+        }
+        // [j][row], two rows a store
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+            for (int r = 0; r < 6; r += 2) {
+                const int a = 3 * r + j, b = 3 * (r + 1) + j;
+                const size_t at = 9 * (size_t)o + 3 * j + r / 2;
+                const int2 y0 = fx_limbs(y[a], ey + rho[r] - fx_exp(y[a])), y1 = fx_limbs(y[b], ey + rho[r + 1] - fx_exp(y[b]));
+                const int2 w0 = fx_limbs(w[a], ew + rho[r] - fx_exp(w[a])), w1 = fx_limbs(w[b], ew + rho[r + 1] - fx_exp(w[b]));
+                Yq[at] = make_int4(y0.x, y0.y, y1.x, y1.y);
+                Wq[at] = make_int4(w0.x, w0.y, w1.x, w1.y);
+            }
+        ex[o] = make_int2(by ? FX_NAN : ey, bw ? FX_NAN : ew);
     }
 }
 
-// S (N x N, row-major, lower triangle) and rhs = ea
-template <typename R>
-__device__ void stage_schur(const BatchProblem &p, const Arenas<R> &ar, double mu)
+// FP64 form: S (N x N, row-major, lower triangle) and rhs = ea, a warp per
+// camera and per camera pair, in block fixed point (fx6_unit; sm: its shared
+// memory, F6_WARP_WORDS per warp).  On the FP64 pipe (two multiply-adds a
+// clock) this was 46% of a solve.
+constexpr int F6_WARP_WORDS = F6_SY + F6_SW;
+
+__device__ void stage_schur(const BatchProblem &p, const Arenas<double> &ar, double mu, int2 *sm)
 {
     const int N = p.N;
     double *S = ar.d + p.d_S, *rhs = ar.d + p.d_rhs;
     for (long long e = threadIdx.x; e < (long long)N * N; e += blockDim.x) S[e] = 0.0;
     __syncthreads();
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, nw = blockDim.x / 32;
-    const R *Y = ar.r + p.r_Y, *W = ar.r + p.r_W;
+    const int warp = threadIdx.x / 32, nw = blockDim.x / 32;
+    int2 *sy = sm + warp * F6_WARP_WORDS, *sw = sy + F6_SY;
+    const FxArgs fx = fx_args(p, ar);
     const double *U = ar.d + p.d_U, *g = ar.d + p.d_g;
-    const int *opt = ar.i + p.i_obs_pt, *cs = ar.i + p.i_cam_start, *co = ar.i + p.i_cam_obs;
-    // diagonal blocks and ea
+    const int *cs = ar.i + p.i_cam_start, *pst = ar.i + p.i_pair_start, *pkl = ar.i + p.i_pair_kl;
     for (int k = warp; k < p.nc; k += nw) {
-        double acc[27];
-        for (int v = 0; v < 27; ++v) acc[v] = 0.0;
-        for (int t = cs[k] + lane; t < cs[k + 1]; t += 32) {
-            const int a = co[t];
-            const R *y = Y + 18 * (size_t)a, *w = W + 18 * (size_t)a;
-            const double *gb = g + N + 3 * (size_t)opt[a];
-            int v = 0;
-            for (int r = 0; r < 6; ++r)
-                for (int c = 0; c <= r; ++c, ++v)
-                    acc[v] += (double)(y[3 * r] * w[3 * c] + y[3 * r + 1] * w[3 * c + 1] + y[3 * r + 2] * w[3 * c + 2]);
-            for (int r = 0; r < 6; ++r)
-                acc[21 + r] += (double)y[3 * r] * gb[0] + (double)y[3 * r + 1] * gb[1] + (double)y[3 * r + 2] * gb[2];
-        }
-        for (int v = 0; v < 27; ++v) acc[v] = warp_sum(acc[v]);
-        if (lane == 0) {
-            int v = 0;
-            for (int r = 0; r < 6; ++r)
-                for (int c = 0; c <= r; ++c, ++v) {
-                    const double uu = U[36 * k + r * 6 + c];
-                    S[(size_t)(6 * k + r) * N + 6 * k + c] = (r == c ? uu + mu : uu) - acc[v];
-                }
-            for (int r = 0; r < 6; ++r) rhs[6 * k + r] = g[6 * k + r] - acc[21 + r];
-        }
-    }
-    // off-diagonal blocks: groups of `lpp` lanes per camera pair (8, 16 or 32,
-    // the autotuner's choice for the problem's size bucket), lanes strided
-    // over the pair's common points, fixed-order shuffle reduction
-    const int *pst = ar.i + p.i_pair_start, *pkl = ar.i + p.i_pair_kl, *pa = ar.i + p.i_pair_a,
-              *pb = ar.i + p.i_pair_b;
-    const int lpp = (p.flags & 0xff) ? (p.flags & 0xff) : 32;
-    const int gpw = 32 / lpp;                       // groups per warp
-    const int grp = warp * gpw + lane / lpp, ng = nw * gpw, gl = lane % lpp;
-    const int qmax = (p.n_pairs + ng - 1) / ng * ng;  // keep whole warps in the loop for the shuffles
-    for (int q = grp; q < qmax; q += ng) {
-        double acc[36];
-        for (int v = 0; v < 36; ++v) acc[v] = 0.0;
-        if (q < p.n_pairs) {
-            for (int t = pst[q] + gl; t < pst[q + 1]; t += lpp) {
-                const R *y = Y + 18 * (size_t)pa[t], *w = W + 18 * (size_t)pb[t];
-                for (int r = 0; r < 6; ++r)
-                    for (int c = 0; c < 6; ++c)
-                        acc[r * 6 + c] +=
-                            (double)(y[3 * r] * w[3 * c] + y[3 * r + 1] * w[3 * c + 1] + y[3 * r + 2] * w[3 * c + 2]);
+        const int n = cs[k + 1] - cs[k];
+        auto emit = [&](int, int r, int c, double x) {
+            if (c == 6) {
+                rhs[6 * k + r] = g[6 * k + r] - x;
+            } else {
+                const double uu = U[36 * k + r * 6 + c];
+                S[(size_t)(6 * k + r) * N + 6 * k + c] = (r == c ? uu + mu : uu) - x;
+            }
+        };
+        if (n > 0) {
+            fx6_unit<true, false>(fx, SchurUnit{k, cs[k], n, 0}, k, k, sy, sw, emit);
+        } else if ((threadIdx.x & 31) == 0) {  // a camera without observations
+            for (int v = 0; v < n_out<6, true>(); ++v) {
+                int r, c;
+                out_rc<6, true>(v, r, c);
+                emit(v, r, c, 0.0);
             }
         }
-        for (int v = 0; v < 36; ++v)
-            for (int off = lpp / 2; off > 0; off >>= 1) acc[v] += __shfl_down_sync(0xffffffffu, acc[v], off, lpp);
-        if (gl == 0 && q < p.n_pairs) {
-            const int k = pkl[2 * q], l = pkl[2 * q + 1];
-            for (int r = 0; r < 6; ++r)
-                for (int c = 0; c < 6; ++c) S[(size_t)(6 * k + r) * N + 6 * l + c] = -acc[r * 6 + c];
-        }
+        __syncwarp();
+    }
+    for (int q = warp; q < p.n_pairs; q += nw) {
+        const int k = pkl[2 * q], l = pkl[2 * q + 1];
+        fx6_unit<false, false>(fx, SchurUnit{q, pst[q], pst[q + 1] - pst[q], 0}, k, l, sy, sw,
+                               [&](int, int r, int c, double x) { S[(size_t)(6 * k + r) * N + 6 * l + c] = -x; });
+        __syncwarp();
     }
 }
 
-// Right-looking column Cholesky of the lower triangle of S (FP64), then
-// L y = rhs and L^T x = y.  Returns 0, or 1 on a non-positive / non-finite
-// pivot (the reference's status, SPD_inv.cl:66-107).
-__device__ int stage_cholesky_solve(double *S, int N, double *rhs, double *x, double *sh, int *shi)
+// Cholesky of the lower triangle of S (FP64, N x N) with L y = rhs carried
+// along, then L^T x = y; both forms.  Returns 0, or 1 on a non-positive /
+// non-finite pivot (the reference's status, SPD_inv.cl:66-107).
+//
+// By panels of chol_width(N) columns in shared memory (P, chol_smem(N) bytes):
+// the panel's columns are eliminated there in LDL^T form, one barrier per column
+// (rhs is the row below; thread 0, whose entry is the next pivot, takes its
+// reciprocal), then scaled by the roots, all at once, and the rest of S
+// takes the panel's product from shared memory in one pass: rows cut into
+// limbs relative to their largest value (|L_ik| <= sqrt(S_ii), so the cut is
+// 2^-57 of the row's own scale), products on the integer pipe, one FP64
+// instruction per entry and panel.  Column by column in global memory every
+// column waited for three barriers and several L2 round trips (9,000 cycles a
+// column), and S was read and written N times: 30% of a mixed solve.
+// The width depends on N alone, so a result does not depend on the batch.
+__host__ __device__ inline int chol_width(int N) { return N <= 384 ? 16 : N <= 768 ? 8 : N <= 1536 ? 4 : N <= 3072 ? 2 : 1; }
+__host__ __device__ inline size_t chol_smem(int N)
 {
-    if (threadIdx.x == 0) shi[0] = 0;
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    for (int k = 0; k < N; ++k) {
-        if (threadIdx.x == 0) {
-            const double d = S[(size_t)k * N + k];
-            if (!(d > 0.0) || !isfinite(d)) {
-                shi[0] = 1;
-            } else {
-                // one root on the column chain: L_kk = d / sqrt(d); the forward
-                // solve rides along (y_k = rhs_k / L_kk), and 1 / L_kk waits in
-                // x[k] for the back solve
-                const double r = rsqrt(d);
-                S[(size_t)k * N + k] = d * r;
-                const double yk = rhs[k] * r;
-                rhs[k] = yk;
-                x[k] = r;
-                sh[0] = r;
-                sh[1] = yk;
+    return sizeof(double) * (size_t)(N + 1) * (size_t)(chol_width(N) + 1) + sizeof(int) * (size_t)(N + 2);
+}
+constexpr int CHOL_NB = 16;  // the widest panel
+
+__device__ __forceinline__ double pivot_rcp(double d) { return d > 1e-290 && d < 1e290 ? rcp_fast(d) : 1.0 / d; }
+
+__device__ int stage_cholesky_solve(double *S, int N, double *rhs, double *x, double *sh, double *P)
+{
+    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+    const int nb = chol_width(N), sb = 31 - __clz(nb), ps = nb + 1;
+    int *E = reinterpret_cast<int *>(P + (size_t)(N + 1) * ps);
+    double *dinv = sh + CHOL_NB, *root = sh + 2 * CHOL_NB, *ys = sh + 3 * CHOL_NB;  // sh: the pivots
+    for (int k0 = 0; k0 < N; k0 += nb) {
+        const int w = min(nb, N - k0), m = N - k0;  // columns; rows of S, then rhs as row m
+        for (int e = tid; e < (m + 1) << sb; e += nt) {
+            const int r = e >> sb, c = e & (nb - 1);
+            if (c < w && c <= r) P[r * ps + c] = r < m ? S[(size_t)(k0 + r) * N + k0 + c] : rhs[k0 + c];
+        }
+        __syncthreads();
+        if (tid == 0) {
+            sh[0] = P[0];
+            dinv[0] = pivot_rcp(P[0]);
+        }
+        __syncthreads();
+        for (int c = 0; c < w - 1; ++c) {
+            const double inv = dinv[c];
+            for (int cc = c + 1 + warp; cc < w; cc += nw) {
+                const double f = P[cc * ps + c] * inv;
+                for (int r = cc + lane; r <= m; r += 32) P[r * ps + cc] = fma(-P[r * ps + c], f, P[r * ps + cc]);
+            }
+            if (tid == 0) {  // the entry (c + 1, c + 1) is its own
+                const double d = P[(c + 1) * ps + c + 1];
+                sh[c + 1] = d;
+                dinv[c + 1] = pivot_rcp(d);
+            }
+            __syncthreads();
+        }
+        int bad = 0;
+        if (tid < w) {
+            const double d = sh[tid];
+            bad = !(d > 0.0) || !isfinite(d);
+            const double r = rsqrt(d);
+            root[tid] = r;
+            x[k0 + tid] = r;  // 1 / L_kk, for the back solve
+            const double y = P[m * ps + tid] * r;
+            ys[tid] = y;
+            rhs[k0 + tid] = y;
+        }
+        if (__syncthreads_or(bad)) return 1;
+        // a row a thread: L = a D^-1/2 out to S; below the diagonal block also
+        // rhs -= L y, and the row as limbs in its place
+        for (int r = tid; r < m; r += nt) {
+            double *a = P + r * ps;
+            double dot = 0.0;
+            int er = 1, nf = 0;
+            const int cn = min(w, r + 1);
+            for (int c = 0; c < cn; ++c) {
+                const double l = a[c] * root[c];
+                a[c] = l;
+                S[(size_t)(k0 + r) * N + k0 + c] = l;
+                dot = fma(l, ys[c], dot);
+                er = max(er, fx_exp(l));
+                nf |= fx_nonfinite(l);
+            }
+            if (r < w) continue;
+            rhs[k0 + r] -= dot;
+            for (int c = 0; c < w; ++c) *reinterpret_cast<int2 *>(a + c) = fx_limbs(a[c], er - fx_exp(a[c]));
+            E[r] = nf ? FX_NAN : er;
+        }
+        __syncthreads();
+        // the rest: S_ij -= sum_k L_ik L_jk, 2 x 2 entries a thread, a warp per pair of rows
+        const int nr = m - w;
+        for (int ti = warp; 2 * ti < nr; ti += nw) {
+            const int i0 = w + 2 * ti, i1 = min(i0 + 1, m - 1);
+            const int2 *a0 = reinterpret_cast<const int2 *>(P + i0 * ps), *a1 = reinterpret_cast<const int2 *>(P + i1 * ps);
+            const int e0 = E[i0], e1 = E[i1];
+            double *s0 = S + (size_t)(k0 + i0) * N + k0, *s1 = S + (size_t)(k0 + i1) * N + k0;
+            for (int tj = lane; tj <= ti; tj += 32) {
+                const int j0 = w + 2 * tj, j1 = min(j0 + 1, m - 1);
+                const int2 *b0 = reinterpret_cast<const int2 *>(P + j0 * ps), *b1 = reinterpret_cast<const int2 *>(P + j1 * ps);
+                const double v00 = s0[j0], v01 = s0[j1], v10 = s1[j0], v11 = s1[j1];  // all inside S
+                long long h[4] = {0, 0, 0, 0}, c[4] = {0, 0, 0, 0};
+#pragma unroll 4
+                for (int k = 0; k < w; ++k) {
+                    const int2 p0 = a0[k], p1 = a1[k], q0 = b0[k], q1 = b1[k];
+                    fx_mad(p0, q0, h[0], c[0]);
+                    fx_mad(p0, q1, h[1], c[1]);
+                    fx_mad(p1, q0, h[2], c[2]);
+                    fx_mad(p1, q1, h[3], c[3]);
+                }
+                const int f0 = E[j0], f1 = E[j1];
+                auto put = [&](double *at, double v, int n, int e) {
+                    *at = e >= FX_NAN / 2 ? nan("") : fx_add(v, -fx_total(h[n], c[n]), e);
+                };
+                put(s0 + j0, v00, 0, e0 + f0);
+                if (j1 > j0 && j1 <= i0) put(s0 + j1, v01, 1, e0 + f1);
+                if (i1 > i0) {
+                    put(s1 + j0, v10, 2, e1 + f0);
+                    if (j1 > j0) put(s1 + j1, v11, 3, e1 + f1);
+                }
             }
         }
         __syncthreads();
-        if (shi[0]) return 1;
-        const double inv = sh[0], yk = sh[1];
-        for (int i = k + 1 + threadIdx.x; i < N; i += blockDim.x) {
-            const double l = S[(size_t)i * N + k] * inv;
-            S[(size_t)i * N + k] = l;
-            rhs[i] -= l * yk;
-        }
-        __syncthreads();
-        // trailing update, lower triangle: a warp per row, lanes over its columns
-        for (int i = k + 1 + warp; i < N; i += nwarps) {
-            const double lik = S[(size_t)i * N + k];
-            for (int j = k + 1 + lane; j <= i; j += 32) S[(size_t)i * N + j] -= lik * S[(size_t)j * N + k];
-        }
-        __syncthreads();
     }
-    // back: L^T x = y (y in rhs, 1 / L_kk in x[k])
-    for (int k = N - 1; k >= 0; --k) {
-        if (threadIdx.x == 0) x[k] = rhs[k] * x[k];
+    // back: L^T x = y by the same blocks, y in P: warp 0 solves a block, a lane
+    // per unknown, then every earlier unknown takes the block's sixteen
+    double *xb = sh;
+    for (int i = tid; i < N; i += nt) P[i] = rhs[i];
+    __syncthreads();
+    for (int k0 = (N - 1) / nb * nb; k0 >= 0; k0 -= nb) {
+        const int w = min(nb, N - k0);
+        if (warp == 0) {
+            const bool on = lane < w;
+            double y = on ? P[k0 + lane] : 0.0, l[CHOL_NB];
+            const double inv = on ? x[k0 + lane] : 0.0;
+#pragma unroll
+            for (int k = 0; k < CHOL_NB; ++k) l[k] = k < w && lane < k ? S[(size_t)(k0 + k) * N + k0 + lane] : 0.0;
+            double xv = 0.0;
+#pragma unroll
+            for (int k = CHOL_NB - 1; k >= 0; --k) {
+                const double xk = __shfl_sync(0xffffffffu, y * inv, k);
+                if (lane == k) xv = xk;
+                y = fma(-l[k], xk, y);
+            }
+            if (on) {
+                xb[lane] = xv;
+                x[k0 + lane] = xv;
+            }
+        }
         __syncthreads();
-        const double xk = x[k];
-        for (int i = threadIdx.x; i < k; i += blockDim.x) rhs[i] -= S[(size_t)k * N + i] * xk;
+        for (int i = tid; i < k0; i += nt) {
+            double s = P[i];
+#pragma unroll 4
+            for (int k = 0; k < w; ++k) s = fma(-S[(size_t)(k0 + k) * N + i], xb[k], s);
+            P[i] = s;
+        }
         __syncthreads();
     }
     return 0;
@@ -1057,7 +1193,7 @@ __device__ double stage_cost_mx(const BatchProblem &p, const Arenas<float> &ar, 
 
 template <typename R>
 __device__ void solve_problem(const BatchProblem &p, const Arenas<R> &ar, const BatchOpts &o, BatchResult *res,
-                              double *sh, int *shi, double *shd)
+                              double *sh, int *shi, double *shd, double *dyn)
 {
     const int N = p.N;
     double *dp = ar.d + p.d_dp, *tab = ar.d + p.d_tab, *tab2 = ar.d + p.d_tab2;
@@ -1133,13 +1269,13 @@ __device__ void solve_problem(const BatchProblem &p, const Arenas<R> &ar, const 
                 __syncthreads();
                 stage_schur_mx(p, ar, mu);
             } else {
-                stage_vinv_y<R>(p, ar, mu);
+                stage_vinv_y(p, ar, mu);
                 __syncthreads();
-                stage_schur<R>(p, ar, mu);
+                stage_schur(p, ar, mu, reinterpret_cast<int2 *>(dyn));
             }
             __syncthreads();
             double *S = ar.d + p.d_S, *rhs = ar.d + p.d_rhs, *x = ar.d + p.d_x;
-            const int st = stage_cholesky_solve(S, N, rhs, x, sh, shi);
+            const int st = stage_cholesky_solve(S, N, rhs, x, sh, dyn);
             if (threadIdx.x == 0) shi[4]++;
             int decided = 0;  // 0: retry with larger mu, 1: accepted, 2: stop
             if (st == 0) {
@@ -1232,6 +1368,7 @@ __global__ void __launch_bounds__(MAX_THREADS) k_batch_lm(const BatchProblem *__
                                                            BatchResult *__restrict__ res)
 {
     const BatchOpts o = *opts;
+    extern __shared__ __align__(16) double dyn[];  // batch_smem bytes: the dense panel, or the FP64 Schur rows
     __shared__ double sh[MAX_THREADS];
     __shared__ double shd[8];
     __shared__ int shi[16];
@@ -1244,7 +1381,7 @@ __global__ void __launch_bounds__(MAX_THREADS) k_batch_lm(const BatchProblem *__
         if (q >= n) break;
         const int pi = order[q];
         const BatchProblem p = probs[pi];
-        solve_problem<R>(p, ar, o, res + pi, sh, shi, shd);
+        solve_problem<R>(p, ar, o, res + pi, sh, shi, shd, dyn);
     }
 }
 
@@ -1357,11 +1494,12 @@ bool build_problem_layout(const psba_problem_desc &p, ProblemLayout &L, std::str
     bp.i_pair_b = iput(pb.data(), pb.size());
     long long r_total = 0;
     // A first: its 48-byte rows stay 16-byte aligned (every region and the
-    // problem's total are multiples of four elements), the others 8-byte
+    // problem's total are multiples of four elements), the others 8-byte; B
+    // behind it: the FP64 form's W limb rows take the place of both
     bp.r_A = r_total; r_total += 12LL * no;
+    bp.r_B = r_total; r_total += 6LL * no;
     bp.r_W = r_total; r_total += 18LL * no;
     bp.r_Y = r_total; r_total += 18LL * no;
-    bp.r_B = r_total; r_total += 6LL * no;
     bp.r_ex = r_total; r_total += 2LL * no;
     // the mixed form's FP32 copies (even counts: FP32 pairs stay 8-byte aligned)
     bp.r_tab32 = r_total; r_total += (long long)CAMTAB32 * nc;
@@ -1412,30 +1550,78 @@ size_t pool_bytes(const ProblemLayout &L, int precision)
     return align256(sizeof(double) * L.dA.size()) + align256(sizeof(int) * L.iA.size()) + align256(rs * L.nr);
 }
 
-cudaError_t launch_batch_lm(int precision, int grid, int threads, cudaStream_t s, const BatchProblem *probs,
+// Dynamic shared memory of the persistent launch: the dense panel of any
+// problem up to max_N, and the FP64 form's Schur rows, one after the other.
+static size_t batch_smem(int precision, int threads, int max_N)
+{
+    // the width steps down as N grows, so a smaller N can need more
+    size_t b = chol_smem(max_N);
+    for (int step : {384, 768, 1536, 3072})
+        if (max_N > step) b = std::max(b, chol_smem(step));
+    if (precision != PSBA_PREC_MIXED) b = std::max(b, sizeof(int2) * F6_WARP_WORDS * (size_t)(threads / 32));
+    return b;
+}
+
+// the kernels' opt-in to more shared memory than 48 KB, once per device
+static cudaError_t batch_attributes()
+{
+    static std::mutex mu;
+    static bool done[MAX_DEVICES] = {};
+    int dev = 0, most = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return e != cudaSuccess ? e : cudaErrorInvalidDevice;
+    std::lock_guard<std::mutex> lk(mu);
+    if (done[dev]) return cudaSuccess;
+    e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    cudaFuncAttributes fa;
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_batch_lm<float>);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_batch_lm<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 most - (int)fa.sharedSizeBytes);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_batch_lm<double>);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_batch_lm<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 most - (int)fa.sharedSizeBytes);
+    done[dev] = e == cudaSuccess;
+    return e;
+}
+
+cudaError_t launch_batch_lm(int precision, int grid, int threads, int max_N, cudaStream_t s, const BatchProblem *probs,
                             const int *order, int n, int *queue, double *darena, int *iarena, void *rarena,
                             const BatchOpts *opts, BatchResult *res)
 {
+    const cudaError_t e = batch_attributes();
+    if (e != cudaSuccess) return e;
+    const size_t smem = batch_smem(precision, threads, max_N);
     if (precision == PSBA_PREC_MIXED) {
         Arenas<float> ar{darena, iarena, (float *)rarena};
-        k_batch_lm<float><<<grid, threads, 0, s>>>(probs, order, n, queue, ar, opts, res);
+        k_batch_lm<float><<<grid, threads, smem, s>>>(probs, order, n, queue, ar, opts, res);
     } else {
         Arenas<double> ar{darena, iarena, (double *)rarena};
-        k_batch_lm<double><<<grid, threads, 0, s>>>(probs, order, n, queue, ar, opts, res);
+        k_batch_lm<double><<<grid, threads, smem, s>>>(probs, order, n, queue, ar, opts, res);
     }
     return cudaGetLastError();  // the caller counts the launch (it may be inside a graph capture)
 }
 
-int batch_blocks_per_sm(int precision, int threads)
+int batch_blocks_per_sm(int precision, int threads, int max_N)
 {
     int per_sm = 1;
+    if (batch_attributes() != cudaSuccess) return 1;
+    const size_t smem = batch_smem(precision, threads, max_N);
     if (precision == PSBA_PREC_MIXED)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_lm<float>, threads, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_lm<float>, threads, smem);
     else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_lm<double>, threads, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_lm<double>, threads, smem);
     return per_sm > 0 ? per_sm : 1;
 }
 
+// Back to the initial estimate, a block per problem.
+__global__ void k_batch_reset(const BatchProblem *__restrict__ probs, double *__restrict__ d)
+{
+    const BatchProblem &p = probs[blockIdx.x];
+    for (int k = threadIdx.x; k < 6 * p.nc; k += blockDim.x) d[p.d_cams + k] = d[p.d_cams0 + k];
+    for (int k = threadIdx.x; k < 3 * p.np; k += blockDim.x) d[p.d_pts + k] = d[p.d_pts0 + k];
+}
 
 struct HostBatch {
     int n = 0;
@@ -1452,6 +1638,7 @@ struct HostBatch {
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int threads = 256;
+    int max_N = 0;  // the largest problem's reduced size
     size_t bytes = 0;
     cudaGraphExec_t graph = nullptr;  // captured [queue reset, persistent launch]
     int graph_key = -1;               // precision * 1024 + threads of the captured graph
@@ -1524,6 +1711,7 @@ int psba_batch_create(const psba_problem_desc *descs, int n, psba_batch **out)
         iA.insert(iA.end(), L.iA.begin(), L.iA.end());
         r_total += L.nr;
         h.probs[q] = L.bp;
+        h.max_N = std::max(h.max_N, L.bp.N);
         work[q] = L.work;
     }
     // longest-first processing order (by observations, then reduced size)
@@ -1582,14 +1770,8 @@ int psba_batch_reset_params(psba_batch *b)
 {
     if (!b) return set_error("null batch"), PSBA_ERR_ARG;
     HostBatch &h = b->hb;
-    for (int q = 0; q < h.n; ++q) {
-        const BatchProblem &p = h.probs[q];
-        cudaMemcpyAsync(h.d_arena + p.d_cams, h.d_arena + p.d_cams0, sizeof(double) * 6 * p.nc,
-                        cudaMemcpyDeviceToDevice, h.stream);
-        if (p.np)
-            cudaMemcpyAsync(h.d_arena + p.d_pts, h.d_arena + p.d_pts0, sizeof(double) * 3 * p.np,
-                            cudaMemcpyDeviceToDevice, h.stream);
-    }
+    k_batch_reset<<<h.n, 256, 0, h.stream>>>(h.d_probs, h.d_arena);
+    note_launch(1);
     const cudaError_t e = cudaStreamSynchronize(h.stream);
     return e == cudaSuccess ? PSBA_OK : cuda_fail(e, "psba_batch_reset_params");
 }
@@ -1624,8 +1806,8 @@ int psba_batch_levmar(psba_batch *b, const psba_opts *opts, psba_batch_result *r
         if (e != cudaSuccess) return cuda_fail(e, "psba_batch_levmar capture");
         cudaMemsetAsync(h.d_queue, 0, sizeof(int), h.stream);
         cudaMemsetAsync(h.d_res, 0, sizeof(BatchResult) * h.n, h.stream);  // every problem starts afresh
-        const int grid = std::min(h.n, batch_blocks_per_sm(opts->precision, h.threads) * sms);
-        launch_batch_lm(opts->precision, grid, h.threads, h.stream, h.d_probs, h.d_order, h.n, h.d_queue,
+        const int grid = std::min(h.n, batch_blocks_per_sm(opts->precision, h.threads, h.max_N) * sms);
+        launch_batch_lm(opts->precision, grid, h.threads, h.max_N, h.stream, h.d_probs, h.d_order, h.n, h.d_queue,
                         h.d_arena, h.i_arena, h.r_arena, h.d_opts, h.d_res);
         e = cudaStreamEndCapture(h.stream, &g);
         if (e == cudaSuccess) e = cudaGraphInstantiate(&h.graph, g, 0);

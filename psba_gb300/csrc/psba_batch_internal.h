@@ -65,10 +65,11 @@ size_t pool_bytes(const ProblemLayout &L, int precision);
 
 // The persistent launch over problems probs[order[0..n)] with state in res[];
 // all three arenas point into one byte pool when called from the server.
-cudaError_t launch_batch_lm(int precision, int grid, int threads, cudaStream_t s, const BatchProblem *probs,
+// max_N: the largest reduced size among the problems.
+cudaError_t launch_batch_lm(int precision, int grid, int threads, int max_N, cudaStream_t s, const BatchProblem *probs,
                             const int *order, int n, int *queue, double *darena, int *iarena, void *rarena,
                             const BatchOpts *opts, BatchResult *res);
-int batch_blocks_per_sm(int precision, int threads);
+int batch_blocks_per_sm(int precision, int threads, int max_N);
 
 }  // namespace batch
 }  // namespace psba

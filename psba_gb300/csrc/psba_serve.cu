@@ -248,11 +248,12 @@ void worker_main(psba_server *s)
         // outer iterations, lighter ones proportionally more
         double wmax = 0.0;
         for (Request *r : active) wmax = std::max(wmax, r->L.work);
-        int max_slot = 0;
+        int max_slot = 0, max_N = 0;
         for (Request *r : active) {
             const double k = std::floor(s->so.slice_iters * wmax / std::max(r->L.work, 1.0));
             s->h_probs[r->slot].slice = (int)std::min<double>(std::max<double>(k, s->so.slice_iters), s->bo.max_iter);
             max_slot = std::max(max_slot, r->slot + 1);
+            max_N = std::max(max_N, r->L.bp.N);
         }
         std::sort(active.begin(), active.end(), [](const Request *a, const Request *b) {
             return a->L.work > b->L.work;
@@ -266,7 +267,7 @@ void worker_main(psba_server *s)
         if (e == cudaSuccess) e = cudaMemsetAsync(s->d_queue, 0, sizeof(int), s->stream);
         if (e == cudaSuccess) e = cudaEventRecord(s->ev0, s->stream);
         if (e == cudaSuccess)
-            e = launch_batch_lm(s->precision, std::min(n, s->grid_cap), s->so.threads, s->stream, s->d_probs,
+            e = launch_batch_lm(s->precision, std::min(n, s->grid_cap), s->so.threads, max_N, s->stream, s->d_probs,
                                 s->d_order, n, s->d_queue, (double *)s->pool, (int *)s->pool, (void *)s->pool,
                                 s->d_opts, s->d_state);
         note_launch(1);
@@ -529,7 +530,7 @@ int psba_server_create(const psba_server_opts *so, const psba_opts *lm, psba_ser
         return e == cudaErrorMemoryAllocation ? PSBA_ERR_NOMEM : PSBA_ERR_CUDA;
     }
     std::memset(s->h_probs, 0, sizeof(BatchProblem) * M);
-    s->grid_cap = batch_blocks_per_sm(s->precision, so->threads) * sms;
+    s->grid_cap = batch_blocks_per_sm(s->precision, so->threads, 6 * std::max(1, so->large_cams > 0 ? so->large_cams : 64)) * sms;
     if (with_large)
         s->large_chol_cap = so->large_chol_ctas > 0 ? std::min(so->large_chol_ctas, sms)
                                                     : std::max(2, sms / so->large_lanes);
