@@ -1623,6 +1623,17 @@ __global__ void k_batch_reset(const BatchProblem *__restrict__ probs, double *__
     for (int k = threadIdx.x; k < 3 * p.np; k += blockDim.x) d[p.d_pts + k] = d[p.d_pts0 + k];
 }
 
+// All problems' parameters, packed for one copy to the host: problem q's
+// cameras, then points, at off[q].
+__global__ void k_batch_pack(const BatchProblem *__restrict__ probs, const long long *__restrict__ off,
+                             const double *__restrict__ d, double *__restrict__ out)
+{
+    const BatchProblem &p = probs[blockIdx.x];
+    double *o = out + off[blockIdx.x];
+    for (int k = threadIdx.x; k < 6 * p.nc; k += blockDim.x) o[k] = d[p.d_cams + k];
+    for (int k = threadIdx.x; k < 3 * p.np; k += blockDim.x) o[6 * p.nc + k] = d[p.d_pts + k];
+}
+
 struct HostBatch {
     int n = 0;
     std::vector<BatchProblem> probs;
@@ -1642,6 +1653,15 @@ struct HostBatch {
     size_t bytes = 0;
     cudaGraphExec_t graph = nullptr;  // captured [queue reset, persistent launch]
     int graph_key = -1;               // precision * 1024 + threads of the captured graph
+    // Reading every problem's parameters one by one took two small copies and
+    // a wait each (22 us; 6.8 ms for 304 problems).  The second read since the
+    // parameters last changed brings all of them over in one copy; a caller
+    // that wants one problem's does not pay for the others.
+    std::mutex read_mu;  // reads may come from several threads
+    int reads = 0;       // since the parameters last changed
+    bool mirrored = false;
+    std::vector<double> mirror;
+    std::vector<long long> mirror_off;
 };
 
 }  // namespace batch
@@ -1680,6 +1700,46 @@ void batch_free(psba_batch *b)
     if (h.ev1) cudaEventDestroy(h.ev1);
     if (h.stream) cudaStreamDestroy(h.stream);
     delete b;
+}
+
+}  // namespace
+
+namespace {
+
+// Every problem's parameters into h.mirror; on an error the mirror stays unused.
+bool read_all(HostBatch &h)
+{
+    h.mirror_off.resize(h.n);
+    long long total = 0;
+    for (int q = 0; q < h.n; ++q) {
+        h.mirror_off[q] = total;
+        total += 6LL * h.probs[q].nc + 3LL * h.probs[q].np;
+    }
+    double *d_out = nullptr;
+    long long *d_off = nullptr;
+    cudaError_t e = cudaMallocAsync(&d_out, sizeof(double) * total, h.stream);
+    if (e == cudaSuccess) e = cudaMallocAsync(&d_off, sizeof(long long) * h.n, h.stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(d_off, h.mirror_off.data(), sizeof(long long) * h.n, cudaMemcpyHostToDevice, h.stream);
+    if (e == cudaSuccess) {
+        k_batch_pack<<<h.n, 256, 0, h.stream>>>(h.d_probs, d_off, h.d_arena, d_out);
+        note_launch(1);
+        h.mirror.resize((size_t)total);
+        e = cudaMemcpyAsync(h.mirror.data(), d_out, sizeof(double) * total, cudaMemcpyDeviceToHost, h.stream);
+    }
+    if (d_out) cudaFreeAsync(d_out, h.stream);
+    if (d_off) cudaFreeAsync(d_off, h.stream);
+    const cudaError_t s = cudaStreamSynchronize(h.stream);
+    if (e == cudaSuccess) e = s;
+    if (e != cudaSuccess) cudaGetLastError();  // the single reads go on, and report what they meet
+    return e == cudaSuccess;
+}
+
+void params_changed(HostBatch &h)
+{
+    std::lock_guard<std::mutex> lk(h.read_mu);
+    h.reads = 0;
+    h.mirrored = false;
 }
 
 }  // namespace
@@ -1770,6 +1830,7 @@ int psba_batch_reset_params(psba_batch *b)
 {
     if (!b) return set_error("null batch"), PSBA_ERR_ARG;
     HostBatch &h = b->hb;
+    params_changed(h);
     k_batch_reset<<<h.n, 256, 0, h.stream>>>(h.d_probs, h.d_arena);
     note_launch(1);
     const cudaError_t e = cudaStreamSynchronize(h.stream);
@@ -1781,6 +1842,7 @@ int psba_batch_levmar(psba_batch *b, const psba_opts *opts, psba_batch_result *r
     if (!b || !opts) return set_error("null argument"), PSBA_ERR_ARG;
     if (opts->refine != 0) return set_error("psba_batch_levmar: refine is for the per-handle solver"), PSBA_ERR_ARG;
     HostBatch &h = b->hb;
+    params_changed(h);
     BatchOpts o;
     o.tau = opts->tau;
     o.stop_thresh = opts->stop_thresh;
@@ -1852,6 +1914,16 @@ int psba_batch_get_params(psba_batch *b, int q, double *cams, double *pts)
     if (!b || q < 0 || q >= b->hb.n || !cams) return set_error("psba_batch_get_params: bad arguments"), PSBA_ERR_ARG;
     HostBatch &h = b->hb;
     const BatchProblem &p = h.probs[q];
+    {
+        std::lock_guard<std::mutex> lk(h.read_mu);
+        if (!h.mirrored && h.n > 2 && ++h.reads == 2) h.mirrored = read_all(h);
+        if (h.mirrored) {
+            const double *m = h.mirror.data() + h.mirror_off[q];
+            std::memcpy(cams, m, sizeof(double) * 6 * p.nc);
+            if (p.np && pts) std::memcpy(pts, m + 6 * p.nc, sizeof(double) * 3 * p.np);
+            return PSBA_OK;
+        }
+    }
     cudaError_t e = cudaMemcpy(cams, h.d_arena + p.d_cams, sizeof(double) * 6 * p.nc, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess && p.np && pts)
         e = cudaMemcpy(pts, h.d_arena + p.d_pts, sizeof(double) * 3 * p.np, cudaMemcpyDeviceToHost);
