@@ -431,19 +431,23 @@ __device__ void stage_schur(const BatchProblem &p, const Arenas<double> &ar, dou
 }
 
 // Cholesky of the lower triangle of S (FP64, N x N) with L y = rhs carried
-// along, then L^T x = y; both forms.  Returns 0, or 1 on a non-positive /
-// non-finite pivot (the reference's status, SPD_inv.cl:66-107).
+// along, then L^T x = y.  Returns 0, or 1 on a non-positive / non-finite pivot
+// (the reference's status, SPD_inv.cl:66-107).
 //
 // By panels of chol_width(N) columns in shared memory (P, chol_smem(N) bytes):
-// the panel's columns are eliminated there in LDL^T form, one barrier per column
-// (rhs is the row below; thread 0, whose entry is the next pivot, takes its
-// reciprocal), then scaled by the roots, all at once, and the rest of S
-// takes the panel's product from shared memory in one pass: rows cut into
-// limbs relative to their largest value (|L_ik| <= sqrt(S_ii), so the cut is
-// 2^-57 of the row's own scale), products on the integer pipe, one FP64
-// instruction per entry and panel.  Column by column in global memory every
-// column waited for three barriers and several L2 round trips (9,000 cycles a
-// column), and S was read and written N times: 30% of a mixed solve.
+// the panel's columns are eliminated there, one barrier per column (rhs is the
+// row below; thread 0, whose entry is the next pivot, takes its reciprocal
+// root), and the rest of S takes the panel's product from shared memory in
+// one pass.  Column by column in global memory every column waited for three
+// barriers and several L2 round trips (9,000 cycles a column), and S was read
+// and written N times: 30% of a mixed solve.
+// Every entry takes the same multiply-adds in the same order as there, so
+// the mixed form (FX false) has the same bits: its FP32 stages turn a last
+// bit of the step into 1e-9 of the parameters within 8 iterations.  The FP64
+// form (FX) forms the rest's products in block fixed point instead: rows cut
+// into limbs relative to their largest value (|L_ik| <= sqrt(S_ii), so the
+// cut is 2^-57 of the row's own scale), one FP64 instruction per entry and
+// panel where the FP64 pipe would take sixteen.
 // The width depends on N alone, so a result does not depend on the batch.
 __host__ __device__ inline int chol_width(int N) { return N <= 384 ? 16 : N <= 768 ? 8 : N <= 1536 ? 4 : N <= 3072 ? 2 : 1; }
 __host__ __device__ inline size_t chol_smem(int N)
@@ -452,14 +456,13 @@ __host__ __device__ inline size_t chol_smem(int N)
 }
 constexpr int CHOL_NB = 16;  // the widest panel
 
-__device__ __forceinline__ double pivot_rcp(double d) { return d > 1e-290 && d < 1e290 ? rcp_fast(d) : 1.0 / d; }
-
+template <bool FX>
 __device__ int stage_cholesky_solve(double *S, int N, double *rhs, double *x, double *sh, double *P)
 {
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
     const int nb = chol_width(N), sb = 31 - __clz(nb), ps = nb + 1;
     int *E = reinterpret_cast<int *>(P + (size_t)(N + 1) * ps);
-    double *dinv = sh + CHOL_NB, *root = sh + 2 * CHOL_NB, *ys = sh + 3 * CHOL_NB;  // sh: the pivots
+    double *root = sh + CHOL_NB, *ys = sh + 2 * CHOL_NB;  // sh: the pivots
     for (int k0 = 0; k0 < N; k0 += nb) {
         const int w = min(nb, N - k0), m = N - k0;  // columns; rows of S, then rhs as row m
         for (int e = tid; e < (m + 1) << sb; e += nt) {
@@ -469,84 +472,103 @@ __device__ int stage_cholesky_solve(double *S, int N, double *rhs, double *x, do
         __syncthreads();
         if (tid == 0) {
             sh[0] = P[0];
-            dinv[0] = pivot_rcp(P[0]);
+            root[0] = rsqrt(P[0]);
         }
         __syncthreads();
+        // column c's L values are formed where they are used, from its entries
+        // (left as they are until the panel is done) and 1 / L_cc
         for (int c = 0; c < w - 1; ++c) {
-            const double inv = dinv[c];
+            const double inv = root[c];
             for (int cc = c + 1 + warp; cc < w; cc += nw) {
                 const double f = P[cc * ps + c] * inv;
-                for (int r = cc + lane; r <= m; r += 32) P[r * ps + cc] = fma(-P[r * ps + c], f, P[r * ps + cc]);
+                for (int r = cc + lane; r <= m; r += 32) P[r * ps + cc] = fma(-(P[r * ps + c] * inv), f, P[r * ps + cc]);
             }
             if (tid == 0) {  // the entry (c + 1, c + 1) is its own
                 const double d = P[(c + 1) * ps + c + 1];
                 sh[c + 1] = d;
-                dinv[c + 1] = pivot_rcp(d);
+                root[c + 1] = rsqrt(d);
             }
             __syncthreads();
         }
         int bad = 0;
         if (tid < w) {
-            const double d = sh[tid];
+            const double d = sh[tid], r = root[tid];
             bad = !(d > 0.0) || !isfinite(d);
-            const double r = rsqrt(d);
-            root[tid] = r;
             x[k0 + tid] = r;  // 1 / L_kk, for the back solve
             const double y = P[m * ps + tid] * r;
             ys[tid] = y;
             rhs[k0 + tid] = y;
         }
         if (__syncthreads_or(bad)) return 1;
-        // a row a thread: L = a D^-1/2 out to S; below the diagonal block also
-        // rhs -= L y, and the row as limbs in its place
+        // a row a thread: L out to S; below the diagonal block also rhs -= L y,
+        // and the row kept for the product
         for (int r = tid; r < m; r += nt) {
             double *a = P + r * ps;
-            double dot = 0.0;
+            double b = r < w ? 0.0 : rhs[k0 + r];
             int er = 1, nf = 0;
             const int cn = min(w, r + 1);
             for (int c = 0; c < cn; ++c) {
                 const double l = a[c] * root[c];
                 a[c] = l;
                 S[(size_t)(k0 + r) * N + k0 + c] = l;
-                dot = fma(l, ys[c], dot);
-                er = max(er, fx_exp(l));
-                nf |= fx_nonfinite(l);
+                b = fma(-l, ys[c], b);
+                if (FX) {
+                    er = max(er, fx_exp(l));
+                    nf |= fx_nonfinite(l);
+                }
             }
             if (r < w) continue;
-            rhs[k0 + r] -= dot;
-            for (int c = 0; c < w; ++c) *reinterpret_cast<int2 *>(a + c) = fx_limbs(a[c], er - fx_exp(a[c]));
-            E[r] = nf ? FX_NAN : er;
+            rhs[k0 + r] = b;
+            if (FX) {
+                for (int c = 0; c < w; ++c) *reinterpret_cast<int2 *>(a + c) = fx_limbs(a[c], er - fx_exp(a[c]));
+                E[r] = nf ? FX_NAN : er;
+            }
         }
         __syncthreads();
         // the rest: S_ij -= sum_k L_ik L_jk, 2 x 2 entries a thread, a warp per pair of rows
         const int nr = m - w;
         for (int ti = warp; 2 * ti < nr; ti += nw) {
             const int i0 = w + 2 * ti, i1 = min(i0 + 1, m - 1);
-            const int2 *a0 = reinterpret_cast<const int2 *>(P + i0 * ps), *a1 = reinterpret_cast<const int2 *>(P + i1 * ps);
-            const int e0 = E[i0], e1 = E[i1];
             double *s0 = S + (size_t)(k0 + i0) * N + k0, *s1 = S + (size_t)(k0 + i1) * N + k0;
             for (int tj = lane; tj <= ti; tj += 32) {
                 const int j0 = w + 2 * tj, j1 = min(j0 + 1, m - 1);
-                const int2 *b0 = reinterpret_cast<const int2 *>(P + j0 * ps), *b1 = reinterpret_cast<const int2 *>(P + j1 * ps);
-                const double v00 = s0[j0], v01 = s0[j1], v10 = s1[j0], v11 = s1[j1];  // all inside S
-                long long h[4] = {0, 0, 0, 0}, c[4] = {0, 0, 0, 0};
+                double v00 = s0[j0], v01 = s0[j1], v10 = s1[j0], v11 = s1[j1];  // all inside S
+                if (FX) {
+                    const int2 *a0 = reinterpret_cast<const int2 *>(P + i0 * ps), *a1 = reinterpret_cast<const int2 *>(P + i1 * ps);
+                    const int2 *b0 = reinterpret_cast<const int2 *>(P + j0 * ps), *b1 = reinterpret_cast<const int2 *>(P + j1 * ps);
+                    long long h[4] = {0, 0, 0, 0}, c[4] = {0, 0, 0, 0};
 #pragma unroll 4
-                for (int k = 0; k < w; ++k) {
-                    const int2 p0 = a0[k], p1 = a1[k], q0 = b0[k], q1 = b1[k];
-                    fx_mad(p0, q0, h[0], c[0]);
-                    fx_mad(p0, q1, h[1], c[1]);
-                    fx_mad(p1, q0, h[2], c[2]);
-                    fx_mad(p1, q1, h[3], c[3]);
+                    for (int k = 0; k < w; ++k) {
+                        const int2 p0 = a0[k], p1 = a1[k], q0 = b0[k], q1 = b1[k];
+                        fx_mad(p0, q0, h[0], c[0]);
+                        fx_mad(p0, q1, h[1], c[1]);
+                        fx_mad(p1, q0, h[2], c[2]);
+                        fx_mad(p1, q1, h[3], c[3]);
+                    }
+                    const int e0 = E[i0], e1 = E[i1], f0 = E[j0], f1 = E[j1];
+                    auto take = [&](double &v, int n, int e) {
+                        v = e >= FX_NAN / 2 ? nan("") : fx_add(v, -fx_total(h[n], c[n]), e);
+                    };
+                    take(v00, 0, e0 + f0);
+                    take(v01, 1, e0 + f1);
+                    take(v10, 2, e1 + f0);
+                    take(v11, 3, e1 + f1);
+                } else {
+                    const double *a0 = P + i0 * ps, *a1 = P + i1 * ps, *b0 = P + j0 * ps, *b1 = P + j1 * ps;
+#pragma unroll 4
+                    for (int k = 0; k < w; ++k) {
+                        const double p0 = -a0[k], p1 = -a1[k], q0 = b0[k], q1 = b1[k];
+                        v00 = fma(p0, q0, v00);
+                        v01 = fma(p0, q1, v01);
+                        v10 = fma(p1, q0, v10);
+                        v11 = fma(p1, q1, v11);
+                    }
                 }
-                const int f0 = E[j0], f1 = E[j1];
-                auto put = [&](double *at, double v, int n, int e) {
-                    *at = e >= FX_NAN / 2 ? nan("") : fx_add(v, -fx_total(h[n], c[n]), e);
-                };
-                put(s0 + j0, v00, 0, e0 + f0);
-                if (j1 > j0 && j1 <= i0) put(s0 + j1, v01, 1, e0 + f1);
+                s0[j0] = v00;
+                if (j1 > j0 && j1 <= i0) s0[j1] = v01;
                 if (i1 > i0) {
-                    put(s1 + j0, v10, 2, e1 + f0);
-                    if (j1 > j0) put(s1 + j1, v11, 3, e1 + f1);
+                    s1[j0] = v10;
+                    if (j1 > j0) s1[j1] = v11;
                 }
             }
         }
@@ -581,7 +603,7 @@ __device__ int stage_cholesky_solve(double *S, int N, double *rhs, double *x, do
         for (int i = tid; i < k0; i += nt) {
             double s = P[i];
 #pragma unroll 4
-            for (int k = 0; k < w; ++k) s = fma(-S[(size_t)(k0 + k) * N + i], xb[k], s);
+            for (int k = w - 1; k >= 0; --k) s = fma(-S[(size_t)(k0 + k) * N + i], xb[k], s);
             P[i] = s;
         }
         __syncthreads();
@@ -1275,7 +1297,7 @@ __device__ void solve_problem(const BatchProblem &p, const Arenas<R> &ar, const 
             }
             __syncthreads();
             double *S = ar.d + p.d_S, *rhs = ar.d + p.d_rhs, *x = ar.d + p.d_x;
-            const int st = stage_cholesky_solve(S, N, rhs, x, sh, dyn);
+            const int st = stage_cholesky_solve<!MX>(S, N, rhs, x, sh, dyn);
             if (threadIdx.x == 0) shi[4]++;
             int decided = 0;  // 0: retry with larger mu, 1: accepted, 2: stop
             if (st == 0) {
