@@ -3,7 +3,7 @@
 // S (Np x Np, lower triangle, Np a multiple of TILE) is factored S = L L^T
 // by one cooperative persistent kernel over TILE x TILE lower tiles.  CTA 0
 // (the panel) walks the diagonal: it applies the last update to each
-// diagonal tile, factors it (cta_potrf, with the forward solve of rhs carried
+// diagonal tile, factors it (panel_factor, with the forward solve of rhs carried
 // along) and forms the sub-diagonal tile below it, which it keeps for the
 // next step.  The other CTAs (helpers) accumulate every other update
 // (left-looking) and solve the remaining tiles against the diagonal
@@ -54,8 +54,7 @@ constexpr int CF_THREADS = PSBA_CHOL_THREADS;
 // (psba_set_wait_limit).  Thread 0 of each CTA stores it here at entry.
 __shared__ long long s_spin_limit;
 constexpr int BJ = PSBA_CHOL_BJ;             // update steps staged per batch in a tile task
-static_assert(BJ >= 2, "the diagonal factor reuses two staging tiles");
-
+static_assert(BJ >= 5, "the panel keeps its tiles in the staging area");
 
 __device__ __forceinline__ int ld_acquire(const int *p)
 {
@@ -64,34 +63,51 @@ __device__ __forceinline__ int ld_acquire(const int *p)
     return v;
 }
 
+__device__ __forceinline__ int ld_relaxed(const int *p)
+{
+    int v;
+    asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
 __device__ __forceinline__ void st_release(int *p, int v)
 {
     asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// Thread 0 waits for flag == epoch; the block then proceeds.  Returns false
-// when the budget ran out or another task already reported a timeout.
-__device__ bool block_wait(const int *flag, int epoch, int *status)
+// One thread's wait for flag == epoch.  The polls are relaxed loads (an acquire
+// a poll slows down the SM's other warps' loads) and the last one an acquire;
+// the status word is looked at every 16 polls, so a poll is one L2 round trip.
+// Returns false when the budget ran out or another task already reported a
+// timeout.
+__device__ __forceinline__ bool poll_flag(const int *flag, int epoch, int *status)
 {
-    __shared__ int ok;
-    if (threadIdx.x == 0) {
-        int good = 0;
-        const long long limit = s_spin_limit;
-        for (long long it = 0; it < limit; ++it) {
-            if (ld_acquire(flag) == epoch) {
-                good = 1;
-                break;
-            }
-            if (ld_acquire(status) == 2) break;
-            __nanosleep(64);
-        }
-        if (!good) atomicExch(status, 2);
-        ok = good;
+    const long long limit = s_spin_limit;
+    for (long long it = 0; it < limit; ++it) {
+        if (ld_relaxed(flag) == epoch && ld_acquire(flag) == epoch) return true;
+        if ((it & 15) == 15 && ld_relaxed(status) == 2) break;
+        __nanosleep(20);
     }
+    atomicExch(status, 2);
+    return false;
+}
+
+// Threads 0 and 32 wait for a flag each (fb may be null); the block then proceeds.
+__device__ void block_wait(const int *fa, const int *fb, int epoch, int *status)
+{
+    if (threadIdx.x == 0) poll_flag(fa, epoch, status);
+    if (threadIdx.x == 32 && fb != nullptr) poll_flag(fb, epoch, status);
     __syncthreads();
-    const bool r = ok != 0;
-    __syncthreads();
-    return r;
+}
+
+// A warp's own wait: its lanes' loads come after lane 0's acquire.
+__device__ __forceinline__ bool warp_wait(const int *flag, int epoch, int *status)
+{
+    int ok = 0;
+    if ((threadIdx.x & 31) == 0) ok = poll_flag(flag, epoch, status);
+    ok = __shfl_sync(0xffffffffu, ok, 0);
+    __syncwarp();
+    return ok != 0;
 }
 
 __device__ __forceinline__ int tile_task(int I, int K, int nb)
@@ -108,341 +124,219 @@ __device__ __forceinline__ void load_tile(double (*dst)[T + 1], const double *S,
 }
 
 // ---------------------------------------------------------------------------
-// Diagonal-tile factor.  GB300 issues one FP64 warp instruction per ~64
-// cycles however many lanes are active, and an FP64 result is ready ~64
-// cycles after issue, so the factor of a 16 x 16 tile is bound by its chain
-// of dependent pivots (d_s, then 1/sqrt(d_s)) and by how much latency the
-// rest adds per column.  The plan below keeps everything but the pivot chain
-// off warp 0 and gives every other thread a fixed, index-free role, in
-// T + 1 phases separated by one barrier each (named barrier 1, the seven warps
-// with a role):
-//   warp 0    phase s: d_s = a[s][s] - (a[s][s-1] / L_{s-1,s-1})^2 (the last
-//             update of the pivot, one column ahead of the others), 1/L_ss
-//             and 1/d_s.
-//   trailing  (warps 2, 3, 6, 7) own the entries a[r][j], 1 <= j <= r, and
-//             b[r] (as column T) in registers.  Phase s applies column s-1:
-//             a[r][j] -= a[r][s-1] a[j][s-1] / d_{s-1}; an entry is published
-//             to shared memory in the phase it becomes final, and its L
-//             value (a[r][j] / L_jj, y_r = b_r / L_rr) written in the next.
-//   inverse   (warps 1, 5) build X = L^-1 one column behind L: entry (i, c)
-//             takes X[i][c] -= L[i][k] X[k][c] in phase k + 2, c <= k < i,
-//             and X[i][c] /= L_ii in its last phase; entries are dealt to
-//             threads by interval colouring, so a thread has one at a time.
-//   warp 4    shares warp 0's sub-partition and takes no part in the phases
-//             (the panel gives it the step's stores and fetches).
-// Each role runs the same short instruction sequence in every lane (operands
-// picked by selects), so a trailing warp issues two FP64 instructions per
-// phase.  The roles run alongside the chain but still slow it (the chain
-// alone: ~710 cycles per column; all roles: ~840); this placement of the
-// roles and the published 1/d_s measured 7% faster than trailing on warps
-// 1, 2, 3, 5 computing 1/d_s themselves.  The plan is built at compile time
-// and copied to shared memory once per launch (divergent reads of constant
-// memory serialise).
+// Diagonal-tile factor and inverse.  An FP64 result is ready ~64 cycles after
+// issue, so the time of a 16 x 16 tile is the number of dependent FP64 steps of
+// its columns, and what stands between them.  A Gauss-Jordan elimination without
+// division has two per column: with the pivot p_s, every entry (r, c) of a row
+// r > s takes
+//     q <- p_s q - a_rs o,   o = a_cs for c > s, x_sc for c < s,
+// where a is what is left of the tile and x, in the places of the columns
+// already eliminated, the rows of its unit factor's inverse (x_rs starts as
+// -a_rs).  Row r of a carries the factor sigma_r = p_0 ... p_(r-1), x_rc the
+// factor sigma_r / sigma_c, and at the end
+//     L_rc = a_rc t_c,  (L^-1)_rc = x_rc sigma_c t_r,  t_c = 1 / sqrt(p_c sigma_c).
+// The only square roots are the 16 of t, all at once.
+// Range: rows and columns are first scaled by 2^-H_r, H_r = floor(log2(a_rr) / 2) of
+// the tile before its last update, which puts the diagonal below 4, and every
+// four columns all entries are scaled by the power of two that brings sigma
+// back to one.  In between sigma grows to 2^30 at most, and shrinks by pivots
+// (in scaled units, of four columns) p q r ... to p^7 q^3 r: it takes four in
+// a row below 2^-60, far under the rounding errors of the tile, to
+// underflow, and the tile is then refused.
+//
+// Roles: warps 0-3 hold one entry of rows 4-15 a thread (and one sigma), warp 4
+// those of rows 0-3, whose columns end early; they meet once a column.  Column
+// s of all is in q[s]: a_is for i >= s, x_si for i < s, so that in the end
+// everything is there.  Warps 5 and 6 take b's update and y, warp 7 the step's
+// fetches.
+// Cycles a tile (N = 528): 1,800 for the last update (at the SM's FP64 rate: one
+// warp instruction per ~19 cycles), 3,950 for 15 columns (263 each, of which
+// the two FP64 steps ~150, the shared-memory round and the barrier ~90), 770 for
+// the roots, 600 for the outputs: 7,100, where an LDL^T elimination with a reciprocal a column
+// and the inverse behind it took 15,000.  What a column does not need is kept
+// out of it: a branch costs ~30 cycles, a sign flip or a comparison in FP64 60.
 
-enum : unsigned char { PF_NONE = 0, PF_OFF, PF_DIAG, PF_D11, PF_B, PF_COL0, PF_B0 };
-constexpr int PF_TRAIL = 128, PF_INV = 64, PF_INV_MAX = 16;
-constexpr int PF_BCOL = T;  // b rides along as column T
+// Beside the 16 entries, q[s] has sigma_s, a zero (sigma's a) and a place for the
+// stores of threads that have nothing to publish: a store under a condition
+// on row and column cost 170 cycles a column in branches.
+constexpr int PF_SIGMA = T, PF_ZERO = T + 1, PF_NONE = T + 2, PF_ROW = T + 3;
+struct PfWork {
+    double (*q)[PF_ROW];  // (q[s][PF_ZERO] = 0 set by the caller)
+    double *t;
+};
 
+// The entry of a thread of warps 0-4: row r, column c (row 0 takes no step).
+// Warp 4 has three lanes an entry for the update; the first goes on with it.
 struct PfEntry {
-    unsigned char kind, r, j;
+    int r, c;
+    bool own;
 };
-struct PfPlan {
-    PfEntry tr[PF_TRAIL][2];
-    unsigned char inv_i[PF_INV][PF_INV_MAX], inv_c[PF_INV][PF_INV_MAX], inv_n[PF_INV];
-};
-
-// last phase in which an entry does work (update, publication or L value)
-__host__ __device__ constexpr int pf_last_busy(const PfEntry &e)
+__device__ __forceinline__ PfEntry pf_entry()
 {
-    return e.kind == PF_OFF ? e.j + 1 : e.kind == PF_DIAG ? e.j + 1 : e.kind == PF_D11 ? 2 : e.kind == PF_B ? e.r + 1 : 1;
+    const int tid = threadIdx.x, lane = tid & 31;
+    PfEntry e{tid < 128 ? 4 : 0, tid < 128 ? tid : lane % 10, tid < 128 ? tid < 126 : lane < 10};
+    for (; e.c > e.r; ++e.r) e.c -= e.r + 1;
+    if (e.r >= T || tid >= 160) e.r = e.c = 0;
+    return e;
 }
 
-constexpr PfPlan make_pf_plan()
+// Named barriers.  The instructions count whole warps, so the warp's lanes come
+// together first (roles split warps here, and a warp that arrives in two
+// parts would be counted twice).
+template <int ID, int N>
+__device__ __forceinline__ void pf_bar()
 {
-    PfPlan p{};
-    PfEntry ents[T * (T + 1) / 2 + T + 1] = {};
-    int n = 0;
-    for (int j = 1; j < T; ++j)
-        for (int r = j + 1; r < T; ++r) ents[n++] = PfEntry{PF_OFF, (unsigned char)r, (unsigned char)j};
-    for (int j = 2; j < T; ++j) ents[n++] = PfEntry{PF_DIAG, (unsigned char)j, (unsigned char)j};
-    ents[n++] = PfEntry{PF_D11, 1, 1};
-    for (int r = 1; r < T; ++r) ents[n++] = PfEntry{PF_B, (unsigned char)r, (unsigned char)PF_BCOL};
-    for (int r = 0; r < T; ++r) ents[n++] = PfEntry{PF_COL0, (unsigned char)r, 0};
-    ents[n++] = PfEntry{PF_B0, 0, (unsigned char)PF_BCOL};
-    // stable sort by last busy phase, latest first
-    for (int a = 1; a < n; ++a) {
-        const PfEntry v = ents[a];
-        int b = a;
-        while (b > 0 && pf_last_busy(ents[b - 1]) < pf_last_busy(v)) {
-            ents[b] = ents[b - 1];
-            --b;
+    __syncwarp();
+    asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(N) : "memory");
+}
+template <int ID, int N>
+__device__ __forceinline__ void pf_arrive()
+{
+    __syncwarp();
+    asm volatile("bar.arrive %0, %1;" ::"n"(ID), "n"(N) : "memory");
+}
+
+// x 2^n by the exponent field: what would be subnormal is zero, what would
+// overflow infinite; infinities and NaN stay
+__device__ __forceinline__ double pf_ldexp(double x, int n)
+{
+    const int h = __double2hiint(x), e = (h >> 20) & 0x7ff, ne = e + n;
+    if (e == 0x7ff) return x;
+    if (e == 0 || ne <= 0) return 0.0;
+    if (ne >= 0x7ff) return __hiloint2double((h & 0x80000000) | 0x7ff00000, 0);
+    return __hiloint2double(h + (n << 20), __double2loint(x));
+}
+
+// The tile's scale H, by one warp
+__device__ __forceinline__ void tile_exp(const double (*a)[T + 1], int *H)
+{
+    const int l = threadIdx.x & (T - 1);
+    H[l] = (((__double2hiint(a[l][l]) >> 20) & 0x7ff) - 1023) >> 1;
+}
+
+// The same without a branch, and n in the exponent field's place
+__device__ __forceinline__ double pf_shift(double x, int n)
+{
+    const int h = __double2hiint(x);
+    const unsigned e = h & 0x7ff00000, ne = e + (unsigned)n;
+    const bool in = ne - 1 < 0x7fefffffu && e != 0x7ff00000u, nan = e == 0x7ff00000u;
+    const int edge = nan ? h : n > 0 && e != 0 ? (h & (int)0x80000000) | 0x7ff00000 : 0;
+    return __hiloint2double(in && e != 0 ? h + n : edge, (in && e != 0) || nan ? __double2loint(x) : 0);
+}
+
+// Warps 0-6 (224 threads): the last update of the diagonal tile a and of b with
+// the previous step's sub-diagonal tile lsub and y (first: none), then the
+// tile's Cholesky factor, to Lg (rows of Np), and its inverse, to X and Ig
+// (lower triangles only).  True in warp 4 when a pivot was not a positive
+// normal number.
+__device__ __forceinline__ bool panel_factor(const double (*a)[T + 1], const int *H, const double (*lsub)[T + 1], double *b, const double *y,
+                             bool first, double (*X)[T + 1], double *Lg, int Np, double *Ig, const PfWork &w, const PfEntry &e)
+{
+    static_assert(CF_THREADS == 256 && T == 16, "the factor is laid out for eight warps and 16 x 16 tiles");
+    constexpr int NE = 160, NT = CF_THREADS - 32;  // threads of warps 0-4 and of warps 0-6
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (warp >= 5) {
+        // b, four lanes a row, when the columns leave the FP64 units room for it
+        pf_bar<4, NT>();
+        if (!first) {
+            const int r = (tid - NE) >> 2, k0 = tid & 3;
+            double v = 0.0;
+#pragma unroll
+            for (int k = 0; k < T; k += 4) v = fma(lsub[r][k0 + k], y[k0 + k], v);
+            v += __shfl_xor_sync(0xffffffffu, v, 1);
+            v += __shfl_xor_sync(0xffffffffu, v, 2);
+            if (k0 == 0) b[r] -= v;
         }
-        ents[b] = v;
+        pf_bar<1, NT>();
+        return false;
     }
-    for (int u = 0; u < PF_TRAIL; ++u) {
-        p.tr[u][0] = ents[u];
-        p.tr[u][1] = PfEntry{PF_NONE, 0, 0};
-    }
-    for (int q = PF_TRAIL; q < n; ++q) p.tr[q - PF_TRAIL][1] = ents[q];
-    // inverse entries (i, c), i > c, busy in phases [c + 2, i + 1]: generated
-    // by start, each goes to the first thread whose previous entry has ended
-    for (int v = 0; v < PF_INV; ++v) p.inv_n[v] = 0;
-    for (int c = 0; c < T; ++c)
-        for (int i = c + 1; i < T; ++i)
-            for (int v = 0; v < PF_INV; ++v) {
-                const int m = p.inv_n[v];
-                if (m < PF_INV_MAX && (m == 0 || p.inv_i[v][m - 1] + 1 < c + 2)) {
-                    p.inv_i[v][m] = (unsigned char)i;
-                    p.inv_c[v][m] = (unsigned char)c;
-                    p.inv_n[v] = (unsigned char)(m + 1);
-                    break;
-                }
-            }
-    return p;
-}
-
-constexpr PfPlan kPfPlan = make_pf_plan();
-
-constexpr bool pf_plan_ok()
-{
-    // second entries are only busy in phases 1-2; every inverse entry placed
-    int placed = 0;
-    for (int u = 0; u < PF_TRAIL; ++u)
-        if (kPfPlan.tr[u][1].kind != PF_NONE && pf_last_busy(kPfPlan.tr[u][1]) > 2) return false;
-    for (int v = 0; v < PF_INV; ++v) placed += kPfPlan.inv_n[v];
-    return placed == T * (T - 1) / 2;
-}
-static_assert(pf_plan_ok(), "diagonal-tile factor plan");
-
-__constant__ PfPlan c_pf = kPfPlan;
-
-// the factor plan into shared memory (once per launch)
-__device__ void load_pf_plan(PfPlan &dst)
-{
-    const unsigned char *src = reinterpret_cast<const unsigned char *>(&c_pf);
-    unsigned char *d = reinterpret_cast<unsigned char *>(&dst);
-    for (int i = threadIdx.x; i < (int)sizeof(PfPlan); i += blockDim.x) d[i] = src[i];
-    __syncthreads();
-}
-
-// The factor's workspace: one shared block of doubles, so that every access
-// is an offset from one base (fixed per entry, plus a phase constant once
-// the phase loop is unrolled).
-constexpr int PW_ROW = T + 1;            // padded row
-constexpr int PW_A = 0;                  // the tile (published entries, pivots)
-constexpr int PW_L = T * PW_ROW;         // the factor L
-constexpr int PW_LINV = 2 * T * PW_ROW;  // its inverse
-constexpr int PW_BW = 3 * T * PW_ROW;    // b being reduced
-constexpr int PW_INVD = PW_BW + T;       // 1 / L_kk = d_k^-1/2 (final pass)
-constexpr int PW_Y = PW_BW + 2 * T;      // y = L^-1 b
-constexpr int PW_B = PW_BW + 3 * T;      // b (input)
-constexpr int PW_INV2 = PW_BW + 4 * T;   // 1 / d_k (warp 0 publishes it)
-constexpr int PW_ASQ = PW_BW + 5 * T;    // a_k,k-1^2 (published with a_k,k-1)
-constexpr int PW_SIZE = PW_BW + 6 * T;
-
-// One entry of a trailing thread, decoded once per factor into offsets: the
-// entry's row (xo), the other operand of its update (oo: row j of the tile,
-// or b), the source of its L value when that is not the entry itself (lo),
-// the pivot inverse it divides by (qo), where it is published (po) and where
-// its L value goes (dofs), its last update phase (0: none) and the phase its
-// L value is due.
-struct PfSlot {
-    int xo, oo, lo, qo, po, dofs, last, due;
-    bool lself;
-    int sqo;  // entry (j + 1, j): where its square goes when final, else -1
-};
-
-__device__ __forceinline__ PfSlot pf_slot(const PfEntry &e)
-{
-    const int r = e.r, j = e.j;
-    switch (e.kind) {
-    case PF_OFF:
-        return PfSlot{r * PW_ROW, j * PW_ROW, 0, PW_INV2 + j, r * PW_ROW + j, PW_L + r * PW_ROW + j, j, j + 1, true,
-                      r == j + 1 ? PW_ASQ + r : -1};
-    case PF_DIAG:  // d_j is left in a[j][j] by warp 0; its M value (1) is not read
-        return PfSlot{j * PW_ROW, j * PW_ROW, j * PW_ROW + j, PW_INV2 + j, j * PW_ROW + j, PW_L + j * PW_ROW + j, j - 1,
-                      j + 1, false, -1};
-    case PF_D11:
-        return PfSlot{PW_ROW, PW_ROW, PW_ROW + 1, PW_INV2 + 1, 0, PW_L + PW_ROW + 1, 0, 2, false, -1};
-    case PF_B:  // its M value is not read: the final pass forms y from the entry
-        return PfSlot{r * PW_ROW, PW_BW, 0, PW_INV2 + r, PW_BW + r, PW_Y + r, r, r + 1, true, -1};
-    case PF_COL0:
-        return PfSlot{r * PW_ROW, 0, r * PW_ROW, PW_INV2, 0, PW_L + r * PW_ROW, 0, 1, false, -1};
-    case PF_B0:
-        return PfSlot{0, PW_BW, PW_BW, PW_INV2, 0, PW_Y, 0, 1, false, -1};
-    default:
-        return PfSlot{0, 0, 0, 0, 0, 0, 0, 0, true, -1};
-    }
-}
-
-// Phase s >= 1 of one entry: the update v -= a[r][k] (other[k] / d_k),
-// k = s - 1, or its L value, as two FP64 instructions whatever the entry
-// does (loads unconditional and in bounds, operands picked by selects).
-template <int S>
-__device__ __forceinline__ void pf_step(const PfSlot &q, double &v, double ik2, double *W)
-{
-    constexpr int k = S - 1;
-    const bool upd = S <= q.last, lval = S == q.due;
-    const double xk = W[q.xo + k];
-    const double ok = W[q.oo + k];
-    const double lraw = W[q.lo];
-    const double qi = W[q.qo];
-    const double lv = q.lself ? v : lraw;
-    const double pa = upd ? ok : lval ? lv : 0.0;
-    const double qa = upd ? ik2 : lval ? qi : 0.0;
-    const double t = pa * qa;
-    const double xs = upd ? xk : 0.0;  // a select of the value; the sign rides on the FMA
-    v = fma(-xs, t, v);
-    if (upd && S == q.last) {
-        W[q.po] = v;
-        if (q.sqo >= 0) W[q.sqo] = v * v;
-    }
-    if (lval) W[q.dofs] = t;
-}
-
-// Phase S of the whole CTA (see the plan above).
-// The phases synchronise the seven warps with a role (named barrier 1); warp
-// 4 joins the CTA only at the factor's start and end.
-__device__ __forceinline__ void pf_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(CF_THREADS - 32) : "memory"); }
-
-template <int S>
-__device__ __forceinline__ void pf_phase(double *W, int warp, int u, int vi, int wlast, const PfPlan &pf,
-                                         const PfSlot &q0, const PfSlot &q1, double &v0, double &v1,
-                                         double &inv_prev, double &w, int &wi, int n_inv, int &ci, int &cc)
-{
-    if (warp == 0) {
-        // the last phase has no pivot: 1 / sqrt(d_j) for the final pass
-        if (S == T && threadIdx.x < T) W[PW_INVD + threadIdx.x] = rsqrt(W[PW_A + threadIdx.x * PW_ROW + threadIdx.x]);
-        // the pivot chain: d_S = a_SS - a_S,S-1^2 / d_S-1 and 1 / d_S, no root
-        if (S < T && threadIdx.x == 0) {
-            double d = W[PW_A + S * PW_ROW + S];
-            if (S > 0) {
-                double asq;
-                if (S == 1) {
-                    const double a = W[PW_A + PW_ROW];
-                    asq = a * a;
-                } else {
-                    asq = W[PW_ASQ + S];
-                }
-                d = fma(-asq, inv_prev, d);
-                W[PW_A + S * PW_ROW + S] = d;
-            }
-            inv_prev = rcp_fast(d);
-            W[PW_INV2 + S] = inv_prev;
-        }
-    } else if (u >= 0) {
-        // a trailing warp whose entries are all done skips the phase (its
-        // FP64 instructions would hold up the pipe that the chain shares)
-        if (S >= 1 && S <= wlast) {
-            const double ik2 = W[PW_INV2 + (S >= 1 ? S - 1 : 0)];
-            pf_step<S>(q0, v0, ik2, W);
-            if (S <= 2) pf_step<S>(q1, v1, ik2, W);
-        }
-    } else if (vi >= 0) {
-        if (S >= 2) {
-            constexpr int k = S >= 2 ? S - 2 : 0;
-            if (S > ci + 1 && wi + 1 < n_inv) {  // entries are disjoint in time: at most one step
-                ++wi;
-                ci = pf.inv_i[vi][wi];
-                cc = pf.inv_c[vi][wi];
-                w = 0.0;
-            }
-            if (S >= cc + 2 && S <= ci + 1) {
-                w = fma(-W[PW_L + ci * PW_ROW + k], W[PW_LINV + k * PW_ROW + cc], w);
-                if (S == ci + 1) W[PW_LINV + ci * PW_ROW + cc] = w;
-            }
-        }
-    }
-    pf_barrier();
-}
-
-template <int S>
-__device__ __forceinline__ void pf_phases(double *W, int warp, int u, int vi, int wlast, const PfPlan &pf,
-                                          const PfSlot &q0, const PfSlot &q1, double &v0, double &v1,
-                                          double &inv_prev, double &w, int &wi, int n_inv, int &ci, int &cc)
-{
-    if constexpr (S <= T) {
-        pf_phase<S>(W, warp, u, vi, wlast, pf, q0, q1, v0, v1, inv_prev, w, wi, n_inv, ci, cc);
-        pf_phases<S + 1>(W, warp, u, vi, wlast, pf, q0, q1, v0, v1, inv_prev, w, wi, n_inv, ci, cc);
-    }
-}
-
-// All threads (CF_THREADS == 256): Cholesky of the lower triangle of the
-// tile W[PW_A..] into the lower triangle of W[PW_L..], its inverse into the
-// lower triangle of W[PW_LINV..] (the upper triangles are left as they were:
-// nothing reads them), 1 / L_kk into W[PW_INVD..] and y = L^-1 b (b in
-// W[PW_B..]) into W[PW_Y..], following the plan pf (in shared memory).
-// Returns false on a non-positive or non-finite pivot (checked once at the
-// end: a bad pivot only produces non-finite values downstream).
-// warp 4's work during the factor: none
-struct NoSide {
-    __device__ __forceinline__ void run(const int *) {}
-};
-
-template <typename Side = NoSide>
-__device__ bool cta_potrf(double *W, const PfPlan &pf, Side &&side = Side())
-{
-    static_assert(CF_THREADS == 256, "the factor plan is laid out for eight warps");
-    __shared__ int bad, fdone;
-    const int tid = threadIdx.x, warp = tid >> 5;
-    if (tid < T) W[PW_BW + tid] = W[PW_B + tid];
-    if (tid == 0) {
-        bad = 0;
-        fdone = 0;
-    }
-    const int u = (warp == 2 || warp == 3) ? tid - 64 : (warp == 6 || warp == 7) ? tid - 128 : -1;
-    const int vi = warp == 1 ? tid - 32 : warp == 5 ? tid - 128 : -1;
-    PfSlot q0 = pf_slot(PfEntry{PF_NONE, 0, 0}), q1 = q0;
-    double v0 = 0.0, v1 = 0.0;
-    int wlast = 0;  // a trailing warp's last busy phase
-    if (u >= 0) {
-        const PfEntry e0 = pf.tr[u][0], e1 = pf.tr[u][1];
-        q0 = pf_slot(e0);
-        q1 = pf_slot(e1);
-        v0 = W[e0.j == PF_BCOL ? PW_B + e0.r : PW_A + e0.r * PW_ROW + e0.j];
-        v1 = W[e1.j == PF_BCOL ? PW_B + e1.r : PW_A + e1.r * PW_ROW + e1.j];
-        const int busy = e0.kind == PF_NONE ? 0 : pf_last_busy(e0);
-        wlast = __reduce_max_sync(0xffffffffu, max(busy, e1.kind == PF_NONE ? 0 : pf_last_busy(e1)));
-    }
-    // inverse threads: the current entry (ci, cc) in registers, the list read
-    // only when an entry is done
-    const int n_inv = vi >= 0 ? pf.inv_n[vi] : 0;
-    int wi = 0, ci = -2, cc = T;
-    if (n_inv > 0) {
-        ci = pf.inv_i[vi][0];
-        cc = pf.inv_c[vi][0];
-    }
-    __syncthreads();
-    double inv_prev = 0.0, w = 0.0;
-    if (warp == 4) {
-        side.run(&fdone);
+    int r = e.r, c = e.c;
+    const bool own = e.own, sig = tid == 127;
+    double q;
+    if (warp < 4) {
+        q = a[r][c];
+        if (!first)
+#pragma unroll
+            for (int k = 0; k < T; ++k) q = fma(-lsub[r][k], lsub[c][k], q);
     } else {
-        // after the CTA barrier above: until then the panel's side warp may
-        // still be storing the previous tile's inverse from this workspace
-        if (tid < T) W[PW_LINV + tid * PW_ROW + tid] = 1.0;  // M^-1 has a unit diagonal
-        pf_phases<0>(W, warp, u, vi, wlast, pf, q0, q1, v0, v1, inv_prev, w, wi, n_inv, ci, cc);
-        // the phases leave the pivots d_j on the diagonal, the final entries
-        // a_rj below it, M = a_rj / d_j in W[PW_L..], M^-1 in W[PW_LINV..]
-        // and 1 / sqrt(d_j) in W[PW_INVD..]; with D^1/2 = diag(sqrt(d_j)):
-        // L = a D^-1/2, L^-1 = D^-1/2 M^-1, y = D^-1/2 z
-        static_assert(T == 16, "entry (r, j) = (e >> 4, e & 15)");
-        const int rt = tid < 128 ? tid : tid - 32;  // 0 .. 223 over the seven warps with a role
-        for (int e = rt; e < T * T; e += CF_THREADS - 32) {
-            const int r = e >> 4, j = e & (T - 1);
-            if (j <= r) {
-                W[PW_L + r * PW_ROW + j] = W[PW_A + r * PW_ROW + j] * W[PW_INVD + j];
-                W[PW_LINV + r * PW_ROW + j] *= W[PW_INVD + r];
+        const int k0 = lane / 10;  // three lanes an entry
+        double v = 0.0;
+        if (!first && lane < 30)
+#pragma unroll
+            for (int k = 0; k < T; k += 3)
+                if (k0 + k < T) v = fma(lsub[r][k0 + k], lsub[c][k0 + k], v);
+        const double v1 = __shfl_down_sync(0xffffffffu, v, 10), v2 = __shfl_down_sync(0xffffffffu, v, 20);
+        q = a[r][c] - (v + (v1 + v2));
+        if (!own) r = c = 0;
+    }
+    q = pf_shift(q, -(H[r] + H[c]) * (1 << 20));
+    if (sig) {
+        c = PF_SIGMA;
+        q = 1.0;
+    }
+    const int ra = sig ? PF_ZERO : r, to = sig ? PF_SIGMA : PF_NONE;
+    w.q[0][own && c == 0 ? r : to] = q;
+    const int steps = warp == 0 ? 8 : warp == 1 ? 11 : warp == 2 ? 14 : warp == 3 ? 15 : 3;  // the warp's last row
+    pf_bar<2, NE>();
+    const double *qs = w.q[0];
+    double *qn = w.q[1];
+#pragma unroll
+    for (int g = -1; g < T - 1; g += 4) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int s = g + j;
+            if (s < 0) continue;
+            if (s < steps) {
+                // (past its row's steps a thread goes on with values that nobody reads)
+                const double p = qs[s], ar = qs[ra];
+                const double f = fma(p, q, -(ar * qs[c]));  // (the smaller product is the rounded one)
+                // a sign flip in FP64 arithmetic would be one more dependent step
+                q = c == s ? __hiloint2double(__double2hiint(ar) ^ (int)0x80000000, __double2loint(ar)) : f;
+                if (j == 3) {
+                    const int e = (__double2hiint(p) & 0x7ff00000) + (__double2hiint(qs[PF_SIGMA]) & 0x7ff00000);
+                    q = pf_shift(q, (2046 << 20) - e);
+                }
+                qn[c == s + 1 ? r : r == s + 1 ? c : to] = q;
             }
-            if (e < T) W[PW_Y + e] = W[PW_BW + e] * W[PW_INVD + e];
+            qs += PF_ROW;
+            qn += PF_ROW;
+            pf_bar<2, NE>();
         }
-        if (tid == 0) *(volatile int *)&fdone = 1;
+        if (g == 7) pf_arrive<4, NT>();
     }
-    if (tid < T) {
-        const double d = W[PW_A + tid * PW_ROW + tid];
-        if (!(d >= DBL_MIN) || !isfinite(d)) bad = 1;  // the reciprocal flushes subnormals
+    // t; meanwhile the others' factors of it
+    const int l = lane & (T - 1);
+    const double p = w.q[l][l], sg = w.q[l][PF_SIGMA], d = p * sg;
+    if (warp == 4) w.t[l] = rsqrt(d);
+    if (sig) c = 0;
+    const double lr = pf_shift(w.q[c][r], H[r] * (1 << 20)), sc = w.q[c][PF_SIGMA];
+    const double x = pf_shift(r == c ? sc : w.q[r][c] * sc, -H[c] * (1 << 20));
+    pf_bar<2, NE>();
+    if (own) {
+        const double xr = x * w.t[r];
+        X[r][c] = xr;
+        Ig[r * T + c] = xr;
+        Lg[(size_t)r * Np + c] = lr * w.t[c];
     }
-    __syncthreads();
-    return bad == 0;
+    pf_bar<1, NT>();
+    // the pivot itself is p 2^2H / sigma
+    return warp == 4 && __any_sync(0xffffffffu, !(p > 0.0 && d >= DBL_MIN && pf_ldexp(p, 2 * H[l]) >= DBL_MIN * sg &&
+                                                  d <= DBL_MAX));
+}
+
+// y = L^-1 b by warps 5 and 6, four lanes a row
+__device__ __forceinline__ void panel_y(const double (*X)[T + 1], const double *b, double *y, double *yg)
+{
+    const int r = ((int)threadIdx.x - 160) >> 2, k0 = threadIdx.x & 3;
+    double v = 0.0;
+#pragma unroll
+    for (int k = 0; k < T; k += 4) v = fma(k0 + k <= r ? X[r][k0 + k] : 0.0, b[k0 + k], v);
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    if (k0 == 0) {
+        y[r] = v;
+        yg[r] = v;
+    }
 }
 
 // The single-CTA back solve over the factor (S lower = L, Linv = diagonal
@@ -571,8 +465,9 @@ __device__ __forceinline__ void tri_of(int e, int &r, int &c)
     c = e - r * (r + 1) / 2;
 }
 
-template <bool WITH_B, int NT = CF_THREADS>
+template <bool WITH_B>
 struct LowerUpdate {
+    static constexpr int NT = CF_THREADS;
     static constexpr int NTRI = T * (T + 1) / 2;
     static constexpr int NE = NTRI + (WITH_B ? T : 0);
     static constexpr int PER = (NE * T + NT - 1) / NT;
@@ -580,19 +475,14 @@ struct LowerUpdate {
     static constexpr int PART = NACC * NT;                  // doubles of partial sums
 };
 
-// NT == CF_THREADS: the whole CTA, CTA barriers.  NT == CF_THREADS - 32: every
-// warp but warp 4 (the panel's), on named barrier 1.
-template <bool WITH_B, int NT = CF_THREADS>
+template <bool WITH_B>
 __device__ void update_lower(double (*a)[T + 1], const double (*L)[T + 1], double *b, const double *y, double *part)
 {
-    static_assert(NT == CF_THREADS || NT == CF_THREADS - 32, "whole CTA or all warps but warp 4");
-    using U = LowerUpdate<WITH_B, NT>;
+    constexpr int NT = CF_THREADS;
+    using U = LowerUpdate<WITH_B>;
     constexpr int NTRI = U::NTRI, NE = U::NE, PER = U::PER, NACC = U::NACC;
-    auto sync = [] {
-        if (NT == CF_THREADS) __syncthreads();
-        else asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
-    };
-    const int tid = NT == CF_THREADS ? (int)threadIdx.x : (int)threadIdx.x - ((int)threadIdx.x >= 160 ? 32 : 0);
+    auto sync = [] { __syncthreads(); };
+    const int tid = threadIdx.x;
     const int f0 = tid * PER, e0 = f0 / T;
     const double *xs[NACC], *ys[NACC];
     double p[NACC];
@@ -642,75 +532,38 @@ __device__ void update_lower(double (*a)[T + 1], const double (*L)[T + 1], doubl
     sync();
 }
 
-// The panel's last update of the diagonal tile and of b, a -= L L^T and
-// b -= L y over the lower triangle, one output per thread (152 outputs, 224
-// threads on named barrier 1): sixteen multiply-adds in two interleaved
-// chains of eight, then one subtraction.  One pass, where update_lower's
-// even deal of the products needs partial sums, a barrier and a second pass.
-__device__ void update_lower_panel(double (*a)[T + 1], const double (*L)[T + 1], double *b, const double *y)
+// A Linv^T with the lower triangle of Linv, out(r, c, v) with v = sum_{k <= c}
+// A[r][k] Linv[c][k]: columns c and T-1-c of a row go to one thread, T + 1
+// products.  Called by the first TT / 2 threads (the products are at one FP64
+// warp instruction per 64 cycles and SM quarter either way, ~1,100 cycles).
+template <typename Out>
+__device__ __forceinline__ void tile_trsm(const double (*A)[T + 1], const double (*Li)[T + 1], Out out)
 {
-    constexpr int NT = CF_THREADS - 32, NTRI = T * (T + 1) / 2, NE = NTRI + T;
-    static_assert(NE <= NT, "one output per thread");
-    const int tid = (int)threadIdx.x - ((int)threadIdx.x >= 160 ? 32 : 0);
-    if (tid < NE) {
-        int r = 0, c = 0;
-        const double *xr, *yr;
-        double *dst;
-        if (tid < NTRI) {
-            tri_of(tid, r, c);
-            xr = L[r];
-            yr = L[c];
-            dst = &a[r][c];
-        } else {
-            xr = L[tid - NTRI];
-            yr = y;
-            dst = b + (tid - NTRI);
-        }
-        double s0 = 0.0, s1 = 0.0;
+    const int r = threadIdx.x / (T / 2), c0 = threadIdx.x % (T / 2), c1 = T - 1 - c0;
+    double x[T + 1], y[T + 1];
+    // the products' factors first, so that the chain waits for no load
 #pragma unroll
-        for (int k = 0; k < T; k += 2) {
-            s0 = fma(xr[k], yr[k], s0);
-            s1 = fma(xr[k + 1], yr[k + 1], s1);
-        }
-        *dst -= s0 + s1;
+    for (int i = 0; i <= T; ++i) {
+        const bool first = i <= c0;
+        const int c = first ? c0 : c1, k = first ? i : i - c0 - 1;
+        x[i] = A[r][k];
+        y[i] = Li[c][k];
     }
-    asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
-}
-
-// out = A Linv^T restricted to the lower triangle of Linv (out[r][c] =
-// sum_{k <= c} A[r][k] Linv[c][k]): columns c and T-1-c of a row go to one
-// thread, T + 1 products each.
-__device__ void tile_trsm(double (*out)[T + 1], const double (*A)[T + 1], const double (*Li)[T + 1])
-{
-    for (int p = threadIdx.x; p < TT / 2; p += CF_THREADS) {
-        const int r = p / (T / 2), c0 = p % (T / 2), c1 = T - 1 - c0;
-        double s0 = 0.0, s1 = 0.0;
+    double s0 = 0.0, s1 = 0.0;
 #pragma unroll
-        for (int i = 0; i < T + 1; ++i) {
-            const bool first = i <= c0;
-            const int c = first ? c0 : c1, k = first ? i : i - c0 - 1;
-            const double v = fma(A[r][k], Li[c][k], first ? s0 : s1);
-            s0 = first ? v : s0;
-            s1 = first ? s1 : v;
-        }
-        out[r][c0] = s0;
-        out[r][c1] = s1;
+    for (int i = 0; i <= T; ++i) {
+        const bool first = i <= c0;
+        const double v = fma(x[i], y[i], first ? s0 : s1);
+        s0 = first ? v : s0;
+        s1 = first ? s1 : v;
     }
+    out(r, c0, s0);
+    out(r, c1, s1);
 }
 
 __device__ __forceinline__ void store_tile(double *S, int Np, int I, int K, const double (*t)[T + 1])
 {
     for (int e = threadIdx.x; e < TT; e += CF_THREADS) S[(size_t)(I * T + e / T) * Np + K * T + e % T] = t[e / T][e % T];
-}
-
-// Thread 0 reads the status word; every thread gets the same answer.
-__device__ bool block_failed(const int *status)
-{
-    __shared__ int f;
-    __syncthreads();
-    if (threadIdx.x == 0) f = ld_acquire(status) != 0;
-    __syncthreads();
-    return f != 0;
 }
 
 // After the CTA barrier, thread 0's release store orders every thread's
@@ -721,57 +574,9 @@ __device__ __forceinline__ void block_release(int *flag, int epoch)
     if (threadIdx.x == 0) st_release(flag, epoch);
 }
 
-// Warp 4 of the panel during a factor (it shares warp 0's sub-partition, has
-// no part in the plan and skips the factor's phase barriers): it raises the
-// flags of the previous step's outputs (stored before that step ended; the
-// release store waits for them here, off the pivot chain), then waits for
-// the flags of the next step's tiles (the sub-diagonal SUB(I) and the
-// diagonal PD(I+1) with its b) and copies those tiles into staging buffers.
-// It stops waiting when the factor is done (*fdone, set by thread 0 after
-// the last phase) or its budget runs out; *done says whether the tiles are
-// there, else the panel loads them itself after the factor.
-struct PanelSide {
-    int *rel0, *rel1;          // flags to raise (null: none)
-    const int *fa, *fb;        // flags the next tiles need (null: none)
-    const double *Smat, *rhs;
-    double (*asub)[T + 1], (*anext)[T + 1];
-    double *bnext;
-    int *done;
-    int epoch, Np, I;
-    bool want;                 // a next step exists
-
-    __device__ void run(const int *fdone)
-    {
-        const int lane = threadIdx.x & 31;
-        if (lane == 0) {
-            if (rel0) st_release(rel0, epoch);
-            if (rel1) st_release(rel1, epoch);
-        }
-        if (!want) return;
-        bool up = false;
-        const long long limit = s_spin_limit;
-        for (long long it = 0; it < limit; ++it) {
-            // every lane acquires the flags itself, so its own loads below are ordered after them
-            up = (fa == nullptr || ld_acquire(fa) == epoch) && (fb == nullptr || ld_acquire(fb) == epoch);
-            if (up || *(const volatile int *)fdone) break;
-            __nanosleep(64);
-        }
-        if (!up) return;
-        for (int e = lane; e < 2 * TT; e += 32) {
-            const int t = e / TT, r = (e % TT) / T, c = e % T;
-            const double v = __ldcg(Smat + (size_t)((I + 1) * T + r) * Np + (I + t) * T + c);
-            if (t == 0) asub[r][c] = v;
-            else anext[r][c] = v;
-        }
-        if (lane < T) bnext[lane] = __ldcg(rhs + (I + 1) * T + lane);
-        __syncwarp();
-        if (lane == 0) *done = 1;
-    }
-};
-
 // Flags: tile (I, K) at tile_task(I, K); that slot is raised for the
-// diagonal tile (I, I) when L_II, its inverse and y_I are stored, and for the
-// sub-diagonal tile (I+1, I) when L_{I+1,I} is stored.  The partial diagonal
+// diagonal tile (I, I) when L_II and its inverse are stored, and for the
+// sub-diagonal tile (I+1, I) when L_{I+1,I} and y_I are stored.  The partial diagonal
 // PD(I) = A_II - sum_{J <= I-2} L_IJ L_IJ^T (with b_I likewise) raises
 // n_fact + I; the partial sub-diagonal SUB(I) = A_{I+1,I} - sum_{J <= I-1}
 // L_{I+1,J} L_IJ^T raises n_fact + nb + I; the second-subdiagonal tile
@@ -780,9 +585,8 @@ struct PanelSide {
 //
 // The factor with the forward solve of rhs carried along.  CTA 0 (the panel)
 // walks the diagonal: step I applies the last update to PD(I) with L_{I,I-1}
-// (its own, kept in shared memory), factors the tile (cta_potrf), forms
-// L_{I+1,I} = SUB(I) Linv_II^T and keeps it, then stores L_II, Linv_II, y_I
-// and L_{I+1,I}.  The other CTAs (helpers) run the task list: the tiles
+// (its own, kept in shared memory), factors the tile and stores L_II and Linv_II
+// (panel_factor), then forms L_{I+1,I} = SUB(I) Linv_II^T, which it keeps, and y_I.  The other CTAs (helpers) run the task list: the tiles
 // (I, K) with I >= K + 2 (left-looking updates, then the triangular solve
 // with Linv_KK), and the PD and SUB accumulations, in the order
 //   P(0), C(0), PD(2), SUB(1), P(1), C(1), PD(3), SUB(2), P(2), ...
@@ -799,111 +603,97 @@ __global__ void __launch_bounds__(CF_THREADS, 1) k_chol_dataflow(int Np, int nb,
                                                               int *__restrict__ flags, int epoch,
                                                               int *__restrict__ status, long long spin_limit)
 {
-    static_assert(BJ >= 6, "the panel keeps six tiles in the staging area");
     static_assert(LowerUpdate<true>::PART <= BJ * T * (T + 1), "update_lower's partial sums fit in the staging area");
     __shared__ double a[T][T + 1], linv[T][T + 1];
     __shared__ double bi[BJ][T][T + 1], bk[BJ][T][T + 1], by[BJ][T];
     __shared__ double bvec[T];
     __shared__ int ready_n;
     const int n_fact = nb * (nb + 1) / 2;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     double *part = &bk[0][0][0];
     if (tid == 0) s_spin_limit = spin_limit;
     __syncthreads();
     if (blockIdx.x == 0) {
-        // ---- panel.  Step I: warp 4 stores step I-1's outputs (L_{I-1,I-1},
-        // its inverse, y_{I-1}, L_{I,I-1}) and raises their flags while the
-        // other warps apply the last update to the diagonal tile; during the
-        // factor warp 4 fetches the tiles of step I+1 (PanelSide); then
-        // L_{I+1,I} is formed.  The panel tracks failure itself (a bad pivot of
-        // its own, a wait that ran out), so it never reads the status word.
-        double(*lsub)[T + 1] = bi[2];  // L_{I,I-1} from the previous step
-        double(*asub)[T + 1] = bi[3];
-        static_assert(LowerUpdate<true>::PART <= 2 * T * (T + 1) && LowerUpdate<true, CF_THREADS - 32>::PART <= 2 * T * (T + 1),
-                      "update_lower's partial sums fit in bk[0..1]");
-        static_assert(2 * T * (T + 1) + PW_SIZE <= BJ * T * (T + 1), "the factor workspace fits after the partial sums");
-        double *W = &bk[2][0][0];  // bk[0..1] hold update_lower's partial sums
-        double(*wa)[T + 1] = reinterpret_cast<double(*)[T + 1]>(W + PW_A);
-        double(*wl)[T + 1] = reinterpret_cast<double(*)[T + 1]>(W + PW_L);
-        double(*wli)[T + 1] = reinterpret_cast<double(*)[T + 1]>(W + PW_LINV);
-        double(*anext)[T + 1] = bi[5];  // the next diagonal tile, fetched during the factor
-        double *bnext = by[0];
-        __shared__ PfPlan s_pf;
-        __shared__ int pf_done;
-        load_pf_plan(s_pf);
-        bool failed = false;
-        const int warp = tid >> 5, lane = tid & 31;
-        load_tile(wa, S, Np, 0, 0);
-        if (tid < T) W[PW_B + tid] = __ldcg(rhs + tid);
+        // ---- panel.  Step I: warps 0-6 update and factor the diagonal tile;
+        // warp 4 raises its flag; warps 0-3 form L_{I+1,I}, warps 5 and 6 y_I, and
+        // warp 7, which raises their flag when the next step begins, fetches
+        // SUB(I) and then PD(I+1) with its b as they come.  The panel tracks failure
+        // itself (a bad pivot, a wait that ran out): it then leaves the loop
+        // and raises all flags that are left.
+        double(*lsub)[T + 1] = bi[2], (*asub)[T + 1] = bi[3], (*wli)[T + 1] = bi[4];
+        double(*pfq)[PF_ROW] = reinterpret_cast<double(*)[PF_ROW]>(&bk[0][0][0]);
+        const PfWork pw{pfq, by[3]};
+        const PfEntry pe = pf_entry();
+        __shared__ int hexp[2][T], stop[2];  // by the step's parity
+        if (tid < 2) stop[tid] = 0;
+        if (tid < T) pfq[tid][PF_ZERO] = 0.0;
+        load_tile(bi[0], S, Np, 0, 0);
+        if (tid < T) by[0][tid] = __ldcg(rhs + tid);
         __syncthreads();
-        for (int I = 0; I < nb; ++I) {
-            const int td = tile_task(I, I, nb);
-            if (I >= 1) {
-                // warp 4 stores step I-1's outputs and raises their flags (its
-                // release waits for the stores, off the pivot chain) while the
-                // other warps apply the last update to the diagonal tile
-                if (warp == 4) {
-                    if (!failed) {
-                        const int Jp = I - 1;
-                        for (int e2 = lane; e2 < TT; e2 += 32) {
-                            const int r = e2 / T, c = e2 % T;
-                            S[(size_t)(Jp * T + r) * Np + Jp * T + c] = wl[r][c];
-                            Linv[(size_t)Jp * TT + e2] = wli[r][c];
-                            S[(size_t)(I * T + r) * Np + Jp * T + c] = lsub[r][c];
-                        }
-                        if (lane < T) rhs[Jp * T + lane] = W[PW_Y + lane];
+        if (warp == 7) tile_exp(bi[0], hexp[0]);
+        __syncthreads();
+        bool failed = false;
+        int I = 0;
+        for (; I < nb && !failed; ++I) {
+            const int cur = I & 1;
+            double *wy = by[2];
+            if (warp == 7) {
+                if (I >= 1 && lane == 0) st_release(flags + tile_task(I, I - 1, nb), epoch);
+                if (I + 1 < nb) {
+                    const double *src = S + (size_t)((I + 1) * T + (lane >> 3)) * Np + I * T + 2 * (lane & 7);
+                    bool ok = I == 0 || warp_wait(flags + n_fact + nb + I, epoch, status);
+                    double2 v[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) v[q] = __ldcg(reinterpret_cast<const double2 *>(src + (size_t)(4 * q) * Np));
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        double *d = &asub[4 * q + (lane >> 3)][2 * (lane & 7)];
+                        d[0] = v[q].x;
+                        d[1] = v[q].y;
+                    }
+                    pf_arrive<3, 160>();
+                    ok = (I == 0 || warp_wait(flags + n_fact + I + 1, epoch, status)) && ok;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) v[q] = __ldcg(reinterpret_cast<const double2 *>(src + (size_t)(4 * q) * Np + T));
+                    if (lane < T) by[cur ^ 1][lane] = __ldcg(rhs + (I + 1) * T + lane);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        double *d = &bi[cur ^ 1][4 * q + (lane >> 3)][2 * (lane & 7)];
+                        d[0] = v[q].x;
+                        d[1] = v[q].y;
                     }
                     __syncwarp();
-                    if (lane == 0) {
-                        st_release(flags + tile_task(I - 1, I - 1, nb), epoch);
-                        st_release(flags + tile_task(I, I - 1, nb), epoch);
-                    }
-                } else if (!failed) {
-                    update_lower_panel(wa, lsub, W + PW_B, W + PW_Y);
-                }
-            }
-            if (tid == 0) pf_done = 0;
-            if (!failed) {
-                PanelSide side{nullptr, nullptr,
-                               I >= 1 ? flags + n_fact + nb + I : nullptr,
-                               I + 1 >= 2 ? flags + n_fact + I + 1 : nullptr,
-                               S, rhs, asub, anext, bnext, &pf_done, epoch, Np, I, I + 1 < nb};
-                const bool good = cta_potrf(W, s_pf, side);
-                if (!good) {
-                    failed = true;
-                    if (tid == 0) atomicCAS(status, 0, 1);
+                    tile_exp(bi[cur ^ 1], hexp[cur ^ 1]);
+                    if (lane == 0 && !ok) stop[cur] = 1;
                 }
             } else {
-                __syncthreads();
-            }
-            if (I + 1 < nb) {
-                // the tile and b are free after the factor: the next diagonal tile goes there
-                if (pf_done) {
-                    for (int e2 = tid; e2 < TT; e2 += CF_THREADS) wa[e2 / T][e2 % T] = anext[e2 / T][e2 % T];
-                    if (tid < T) W[PW_B + tid] = bnext[tid];
-                } else {
-                    if (I >= 1 && !block_wait(flags + n_fact + nb + I, epoch, status)) failed = true;
-                    if (I + 1 >= 2 && !block_wait(flags + n_fact + I + 1, epoch, status)) failed = true;
-                    for (int e2 = tid; e2 < TT; e2 += CF_THREADS) {
-                        const int r = e2 / T, c = e2 % T;
-                        asub[r][c] = __ldcg(S + (size_t)((I + 1) * T + r) * Np + I * T + c);
-                        wa[r][c] = __ldcg(S + (size_t)((I + 1) * T + r) * Np + (I + 1) * T + c);
+                const bool bad = panel_factor(bi[cur], hexp[cur], lsub, by[cur], wy, I == 0, wli,
+                                              S + (size_t)(I * T) * Np + I * T, Np, Linv + (size_t)I * TT, pw, pe);
+                if (warp == 4 && lane == 0) {
+                    if (bad) {
+                        atomicCAS(status, 0, 1);
+                        stop[cur] = 1;
                     }
-                    if (tid < T) W[PW_B + tid] = __ldcg(rhs + (I + 1) * T + tid);
+                    st_release(flags + tile_task(I, I, nb), epoch);
                 }
-                __syncthreads();
-                if (!failed) tile_trsm(lsub, asub, wli);
-                __syncthreads();
+                if (warp >= 5) panel_y(wli, by[cur], wy, rhs + I * T);
+                if (warp < 4 && I + 1 < nb) {
+                    pf_bar<3, 160>();  // SUB(I) is there
+                    double *Lg = S + (size_t)((I + 1) * T) * Np + I * T;
+                    tile_trsm(asub, wli, [&](int r, int c, double v) {
+                        lsub[r][c] = v;
+                        Lg[(size_t)r * Np + c] = v;
+                    });
+                }
             }
+            __syncthreads();
+            failed = stop[cur] != 0;
         }
-        // the last step's outputs
-        if (!failed) {
-            store_tile(S, Np, nb - 1, nb - 1, wl);
-            for (int e2 = tid; e2 < TT; e2 += CF_THREADS) Linv[(size_t)(nb - 1) * TT + e2] = wli[e2 / T][e2 % T];
-            if (tid < T) rhs[(nb - 1) * T + tid] = W[PW_Y + tid];
-        }
-        __syncthreads();
-        if (tid == 0) st_release(flags + tile_task(nb - 1, nb - 1, nb), epoch);
+        if (tid == 0 && failed)
+            for (int J = I - 1; J < nb; ++J) {
+                st_release(flags + tile_task(J, J, nb), epoch);
+                if (J + 1 < nb) st_release(flags + tile_task(J + 1, J, nb), epoch);
+            }
         return;
     }
     // ---- helpers
@@ -926,15 +716,15 @@ __global__ void __launch_bounds__(CF_THREADS, 1) k_chol_dataflow(int Np, int nb,
             if (tid == 0) ready_n = nmax;
             __syncthreads();
             if (tid < nmax) {
-                const bool ok = ld_acquire(flags + tile_task(I, J + tid, nb)) == epoch &&
-                                (kind == 0 || ld_acquire(flags + tile_task(K, J + tid, nb)) == epoch);
-                if (!ok) atomicMin(&ready_n, tid);
+                // the diagonal's other flag is that of y_J
+                const int fi = ld_acquire(flags + tile_task(I, J + tid, nb));
+                const int fk = ld_acquire(flags + tile_task(kind != 0 ? K : J + tid + 1, J + tid, nb));
+                if (fi != epoch || fk != epoch) atomicMin(&ready_n, tid);
             }
             __syncthreads();
             int n = ready_n;
             if (n == 0) {  // the next step is not done yet: wait for it alone
-                block_wait(flags + tile_task(I, J, nb), epoch, status);
-                if (kind != 0) block_wait(flags + tile_task(K, J, nb), epoch, status);
+                block_wait(flags + tile_task(I, J, nb), flags + tile_task(kind != 0 ? K : J + 1, J, nb), epoch, status);
                 n = 1;
             }
             for (int e2 = tid; e2 < n * TT; e2 += CF_THREADS) {
@@ -967,54 +757,55 @@ __global__ void __launch_bounds__(CF_THREADS, 1) k_chol_dataflow(int Np, int nb,
             // the panel raises Linv_JJ.  PD and SUB solve it here themselves
             // (the same arithmetic, so the same bits) as soon as Linv_JJ is
             // up, which saves the panel a hand-off per step.
+            // Warps 0-3 solve it, the others meanwhile fetch L_{K,J} or y_J.
             const int Jl = I - 2;
-            block_wait(flags + n_fact + 2 * nb + Jl, epoch, status);
-            block_wait(flags + tile_task(Jl, Jl, nb), epoch, status);
-            if (kind == 1) block_wait(flags + tile_task(K, Jl, nb), epoch, status);
-            for (int e2 = tid; e2 < TT; e2 += CF_THREADS) {
-                const int r = e2 / T, c = e2 % T;
-                bi[1][r][c] = __ldcg(pre + (size_t)Jl * TT + e2);
-                linv[r][c] = __ldcg(Linv + (size_t)Jl * TT + e2);
-                if (kind == 1) bi[2][r][c] = __ldcg(S + (size_t)(K * T + r) * Np + Jl * T + c);
+            if (warp < 4) {
+                warp_wait(flags + n_fact + 2 * nb + Jl, epoch, status);
+                const double p0 = __ldcg(pre + (size_t)Jl * TT + tid), p1 = __ldcg(pre + (size_t)Jl * TT + TT / 2 + tid);
+                const int r = tid / T, c = tid % T;
+                bi[1][r][c] = p0;
+                bi[1][r + T / 2][c] = p1;
+                warp_wait(flags + tile_task(Jl, Jl, nb), epoch, status);
+                const double l0 = __ldcg(Linv + (size_t)Jl * TT + tid), l1 = __ldcg(Linv + (size_t)Jl * TT + TT / 2 + tid);
+                linv[r][c] = l0;
+                linv[r + T / 2][c] = l1;
+                pf_bar<3, TT / 2>();
+                tile_trsm(bi[1], linv, [&](int i, int j, double v) { bi[0][i][j] = v; });
+            } else {
+                const int u = tid - TT / 2, r = u / T, c = u % T;
+                warp_wait(flags + tile_task(Jl + 1, Jl, nb), epoch, status);
+                if (kind == 1) {
+                    const double *src = S + (size_t)(K * T + r) * Np + Jl * T + c;
+                    const double v0 = __ldcg(src), v1 = __ldcg(src + (size_t)(T / 2) * Np);
+                    bi[2][r][c] = v0;
+                    bi[2][r + T / 2][c] = v1;
+                } else if (u < T) {
+                    by[0][u] = __ldcg(rhs + Jl * T + u);
+                }
             }
-            if (kind == 0 && tid < T) by[0][tid] = __ldcg(rhs + Jl * T + tid);
-            __syncthreads();
-            tile_trsm(bi[0], bi[1], linv);
             __syncthreads();
             if (kind == 0) {
                 update_lower<true>(a, bi[0], bvec, by[0], part);
-            } else {
-                for (int e2 = tid; e2 < TT; e2 += CF_THREADS) {
-                    const int r = e2 / T, c = e2 % T;
-                    double sacc = a[r][c];
-#pragma unroll
-                    for (int k = 0; k < T; ++k) sacc = fma(-bi[0][r][k], bi[2][c][k], sacc);
-                    a[r][c] = sacc;
-                }
-                __syncthreads();
-            }
-        } else if (kind == 2) {
-            // the second-subdiagonal tile before its solve, for PD(K + 2) and SUB(K + 1)
-            for (int e2 = tid; e2 < TT; e2 += CF_THREADS) pre[(size_t)K * TT + e2] = a[e2 / T][e2 % T];
-            block_release(flags + n_fact + 2 * nb + K, epoch);
-        }
-        const bool failed = block_failed(status);
-        if (kind == 0) {
-            if (!failed) {
                 store_tile(S, Np, I, I, a);
                 if (tid < T) rhs[I * T + tid] = bvec[tid];
+            } else {
+                const int r = tid / T, c = tid % T;
+                double sacc = a[r][c];
+#pragma unroll
+                for (int k = 0; k < T; ++k) sacc = fma(-bi[0][r][k], bi[2][c][k], sacc);
+                S[(size_t)(I * T + r) * Np + K * T + c] = sacc;
             }
-        } else if (kind == 1) {
-            if (!failed) store_tile(S, Np, I, K, a);
         } else {
-            block_wait(flags + tile_task(K, K, nb), epoch, status);
+            if (kind == 2) {
+                // the second-subdiagonal tile before its solve, for PD(K + 2) and SUB(K + 1)
+                for (int e2 = tid; e2 < TT; e2 += CF_THREADS) pre[(size_t)K * TT + e2] = a[e2 / T][e2 % T];
+                block_release(flags + n_fact + 2 * nb + K, epoch);
+            }
+            block_wait(flags + tile_task(K, K, nb), nullptr, epoch, status);
             for (int e2 = tid; e2 < TT; e2 += CF_THREADS) linv[e2 / T][e2 % T] = __ldcg(Linv + (size_t)K * TT + e2);
             __syncthreads();
-            if (!block_failed(status)) {
-                tile_trsm(bi[0], a, linv);
-                __syncthreads();
-                store_tile(S, Np, I, K, bi[0]);
-            }
+            if (warp < 4)
+                tile_trsm(a, linv, [&](int r, int c, double v) { S[(size_t)(I * T + r) * Np + K * T + c] = v; });
         }
         block_release(flags + mark, epoch);
         __syncthreads();
