@@ -100,14 +100,59 @@ __device__ void block_wait(const int *fa, const int *fb, int epoch, int *status)
     __syncthreads();
 }
 
-// A warp's own wait: its lanes' loads come after lane 0's acquire.
-__device__ __forceinline__ bool warp_wait(const int *flag, int epoch, int *status)
+// Mail.  What the chain of panel steps waits for goes from CTA to CTA as
+// 16-byte packets, a value and the launch's epoch, each written and read whole
+// (one 128-bit access).  A packet is its own flag: the reader polls the values
+// themselves, so a hand-off is a store and a poll, ~1 us less than store, fence,
+// flag, poll and load.  Per block column K: L_KK^-1 and PD(K) by lower triangle
+// rows (PD's b behind it), L_{K+1,K}, SUB(K) and the pre-solve (K+2, K) by rows, y_K.
+constexpr int TRI = T * (T + 1) / 2;
+constexpr int ML_INV = 0, ML_PD = ML_INV + TRI, ML_SUBD = ML_PD + TRI + T, ML_SUB = ML_SUBD + TT, ML_PRE = ML_SUB + TT,
+              ML_Y = ML_PRE + TT, ML_COLUMN = ML_Y + T;
+static_assert(ML_COLUMN == CHOL_MAIL, "the packets of a block column");
+
+__device__ __forceinline__ int tri_at(int r, int c) { return r * (r + 1) / 2 + c; }
+
+// row and column of entry e of a lower triangle by rows
+__device__ __forceinline__ void tri_of(int e, int &r, int &c)
 {
-    int ok = 0;
-    if ((threadIdx.x & 31) == 0) ok = poll_flag(flag, epoch, status);
-    ok = __shfl_sync(0xffffffffu, ok, 0);
-    __syncwarp();
-    return ok != 0;
+    r = (int)((sqrtf(8.0f * (float)e + 1.0f) - 1.0f) * 0.5f);
+    while ((r + 1) * (r + 2) / 2 <= e) ++r;
+    while (r * (r + 1) / 2 > e) --r;
+    c = e - r * (r + 1) / 2;
+}
+
+__device__ __forceinline__ void mail_put(ulonglong2 *p, double v, int epoch)
+{
+    asm volatile("{ .reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.gpu.global.b128 [%0], t; }" ::"l"(p),
+                 "l"(__double_as_longlong(v)), "l"((long long)epoch)
+                 : "memory");
+}
+
+// The thread's n <= N packets p[0], p[stride], ...; waits for all.  False when the
+// budget ran out, or another task failed or timed out.
+template <int N>
+__device__ __forceinline__ bool mail_get(const ulonglong2 *p, int stride, int n, double (&v)[N], int epoch, int *status)
+{
+    const long long limit = s_spin_limit;
+    for (long long it = 0; it < limit; ++it) {
+        bool ok = true;
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            long long x = 0, tag = epoch;
+            if (j < n)
+                asm volatile("{ .reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+                             : "=l"(x), "=l"(tag)
+                             : "l"(p + j * stride)
+                             : "memory");
+            v[j] = __longlong_as_double(x);
+            ok = ok && tag == epoch;
+        }
+        if (ok) return true;
+        if ((it & 15) == 15 && ld_relaxed(status) != 0) return false;
+    }
+    atomicCAS(status, 0, 2);
+    return false;
 }
 
 __device__ __forceinline__ int tile_task(int I, int K, int nb)
@@ -139,10 +184,10 @@ __device__ __forceinline__ void load_tile(double (*dst)[T + 1], const double *S,
 // Range: rows and columns are first scaled by 2^-H_r, H_r = floor(log2(a_rr) / 2) of
 // the tile before its last update, which puts the diagonal below 4, and every
 // four columns all entries are scaled by the power of two that brings sigma
-// back to one.  In between sigma grows to 2^30 at most, and shrinks by pivots
-// (in scaled units, of four columns) p q r ... to p^7 q^3 r: it takes four in
-// a row below 2^-60, far under the rounding errors of the tile, to
-// underflow, and the tile is then refused.
+// back to one.  In between sigma grows to 2^30 at most, and four columns of
+// pivots D_0 ... D_3 (scaled) shrink it to D_0^8 D_1^4 D_2^2 D_3: it takes four
+// in a row below 2^-60, far under the rounding errors of the tile, to underflow,
+// and the tile is then refused.
 //
 // Roles: warps 0-3 hold one entry of rows 4-15 a thread (and one sigma), warp 4
 // those of rows 0-3, whose columns end early; they meet once a column.  Column
@@ -226,11 +271,12 @@ __device__ __forceinline__ double pf_shift(double x, int n)
 
 // Warps 0-6 (224 threads): the last update of the diagonal tile a and of b with
 // the previous step's sub-diagonal tile lsub and y (first: none), then the
-// tile's Cholesky factor, to Lg (rows of Np), and its inverse, to X and Ig
-// (lower triangles only).  True in warp 4 when a pivot was not a positive
+// tile's Cholesky factor, to Lg (rows of Np), and its inverse, to X, Ig and the
+// mail (lower triangles only).  True in warp 4 when a pivot was not a positive
 // normal number.
 __device__ __forceinline__ bool panel_factor(const double (*a)[T + 1], const int *H, const double (*lsub)[T + 1], double *b, const double *y,
-                             bool first, double (*X)[T + 1], double *Lg, int Np, double *Ig, const PfWork &w, const PfEntry &e)
+                             bool first, double (*X)[T + 1], double *Lg, int Np, double *Ig, ulonglong2 *mail, int epoch, const PfWork &w,
+                             const PfEntry &e)
 {
     static_assert(CF_THREADS == 256 && T == 16, "the factor is laid out for eight warps and 16 x 16 tiles");
     constexpr int NE = 160, NT = CF_THREADS - 32;  // threads of warps 0-4 and of warps 0-6
@@ -315,6 +361,7 @@ __device__ __forceinline__ bool panel_factor(const double (*a)[T + 1], const int
     if (own) {
         const double xr = x * w.t[r];
         X[r][c] = xr;
+        mail_put(mail + ML_INV + tri_at(r, c), xr, epoch);
         Ig[r * T + c] = xr;
         Lg[(size_t)r * Np + c] = lr * w.t[c];
     }
@@ -325,7 +372,8 @@ __device__ __forceinline__ bool panel_factor(const double (*a)[T + 1], const int
 }
 
 // y = L^-1 b by warps 5 and 6, four lanes a row
-__device__ __forceinline__ void panel_y(const double (*X)[T + 1], const double *b, double *y, double *yg)
+__device__ __forceinline__ void panel_y(const double (*X)[T + 1], const double *b, double *y, double *yg, ulonglong2 *mail,
+                                        int epoch)
 {
     const int r = ((int)threadIdx.x - 160) >> 2, k0 = threadIdx.x & 3;
     double v = 0.0;
@@ -335,6 +383,7 @@ __device__ __forceinline__ void panel_y(const double (*X)[T + 1], const double *
     v += __shfl_xor_sync(0xffffffffu, v, 2);
     if (k0 == 0) {
         y[r] = v;
+        mail_put(mail + ML_Y + r, v, epoch);
         yg[r] = v;
     }
 }
@@ -457,14 +506,6 @@ __device__ void cta_back(int Np, int nb, const double *__restrict__ S, const dou
 // elements, whose partial sums go to part[NACC t ...].  Each element then
 // subtracts its partial sums in k order.  The accumulator and operands of a
 // product are picked by selects, so a warp issues one FMA per product.
-__device__ __forceinline__ void tri_of(int e, int &r, int &c)
-{
-    r = (int)((sqrtf(8.0f * (float)e + 1.0f) - 1.0f) * 0.5f);
-    while ((r + 1) * (r + 2) / 2 <= e) ++r;
-    while (r * (r + 1) / 2 > e) --r;
-    c = e - r * (r + 1) / 2;
-}
-
 template <bool WITH_B>
 struct LowerUpdate {
     static constexpr int NT = CF_THREADS;
@@ -576,19 +617,19 @@ __device__ __forceinline__ void block_release(int *flag, int epoch)
 
 // Flags: tile (I, K) at tile_task(I, K); that slot is raised for the
 // diagonal tile (I, I) when L_II and its inverse are stored, and for the
-// sub-diagonal tile (I+1, I) when L_{I+1,I} and y_I are stored.  The partial diagonal
-// PD(I) = A_II - sum_{J <= I-2} L_IJ L_IJ^T (with b_I likewise) raises
-// n_fact + I; the partial sub-diagonal SUB(I) = A_{I+1,I} - sum_{J <= I-1}
-// L_{I+1,J} L_IJ^T raises n_fact + nb + I; the second-subdiagonal tile
-// (K+2, K) raises n_fact + 2 nb + K when its accumulation (before its solve)
-// is in pre[K].
+// sub-diagonal tile (I+1, I) when L_{I+1,I} and y_I are stored.  By mail go, beside
+// these, the partial diagonal PD(I) = A_II - sum_{J <= I-2} L_IJ L_IJ^T (with
+// b_I likewise), the partial sub-diagonal SUB(I) = A_{I+1,I} -
+// sum_{J <= I-1} L_{I+1,J} L_IJ^T, and the second-subdiagonal tile (K+2, K)
+// after its accumulation, before its solve.
 //
 // The factor with the forward solve of rhs carried along.  CTA 0 (the panel)
 // walks the diagonal: step I applies the last update to PD(I) with L_{I,I-1}
 // (its own, kept in shared memory), factors the tile and stores L_II and Linv_II
-// (panel_factor), then forms L_{I+1,I} = SUB(I) Linv_II^T, which it keeps, and y_I.  The other CTAs (helpers) run the task list: the tiles
-// (I, K) with I >= K + 2 (left-looking updates, then the triangular solve
-// with Linv_KK), and the PD and SUB accumulations, in the order
+// (panel_factor), then forms L_{I+1,I} = SUB(I) Linv_II^T, which it keeps, and
+// y_I.  The other CTAs (helpers) run the task list: the tiles (I, K) with
+// I >= K + 2 (left-looking updates, then the triangular solve with Linv_KK),
+// and the PD and SUB accumulations, in the order
 //   P(0), C(0), PD(2), SUB(1), P(1), C(1), PD(3), SUB(2), P(2), ...
 // (P = panel step, C(K) = the tiles of column K) -- every task depends only on
 // tasks before it, each helper takes every (G-1)-th task in that order and
@@ -599,7 +640,7 @@ __global__ void __launch_bounds__(CF_THREADS, 1) k_chol_dataflow(int Np, int nb,
                                                               double *__restrict__ S,
                                                               double *__restrict__ Linv,
                                                               double *__restrict__ rhs,
-                                                              double *__restrict__ pre,
+                                                              ulonglong2 *__restrict__ mail,
                                                               int *__restrict__ flags, int epoch,
                                                               int *__restrict__ status, long long spin_limit)
 {
@@ -608,7 +649,6 @@ __global__ void __launch_bounds__(CF_THREADS, 1) k_chol_dataflow(int Np, int nb,
     __shared__ double bi[BJ][T][T + 1], bk[BJ][T][T + 1], by[BJ][T];
     __shared__ double bvec[T];
     __shared__ int ready_n;
-    const int n_fact = nb * (nb + 1) / 2;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     double *part = &bk[0][0][0];
     if (tid == 0) s_spin_limit = spin_limit;
@@ -632,6 +672,9 @@ __global__ void __launch_bounds__(CF_THREADS, 1) k_chol_dataflow(int Np, int nb,
         __syncthreads();
         if (warp == 7) tile_exp(bi[0], hexp[0]);
         __syncthreads();
+        int pd_r[5], pd_c[5];  // warp 7's places in PD's mail
+#pragma unroll
+        for (int q = 0; q < 5; ++q) tri_of(min(lane + 32 * q, TRI - 1), pd_r[q], pd_c[q]);
         bool failed = false;
         int I = 0;
         for (; I < nb && !failed; ++I) {
@@ -640,35 +683,38 @@ __global__ void __launch_bounds__(CF_THREADS, 1) k_chol_dataflow(int Np, int nb,
             if (warp == 7) {
                 if (I >= 1 && lane == 0) st_release(flags + tile_task(I, I - 1, nb), epoch);
                 if (I + 1 < nb) {
-                    const double *src = S + (size_t)((I + 1) * T + (lane >> 3)) * Np + I * T + 2 * (lane & 7);
-                    bool ok = I == 0 || warp_wait(flags + n_fact + nb + I, epoch, status);
-                    double2 v[4];
+                    double(*an)[T + 1] = bi[cur ^ 1], *bn = by[cur ^ 1];
+                    bool ok = true;
+                    if (I == 0) {  // no updates before these
+                        for (int e = lane; e < TT; e += 32) {
+                            const double *src = S + (size_t)(T + e / T) * Np + e % T;
+                            asub[e / T][e % T] = __ldcg(src);
+                            an[e / T][e % T] = __ldcg(src + T);
+                        }
+                        if (lane < T) bn[lane] = __ldcg(rhs + T + lane);
+                        pf_arrive<3, 160>();
+                    } else {
+                        double v[8];
+                        ok = mail_get(mail + (size_t)I * ML_COLUMN + ML_SUB + lane, 32, 8, v, epoch, status);
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) v[q] = __ldcg(reinterpret_cast<const double2 *>(src + (size_t)(4 * q) * Np));
+                        for (int q = 0; q < 8; ++q) asub[2 * q + (lane >> 4)][lane & 15] = v[q];
+                        pf_arrive<3, 160>();
+                        double u[5];
+                        ok = mail_get(mail + (size_t)(I + 1) * ML_COLUMN + ML_PD + lane, 32, lane < 24 ? 5 : 4, u, epoch, status) && ok;
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        double *d = &asub[4 * q + (lane >> 3)][2 * (lane & 7)];
-                        d[0] = v[q].x;
-                        d[1] = v[q].y;
-                    }
-                    pf_arrive<3, 160>();
-                    ok = (I == 0 || warp_wait(flags + n_fact + I + 1, epoch, status)) && ok;
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) v[q] = __ldcg(reinterpret_cast<const double2 *>(src + (size_t)(4 * q) * Np + T));
-                    if (lane < T) by[cur ^ 1][lane] = __ldcg(rhs + (I + 1) * T + lane);
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        double *d = &bi[cur ^ 1][4 * q + (lane >> 3)][2 * (lane & 7)];
-                        d[0] = v[q].x;
-                        d[1] = v[q].y;
+                        for (int q = 0; q < 5; ++q) {
+                            const int e = lane + 32 * q;
+                            if (e < TRI) an[pd_r[q]][pd_c[q]] = u[q];
+                            else if (e < TRI + T) bn[e - TRI] = u[q];
+                        }
                     }
                     __syncwarp();
                     tile_exp(bi[cur ^ 1], hexp[cur ^ 1]);
-                    if (lane == 0 && !ok) stop[cur] = 1;
+                    if (!ok) stop[cur] = 1;
                 }
             } else {
                 const bool bad = panel_factor(bi[cur], hexp[cur], lsub, by[cur], wy, I == 0, wli,
-                                              S + (size_t)(I * T) * Np + I * T, Np, Linv + (size_t)I * TT, pw, pe);
+                                              S + (size_t)(I * T) * Np + I * T, Np, Linv + (size_t)I * TT, mail + (size_t)I * ML_COLUMN, epoch, pw, pe);
                 if (warp == 4 && lane == 0) {
                     if (bad) {
                         atomicCAS(status, 0, 1);
@@ -676,11 +722,12 @@ __global__ void __launch_bounds__(CF_THREADS, 1) k_chol_dataflow(int Np, int nb,
                     }
                     st_release(flags + tile_task(I, I, nb), epoch);
                 }
-                if (warp >= 5) panel_y(wli, by[cur], wy, rhs + I * T);
+                if (warp >= 5) panel_y(wli, by[cur], wy, rhs + I * T, mail + (size_t)I * ML_COLUMN, epoch);
                 if (warp < 4 && I + 1 < nb) {
                     pf_bar<3, 160>();  // SUB(I) is there
                     double *Lg = S + (size_t)((I + 1) * T) * Np + I * T;
                     tile_trsm(asub, wli, [&](int r, int c, double v) {
+                        mail_put(mail + (size_t)I * ML_COLUMN + ML_SUBD + r * T + c, v, epoch);
                         lsub[r][c] = v;
                         Lg[(size_t)r * Np + c] = v;
                     });
@@ -697,10 +744,11 @@ __global__ void __launch_bounds__(CF_THREADS, 1) k_chol_dataflow(int Np, int nb,
         return;
     }
     // ---- helpers
+    int inv_r, inv_c;  // the thread's place in an inverse's mail
+    tri_of(min(tid, TRI - 1), inv_r, inv_c);
     for (int t = blockIdx.x - 1; t < n_tasks; t += gridDim.x - 1) {
         const int I = tasks[t].x, K = tasks[t].y;
         const int kind = I - K;  // 0: PD(I), 1: SUB(K), >= 2: tile (I, K)
-        const int mark = kind == 0 ? n_fact + I : kind == 1 ? n_fact + nb + K : tile_task(I, K, nb);
         load_tile(a, S, Np, I, K);
         if (kind == 0 && tid < T) bvec[tid] = __ldcg(rhs + I * T + tid);
         __syncthreads();
@@ -753,61 +801,58 @@ __global__ void __launch_bounds__(CF_THREADS, 1) k_chol_dataflow(int Np, int nb,
         }
         if (kind <= 1) {
             // Last step, J = I - 2: L_{I,J} is the second-subdiagonal tile, whose
-            // own task publishes it before its solve (PRE) and solves it once
-            // the panel raises Linv_JJ.  PD and SUB solve it here themselves
+            // own task mails it before its solve and solves it for the others
+            // once the panel raises Linv_JJ.  PD and SUB solve it here themselves
             // (the same arithmetic, so the same bits) as soon as Linv_JJ is
-            // up, which saves the panel a hand-off per step.
+            // there, which saves the panel a hand-off per step.
             // Warps 0-3 solve it, the others meanwhile fetch L_{K,J} or y_J.
             const int Jl = I - 2;
+            const ulonglong2 *from = mail + (size_t)Jl * ML_COLUMN;
             if (warp < 4) {
-                warp_wait(flags + n_fact + 2 * nb + Jl, epoch, status);
-                const double p0 = __ldcg(pre + (size_t)Jl * TT + tid), p1 = __ldcg(pre + (size_t)Jl * TT + TT / 2 + tid);
-                const int r = tid / T, c = tid % T;
-                bi[1][r][c] = p0;
-                bi[1][r + T / 2][c] = p1;
-                warp_wait(flags + tile_task(Jl, Jl, nb), epoch, status);
-                const double l0 = __ldcg(Linv + (size_t)Jl * TT + tid), l1 = __ldcg(Linv + (size_t)Jl * TT + TT / 2 + tid);
-                linv[r][c] = l0;
-                linv[r + T / 2][c] = l1;
+                double v[2];
+                mail_get(from + ML_PRE + tid, TT / 2, 2, v, epoch, status);
+                bi[1][tid / T][tid % T] = v[0];
+                bi[1][tid / T + T / 2][tid % T] = v[1];
+                mail_get(from + ML_INV + tid, TT / 2, tid < TRI - TT / 2 ? 2 : 1, v, epoch, status);
+                linv[inv_r][inv_c] = v[0];
+                if (tid < TRI - TT / 2) linv[T - 1][tid + TT / 2 - tri_at(T - 1, 0)] = v[1];
                 pf_bar<3, TT / 2>();
-                tile_trsm(bi[1], linv, [&](int i, int j, double v) { bi[0][i][j] = v; });
+                tile_trsm(bi[1], linv, [&](int i, int j, double x) { bi[0][i][j] = x; });
             } else {
-                const int u = tid - TT / 2, r = u / T, c = u % T;
-                warp_wait(flags + tile_task(Jl + 1, Jl, nb), epoch, status);
+                const int u = tid - TT / 2;
+                double v[2];
                 if (kind == 1) {
-                    const double *src = S + (size_t)(K * T + r) * Np + Jl * T + c;
-                    const double v0 = __ldcg(src), v1 = __ldcg(src + (size_t)(T / 2) * Np);
-                    bi[2][r][c] = v0;
-                    bi[2][r + T / 2][c] = v1;
+                    mail_get(from + ML_SUBD + u, TT / 2, 2, v, epoch, status);
+                    bi[2][u / T][u % T] = v[0];
+                    bi[2][u / T + T / 2][u % T] = v[1];
                 } else if (u < T) {
-                    by[0][u] = __ldcg(rhs + Jl * T + u);
+                    mail_get(from + ML_Y + u, 0, 1, v, epoch, status);
+                    by[0][u] = v[0];
                 }
             }
             __syncthreads();
+            const int r = tid / T, c = tid % T;
             if (kind == 0) {
                 update_lower<true>(a, bi[0], bvec, by[0], part);
-                store_tile(S, Np, I, I, a);
-                if (tid < T) rhs[I * T + tid] = bvec[tid];
+                ulonglong2 *to = mail + (size_t)I * ML_COLUMN + ML_PD;
+                if (c <= r) mail_put(to + tri_at(r, c), a[r][c], epoch);
+                if (tid < T) mail_put(to + TRI + tid, bvec[tid], epoch);
             } else {
-                const int r = tid / T, c = tid % T;
                 double sacc = a[r][c];
 #pragma unroll
                 for (int k = 0; k < T; ++k) sacc = fma(-bi[0][r][k], bi[2][c][k], sacc);
-                S[(size_t)(I * T + r) * Np + K * T + c] = sacc;
+                mail_put(mail + (size_t)K * ML_COLUMN + ML_SUB + tid, sacc, epoch);
             }
         } else {
-            if (kind == 2) {
-                // the second-subdiagonal tile before its solve, for PD(K + 2) and SUB(K + 1)
-                for (int e2 = tid; e2 < TT; e2 += CF_THREADS) pre[(size_t)K * TT + e2] = a[e2 / T][e2 % T];
-                block_release(flags + n_fact + 2 * nb + K, epoch);
-            }
+            // the second-subdiagonal tile before its solve, for PD(K + 2) and SUB(K + 1)
+            if (kind == 2) mail_put(mail + (size_t)K * ML_COLUMN + ML_PRE + tid, a[tid / T][tid % T], epoch);
             block_wait(flags + tile_task(K, K, nb), nullptr, epoch, status);
             for (int e2 = tid; e2 < TT; e2 += CF_THREADS) linv[e2 / T][e2 % T] = __ldcg(Linv + (size_t)K * TT + e2);
             __syncthreads();
             if (warp < 4)
                 tile_trsm(a, linv, [&](int r, int c, double v) { S[(size_t)(I * T + r) * Np + K * T + c] = v; });
+            block_release(flags + tile_task(I, K, nb), epoch);
         }
-        block_release(flags + mark, epoch);
         __syncthreads();
     }
 }
@@ -1122,10 +1167,11 @@ void launch_chol_dataflow(const DeviceProblem &d, int epoch, double *x_out, cuda
         int n_tasks = d.chol_n_tasks;
         const int grid = chol_grid(n_tasks + 1, d.chol_grid_cap);
         const int2 *tasks = d.chol_tasks;
-        double *S = d.S, *Linv = d.Linv, *rhs = d.rhs, *pre = d.chol_pre;
+        double *S = d.S, *Linv = d.Linv, *rhs = d.rhs;
+        ulonglong2 *mail = d.chol_mail;
         int *flags = d.chol_flags, *status = d.status;
         long long spin = d.wait_limit;
-        void *args[] = {&Np, &nb, &n_tasks, (void *)&tasks, &S, &Linv, &rhs, &pre, &flags, &epoch, &status, &spin};
+        void *args[] = {&Np, &nb, &n_tasks, (void *)&tasks, &S, &Linv, &rhs, &mail, &flags, &epoch, &status, &spin};
         cudaMemsetAsync(d.status, 0, 2 * sizeof(int), s);
         cudaLaunchCooperativeKernel((const void *)k_chol_dataflow, dim3(grid), dim3(CF_THREADS), args, 0, s);
         note_launch(1);
@@ -1535,7 +1581,7 @@ extern "C" int psba_eval_dense_solve(int n, const double *S, const double *b, do
     std::vector<int2> tasks;
     chol_task_list(nb, tasks);
     d.chol_n_tasks = (int)tasks.size();
-    d.chol_n_flags = nb * (nb + 1) / 2 + 3 * nb;
+    d.chol_n_flags = nb * (nb + 1) / 2;
     std::vector<double> hS((size_t)Np * Np, 0.0), hb(Np, 0.0);
     for (int r = 0; r < Np; ++r)
         for (int c = 0; c <= r; ++c) hS[(size_t)r * Np + c] = (r < n && c < n) ? S[(size_t)r * n + c] : (r == c ? 1.0 : 0.0);
@@ -1552,7 +1598,7 @@ extern "C" int psba_eval_dense_solve(int n, const double *S, const double *b, do
     get(&d.rhs, (size_t)Np);
     get(&d.xsol, (size_t)Np);
     get(&d.Linv, (size_t)Np * TILE);
-    get(&d.chol_pre, (size_t)nb * TILE * TILE);
+    get(&d.chol_mail, (size_t)nb * CHOL_MAIL);
     get(&d.chol_tasks, tasks.size());
     get(&d.chol_flags, (size_t)d.chol_n_flags);
     get(&d.status, 4);
@@ -1561,6 +1607,7 @@ extern "C" int psba_eval_dense_solve(int n, const double *S, const double *b, do
     if (e == cudaSuccess && !tasks.empty())
         e = cudaMemcpyAsync(d.chol_tasks, tasks.data(), sizeof(int2) * tasks.size(), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(d.chol_flags, 0, sizeof(int) * d.chol_n_flags, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d.chol_mail, 0, sizeof(*d.chol_mail) * nb * CHOL_MAIL, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(d.status, 0, sizeof(int) * 4, st);
     if (e == cudaSuccess) {
         launch_chol_dataflow(d, 1, d.xsol, st);

@@ -107,6 +107,7 @@ constexpr int CAMTAB = 56;  // doubles per camera table entry (CamTab)
 constexpr int CAMTAB32 = 40;  // floats per FP32 camera table entry: M, D, fx, sk, fy (the mixed Jacobian)
 constexpr int RES_TAB2F = 18;  // FP32 pairs per camera of the mixed projection: M, t, fx sk cx fy cy, a pad (16-byte rows)
 constexpr int TILE = 16;    // dense Cholesky tile size
+constexpr int CHOL_MAIL = 1072;  // packets of the dense factor's mail per block column
 constexpr int SCHUR_CHUNK = 32;  // pair-list entries an off-diagonal unit stages at a time (11/16-parameter cameras, FP32)
 constexpr int MX_UNIT = 256;     // 6-parameter cameras, FP32 products: pair-list entries per warp unit
 constexpr int DIAG_CHUNK = 16;   // observations a diagonal unit stages at a time (11/16-parameter cameras, FP32)
@@ -271,9 +272,9 @@ struct DeviceProblem {
     int2 *chol_tasks = nullptr;   // helper tasks of the dense factor, in dependency order
     int chol_n_tasks = 0;
     int chol_grid_cap = 0;        // CTAs of the dense factor at most (0: one per SM)
-    long long wait_limit = DEFAULT_WAIT_LIMIT;  // polls per device-side wait (dense factor flags)
-    double *chol_pre = nullptr;   // second-subdiagonal tiles before their solve (Np / TILE tiles)
-    int *chol_flags = nullptr;    // one flag per dataflow task (value = epoch when done)
+    long long wait_limit = DEFAULT_WAIT_LIMIT;  // polls per device-side wait (dense factor flags and mail)
+    ulonglong2 *chol_mail = nullptr;  // hand-offs of the dense factor's chain: CHOL_MAIL packets (value, epoch) per block column
+    int *chol_flags = nullptr;    // one flag per tile (value = epoch when done)
     int chol_n_flags = 0;
     double *dp = nullptr;         // N + 3 np
     double *eb = nullptr;         // 3 np

@@ -1060,12 +1060,13 @@ int create_impl(const psba_problem_desc *p, psba_handle *h)
         std::vector<int2> tasks;
         chol_task_list(nb, tasks);
         d.chol_n_tasks = (int)tasks.size();
-        d.chol_n_flags = nb * (nb + 1) / 2 + 3 * nb;
-        TRY(dalloc(h, &d.chol_pre, (size_t)nb * TILE * TILE));
+        d.chol_n_flags = nb * (nb + 1) / 2;
+        TRY(dalloc(h, &d.chol_mail, (size_t)nb * CHOL_MAIL));
         TRY(dalloc(h, &d.chol_tasks, tasks.size()));
         TRY(dalloc(h, &d.chol_flags, (size_t)d.chol_n_flags));
         TRY(upload(h, d.chol_tasks, tasks.data(), tasks.size()));
         PSBA_CUDA_TRY(cudaMemsetAsync(d.chol_flags, 0, sizeof(int) * d.chol_n_flags, h->stream));
+        PSBA_CUDA_TRY(cudaMemsetAsync(d.chol_mail, 0, sizeof(*d.chol_mail) * nb * CHOL_MAIL, h->stream));
     }
     TRY(dalloc(h, &d.dp, nt));
     TRY(dalloc(h, &d.eb, 3 * (size_t)np));
