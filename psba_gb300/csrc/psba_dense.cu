@@ -92,11 +92,11 @@ __device__ __forceinline__ bool poll_flag(const int *flag, int epoch, int *statu
     return false;
 }
 
-// Threads 0 and 32 wait for a flag each (fb may be null); the block then proceeds.
+// Threads 0 and 32 wait for a flag each; the block then proceeds.
 __device__ void block_wait(const int *fa, const int *fb, int epoch, int *status)
 {
     if (threadIdx.x == 0) poll_flag(fa, epoch, status);
-    if (threadIdx.x == 32 && fb != nullptr) poll_flag(fb, epoch, status);
+    if (threadIdx.x == 32) poll_flag(fb, epoch, status);
     __syncthreads();
 }
 
@@ -192,15 +192,15 @@ __device__ __forceinline__ void load_tile(double (*dst)[T + 1], const double *S,
 // Roles: warps 0-3 hold one entry of rows 4-15 a thread (and one sigma), warp 4
 // those of rows 0-3, whose columns end early; they meet once a column.  Column
 // s of all is in q[s]: a_is for i >= s, x_si for i < s, so that in the end
-// everything is there.  Warps 5 and 6 take b's update and y, warp 7 the step's
-// fetches.
-// Cycles a tile (N = 528): 1,800 for the last update (at the SM's FP64 rate: one
-// warp instruction per ~19 cycles), 3,950 for 15 columns (263 each, of which
-// the two FP64 steps ~150, the shared-memory round and the barrier ~90), 770 for
-// the roots, 600 for the outputs: 7,100, where an LDL^T elimination with a reciprocal a column
-// and the inverse behind it took 15,000.  What a column does not need is kept
-// out of it: a branch costs ~30 cycles, a sign flip or a comparison in FP64 60.
-
+// everything is there.  Warp 5 takes b's update and y, warp 7 the step's fetches.
+// Cycles a tile (N = 528): 1,850 for the last update (at the SM's FP64 rate: one
+// warp instruction per ~19 cycles), 4,150 for 15 columns (277 each, of which
+// the two FP64 steps ~150, the shared-memory round and the barrier ~90), 400 to
+// the inverse but for t, and 1,800 for the sub-diagonal tile, beside which the
+// roots (770 by themselves) are taken.  A panel step is 8,900 of these; with an
+// LDL^T elimination, a reciprocal a column and the inverse behind it, the tile
+// alone took 15,000.  What a column does not need is kept out of it: a branch
+// costs ~30 cycles, a sign flip or a comparison in FP64 60.
 // Beside the 16 entries, q[s] has sigma_s, a zero (sigma's a) and a place for the
 // stores of threads that have nothing to publish: a store under a condition
 // on row and column cost 170 cycles a column in branches.
@@ -271,30 +271,28 @@ __device__ __forceinline__ double pf_shift(double x, int n)
 
 // Warps 0-6 (224 threads): the last update of the diagonal tile a and of b with
 // the previous step's sub-diagonal tile lsub and y (first: none), then the
-// tile's Cholesky factor, to Lg (rows of Np), and its inverse, to X, Ig and the
-// mail (lower triangles only).  True in warp 4 when a pivot was not a positive
-// normal number.
-__device__ __forceinline__ bool panel_factor(const double (*a)[T + 1], const int *H, const double (*lsub)[T + 1], double *b, const double *y,
-                             bool first, double (*X)[T + 1], double *Lg, int Np, double *Ig, ulonglong2 *mail, int epoch, const PfWork &w,
-                             const PfEntry &e)
+// elimination.  X gets the inverse but for t (rows r to be multiplied by t_r),
+// w.q the rest.
+__device__ __forceinline__ void panel_factor(const double (*a)[T + 1], const int *H, const double (*lsub)[T + 1], double *b,
+                                             const double *y, bool first, double (*X)[T + 1], const PfWork &w,
+                                             const PfEntry &e)
 {
     static_assert(CF_THREADS == 256 && T == 16, "the factor is laid out for eight warps and 16 x 16 tiles");
     constexpr int NE = 160, NT = CF_THREADS - 32;  // threads of warps 0-4 and of warps 0-6
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (warp >= 5) {
-        // b, four lanes a row, when the columns leave the FP64 units room for it
+        // b (warp 5, two lanes a row), when the columns leave the FP64 units room for it
         pf_bar<4, NT>();
-        if (!first) {
-            const int r = (tid - NE) >> 2, k0 = tid & 3;
+        if (!first && warp == 5) {
+            const int r = lane >> 1, k0 = lane & 1;
             double v = 0.0;
 #pragma unroll
-            for (int k = 0; k < T; k += 4) v = fma(lsub[r][k0 + k], y[k0 + k], v);
+            for (int k = 0; k < T; k += 2) v = fma(lsub[r][k0 + k], y[k0 + k], v);
             v += __shfl_xor_sync(0xffffffffu, v, 1);
-            v += __shfl_xor_sync(0xffffffffu, v, 2);
             if (k0 == 0) b[r] -= v;
         }
         pf_bar<1, NT>();
-        return false;
+        return;
     }
     int r = e.r, c = e.c;
     const bool own = e.own, sig = tid == 127;
@@ -350,42 +348,65 @@ __device__ __forceinline__ bool panel_factor(const double (*a)[T + 1], const int
         }
         if (g == 7) pf_arrive<4, NT>();
     }
-    // t; meanwhile the others' factors of it
-    const int l = lane & (T - 1);
-    const double p = w.q[l][l], sg = w.q[l][PF_SIGMA], d = p * sg;
-    if (warp == 4) w.t[l] = rsqrt(d);
-    if (sig) c = 0;
-    const double lr = pf_shift(w.q[c][r], H[r] * (1 << 20)), sc = w.q[c][PF_SIGMA];
-    const double x = pf_shift(r == c ? sc : w.q[r][c] * sc, -H[c] * (1 << 20));
-    pf_bar<2, NE>();
     if (own) {
-        const double xr = x * w.t[r];
-        X[r][c] = xr;
-        mail_put(mail + ML_INV + tri_at(r, c), xr, epoch);
-        Ig[r * T + c] = xr;
-        Lg[(size_t)r * Np + c] = lr * w.t[c];
+        const double sc = w.q[c][PF_SIGMA];
+        X[r][c] = pf_shift(r == c ? sc : w.q[r][c] * sc, -H[c] * (1 << 20));
     }
     pf_bar<1, NT>();
-    // the pivot itself is p 2^2H / sigma
-    return warp == 4 && __any_sync(0xffffffffu, !(p > 0.0 && d >= DBL_MIN && pf_ldexp(p, 2 * H[l]) >= DBL_MIN * sg &&
-                                                  d <= DBL_MAX));
 }
 
-// y = L^-1 b by warps 5 and 6, four lanes a row
-__device__ __forceinline__ void panel_y(const double (*X)[T + 1], const double *b, double *y, double *yg, ulonglong2 *mail,
-                                        int epoch)
+// y = L^-1 b by warp 5, two lanes a row
+__device__ __forceinline__ void panel_y(const double (*X)[T + 1], const double *b, const double *t, double *y, double *yg,
+                                        ulonglong2 *mail, int epoch)
 {
-    const int r = ((int)threadIdx.x - 160) >> 2, k0 = threadIdx.x & 3;
+    const int r = (threadIdx.x & 31) >> 1, k0 = threadIdx.x & 1;
     double v = 0.0;
 #pragma unroll
-    for (int k = 0; k < T; k += 4) v = fma(k0 + k <= r ? X[r][k0 + k] : 0.0, b[k0 + k], v);
+    for (int k = 0; k < T; k += 2) v = fma(k0 + k <= r ? X[r][k0 + k] : 0.0, b[k0 + k], v);
     v += __shfl_xor_sync(0xffffffffu, v, 1);
-    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    v *= t[r];
     if (k0 == 0) {
         y[r] = v;
         mail_put(mail + ML_Y + r, v, epoch);
         yg[r] = v;
     }
+}
+
+// Warps 4-6 after it, beside the others' sub-diagonal tile: t (warp 4), then the
+// inverse, to the mail and Ig (lower triangle), and y (warp 5).  (The solves use
+// the diagonal tiles' inverses only: L_II itself is not kept.)  True in warp 4
+// when a pivot was not a positive normal number.  t is announced on barrier 5
+// to warps 0-3 (if they wait).
+struct PfOut {
+    int r[2], c[2];  // the thread's entries of the triangle
+};
+
+__device__ __forceinline__ bool panel_finish(const double (*X)[T + 1], const int *H, const double *b, double *y, bool waited,
+                                             double *Ig, double *yg, ulonglong2 *mail, int epoch,
+                                             const PfWork &w, const PfOut &o)
+{
+    const int tid = threadIdx.x, lane = tid & 31;
+    bool bad = false;
+    if (tid < 160) {
+        const int l = lane & (T - 1);
+        const double p = w.q[l][l], sg = w.q[l][PF_SIGMA], d = p * sg;
+        w.t[l] = rsqrt(d);
+        if (waited) pf_arrive<5, 160>();
+        // the pivot itself is p 2^2H / sigma
+        bad = __any_sync(0xffffffffu,
+                         !(p > 0.0 && d >= DBL_MIN && pf_ldexp(p, 2 * H[l]) >= DBL_MIN * sg && d <= DBL_MAX));
+    }
+    pf_bar<6, 96>();
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const int r = o.r[j], c = o.c[j];
+        if (r >= T) continue;
+        const double xr = X[r][c] * w.t[r];
+        mail_put(mail + ML_INV + tri_at(r, c), xr, epoch);
+        Ig[r * T + c] = xr;
+    }
+    if (tid >= 160 && tid < 192) panel_y(X, b, w.t, y, yg, mail, epoch);
+    return bad;
 }
 
 // The single-CTA back solve over the factor (S lower = L, Linv = diagonal
@@ -573,9 +594,9 @@ __device__ void update_lower(double (*a)[T + 1], const double (*L)[T + 1], doubl
     sync();
 }
 
-// A Linv^T with the lower triangle of Linv, out(r, c, v) with v = sum_{k <= c}
-// A[r][k] Linv[c][k]: columns c and T-1-c of a row go to one thread, T + 1
-// products.  Called by the first TT / 2 threads (the products are at one FP64
+// A Linv^T with the lower triangle of Linv: v_rc = sum_{k <= c} A[r][k] Linv[c][k],
+// columns c0 and c1 = T-1-c0 of a row to one thread, T + 1 products, which
+// out(r, c0, c1, v0, v1) gets.  Called by the first TT / 2 threads (the products are at one FP64
 // warp instruction per 64 cycles and SM quarter either way, ~1,100 cycles).
 template <typename Out>
 __device__ __forceinline__ void tile_trsm(const double (*A)[T + 1], const double (*Li)[T + 1], Out out)
@@ -598,8 +619,7 @@ __device__ __forceinline__ void tile_trsm(const double (*A)[T + 1], const double
         s0 = first ? v : s0;
         s1 = first ? s1 : v;
     }
-    out(r, c0, s0);
-    out(r, c1, s1);
+    out(r, c0, c1, s0, s1);
 }
 
 __device__ __forceinline__ void store_tile(double *S, int Np, int I, int K, const double (*t)[T + 1])
@@ -615,18 +635,17 @@ __device__ __forceinline__ void block_release(int *flag, int epoch)
     if (threadIdx.x == 0) st_release(flag, epoch);
 }
 
-// Flags: tile (I, K) at tile_task(I, K); that slot is raised for the
-// diagonal tile (I, I) when L_II and its inverse are stored, and for the
-// sub-diagonal tile (I+1, I) when L_{I+1,I} and y_I are stored.  By mail go, beside
-// these, the partial diagonal PD(I) = A_II - sum_{J <= I-2} L_IJ L_IJ^T (with
-// b_I likewise), the partial sub-diagonal SUB(I) = A_{I+1,I} -
-// sum_{J <= I-1} L_{I+1,J} L_IJ^T, and the second-subdiagonal tile (K+2, K)
-// after its accumulation, before its solve.
+// Flags: tile (I, K), I > K, at tile_task(I, K), raised when it is stored (and
+// y_K with (K+1, K)).  By mail go, beside that, the diagonal inverses, the
+// sub-diagonal tiles and y, the partial diagonal PD(I) =
+// A_II - sum_{J <= I-2} L_IJ L_IJ^T (with b_I likewise), the partial sub-diagonal
+// SUB(I) = A_{I+1,I} - sum_{J <= I-1} L_{I+1,J} L_IJ^T, and the
+// second-subdiagonal tile (K+2, K) after its accumulation, before its solve.
 //
 // The factor with the forward solve of rhs carried along.  CTA 0 (the panel)
 // walks the diagonal: step I applies the last update to PD(I) with L_{I,I-1}
-// (its own, kept in shared memory), factors the tile and stores L_II and Linv_II
-// (panel_factor), then forms L_{I+1,I} = SUB(I) Linv_II^T, which it keeps, and
+// (its own, kept in shared memory), factors the tile (panel_factor), stores
+// Linv_II (panel_finish; nothing reads L_II) and forms L_{I+1,I} = SUB(I) Linv_II^T, which it keeps, and
 // y_I.  The other CTAs (helpers) run the task list: the tiles (I, K) with
 // I >= K + 2 (left-looking updates, then the triangular solve with Linv_KK),
 // and the PD and SUB accumulations, in the order
@@ -655,9 +674,10 @@ __global__ void __launch_bounds__(CF_THREADS, 1) k_chol_dataflow(int Np, int nb,
     __syncthreads();
     if (blockIdx.x == 0) {
         // ---- panel.  Step I: warps 0-6 update and factor the diagonal tile;
-        // warp 4 raises its flag; warps 0-3 form L_{I+1,I}, warps 5 and 6 y_I, and
-        // warp 7, which raises their flag when the next step begins, fetches
-        // SUB(I) and then PD(I+1) with its b as they come.  The panel tracks failure
+        // warps 0-3 form L_{I+1,I} (the columns' factor t last, so that its
+        // roots are not waited for), while warps 4-6 finish the tile's outputs and
+        // y_I; warp 7, which raises L_{I+1,I}'s flag when the next step begins,
+        // fetches SUB(I) and then PD(I+1) with its b as they come.  The panel tracks failure
         // itself (a bad pivot, a wait that ran out): it then leaves the loop
         // and raises all flags that are left.
         double(*lsub)[T + 1] = bi[2], (*asub)[T + 1] = bi[3], (*wli)[T + 1] = bi[4];
@@ -672,6 +692,10 @@ __global__ void __launch_bounds__(CF_THREADS, 1) k_chol_dataflow(int Np, int nb,
         __syncthreads();
         if (warp == 7) tile_exp(bi[0], hexp[0]);
         __syncthreads();
+        PfOut po{{T, T}, {0, 0}};
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+            if (warp >= 4 && warp < 7 && tid - 128 + 96 * j < TRI) tri_of(tid - 128 + 96 * j, po.r[j], po.c[j]);
         int pd_r[5], pd_c[5];  // warp 7's places in PD's mail
 #pragma unroll
         for (int q = 0; q < 5; ++q) tri_of(min(lane + 32 * q, TRI - 1), pd_r[q], pd_c[q]);
@@ -713,34 +737,43 @@ __global__ void __launch_bounds__(CF_THREADS, 1) k_chol_dataflow(int Np, int nb,
                     if (!ok) stop[cur] = 1;
                 }
             } else {
-                const bool bad = panel_factor(bi[cur], hexp[cur], lsub, by[cur], wy, I == 0, wli,
-                                              S + (size_t)(I * T) * Np + I * T, Np, Linv + (size_t)I * TT, mail + (size_t)I * ML_COLUMN, epoch, pw, pe);
-                if (warp == 4 && lane == 0) {
-                    if (bad) {
+                ulonglong2 *mc = mail + (size_t)I * ML_COLUMN;
+                panel_factor(bi[cur], hexp[cur], lsub, by[cur], wy, I == 0, wli, pw, pe);
+                if (warp >= 4) {
+                    const bool bad = panel_finish(wli, hexp[cur], by[cur], wy, I + 1 < nb, Linv + (size_t)I * TT,
+                                                  rhs + I * T, mc, epoch, pw, po);
+                    if (tid == 128 && bad) {
                         atomicCAS(status, 0, 1);
                         stop[cur] = 1;
                     }
-                    st_release(flags + tile_task(I, I, nb), epoch);
-                }
-                if (warp >= 5) panel_y(wli, by[cur], wy, rhs + I * T, mail + (size_t)I * ML_COLUMN, epoch);
-                if (warp < 4 && I + 1 < nb) {
+                } else if (I + 1 < nb) {
                     pf_bar<3, 160>();  // SUB(I) is there
                     double *Lg = S + (size_t)((I + 1) * T) * Np + I * T;
-                    tile_trsm(asub, wli, [&](int r, int c, double v) {
-                        mail_put(mail + (size_t)I * ML_COLUMN + ML_SUBD + r * T + c, v, epoch);
-                        lsub[r][c] = v;
-                        Lg[(size_t)r * Np + c] = v;
+                    double v0, v1;
+                    int r, c0, c1;
+                    tile_trsm(asub, wli, [&](int i, int j0, int j1, double x0, double x1) {
+                        r = i;
+                        c0 = j0;
+                        c1 = j1;
+                        v0 = x0;
+                        v1 = x1;
                     });
+                    pf_bar<5, 160>();  // t
+                    v0 *= pw.t[c0];
+                    v1 *= pw.t[c1];
+                    mail_put(mc + ML_SUBD + r * T + c0, v0, epoch);
+                    mail_put(mc + ML_SUBD + r * T + c1, v1, epoch);
+                    lsub[r][c0] = v0;
+                    lsub[r][c1] = v1;
+                    Lg[(size_t)r * Np + c0] = v0;
+                    Lg[(size_t)r * Np + c1] = v1;
                 }
             }
             __syncthreads();
             failed = stop[cur] != 0;
         }
         if (tid == 0 && failed)
-            for (int J = I - 1; J < nb; ++J) {
-                st_release(flags + tile_task(J, J, nb), epoch);
-                if (J + 1 < nb) st_release(flags + tile_task(J + 1, J, nb), epoch);
-            }
+            for (int J = I - 1; J + 1 < nb; ++J) st_release(flags + tile_task(J + 1, J, nb), epoch);
         return;
     }
     // ---- helpers
@@ -817,7 +850,10 @@ __global__ void __launch_bounds__(CF_THREADS, 1) k_chol_dataflow(int Np, int nb,
                 linv[inv_r][inv_c] = v[0];
                 if (tid < TRI - TT / 2) linv[T - 1][tid + TT / 2 - tri_at(T - 1, 0)] = v[1];
                 pf_bar<3, TT / 2>();
-                tile_trsm(bi[1], linv, [&](int i, int j, double x) { bi[0][i][j] = x; });
+                tile_trsm(bi[1], linv, [&](int i, int j0, int j1, double x0, double x1) {
+                    bi[0][i][j0] = x0;
+                    bi[0][i][j1] = x1;
+                });
             } else {
                 const int u = tid - TT / 2;
                 double v[2];
@@ -846,11 +882,18 @@ __global__ void __launch_bounds__(CF_THREADS, 1) k_chol_dataflow(int Np, int nb,
         } else {
             // the second-subdiagonal tile before its solve, for PD(K + 2) and SUB(K + 1)
             if (kind == 2) mail_put(mail + (size_t)K * ML_COLUMN + ML_PRE + tid, a[tid / T][tid % T], epoch);
-            block_wait(flags + tile_task(K, K, nb), nullptr, epoch, status);
-            for (int e2 = tid; e2 < TT; e2 += CF_THREADS) linv[e2 / T][e2 % T] = __ldcg(Linv + (size_t)K * TT + e2);
+            if (tid < TRI) {
+                double v[1];
+                mail_get(mail + (size_t)K * ML_COLUMN + ML_INV + tid, 0, 1, v, epoch, status);
+                linv[inv_r][inv_c] = v[0];
+            }
             __syncthreads();
             if (warp < 4)
-                tile_trsm(a, linv, [&](int r, int c, double v) { S[(size_t)(I * T + r) * Np + K * T + c] = v; });
+                tile_trsm(a, linv, [&](int r, int c0, int c1, double v0, double v1) {
+                    double *row = S + (size_t)(I * T + r) * Np + K * T;
+                    row[c0] = v0;
+                    row[c1] = v1;
+                });
             block_release(flags + tile_task(I, K, nb), epoch);
         }
         __syncthreads();
