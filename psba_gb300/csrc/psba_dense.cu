@@ -967,210 +967,310 @@ __global__ void __launch_bounds__(TS_THREADS) k_tri_solve(int refine, int Np, in
 // ---------------------------------------------------------------------------
 // The triangular solves on a thread-block cluster of TC_CTAS CTAs (one SM
 // each): the back solve after the factor, or (refine = 1) both solves of a
-// refinement residual, added into x.  One SM's FP64 rate bounds a one-CTA solve (N^2 / 2 multiply-adds);
-// the cluster spreads the updates over TC_CTAS SMs and passes each step's
-// solved block through distributed shared memory with one cluster barrier
-// per step (~400 cycles on GB300, against 1-2 us for a flag in L2).
-// Block I of the vector is owned by CTA I mod TC_CTAS, which holds it in
-// shared memory.  Step K: the owner solves block K (16 x 16 product with
-// the diagonal inverse, 256 threads, fixed shuffle tree), publishes it and
-// arrives at the barrier; while the barrier completes, every CTA applies the
-// previous step's block to its other blocks; after it, every CTA reads block
-// K from the owner and first updates the block the next step needs (if it
-// owns it), so the next owner can solve and arrive at once.  The diagonal
-// inverse entries and the coefficients of both updates are loaded a step
-// ahead, after the arrive.  The forward solve runs the same steps in the
-// other direction over the rows of L.  Each vector entry takes its updates
-// in step order: results do not depend on timing.
-constexpr int TC_CTAS = 8, TC_THREADS = 256;
+// refinement residual, added into x.  Block after block, x_p = D_p y_p with the
+// diagonal inverse, then y_r -= C_pr x_p for every later block r: a chain of nb
+// steps, each two 16 x 16 products long when nothing else is waited for.
+// CTA 0 keeps that chain to itself.  Two pairs of its warps take the diagonal
+// product and the update of the next block in turns (four lanes an entry, four
+// terms each, a fixed tree), warps 2 and 3 the update of the block after that,
+// from x_p as soon as it is known.  All blocks from the third on take x_p in the other
+// CTAs: block p is CTA 1 + p mod 7's, which sends it to CTA 0 with all its
+// updates but the last two, two chain steps before it is needed.  x_p and these
+// blocks travel as st.async stores that complete an mbarrier of their own (one
+// per block and pass, used once), ~350 cycles, where one cluster barrier per
+// step, with the solving CTA changing every step, made a step of 3,300
+// cycles.  Each entry takes its updates in step order: results do not depend on
+// timing.  A step is 1,500 cycles, two products of ~500 (six dependent FP64
+// instructions and two shuffles each) and ~500 of barriers and shared memory:
+// N = 528 takes 28 us, with a barrier of the cluster a step 56.
+constexpr int TC_CTAS = 8, TC_THREADS = 256, TC_OWNERS = TC_CTAS - 1;
+constexpr int TC_NEAR = 3;           // blocks up to p + TC_NEAR - 1 take x_p in CTA 0
+constexpr int TC_POLLS = 1 << 20;    // polls per wait (~1 s)
 
-__device__ __forceinline__ void cl_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cl_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ unsigned smem_at(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 
-// v[c] -= sum_r P(r, c) xs[r] for the columns (back) or rows (forward) listed
-// by idx(q), q < n: four threads per entry, four terms each, fixed tree.  The
-// first pass (q < TC_THREADS / 4) takes its four coefficients from first[],
-// loaded by the caller a step ahead; later passes load them here.
-template <typename Coef, typename Idx>
-__device__ __forceinline__ void cl_update(double *v, const double *xs, int n, const double (&first)[4], Coef coef,
-                                          Idx idx)
+__device__ __forceinline__ void mb_init(unsigned long long *b, int count)
 {
-    const int g = threadIdx.x & 3;
-    for (int q0 = 0; q0 < n; q0 += TC_THREADS / 4) {
-        const int q = q0 + (threadIdx.x >> 2);
-        double s = 0.0;
-        int c = 0;
-        if (q < n) {
-            c = idx(q);
-            if (q0 == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_at(b)), "r"(count) : "memory");
+}
+
+__device__ __forceinline__ void mb_expect(unsigned long long *b, int bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_at(b)), "r"(bytes) : "memory");
+}
+
+__device__ __forceinline__ void mb_arrive(unsigned long long *b)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_at(b)) : "memory");
+}
+
+// Waits for the barrier's first phase; *dead is set, and nothing waited for any
+// more, when the polls run out.
+__device__ __forceinline__ void mb_wait(unsigned long long *b, bool *dead)
+{
+    if (*dead) return;
+    for (int it = 0; it < TC_POLLS; ++it) {
+        int ok;
+        asm volatile("{ .reg .pred q; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 q, [%1], 0; selp.s32 %0, 1, 0, q; }"
+                     : "=r"(ok)
+                     : "r"(smem_at(b))
+                     : "memory");
+        if (ok) return;
+    }
+    *dead = true;
+}
+
+// The address of p's place in the shared memory of CTA `rank`
+__device__ __forceinline__ unsigned peer_at(const void *p, int rank)
+{
+    unsigned a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_at(p)), "r"(rank));
+    return a;
+}
+
+// v to another CTA's shared memory, 8 bytes of what its barrier there waits for
+__device__ __forceinline__ void send(unsigned place, unsigned bar, double v)
+{
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(place),
+                 "l"(__double_as_longlong(v)), "r"(bar)
+                 : "memory");
+}
+
+// Four lanes of one output: their sum in all of them
+__device__ __forceinline__ double quad_sum(double s)
+{
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    return s + __shfl_xor_sync(0xffffffffu, s, 2);
+}
+
+__device__ __forceinline__ double dot4(const double (&cf)[4], const double *v)
+{
+    double s = cf[0] * v[0];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) s = fma(first[j], xs[4 * g + j], s);
-            } else {
+    for (int j = 1; j < 4; ++j) s = fma(cf[j], v[j], s);
+    return quad_sum(s);
+}
+
+// The matrix as the chain sees it, by positions (0 is solved first)
+template <bool FWD>
+struct TriView {
+    const double *S, *Linv;
+    int Np, nb;
+    __device__ __forceinline__ int block(int p) const { return FWD ? p : nb - 1 - p; }
+    // terms 4 g .. 4 g + 3 of entry c of the diagonal product at p: a place that
+    // moves by diag_step from one p to the next
+    __device__ __forceinline__ const double *diag_at(int p, int c, int g) const
+    {
+        return Linv + (size_t)block(p) * TT + (FWD ? c * T + 4 * g : 4 * g * T + c);
+    }
+    __device__ __forceinline__ ptrdiff_t diag_step() const { return FWD ? TT : -TT; }
+    __device__ __forceinline__ static void diag(const double *L, int c, int g, double (&v)[4])
+    {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) s = fma(coef(4 * g + j, c), xs[4 * g + j], s);
+        for (int j = 0; j < 4; ++j) v[j] = (FWD ? 4 * g + j <= c : 4 * g + j >= c) ? __ldcg(L + (FWD ? j : j * T)) : 0.0;
+    }
+    // terms of what entry c of the block at r takes of x_p; moves by coef_step when
+    // both move on
+    __device__ __forceinline__ const double *coef_at(int p, int r, int c, int g) const
+    {
+        const int P = block(p) * T, R = block(r) * T;
+        return S + (FWD ? (size_t)(R + c) * Np + P + 4 * g : (size_t)(P + 4 * g) * Np + R + c);
+    }
+    __device__ __forceinline__ ptrdiff_t coef_step() const { return (ptrdiff_t)(FWD ? T : -T) * (Np + 1); }
+    __device__ __forceinline__ void coef(const double *L, double (&v)[4]) const
+    {
+        const unsigned st = FWD ? 1 : Np;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = __ldcg(L + j * st);
+    }
+};
+
+// One solve: base (Np) is the right-hand side, xs takes the solution in every
+// CTA, far (Np) is CTA 0's inbox and the others' blocks, bars 2 nb barriers.
+template <bool FWD>
+__device__ __forceinline__ void tri_pass(const TriView<FWD> &m, int rank, const double *base, double *xs, double *far,
+                                         unsigned long long *bars, double (*yb)[T], double (*near2)[T], bool *dead)
+{
+    const int tid = threadIdx.x, lane = tid & 31, g = tid & 3, nb = m.nb;
+    if (rank == 0) {
+        unsigned long long *bfar = bars, *bx = bars + nb;
+        const int c = (tid & 63) >> 2;
+        if (tid < 64 || (tid >= 128 && tid < 192)) {
+            // the chain: even p by warps 0 and 1, odd p by warps 4 and 5, so that
+            // what follows a step (x to the others, the next coefficients' loads,
+            // ~500 cycles) goes beside the next one
+            const int set = tid >= 128;
+            double dg[4] = {}, cr[4] = {};
+            const double *dp = m.diag_at(min(set, nb - 1), c, g), *cp = m.coef_at(min(set, nb - 1), min(set + 1, nb - 1), c, g);
+            const ptrdiff_t ds = 2 * m.diag_step(), cs = 2 * m.coef_step();
+            if (set < nb) m.diag(dp, c, g, dg);
+            if (set + 1 < nb) m.coef(cp, cr);
+            int at = m.block(set) * T + c;
+            // where x goes: CTAs 1 + g and 5 + g (whose barrier p is x_p's)
+            unsigned to0 = peer_at(xs, 1 + g) + at * (int)sizeof(double), to1 = peer_at(xs, g < 3 ? 5 + g : 0) + at * (int)sizeof(double);
+            unsigned tb0 = peer_at(bars + set, 1 + g), tb1 = peer_at(bars + set, g < 3 ? 5 + g : 0);
+            if (set == 0) {
+                if (g == 0) yb[0][c] = base[at];
+                pf_bar<1, 64>();
+            }
+            for (int p = set; p < nb; p += 2) {
+                if (set) pf_bar<5, 128>();  // y_p is there
+                else if (p > 0) pf_bar<4, 128>();
+                const double x = dot4(dg, yb[set] + 4 * g);
+                if (g == 0) xs[at] = x;
+                if (set) pf_bar<6, 64>();
+                else pf_bar<1, 64>();
+                if (p + 1 < nb) {
+                    const double u = dot4(cr, xs + (at - c) + 4 * g);
+                    double b;
+                    if (p > 0) {
+                        if (set) pf_bar<2, 128>();
+                        else pf_bar<3, 128>();
+                        b = near2[set ^ 1][c];
+                    } else {
+                        b = base[m.block(1) * T + c];
+                    }
+                    if (g == 0) yb[set ^ 1][c] = b - u;
+                    if (set) pf_arrive<4, 128>();
+                    else pf_arrive<5, 128>();
+                }
+                if (lane == 0) mb_arrive(bx + p);
+                send(to0, tb0, x);
+                if (g < 3) send(to1, tb1, x);
+                if (p + 2 < nb) m.diag(dp += ds, c, g, dg);
+                if (p + 3 < nb) m.coef(cp += cs, cr);
+                constexpr int ahead = 2 * (FWD ? T : -T);
+                at += ahead;
+                to0 += ahead * (int)sizeof(double);
+                to1 += ahead * (int)sizeof(double);
+                tb0 += 2 * sizeof(unsigned long long);
+                tb1 += 2 * sizeof(unsigned long long);
+            }
+        } else if (tid >= 64 && tid < 128) {
+            double cf[4], cn[4] = {}, cm[4] = {};
+            const double *cp = m.coef_at(0, min(2, nb - 1), c, g);
+            const ptrdiff_t cs = m.coef_step();
+            if (nb > 2) m.coef(cp, cf);
+            if (nb > 3) m.coef(cp += cs, cn);
+            for (int p = 2; p < nb; ++p) {
+                if (p + 2 < nb) m.coef(cp += cs, cm);
+                if (p >= TC_NEAR) mb_wait(bfar + p, dead);
+                const double b = (p >= TC_NEAR ? far : base)[m.block(p) * T + c];
+                mb_wait(bx + p - 2, dead);
+                const double v = b - dot4(cf, xs + m.block(p - 2) * T + 4 * g);
+                if (g == 0) near2[p & 1][c] = v;
+                // a barrier per parity: the next but one, p + 2, needs an x_p that
+                // the chain has only after it has taken this one
+                if (p & 1) pf_arrive<3, 128>();
+                else pf_arrive<2, 128>();
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    cf[j] = cn[j];
+                    cn[j] = cm[j];
+                }
             }
         }
-        s += __shfl_xor_sync(0xffffffffu, s, 1);
-        s += __shfl_xor_sync(0xffffffffu, s, 2);
-        if (q < n && g == 0) v[c] -= s;
+    } else {
+        // entry c of this CTA's blocks k, k + 4, k + 8, ... (four lanes)
+        const int c = (tid >> 2) & (T - 1), k = tid >> 6;
+        const int p0 = rank - 1 + TC_OWNERS * k, step = TC_OWNERS * (TC_THREADS / 64);
+        auto next = [&](int q) {  // the first of them at q or later
+            return q <= p0 ? p0 : p0 + (q - p0 + step - 1) / step * step;
+        };
+        if (g == 0)
+            for (int p = p0; p < nb; p += step) far[m.block(p) * T + c] = base[m.block(p) * T + c];
+        double cf[4] = {}, cn[4] = {}, cm[4] = {};
+        auto coef = [&](int q, int p, double (&v)[4]) { m.coef(m.coef_at(q, p, c, g), v); };
+        if (next(TC_NEAR) < nb) coef(0, next(TC_NEAR), cf);
+        if (next(TC_NEAR + 1) < nb) coef(1, next(TC_NEAR + 1), cn);
+        for (int q = 0; q < nb; ++q) {
+            int p = next(q + TC_NEAR);
+            const int pn = next(q + 2 + TC_NEAR);
+            if (pn < nb) coef(q + 2, pn, cm);
+            mb_wait(bars + q, dead);
+            const double *xq = xs + m.block(q) * T + 4 * g;
+            if (p < nb) {
+                const double s = dot4(cf, xq);
+                double *mine = far + m.block(p) * T + c;
+                if (g == 0) {
+                    const double v = *mine - s;
+                    if (p == q + TC_NEAR) send(peer_at(mine, 0), peer_at(bars + p, 0), v);
+                    else *mine = v;
+                }
+                for (p += step; p < nb; p += 2 * step) {
+                    double c0[4], c1[4] = {};
+                    const int p1 = p + step;
+                    coef(q, p, c0);
+                    if (p1 < nb) coef(q, p1, c1);
+                    const double s0 = dot4(c0, xq), s1 = dot4(c1, xq);
+                    if (g == 0) {
+                        far[m.block(p) * T + c] -= s0;
+                        if (p1 < nb) far[m.block(p1) * T + c] -= s1;
+                    }
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                cf[j] = cn[j];
+                cn[j] = cm[j];
+            }
+        }
     }
 }
 
-__global__ void __launch_bounds__(TC_THREADS) k_tri_cluster(int refine, int Np, int nb,
+__device__ __forceinline__ void cl_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+size_t tri_smem(int Np, int refine)
+{
+    const size_t passes = refine ? 2 : 1;
+    return passes * (2 * sizeof(double) * Np + 2 * sizeof(unsigned long long) * (Np / T));
+}
+
+__global__ void __launch_bounds__(TC_THREADS, 1) k_tri_cluster(int refine, int Np, int nb,
                                                             const double *__restrict__ S,
                                                             const double *__restrict__ Linv,
                                                             const double *__restrict__ rhs,
                                                             double *__restrict__ x, float2 *__restrict__ x2,
-                                                            const int *__restrict__ status)
+                                                            int *__restrict__ status)
 {
-    static_assert(TC_THREADS == TT, "one thread per term of the 16 x 16 diagonal product");
-    extern __shared__ double vec[];  // Np; this CTA's blocks are the valid ones
-    __shared__ double xb[2][T], xs[2][T];
-    cg::cluster_group cl = cg::this_cluster();
-    const int rank = (int)cl.block_rank(), tid = threadIdx.x;
+    static_assert(T == 16 && TC_CTAS == 8, "two sends a lane reach the other CTAs");
+    extern __shared__ double tri_sm[];  // per pass: x, inbox; then the barriers
+    __shared__ double yb[2][T], near2[2][T];
+    const int rank = (int)cg::this_cluster().block_rank(), tid = threadIdx.x, passes = refine ? 2 : 1;
     if (*status != 0) return;  // the same word for every CTA: all leave together
-    for (int I = rank; I < nb; I += TC_CTAS)
-        if (tid < T) vec[I * T + tid] = rhs[I * T + tid];
-    const int dr = tid / T, dk = tid % T;
-    const int cq = tid >> 2, cg4 = tid & 3;  // one entry of a block, four terms (threads 0..63)
-    auto mine = [&](int I) { return I >= 0 && I < nb && I % TC_CTAS == rank; };
-    // my first block above lo, and the entries of my blocks I with lo < I < hi
-    auto first_above = [&](int lo) { return lo < rank ? rank : rank + ((lo - rank) / TC_CTAS + 1) * TC_CTAS; };
-    auto n_between = [&](int lo, int hi) {
-        const int f = first_above(lo);
-        return f < hi ? ((hi - 1 - f) / TC_CTAS + 1) * T : 0;
-    };
-    auto entry_between = [&](int lo, int q) {  // q-th entry of my blocks above lo, ascending
-        return (first_above(lo) + (q / T) * TC_CTAS) * T + q % T;
-    };
-    // the next step's block update, from coefficients loaded a step ahead
-    auto crit_apply = [&](const double *xs_, const double (&cf)[4], int entry) {
-        double s = 0.0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) s = fma(cf[j], xs_[4 * cg4 + j], s);
-        s += __shfl_xor_sync(0xffffffffu, s, 1);
-        s += __shfl_xor_sync(0xffffffffu, s, 2);
-        if (cq < T && cg4 == 0) vec[entry] -= s;
-    };
-    __syncthreads();
-    // Every register loaded for the next step goes to the other half of a
-    // ping-pong pair (the loop is unrolled by two), so nothing waits for a
-    // load until the step that uses it; all loads are issued after the
-    // arrive (a load in flight at the arrive would hold up its release).
+    unsigned long long *bars = reinterpret_cast<unsigned long long *>(tri_sm + (size_t)2 * passes * Np);
+    for (int i = tid; i < passes * nb; i += TC_THREADS) {
+        unsigned long long *b = bars + (i >= nb ? nb + i : i);
+        mb_init(b, 1);  // a block on its way here: x_p, or in CTA 0 the block at p
+        mb_init(b + nb, 2);  // x_p in CTA 0, from its two warps
+        if (rank != 0 || i % nb >= TC_NEAR) mb_expect(b, T * sizeof(double));
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    cl_sync();
+    bool dead = false;
+    double *xs = tri_sm, *far = tri_sm + (size_t)passes * Np;
     if (refine) {
-        // L y = b: step K solves y_K = Linv_K b_K, then b_I -= L_IK y_K for I > K
-        auto ldiag = [&](int K) {
-            return mine(K) && dk <= dr ? __ldcg(Linv + (size_t)K * TT + dr * T + dk) : 0.0;
-        };
-        auto lcrit = [&](int K, double (&cf)[4]) {  // rows of block K+1, columns of block K
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                cf[j] = (cq < T && mine(K + 1)) ? __ldcg(S + (size_t)((K + 1) * T + cq) * Np + K * T + 4 * cg4 + j)
-                                                : 0.0;
-        };
-        auto ldef = [&](int P, double (&df)[4]) {  // rows of my blocks above P + 1, columns of block P
-            const int n = n_between(P + 1, nb);
-            const int i = cq < n ? entry_between(P + 1, cq) : 0;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) df[j] = cq < n ? __ldcg(S + (size_t)i * Np + P * T + 4 * cg4 + j) : 0.0;
-        };
-        int pend = -1;
-        auto step = [&](int K, double &pl, double &pln, double (&cf)[4], double (&cfn)[4], double (&df)[4],
-                        double (&dfn)[4]) {
-            if (mine(K)) {
-                const double yv = half_warp_sum(pl * vec[K * T + dk]);
-                if (dk == 0) xb[K & 1][dr] = yv;
-            }
-            __syncthreads();
-            if (mine(K) && tid < T) vec[K * T + tid] = xb[K & 1][tid];
-            cl_arrive();
-            pln = K + 1 < nb ? ldiag(K + 1) : 0.0;
-            lcrit(K + 1, cfn);
-            ldef(K, dfn);
-            if (pend >= 0) {  // the previous step's block, applied to my blocks above pend + 1
-                const int P = pend;
-                cl_update(vec, xs[P & 1], n_between(P + 1, nb), df,
-                          [&](int r, int i) { return __ldcg(S + (size_t)i * Np + P * T + r); },
-                          [&](int q) { return entry_between(P + 1, q); });
-            }
-            cl_wait();
-            if (tid < T) xs[K & 1][tid] = cl.map_shared_rank(&xb[K & 1][0], K % TC_CTAS)[tid];
-            __syncthreads();
-            if (mine(K + 1)) crit_apply(xs[K & 1], cf, (K + 1) * T + cq);
-            __syncthreads();
-            pend = K;
-        };
-        double plA = ldiag(0), plB = 0.0, cfA[4], cfB[4], dfA[4] = {0.0, 0.0, 0.0, 0.0}, dfB[4];
-        lcrit(0, cfA);
-        for (int K = 0; K < nb; K += 2) {
-            step(K, plA, plB, cfA, cfB, dfA, dfB);
-            if (K + 1 < nb) step(K + 1, plB, plA, cfB, cfA, dfB, dfA);
-        }
-        // the last step's block reaches no block above it; every CTA has read
-        // it before the back solve's first step rewrites its buffer
-        cl_arrive();
-        cl_wait();
+        tri_pass(TriView<true>{S, Linv, Np, nb}, rank, rhs, xs, far, bars, yb, near2, &dead);
+        __syncthreads();
+        tri_pass(TriView<false>{S, Linv, Np, nb}, rank, xs, xs + Np, far + Np, bars + 2 * nb, yb, near2, &dead);
+        xs += Np;
+    } else {
+        tri_pass(TriView<false>{S, Linv, Np, nb}, rank, rhs, xs, far, bars, yb, near2, &dead);
     }
-    {
-        // L^T x = y: step K solves x_K = Linv_K^T y_K, then y_I -= L_KI^T x_K for I < K
-        auto ldiag = [&](int K) {
-            return mine(K) && dk >= dr ? __ldcg(Linv + (size_t)K * TT + dk * T + dr) : 0.0;
-        };
-        auto lcrit = [&](int K, double (&cf)[4]) {  // rows of block K, columns of block K-1
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                cf[j] = (cq < T && mine(K - 1)) ? __ldcg(S + (size_t)(K * T + 4 * cg4 + j) * Np + (K - 1) * T + cq)
-                                                : 0.0;
-        };
-        auto ldef = [&](int P, double (&df)[4]) {  // rows of block P, columns of my blocks below P - 1
-            const int n = n_between(-1, P - 1);
-            const int c = cq < n ? entry_between(-1, cq) : 0;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) df[j] = cq < n ? __ldcg(S + (size_t)(P * T + 4 * cg4 + j) * Np + c) : 0.0;
-        };
-        int pend = -1;
-        auto step = [&](int K, double &pl, double &pln, double (&cf)[4], double (&cfn)[4], double (&df)[4],
-                        double (&dfn)[4]) {
-            if (mine(K)) {
-                const double xv = half_warp_sum(pl * vec[K * T + dk]);
-                if (dk == 0) xb[K & 1][dr] = xv;
-            }
-            __syncthreads();
-            // x_K replaces y_K in the owner's vector (no global store before the release)
-            if (mine(K) && tid < T) vec[K * T + tid] = xb[K & 1][tid];
-            cl_arrive();
-            pln = K > 0 ? ldiag(K - 1) : 0.0;
-            lcrit(K - 1, cfn);
-            ldef(K, dfn);
-            if (pend >= 0) {  // the previous step's block, applied to my blocks below pend - 1
-                const int P = pend;
-                cl_update(vec, xs[P & 1], n_between(-1, P - 1), df,
-                          [&](int r, int c) { return __ldcg(S + (size_t)(P * T + r) * Np + c); },
-                          [&](int q) { return entry_between(-1, q); });
-            }
-            cl_wait();
-            if (tid < T) xs[K & 1][tid] = cl.map_shared_rank(&xb[K & 1][0], K % TC_CTAS)[tid];
-            __syncthreads();
-            if (mine(K - 1)) crit_apply(xs[K & 1], cf, (K - 1) * T + cq);
-            __syncthreads();
-            pend = K;
-        };
-        double plA = ldiag(nb - 1), plB = 0.0, cfA[4], cfB[4], dfA[4] = {0.0, 0.0, 0.0, 0.0}, dfB[4];
-        lcrit(nb - 1, cfA);
-        for (int K = nb - 1; K >= 0; K -= 2) {
-            step(K, plA, plB, cfA, cfB, dfA, dfB);
-            if (K - 1 >= 0) step(K - 1, plB, plA, cfB, cfA, dfB, dfA);
+    if (dead) atomicCAS(status, 0, 2);
+    __syncthreads();
+    // every block sent to a CTA has been waited for there; a CTA that gave up
+    // stays until all have sent
+    cl_sync();
+    if (rank == 0)
+        for (int i = tid; i < Np; i += TC_THREADS) {
+            const double xv = refine ? x[i] + xs[i] : xs[i];
+            x[i] = xv;
+            if (x2) x2[i] = split2f(xv);
         }
-        // no CTA may leave while another can still read its shared memory
-        cl_arrive();
-        cl_wait();
-        for (int I = rank; I < nb; I += TC_CTAS)
-            if (tid < T) {
-                const double xv = refine ? x[I * T + tid] + vec[I * T + tid] : vec[I * T + tid];
-                x[I * T + tid] = xv;
-                if (x2) x2[I * T + tid] = split2f(xv);
-            }
-    }
 }
 
 // The triangular solves after the factor: the back solve of d.rhs into x
@@ -1185,8 +1285,10 @@ void launch_tri(const DeviceProblem &d, int refine, double *x, cudaStream_t s)
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(TC_CTAS);
     cfg.blockDim = dim3(TC_THREADS);
-    cfg.dynamicSmemBytes = sizeof(double) * Np;
+    cfg.dynamicSmemBytes = tri_smem(Np, refine);
     cfg.stream = s;
+    if (cfg.dynamicSmemBytes > 40 * 1024)  // above the default limit (as for k_cholmod: the same value always)
+        cudaFuncSetAttribute(k_tri_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tri_smem(4096, 1));
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = TC_CTAS;
@@ -1195,7 +1297,7 @@ void launch_tri(const DeviceProblem &d, int refine, double *x, cudaStream_t s)
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const double *S = d.S, *Linv = d.Linv, *rhs = d.rhs;
-    cudaLaunchKernelEx(&cfg, k_tri_cluster, refine, Np, nb, S, Linv, rhs, x, x2, (const int *)d.status);
+    cudaLaunchKernelEx(&cfg, k_tri_cluster, refine, Np, nb, S, Linv, rhs, x, x2, d.status);
 #else
     k_tri_solve<<<1, TS_THREADS, sizeof(double) * Np, s>>>(refine, Np, nb, d.S, d.Linv, d.rhs, x, x2, d.status);
 #endif
