@@ -138,12 +138,15 @@ __global__ void __launch_bounds__(FV_THREADS) k_schur_fxv(FxArgs g, const SchurU
     constexpr int SY = 3 * RP + 2, SW = 3 * CP + 2, NW = FV_THREADS / 32;
     constexpr int NV = n_out<CNP, DIAG>(), PER = (NV + FV_THREADS - 1) / FV_THREADS;
     constexpr int PIECES = 3 * RP / 2;  // 16-byte pieces of a row
-    __shared__ __align__(16) int2 sy[FX_CHUNK * SY], sw[FX_CHUNK * SW];
+    // this chunk's rows and, where 48 KB hold them (CNP 11), the next one's, which
+    // are then under way while this one is summed; else they are fetched after it
+    constexpr int NB = 2 * 8 * FX_CHUNK * (SY + SW) + 8 * NW * RP * CP <= 48 * 1024 ? 2 : 1;
+    __shared__ __align__(16) int2 sys[NB][FX_CHUNK * SY], sws[NB][FX_CHUNK * SW];
     __shared__ long long st[NW][RP * CP];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const SchurUnit u = units[blockIdx.x];
     const int *pa = DIAG ? g.cam_obs + u.begin : g.pa + u.begin, *pb = DIAG ? pa : g.pb + u.begin;
-    for (int e = tid; e < FX_CHUNK * SW; e += FV_THREADS) sw[e] = make_int2(0, 0);  // the padding columns
+    for (int e = tid; e < NB * FX_CHUNK * SW; e += FV_THREADS) sws[0][e] = make_int2(0, 0);  // the padding columns
     double acc[PER];
     int at[PER], we[PER];
 #pragma unroll
@@ -160,28 +163,41 @@ __global__ void __launch_bounds__(FV_THREADS) k_schur_fxv(FxArgs g, const SchurU
                                     DIAG ? u.slot : __ldg(g.pair_kl + 2 * u.slot + 1), r, c);
         }
     }
-    int ey = 0, e = 0, pt = 0;
+    // entry lane of a chunk, in every warp: its observations two chunks ahead,
+    // its exponents and (DIAG) its point one chunk ahead, with the rows
+    int an = 0, bn = 0, eyn = 0, en = 0, ptn = 0;
+    auto indices = [&](int t0) {
+        const int t = min(t0 + lane, u.count - 1);
+        an = __ldg(pa + t);
+        bn = DIAG ? an : __ldg(pb + t);
+    };
     auto fetch = [&](int t0) {
         const int n = min(FX_CHUNK, u.count - t0);
-        for (int p = tid; p < n * PIECES; p += FV_THREADS) {
-            const int t = p / PIECES, part = p % PIECES;
+        int2 *sy = sys[(t0 / FX_CHUNK) & (NB - 1)], *sw = sws[(t0 / FX_CHUNK) & (NB - 1)];
+#pragma unroll
+        for (int m = 0; m < (FX_CHUNK * PIECES + FV_THREADS - 1) / FV_THREADS; ++m) {
+            const int p = tid + FV_THREADS * m, t = p / PIECES, part = p % PIECES;
+            const int ia = __shfl_sync(0xffffffffu, an, t & 31), ib = DIAG ? ia : __shfl_sync(0xffffffffu, bn, t & 31);
+            if (t >= n) continue;
             const int wd = (part / (RP / 2)) * CP + 2 * (part % (RP / 2));
-            cp_async16(sy + t * SY + 2 * part, g.Yq + 3 * RP * (size_t)__ldg(pa + t0 + t) + 2 * part);
-            cp_async16(sw + t * SW + wd, g.Wq + 3 * RP * (size_t)__ldg(pb + t0 + t) + 2 * part);
+            cp_async16(sy + t * SY + 2 * part, g.Yq + 3 * RP * (size_t)ia + 2 * part);
+            cp_async16(sw + t * SW + wd, g.Wq + 3 * RP * (size_t)ib + 2 * part);
         }
-        e = -(1 << 20);
-        if (lane < n) {  // every warp: entry lane's exponents
-            const int a = __ldg(pa + t0 + lane);
-            const int2 xa = __ldg(g.ex + a);
-            ey = xa.x;
-            e = ey + (DIAG ? xa.y : __ldg(&g.ex[__ldg(pb + t0 + lane)].y));
-            if (DIAG) pt = __ldg(g.obs_pt + a);
+        en = -(1 << 20);
+        if (lane < n) {
+            const int2 xa = __ldg(g.ex + an);
+            eyn = xa.x;
+            en = eyn + (DIAG ? xa.y : __ldg(&g.ex[bn].y));
+            if (DIAG) ptn = __ldg(g.obs_pt + an);
         }
+        if (t0 + FX_CHUNK < u.count) indices(t0 + FX_CHUNK);
     };
+    indices(0);
     __syncthreads();
     fetch(0);
     for (int t0 = 0; t0 < u.count; t0 += FX_CHUNK) {
-        const int n = min(FX_CHUNK, u.count - t0);
+        const int n = min(FX_CHUNK, u.count - t0), e = en, ey = eyn, pt = ptn;
+        int2 *sy = sys[(t0 / FX_CHUNK) & (NB - 1)], *sw = sws[(t0 / FX_CHUNK) & (NB - 1)];
         const int E = __reduce_max_sync(0xffffffffu, e);
         const int d = E - e;
         bool bad = E >= FX_NAN / 2;  // the same in every warp
@@ -199,9 +215,9 @@ __global__ void __launch_bounds__(FV_THREADS) k_schur_fxv(FxArgs g, const SchurU
             Eg = __reduce_max_sync(0xffffffffu, lane < n ? ey + eg : -(1 << 20));
             bad |= __any_sync(0xffffffffu, nf);
         }
-        const int eyt = ey;
         cp_async_wait();
         __syncthreads();
+        if (NB == 2 && t0 + FX_CHUNK < u.count) fetch(t0 + FX_CHUNK);
         if (!bad) {
             if (lane < n) {
                 // entry lane's W row, d bits down; the warps share out the row
@@ -218,7 +234,7 @@ __global__ void __launch_bounds__(FV_THREADS) k_schur_fxv(FxArgs g, const SchurU
             if (DIAG) {
                 if (CNP < RP) __syncthreads();  // gb takes the place of the padding column that the shift has rewritten
                 if (lane < n && warp < 3)
-                    sw[lane * SW + warp * CP + CNP] = fx_limbs(gv[warp], Eg - eyt - fx_exp(gv[warp]));
+                    sw[lane * SW + warp * CP + CNP] = fx_limbs(gv[warp], Eg - ey - fx_exp(gv[warp]));
             }
         }
         __syncthreads();
@@ -241,7 +257,7 @@ __global__ void __launch_bounds__(FV_THREADS) k_schur_fxv(FxArgs g, const SchurU
                 }
         }
         __syncthreads();
-        if (t0 + FX_CHUNK < u.count) fetch(t0 + FX_CHUNK);
+        if (NB == 1 && t0 + FX_CHUNK < u.count) fetch(t0 + FX_CHUNK);
 #pragma unroll
         for (int p = 0; p < PER; ++p) {
             if (at[p] < 0) continue;
