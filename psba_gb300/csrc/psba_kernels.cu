@@ -947,6 +947,75 @@ __global__ void __launch_bounds__(CAM_THREADS, 1) k_camera_partial(const CamUnit
     }
 }
 
+// The FP64 sums of few units: PARTS CTAs a unit, each with every PARTS-th third
+// or ninth of the 27 values (blockIdx.y), in the same order as one CTA sums
+// them.  A unit is 1,024 observations x 54 multiply-adds, ~17 us at one SM's
+// FP64 rate, which few cameras leave most SMs without (7 cameras, 7 units:
+// 22.7 -> 10.4 us; 41 cameras in three parts 24.4 -> 14.0).  With more units than SMs the rows' loads, once per part, cost more.
+template <int PARTS, int P>
+__device__ __forceinline__ void camera_part(const CamUnit &u, const int *__restrict__ cam_obs, const double *__restrict__ A,
+                                            const double *__restrict__ ex, double (&acc)[CAM_NV / PARTS])
+{
+    constexpr int N = CAM_NV / PARTS;
+#pragma unroll
+    for (int j = 0; j < N; ++j) acc[j] = 0.0;
+    const int k0 = threadIdx.x * CAM_PER, k1 = min(u.count, k0 + CAM_PER);
+#pragma unroll 2
+    for (int kk = k0; kk < k1; ++kk) {
+        const int o = __ldg(cam_obs + u.begin + kk);
+        double a[12], e2[2];
+        ldn<double, 12>(A + 12 * (size_t)o, a);
+        ld2<double>(ex + 2 * (size_t)o, e2[0], e2[1]);
+        int v = 0;
+#pragma unroll
+        for (int r = 0; r < 6; ++r)
+#pragma unroll
+            for (int c = r; c < 6; ++c, ++v)
+                if (v / N == P) acc[v % N] = acc[v % N] + a[r] * a[c] + a[6 + r] * a[6 + c];
+#pragma unroll
+        for (int q = 0; q < 6; ++q)
+            if ((21 + q) / N == P) acc[(21 + q) % N] = acc[(21 + q) % N] + a[q] * e2[0] + a[6 + q] * e2[1];
+    }
+}
+
+template <int PARTS, int P = 0>
+__device__ __forceinline__ void camera_part_of(int p, const CamUnit &u, const int *__restrict__ cam_obs,
+                                               const double *__restrict__ A, const double *__restrict__ ex,
+                                               double (&acc)[CAM_NV / PARTS])
+{
+    if constexpr (P < PARTS) {
+        if (p == P) camera_part<PARTS, P>(u, cam_obs, A, ex, acc);
+        else camera_part_of<PARTS, P + 1>(p, u, cam_obs, A, ex, acc);
+    }
+}
+
+template <int PARTS>
+__global__ void __launch_bounds__(CAM_THREADS) k_camera_part(const CamUnit *__restrict__ units,
+                                                             const int *__restrict__ cam_obs, const double *__restrict__ A,
+                                                             const double *__restrict__ ex, double *__restrict__ partial)
+{
+    constexpr int N = CAM_NV / PARTS;
+    static_assert(N * PARTS == CAM_NV && CAM_THREADS == 128, "camera unit layout");
+    __shared__ double red[N][CAM_THREADS + 1];
+    const CamUnit u = units[blockIdx.x];
+    const int t = threadIdx.x;
+    double acc[N];
+    camera_part_of<PARTS>(blockIdx.y, u, cam_obs, A, ex, acc);
+#pragma unroll
+    for (int v = 0; v < N; ++v) red[v][t] = acc[v];
+    __syncthreads();
+    const int v = t >> 2, g = t & 3;
+    double s = 0.0;
+    if (v < N) {
+#pragma unroll 8
+        for (int q = 0; q < CAM_THREADS / 4; ++q) s += red[v][g * (CAM_THREADS / 4) + q];
+    }
+    // (s0 + s1) + (s2 + s3): the lanes of a value are neighbours
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    if (v < N && g == 0) partial[(size_t)blockIdx.x * CAM_NV + blockIdx.y * N + v] = s;
+}
+
 __global__ void k_camera_finish(int nc, const int *__restrict__ unit_start,
                                 const double *__restrict__ partial, double coeff,
                                 double *__restrict__ U, double *__restrict__ g,
@@ -980,7 +1049,11 @@ void launch_camera_blocks(const DeviceProblem &d, double coeff, cudaStream_t s)
 {
     if (d.cnp != 6) return launch_camera_blocks_v(d, coeff, s);
     if (d.n_cam_units > 0) {
-        if (d.prec == PSBA_PREC_FP64)
+        if (d.prec == PSBA_PREC_FP64 && d.n_cam_units <= 2 * 152 / 9)  // up to two CTAs per SM
+            k_camera_part<9><<<dim3(d.n_cam_units, 9), CAM_THREADS, 0, s>>>(d.cam_units, d.cam_obs, d.A, d.ex, d.cam_partial);
+        else if (d.prec == PSBA_PREC_FP64 && d.n_cam_units <= 152)
+            k_camera_part<3><<<dim3(d.n_cam_units, 3), CAM_THREADS, 0, s>>>(d.cam_units, d.cam_obs, d.A, d.ex, d.cam_partial);
+        else if (d.prec == PSBA_PREC_FP64)
             k_camera_partial<double><<<d.n_cam_units, CAM_THREADS, 0, s>>>(d.cam_units, d.cam_obs, d.A, d.ex,
                                                                              d.cam_partial);
         else
