@@ -16,11 +16,11 @@ estimate.  The metric is LM iterations per second.
   than L2 anyway).
 * e2e: the same metric through the C ABI from host buffers: psba_create
   (upload, index lists) + psba_levmar + psba_get_params per step, host clock.
-* roofline: the dominant kernel, k_schur (the Schur complement's
-  off-diagonal blocks in equal chunks of the pair list, and its diagonal
-  blocks in the same launch; one launch per LM trial), timed live with CUDA
-  events inside the timed solves; FP64-bound, so its peak is the measured
-  FP64 FMA rate.  roofline_chol: the dense solve (k_chol_dataflow +
+* roofline: the dominant kernel, k_schur_fx6 (the Schur complement's
+  off-diagonal and diagonal blocks, one launch per LM trial), timed live with
+  CUDA events inside the timed solves.  Its sums are in 57-bit fixed point on the
+  integer multiply pipe; the peak is the measured FP64 FMA rate that FP64 sums
+  would be bound by, so the fraction can exceed one.  roofline_chol: the dense solve (k_chol_dataflow +
   k_tri_cluster); roofline_mixed: the mixed form's Schur products
   (k_schur_f32) against the FP32 FMA rate and HBM.
 * matched_cost: solves at matched final cost, on the bench problem and
@@ -73,8 +73,8 @@ UNIT = "iterations/s"
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per launch, from
 # one ncu capture of this workload's kernels.
-SCHUR_TRAFFIC = 250.1e6
-CHOL_TRAFFIC = 1.30e6  # S (2.2 MB) stays in L2 between the Schur stage and the factor
+SCHUR_TRAFFIC = 275.4e6  # k_schur_fx6: 248.9 MB read + 26.5 MB written
+CHOL_TRAFFIC = 1.6e6  # S (2.2 MB) stays in L2 between the Schur stage and the factor
 SCHUR_F32_TRAFFIC = 83.1e6  # k_schur_f32, mixed form: 79.8 MB read + 3.3 MB written
 MATCH_TOL = 1e-6  # matched final cost: within 1e-6 relative of the FP64 converged cost
 
@@ -838,7 +838,7 @@ def main():
         h2d, d2h = a, b
     e2e_value = e2e_iters / e2e_s if e2e_s > 0 else None
 
-    # ---- rooflines: the dominant kernel (k_schur), the dense solve and the whole Schur stage
+    # ---- rooflines: the dominant kernel (k_schur_fx6), the dense solve and the whole Schur stage
     peak_gbs, peak_kind = measured_peaks()
     fp64_peak = P.measure_peak("fp64")
     # the FP64 tensor cores (mma.sync m8n8k4 / m16n8k16) against the FP64 FMA
@@ -852,9 +852,9 @@ def main():
     achieved_gbs = schur_bytes(sc) / schur_avg_s / 1e9
     fp64_achieved = schur_flops(cfg) / schur_avg_s / 1e12
     chol_avg_s = live["cholesky"][0] / max(live["cholesky"][1], 1) / 1e3
-    # k_schur (the "schur_off" stage: the diagonal units run in the same
+    # k_schur_fx6 (the "schur_off" stage: the diagonal units run in the same
     # launch): 6x6x3 FMAs per camera-pair entry and (21 + 6) x 3 per
-    # observation; algorithmic bytes are Y and W of every observation (FP64),
+    # observation; algorithmic bytes are Y and W of every observation (64 bits),
     # the two pair-entry lists and the camera-sorted observation list
     soff_avg_s = live["schur_off"][0] / max(live["schur_off"][1], 1) / 1e3
     soff_flops = schur_flops(cfg)
@@ -901,8 +901,9 @@ def main():
         "final_cost": costs[-1], "wall_ms_per_step": 1e3 * wall / args.steps,
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h),
                 "steps": args.e2e_steps},
-        "roofline": {"kernel": "k_schur: off-diagonal and diagonal blocks of the Schur complement, one launch "
-                               "per LM trial (the largest share of the launch list)",
+        "roofline": {"kernel": "k_schur_fx6: off-diagonal and diagonal blocks of the Schur complement, one launch "
+                               "per LM trial (the largest share of the launch list); 57-bit fixed-point sums, "
+                               "three integer multiply-adds a product, against the FP64 FMA rate",
                      "bound": "fp64", "achieved": soff_flops / soff_avg_s / 1e12, "peak": fp64_peak,
                      "unit": "TFLOP/s", "frac": soff_flops / soff_avg_s / 1e12 / fp64_peak,
                      "peak_source": "measured FP64 FMA rate (psba_measure_peak); MEASURED_PEAKS.json "
@@ -921,10 +922,10 @@ def main():
                      "hbm": {"achieved": chol_bytes / chol_avg_s / 1e9, "peak": peak_gbs, "unit": "GB/s",
                              "frac": chol_bytes / chol_avg_s / 1e9 / peak_gbs, "algorithmic_bytes": chol_bytes,
                              "peak_source": peak_kind}},
-        "roofline_schur": {"kernel": "schur (k_schur + k_schur_reduce), per trial",
+        "roofline_schur": {"kernel": "schur (k_schur_fx6 + k_schur_reduce), per trial",
                            "bound": "fp64", "achieved": fp64_achieved, "peak": fp64_peak, "unit": "TFLOP/s",
                            "frac": fp64_achieved / fp64_peak, "flops": schur_flops(cfg),
-                           "traffic": SCHUR_TRAFFIC, "traffic_kernel": "k_schur",
+                           "traffic": SCHUR_TRAFFIC, "traffic_kernel": "k_schur_fx6",
                            "avg_ms": schur_avg_s * 1e3,
                            "hbm": {"achieved": achieved_gbs, "peak": peak_gbs, "unit": "GB/s",
                                    "frac": achieved_gbs / peak_gbs, "algorithmic_bytes": schur_bytes(sc),

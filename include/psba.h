@@ -188,8 +188,7 @@ int psba_levmar_resume(psba_handle *h, const psba_opts *opts, double mu, int nu,
                        psba_result *res);
 
 /* Bound of the handle's device-side waits: the dense factor's waits on its
- * task flags and the Y kernel's wait for its bulk copies, in polls (0: the
- * default, 2^22, about half a second).  A wait that runs out ends its kernel
+ * tile flags and hand-offs, in polls (0: the default, 2^22, a second or two).  A wait that runs out ends its kernel
  * with a status the driver reads; the solve then returns PSBA_ERR_STATE and
  * the handle stays usable.  No reference counterpart: the reference's
  * device-side enqueue chain has no waits of its own (CL_files/SPD_inv.cl:165-179). */
@@ -317,7 +316,7 @@ int psba_batch_get_params(psba_batch *b, int problem, double *cams, double *pts)
 int psba_batch_reset_params(psba_batch *b);
 /* Tile/segment shape knobs set by the autotuner (psba_gb300.batch.autotune):
  * threads per CTA (128, 256, 512) and, per problem, lanes per camera pair in
- * the Schur stage (8, 16, 32). */
+ * the mixed form's Schur stage (8, 16, 32; the FP64 form always takes a warp). */
 int psba_batch_set_threads(psba_batch *b, int threads);
 int psba_batch_set_lanes_per_pair(psba_batch *b, const int *lanes);
 size_t psba_batch_device_bytes(psba_batch *b);
@@ -353,7 +352,7 @@ typedef struct psba_server_opts {
     int max_active;          /* resident problems of the batch lane at once (default 1024) */
     int slice_iters;         /* outer LM iterations of the heaviest problem per launch (default 1) */
     int threads;             /* CTA size of the persistent launch: 128, 256, 512 (default 256) */
-    int lanes_per_pair;      /* lanes per camera pair in the Schur stage: 8, 16, 32 (default 32) */
+    int lanes_per_pair;      /* lanes per camera pair in the mixed form's Schur stage: 8, 16, 32 (default 32) */
     int large_cams;          /* requests with more cameras run on the large lane (default 40; 0: no large lane) */
     int large_lanes;         /* large-lane host threads, each solving one request at a time (default 8) */
     double large_share;      /* share of hbm_budget_bytes reserved for the large lane (default 0.25) */

@@ -3,7 +3,7 @@
 ``Batch`` wraps psba_batch_* of include/psba.h: every problem runs the
 reference's levmar() control flow (PSBA/levmar.cpp:45-256) inside one CTA of
 a persistent kernel.  ``autotune`` picks the tile/segment shape per size
-bucket -- lanes per camera pair in the Schur stage for each bucket of
+bucket -- lanes per camera pair in the mixed form's Schur stage for each bucket of
 problems (bucketed by the mean number of common points per camera pair), and
 threads per CTA for the batch -- by timing one LM iteration of the batch for
 each candidate (coordinate descent, best of two runs).
