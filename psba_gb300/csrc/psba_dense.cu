@@ -7,8 +7,9 @@
 // along) and forms the sub-diagonal tile below it, which it keeps for the
 // next step.  The other CTAs (helpers) accumulate every other update
 // (left-looking) and solve the remaining tiles against the diagonal
-// inverses, in a fixed dependency order; waits are bounded spins on per-task
-// flags in global memory (acquire/release).  After the factor, the back
+// inverses, in a fixed dependency order; waits are bounded spins on per-tile
+// flags in global memory (acquire/release) or on the values themselves, sent
+// with the launch's epoch (mail).  After the factor, the back
 // solve L^T x = y runs on a thread-block cluster (k_tri_cluster; k_tri_solve,
 // one CTA, when PSBA_TRI_CLUSTER is 0).  On request one step of iterative
 // refinement follows: r = b - S x in FP64 against a copy of S taken before
@@ -18,8 +19,8 @@
 // This replaces the reference's explicit inverse (SPD_inv.cl: 3x3-block
 // Cholesky chain, kern_trigMat_inv, kern_trigMat_mul, then matVec_mul) with
 // two triangular solves.  The failure test is the reference's: a non-positive
-// or non-finite pivot (SPD_inv.cl:66-107) sets status 1; every task still
-// raises its flag, so nothing waits forever.  A spin that runs out of its
+// or non-finite pivot (SPD_inv.cl:66-107) sets status 1; every flag is still
+// raised and waits for mail end at the status, so nothing waits forever.  A spin that runs out of its
 // iteration budget sets status 2 and the kernel completes.
 #include <cfloat>
 #include <cooperative_groups.h>
@@ -49,8 +50,8 @@ constexpr int TT = TILE * TILE;
 #define PSBA_CHOL_PER_SM 1  // the panel's FP64 chain runs alone on its SM
 #endif
 constexpr int CF_THREADS = PSBA_CHOL_THREADS;
-// Polls per wait (each poll an acquire load and a 64 ns sleep; the default,
-// 2^22, is ~0.5 s) come from the launch: a handle can shorten the bound
+// Polls per wait (each one L2 round trip; the default, 2^22, is a second or
+// two) come from the launch: a handle can shorten the bound
 // (psba_set_wait_limit).  Thread 0 of each CTA stores it here at entry.
 __shared__ long long s_spin_limit;
 constexpr int BJ = PSBA_CHOL_BJ;             // update steps staged per batch in a tile task
@@ -622,11 +623,6 @@ __device__ __forceinline__ void tile_trsm(const double (*A)[T + 1], const double
     out(r, c0, c1, s0, s1);
 }
 
-__device__ __forceinline__ void store_tile(double *S, int Np, int I, int K, const double (*t)[T + 1])
-{
-    for (int e = threadIdx.x; e < TT; e += CF_THREADS) S[(size_t)(I * T + e / T) * Np + K * T + e % T] = t[e / T][e % T];
-}
-
 // After the CTA barrier, thread 0's release store orders every thread's
 // earlier writes (the barrier puts them before it) ahead of the flag.
 __device__ __forceinline__ void block_release(int *flag, int epoch)
@@ -1141,8 +1137,8 @@ __device__ __forceinline__ void tri_pass(const TriView<FWD> &m, int rank, const 
                 if (p + 3 < nb) m.coef(cp += cs, cr);
                 constexpr int ahead = 2 * (FWD ? T : -T);
                 at += ahead;
-                to0 += ahead * (int)sizeof(double);
-                to1 += ahead * (int)sizeof(double);
+                to0 += (unsigned)(ahead * (int)sizeof(double));
+                to1 += (unsigned)(ahead * (int)sizeof(double));
                 tb0 += 2 * sizeof(unsigned long long);
                 tb1 += 2 * sizeof(unsigned long long);
             }

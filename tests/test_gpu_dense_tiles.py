@@ -1,7 +1,7 @@
 """The dense solve at the edges of its 16 x 16 tiles.
 
 Sizes around one, two and three tiles, where the panel has no sub-diagonal
-tile, one, or the first tasks of the other CTAs:
+tile, one, or the first tasks of the other CTAs (and the largest):
 * the residual: a Cholesky solve's backward error is within (n + 1) eps of
   sqrt(a_ii a_jj) per entry, and the products with the tiles' explicit inverses
   multiply it by the tile factor's condition, sqrt(1e2) at most here; the
@@ -36,6 +36,18 @@ def system(n, seed):
 @pytest.mark.parametrize("n", SIZES)
 def test_residual(n):
     A, b = system(n, n)
+    st, x = P.dense_solve(np.tril(A), b)
+    assert st == 0
+    d = np.sqrt(np.diag(A))
+    bound = 4 * 10 * (n + 1) * np.finfo(float).eps * d * (d @ np.abs(x))
+    assert np.all(np.abs(A @ x - b) <= bound)
+
+
+@pytest.mark.parametrize("n", [2528, 2561, 4096])  # the back solve's shared memory below and above 40 KB, the largest
+def test_residual_large(n):
+    rng = np.random.default_rng(n)
+    B = rng.normal(size=(n, 64))
+    A, b = B @ B.T / 64 + 3 * np.eye(n), rng.normal(size=n)  # condition below 100
     st, x = P.dense_solve(np.tril(A), b)
     assert st == 0
     d = np.sqrt(np.diag(A))
