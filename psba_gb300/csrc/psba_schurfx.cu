@@ -315,13 +315,40 @@ __global__ void __launch_bounds__(FV_THREADS) k_camera_fx(const CamUnit *__restr
             at[p] = (v - NU) * CP + CNP;
         }
     }
+    // the thread's LD values of a chunk: the next chunk's are on their way while
+    // this one is summed, and their observations' indices one chunk before that
+    // (52 cameras: 99.4 -> 81.9 us)
+    constexpr int LD = (FX_CHUNK * 2 * NC + FV_THREADS - 1) / FV_THREADS;
+    int oi[LD];
+    double v[LD];
+    auto indices = [&](int t0) {
+#pragma unroll
+        for (int m = 0; m < LD; ++m) {
+            const int t = t0 + (tid + FV_THREADS * m) / (2 * NC);
+            oi[m] = t < min(u.count, t0 + FX_CHUNK) ? __ldg(cam_obs + u.begin + t) : -1;
+        }
+    };
+    auto values = [&] {
+#pragma unroll
+        for (int m = 0; m < LD; ++m) {
+            const int k = (tid + FV_THREADS * m) % (2 * NC), i = k / NC, c = k % NC;
+            if (oi[m] >= 0) v[m] = c < CNP ? __ldg(A + 2 * CNP * (size_t)oi[m] + i * CNP + c) : __ldg(ex + 2 * (size_t)oi[m] + i);
+        }
+    };
+    indices(0);
+    values();
+    if (FX_CHUNK < u.count) indices(FX_CHUNK);
     for (int t0 = 0; t0 < u.count; t0 += FX_CHUNK) {
         const int n = min(FX_CHUNK, u.count - t0);
         __syncthreads();  // the last chunk's limbs are read
-        for (int e = tid; e < n * 2 * NC; e += FV_THREADS) {
-            const int t = e / (2 * NC), k = e % (2 * NC), i = k / NC, c = k % NC;
-            const size_t o = __ldg(cam_obs + u.begin + t0 + t);
-            sa[t * ST + i * CP + c] = __double_as_longlong(c < CNP ? __ldg(A + 2 * CNP * o + i * CNP + c) : __ldg(ex + 2 * o + i));
+#pragma unroll
+        for (int m = 0; m < LD; ++m) {
+            const int e = tid + FV_THREADS * m, t = e / (2 * NC), k = e % (2 * NC);
+            if (t < n) sa[t * ST + k / NC * CP + k % NC] = __double_as_longlong(v[m]);
+        }
+        if (t0 + FX_CHUNK < u.count) {
+            values();
+            if (t0 + 2 * FX_CHUNK < u.count) indices(t0 + 2 * FX_CHUNK);
         }
         __syncthreads();
         // a warp per column, a lane per observation
