@@ -1561,12 +1561,19 @@ __global__ void k_schur_reduce(int n_pairs, int nc, int Np, const int *__restric
     S[(size_t)(6 * k + r) * Np + 6 * k + c] = (r == c ? uu + mu : uu) - sum;
 }
 
-__global__ void k_pad_identity(int N, int Np, double *S, double *rhs)
+// S zeroed, with the identity on its padding rows (and zeros in rhs there): one
+// launch where a memset before the reduction and a one-warp kernel behind it took
+// ~2 us more of every trial
+__global__ void __launch_bounds__(256) k_clear_padded(int N, int Np, double *S, double *rhs)
 {
-    const int i = N + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= Np) return;
-    S[(size_t)i * Np + i] = 1.0;
-    rhs[i] = 0.0;
+    const unsigned half = Np / 2, total = half * Np;  // Np <= 4096, a multiple of 16
+    const unsigned first = blockIdx.x * 256 + threadIdx.x;
+    for (unsigned e = first; e < total; e += gridDim.x * 256) {
+        const unsigned r = e / half, c = 2 * (e - r * half);
+        const bool pad = (int)r >= N && c == (r & ~1u);
+        reinterpret_cast<double2 *>(S)[e] = make_double2(pad && r == c ? 1.0 : 0.0, pad && r != c ? 1.0 : 0.0);
+    }
+    if (first < (unsigned)(Np - N)) rhs[N + first] = 0.0;
 }
 
 void launch_schur_off(const DeviceProblem &d, cudaStream_t s)
@@ -1591,15 +1598,13 @@ void launch_schur_diag(const DeviceProblem &d, cudaStream_t s)
 
 void launch_schur_reduce(const DeviceProblem &d, double mu, cudaStream_t s)
 {
-    cudaMemsetAsync(d.S, 0, sizeof(double) * (size_t)d.Np * d.Np, s);
-    if (d.cnp != 6) {
-        launch_schur_reduce_v(d, mu, s);
-        if (d.Np > d.N) {
-            k_pad_identity<<<1, TILE, 0, s>>>(d.N, d.Np, d.S, d.rhs);
-            note_launch(1);
-        }
-        return;
+    if (d.Np > d.N) {
+        k_clear_padded<<<std::min(ceil_div((long long)d.Np * d.Np / 2, 256), 152 * 8), 256, 0, s>>>(d.N, d.Np, d.S, d.rhs);
+        note_launch(1);
+    } else {
+        cudaMemsetAsync(d.S, 0, sizeof(double) * (size_t)d.Np * d.Np, s);
     }
+    if (d.cnp != 6) return launch_schur_reduce_v(d, mu, s);
     double *off_partial = d.schur_partial;
     double *diag_partial = d.schur_partial + off_partial_slots(d) * 36;
     const int total = d.n_pairs * 36 + d.nc * DIAG_NV;
@@ -1611,10 +1616,6 @@ void launch_schur_reduce(const DeviceProblem &d, double mu, cudaStream_t s)
                                                           diag_partial, d.U, d.g,
                                                           mu, d.S, d.rhs);
     note_launch(1);
-    if (d.Np > d.N) {
-        k_pad_identity<<<1, TILE, 0, s>>>(d.N, d.Np, d.S, d.rhs);
-        note_launch(1);
-    }
 }
 
 void launch_schur(const DeviceProblem &d, double mu, cudaStream_t s)
