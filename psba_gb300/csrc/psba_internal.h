@@ -336,9 +336,9 @@ void launch_update_params(const DeviceProblem &d, cudaStream_t s);
 
 // Deterministic reductions and vector helpers.
 void launch_sum_partials(const double *partial, int n, double *dst, cudaStream_t s);
-// |cams|^2 and |pts|^2 (into dst_cams, dst_pts) in one launch: nred blocks over the points, one over the
-// cameras, the last block summing the points' partials in index order
-void launch_param_norm(const DeviceProblem &d, int nred, double *partial, double *dst_cams, double *dst_pts,
+// cams += dpa, pts += dpb, then |cams|^2 and |pts|^2 (into dst_cams, dst_pts), in one launch: nred blocks over
+// the points, one over the cameras, the last block summing the points' partials in index order
+void launch_accept_norm(const DeviceProblem &d, int nred, double *partial, double *dst_cams, double *dst_pts,
                        cudaStream_t s);
 void launch_max_uvdiag(const DeviceProblem &d, double *dst, cudaStream_t s);
 void launch_dot(const double *x, const double *y, long long n, double *partial, int nblocks,

@@ -2004,21 +2004,31 @@ __global__ void k_sumsq_partial(const double *__restrict__ x, const double *__re
     if (threadIdx.x == 0) partial[blockIdx.x] = r[0];
 }
 
-// The parameters' squared norms for the LM stop test (levmar.cpp:150-152):
-// blocks below nred stride over the points' coordinates, block nred over
-// the cameras' parameters; fixed-order sums in every block and in the last.
-__global__ void __launch_bounds__(256) k_param_norm(const double *__restrict__ cams, int ncv,
-                                                    const double *__restrict__ pts, long long npv, int nred,
-                                                    double *__restrict__ partial, int *__restrict__ ticket,
-                                                    double *__restrict__ dst_cams, double *__restrict__ dst_pts)
+// Accept an LM step, cams += dpa and pts += dpb (compute_newp.cl + update_p.cl),
+// and the new parameters' squared norms for the stop test (levmar.cpp:150-152):
+// blocks below nred stride over the points' coordinates, block nred over the
+// cameras' parameters; fixed-order sums in every block and in the last.  (One
+// launch: a separate update before the norms took ~3 us more of an iteration.)
+__global__ void __launch_bounds__(256) k_accept_norm(double *__restrict__ cams, int ncv, double *__restrict__ pts,
+                                                     long long npv, const double *__restrict__ dp, int nred,
+                                                     double *__restrict__ partial, int *__restrict__ ticket,
+                                                     double *__restrict__ dst_cams, double *__restrict__ dst_pts)
 {
     __shared__ double r[256];
     double a = 0.0;
     if ((int)blockIdx.x < nred) {
         const long long stride = (long long)nred * 256;
-        for (long long k = (long long)blockIdx.x * 256 + threadIdx.x; k < npv; k += stride) a = fma(pts[k], pts[k], a);
+        for (long long k = (long long)blockIdx.x * 256 + threadIdx.x; k < npv; k += stride) {
+            const double x = pts[k] + dp[ncv + k];
+            pts[k] = x;
+            a = fma(x, x, a);
+        }
     } else {
-        for (int k = threadIdx.x; k < ncv; k += 256) a = fma(cams[k], cams[k], a);
+        for (int k = threadIdx.x; k < ncv; k += 256) {
+            const double x = cams[k] + dp[k];
+            cams[k] = x;
+            a = fma(x, x, a);
+        }
     }
     r[threadIdx.x] = a;
     __syncthreads();
@@ -2036,11 +2046,11 @@ __global__ void __launch_bounds__(256) k_param_norm(const double *__restrict__ c
     }
 }
 
-void launch_param_norm(const DeviceProblem &d, int nred, double *partial, double *dst_cams, double *dst_pts,
-                       cudaStream_t s)
+void launch_accept_norm(const DeviceProblem &d, int nred, double *partial, double *dst_cams, double *dst_pts,
+                        cudaStream_t s)
 {
-    k_param_norm<<<nred + 1, 256, 0, s>>>(d.cams, d.N, d.pts, 3LL * d.np, nred, partial, d.tickets + 2, dst_cams,
-                                          dst_pts);
+    k_accept_norm<<<nred + 1, 256, 0, s>>>(d.cams, d.N, d.pts, 3LL * d.np, d.dp, nred, partial, d.tickets + 2, dst_cams,
+                                           dst_pts);
     note_launch(1);
 }
 
@@ -2051,7 +2061,7 @@ void launch_dot(const double *x, const double *y, long long n, double *partial, 
     k_sum_partials<<<1, 256, 0, s>>>(partial, nblocks, dst); note_launch(1);
 }
 
-// Accept a step: cams += dpa, pts += dpb (compute_newp.cl + update_p.cl).
+// Accept a trust-region step: cams += dpa, pts += dpb.
 __global__ void k_update_params(int ncp, int npp, double *cams, double *pts, const double *dp)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;

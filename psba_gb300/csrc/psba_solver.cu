@@ -372,10 +372,10 @@ void enqueue_step(psba_handle *h, double mu)
     }
 }
 
-void enqueue_param_norm(psba_handle *h)
+void enqueue_accept(psba_handle *h)
 {
     DeviceProblem &d = h->d;
-    launch_param_norm(d, h->nred, d.red_partial + 4, h->scratch + SC_PL2A, h->scratch + SC_PL2B, h->stream);
+    launch_accept_norm(d, h->nred, d.red_partial + 4, h->scratch + SC_PL2A, h->scratch + SC_PL2B, h->stream);
 }
 
 void trace_push(psba_result *res, int itno, int kind, int acc, double damping, double rho, double cost,
@@ -476,8 +476,7 @@ int levmar_impl(psba_handle *h, const psba_opts *o, int *itno, psba_result *res,
                     tmp = 1.0 - tmp * tmp * tmp;
                     mu = mu * ((tmp >= (1.0 / 3.0)) ? tmp : (1.0 / 3.0));
                     nu = 2;
-                    launch_update_params(d, h->stream);
-                    enqueue_param_norm(h);
+                    enqueue_accept(h);
                     TRY(check_launch());
                     have_pl2_pending = true;
                     ex_L2 = new_ex_L2;
