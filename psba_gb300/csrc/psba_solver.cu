@@ -280,12 +280,17 @@ void enqueue_cost_current(psba_handle *h, double *ex_out)
     launch_residual(d, d.camtab, d.pts, nullptr, ex_out, d.red_partial, nb, h->scratch + SC_COST, h->stream);
 }
 
+// The FP32 table of the mixed Jacobian, where there is one
+float *linearize_tab32(const DeviceProblem &d) { return d.prec == PSBA_PREC_MIXED && d.cnp == 6 ? d.camtab32 : nullptr; }
+
 // Cost at p + step (into scal->new_cost).
 #ifndef PSBA_MIXED_DF_COST
 #define PSBA_MIXED_DF_COST 1  // the mixed form's LM trial cost in double-float FP32 arithmetic (else FP64)
 #endif
 
-void enqueue_cost_trial(psba_handle *h, const double *step)
+// tables: the camera tables at p + step complete, for a linearization there if the
+// step is accepted (~6 us of a launch that it then does without).
+void enqueue_cost_trial(psba_handle *h, const double *step, bool tables = false)
 {
     DeviceProblem &d = h->d;
     StageScope sc(h, ST_COST);
@@ -296,22 +301,24 @@ void enqueue_cost_trial(psba_handle *h, const double *step)
     // has just split into FP32 pairs): the double-float cost
     const bool df = PSBA_MIXED_DF_COST && d.prec == PSBA_PREC_MIXED && d.cnp == 6 && !d.wt && step == d.dp &&
                     (size_t)d.nc * RES_TAB2F * sizeof(float2) <= 48 * 1024;
-    launch_cam_tables(d, d.cams, step, d.camtab_new, h->stream, nullptr, df ? d.tab2f : nullptr);
+    launch_cam_tables(d, d.cams, step, d.camtab_new, h->stream, tables ? linearize_tab32(d) : nullptr,
+                      df || (tables && linearize_df(d)) ? d.tab2f : nullptr, tables ? 1 : 0);
     if (df)
         launch_residual_df(d, part, nb, &d.scal->new_cost, h->stream);
     else
         launch_residual(d, d.camtab_new, d.pts, step + d.N, nullptr, part, nb, &d.scal->new_cost, h->stream);
 }
 
-// Jacobian, U, V, W, g with factor coeff at the current parameters.
-void enqueue_linearize(psba_handle *h, double coeff)
+// Jacobian, U, V, W, g with factor coeff at the current parameters.  tables: the
+// camera tables are those of the trial that has just been accepted.
+void enqueue_linearize(psba_handle *h, double coeff, bool tables = false)
 {
     DeviceProblem &d = h->d;
     {
         StageScope sc(h, ST_LINEARIZE);
-        launch_cam_tables(d, d.cams, nullptr, d.camtab, h->stream,
-                          d.prec == PSBA_PREC_MIXED && d.cnp == 6 ? d.camtab32 : nullptr,
-                          linearize_df(d) ? d.tab2f : nullptr, 1);
+        if (!tables)
+            launch_cam_tables(d, d.cams, nullptr, d.camtab, h->stream, linearize_tab32(d),
+                              linearize_df(d) ? d.tab2f : nullptr, 1);
         launch_linearize(d, coeff, h->stream);
     }
     {
@@ -429,8 +436,10 @@ int levmar_impl(psba_handle *h, const psba_opts *o, int *itno, psba_result *res,
 
     int iter_flag = PSBA_ITER_CONTINUE;
     bool have_pl2_pending = false;
+    bool tables = false;  // d.camtab is the accepted trial's
     for (; *itno < o->max_iter && iter_flag == PSBA_ITER_CONTINUE; (*itno)++) {
-        enqueue_linearize(h, 1.0);
+        enqueue_linearize(h, 1.0, tables);
+        tables = false;
         if (res) res->n_linearizations++;
         h->linearized = 1;
         if (first) {
@@ -445,7 +454,7 @@ int levmar_impl(psba_handle *h, const psba_opts *o, int *itno, psba_result *res,
         while (true) {
             enqueue_reduced(h, mu);
             enqueue_step(h, mu);
-            enqueue_cost_trial(h, d.dp);
+            enqueue_cost_trial(h, d.dp, true);
             TRY(check_launch());
             TrialScalars ts;
             TRY(read_trial(h, &ts));
@@ -477,6 +486,8 @@ int levmar_impl(psba_handle *h, const psba_opts *o, int *itno, psba_result *res,
                     mu = mu * ((tmp >= (1.0 / 3.0)) ? tmp : (1.0 / 3.0));
                     nu = 2;
                     enqueue_accept(h);
+                    std::swap(d.camtab, d.camtab_new);
+                    tables = true;
                     TRY(check_launch());
                     have_pl2_pending = true;
                     ex_L2 = new_ex_L2;
