@@ -310,10 +310,10 @@ __device__ void vinv3(const double *Vi, double mu, double *out)
     out[5] = -(-a12 * a12 + a11 * a22) / T;
 }
 
-// FP64 form: V^-1, and Y = W V^-1 and W as limb rows (psba_fixed.h).  W's take the
-// place of the Jacobian rows (12 + 6 doubles per observation) and the rows'
-// exponents that of the residuals: both have been summed, and the next
-// linearization writes them afresh.
+// FP64 form: V^-1, and Y = W V^-1 and W as limb rows and third pieces
+// (psba_fixed.h).  W's limbs take the place of the Jacobian rows (12 + 6 doubles
+// per observation) and the rows' exponents that of the residuals: both have
+// been summed, and the next linearization writes them afresh.
 __device__ FxArgs fx_args(const BatchProblem &p, const Arenas<double> &ar)
 {
     return FxArgs{ar.i + p.i_pair_a,
@@ -322,6 +322,8 @@ __device__ FxArgs fx_args(const BatchProblem &p, const Arenas<double> &ar)
                   ar.i + p.i_obs_pt,
                   reinterpret_cast<const int2 *>(ar.r + p.r_Y),
                   reinterpret_cast<const int2 *>(ar.r + p.r_A),
+                  reinterpret_cast<const int2 *>(ar.r + p.r_fx),
+                  reinterpret_cast<const int2 *>(ar.r + p.r_fx) + fx_low_words(6) * (size_t)p.no,
                   reinterpret_cast<const int2 *>(ar.r + p.r_ex),
                   ar.r + p.r_W,
                   ar.d + p.d_Vinv,
@@ -341,6 +343,7 @@ __device__ void stage_vinv_y(const BatchProblem &p, const Arenas<double> &ar, do
     const int *opt = ar.i + p.i_obs_pt, *ocam = ar.i + p.i_obs_cam;
     const double *W = ar.r + p.r_W, *U = ar.d + p.d_U;
     int4 *Yq = reinterpret_cast<int4 *>(ar.r + p.r_Y), *Wq = reinterpret_cast<int4 *>(ar.r + p.r_A);
+    int4 *Yl = reinterpret_cast<int4 *>(ar.r + p.r_fx), *Wl = Yl + 3 * (size_t)p.no;
     int2 *ex = reinterpret_cast<int2 *>(ar.r + p.r_ex);
     for (int o = threadIdx.x; o < p.no; o += blockDim.x) {
         const double *s = Vi + 6 * (size_t)opt[o], *u = U + 36 * (size_t)ocam[o];
@@ -368,27 +371,34 @@ __device__ void stage_vinv_y(const BatchProblem &p, const Arenas<double> &ar, do
                 by |= fx_nonfinite(y[3 * r + j]);
             }
         }
-        // [j][row], two rows a store
+        // [j][row], two rows a store; the third pieces [j][row / 3][4]
 #pragma unroll
-        for (int j = 0; j < 3; ++j)
+        for (int j = 0; j < 3; ++j) {
+            unsigned fy[6], fw[6];
 #pragma unroll
             for (int r = 0; r < 6; r += 2) {
                 const int a = 3 * r + j, b = 3 * (r + 1) + j;
                 const size_t at = 9 * (size_t)o + 3 * j + r / 2;
-                const int2 y0 = fx_limbs(y[a], ey + rho[r] - fx_exp(y[a])), y1 = fx_limbs(y[b], ey + rho[r + 1] - fx_exp(y[b]));
-                const int2 w0 = fx_limbs(w[a], ew + rho[r] - fx_exp(w[a])), w1 = fx_limbs(w[b], ew + rho[r + 1] - fx_exp(w[b]));
-                Yq[at] = make_int4(y0.x, y0.y, y1.x, y1.y);
-                Wq[at] = make_int4(w0.x, w0.y, w1.x, w1.y);
+                const Fx3 y0 = fx_limbs3(y[a], ey + rho[r] - fx_exp(y[a])), y1 = fx_limbs3(y[b], ey + rho[r + 1] - fx_exp(y[b]));
+                const Fx3 w0 = fx_limbs3(w[a], ew + rho[r] - fx_exp(w[a])), w1 = fx_limbs3(w[b], ew + rho[r + 1] - fx_exp(w[b]));
+                Yq[at] = make_int4(y0.v.x, y0.v.y, y1.v.x, y1.v.y);
+                Wq[at] = make_int4(w0.v.x, w0.v.y, w1.v.x, w1.v.y);
+                fy[r] = y0.f;
+                fy[r + 1] = y1.f;
+                fw[r] = w0.f;
+                fw[r + 1] = w1.f;
             }
+            Yl[3 * (size_t)o + j] = make_int4(fy[0] | fy[1] << 16, fy[2], fy[3] | fy[4] << 16, fy[5]);
+            Wl[3 * (size_t)o + j] = make_int4(fw[0] | fw[1] << 16, fw[2], fw[3] | fw[4] << 16, fw[5]);
+        }
         ex[o] = make_int2(by ? FX_NAN : ey, bw ? FX_NAN : ew);
     }
 }
 
 // FP64 form: S (N x N, row-major, lower triangle) and rhs = ea, a warp per
 // camera and per camera pair, in block fixed point (fx6_unit; sm: its shared
-// memory, F6_WARP_WORDS per warp).  On the FP64 pipe (two multiply-adds a
+// memory, F6_WORDS per warp).  On the FP64 pipe (two multiply-adds a
 // clock) this was 46% of a solve.
-constexpr int F6_WARP_WORDS = F6_SY + F6_SW;
 
 __device__ void stage_schur(const BatchProblem &p, const Arenas<double> &ar, double mu, int2 *sm)
 {
@@ -397,7 +407,7 @@ __device__ void stage_schur(const BatchProblem &p, const Arenas<double> &ar, dou
     for (long long e = threadIdx.x; e < (long long)N * N; e += blockDim.x) S[e] = 0.0;
     __syncthreads();
     const int warp = threadIdx.x / 32, nw = blockDim.x / 32;
-    int2 *sy = sm + warp * F6_WARP_WORDS, *sw = sy + F6_SY;
+    int2 *mine = sm + warp * F6_WORDS;
     const FxArgs fx = fx_args(p, ar);
     const double *U = ar.d + p.d_U, *g = ar.d + p.d_g;
     const int *cs = ar.i + p.i_cam_start, *pst = ar.i + p.i_pair_start, *pkl = ar.i + p.i_pair_kl;
@@ -412,7 +422,7 @@ __device__ void stage_schur(const BatchProblem &p, const Arenas<double> &ar, dou
             }
         };
         if (n > 0) {
-            fx6_unit<true, false>(fx, SchurUnit{k, cs[k], n, 0}, k, k, sy, sw, emit);
+            fx6_unit<true, false>(fx, SchurUnit{k, cs[k], n, 0}, k, k, mine, emit);
         } else if ((threadIdx.x & 31) == 0) {  // a camera without observations
             for (int v = 0; v < n_out<6, true>(); ++v) {
                 int r, c;
@@ -424,7 +434,7 @@ __device__ void stage_schur(const BatchProblem &p, const Arenas<double> &ar, dou
     }
     for (int q = warp; q < p.n_pairs; q += nw) {
         const int k = pkl[2 * q], l = pkl[2 * q + 1];
-        fx6_unit<false, false>(fx, SchurUnit{q, pst[q], pst[q + 1] - pst[q], 0}, k, l, sy, sw,
+        fx6_unit<false, false>(fx, SchurUnit{q, pst[q], pst[q + 1] - pst[q], 0}, k, l, mine,
                                [&](int, int r, int c, double x) { S[(size_t)(6 * k + r) * N + 6 * l + c] = -x; });
         __syncwarp();
     }
@@ -1523,6 +1533,9 @@ bool build_problem_layout(const psba_problem_desc &p, ProblemLayout &L, std::str
     bp.r_W = r_total; r_total += 18LL * no;
     bp.r_Y = r_total; r_total += 18LL * no;
     bp.r_ex = r_total; r_total += 2LL * no;
+    // the FP64 form's third pieces of the limb rows, in the place of what follows
+    bp.r_fx = r_total;
+    const long long r_end64 = r_total + 2LL * fx_low_words(6) * no;
     // the mixed form's FP32 copies (even counts: FP32 pairs stay 8-byte aligned)
     bp.r_tab32 = r_total; r_total += (long long)CAMTAB32 * nc;
     bp.r_tab2f = r_total; r_total += 2LL * RES_TAB2F * nc;
@@ -1533,7 +1546,7 @@ bool build_problem_layout(const psba_problem_desc &p, ProblemLayout &L, std::str
     bp.r_vinv2f = r_total; r_total += 12LL * np;
     bp.r_dpa2f = r_total; r_total += 2LL * N;
     bp.r_gb32 = r_total; r_total += 4LL * np;
-    L.nr = r_total;
+    L.nr = std::max(r_total, r_end64);
     bp.d_V = dres(6 * (size_t)np);
     bp.d_Vinv = dres(6 * (size_t)np);
     bp.d_U = dres(36 * (size_t)nc);
@@ -1560,7 +1573,7 @@ void rebase_problem(BatchProblem &bp, long long db, long long ib, long long rb)
                          &bp.i_pair_start, &bp.i_pair_kl, &bp.i_pair_a, &bp.i_pair_b})
         *f += ib;
     for (long long *f : {&bp.r_ex, &bp.r_A, &bp.r_B, &bp.r_W, &bp.r_Y, &bp.r_tab32, &bp.r_tab2f, &bp.r_tab2f2,
-                         &bp.r_meas2f, &bp.r_pts2f, &bp.r_x2f, &bp.r_vinv2f, &bp.r_dpa2f, &bp.r_gb32})
+                         &bp.r_meas2f, &bp.r_pts2f, &bp.r_x2f, &bp.r_vinv2f, &bp.r_dpa2f, &bp.r_gb32, &bp.r_fx})
         *f += rb;
 }
 
@@ -1580,7 +1593,7 @@ static size_t batch_smem(int precision, int threads, int max_N)
     size_t b = chol_smem(max_N);
     for (int step : {384, 768, 1536, 3072})
         if (max_N > step) b = std::max(b, chol_smem(step));
-    if (precision != PSBA_PREC_MIXED) b = std::max(b, sizeof(int2) * F6_WARP_WORDS * (size_t)(threads / 32));
+    if (precision != PSBA_PREC_MIXED) b = std::max(b, sizeof(int2) * F6_WORDS * (size_t)(threads / 32));
     return b;
 }
 

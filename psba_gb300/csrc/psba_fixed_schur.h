@@ -15,7 +15,9 @@ struct FxArgs {
     const int *pa, *pb;    // pair entries: observation of camera k, of camera l
     const int *cam_obs;    // observations by camera
     const int *obs_pt;
-    const int2 *Yq, *Wq, *ex;
+    const int2 *Yq, *Wq;   // limbs
+    const int2 *Yl, *Wl;   // third pieces
+    const int2 *ex;
     const double *W, *Vinv;  // for entries with an infinity or a NaN
     const double *U, *gb;
     const int *pair_kl;
@@ -87,20 +89,15 @@ __device__ __forceinline__ void ld_limbs(const int2 *p, int2 *out)
     }
 }
 
-// A TR x TC tile of entry t's products, summed over the NJ inner columns
-template <int TR, int TC, int RP, int CP, int NJ = 3>
-__device__ __forceinline__ void fx_tile(const int2 *y, const int2 *w, long long (&hh)[TR][TC], long long (&hl)[TR][TC])
+// The N <= 4 third pieces of a group
+template <int N>
+__device__ __forceinline__ void ld_lows(const int2 *p, float (&out)[N])
 {
-#pragma unroll
-    for (int j = 0; j < NJ; ++j) {
-        int2 a[TR], b[TC];
-        ld_limbs<TR>(y + j * RP, a);
-        ld_limbs<TC>(w + j * CP, b);
-#pragma unroll
-        for (int p = 0; p < TR; ++p)
-#pragma unroll
-            for (int q = 0; q < TC; ++q) fx_mad(a[p], b[q], hh[p][q], hl[p][q]);
-    }
+    const uint2 v = *reinterpret_cast<const uint2 *>(p);
+    out[0] = (float)(v.x & 0xffffu);
+    if (N > 1) out[1] = (float)(v.x >> 16);
+    if (N > 2) out[2] = (float)(v.y & 0xffffu);
+    if (N > 3) out[3] = (float)(v.y >> 16);
 }
 
 // ---------------------------------------------------------------------------
@@ -109,22 +106,29 @@ __device__ __forceinline__ void fx_tile(const int2 *y, const int2 *w, long long 
 // asynchronous copies (the next chunk's are under way during the sums' end);
 // lane t moves entry t's W row (and gb, DIAG) to the chunk's exponent; lane
 // 4 g + q takes entries g, g + 8, g + 16, g + 24 and quadrant q of the block in
-// two 64-bit integers per output; the eight lane groups' totals meet in
-// shared memory, and a lane per output adds them to its FP64 sum.
-// Camera block (k, l), sy and sw: F6_SY and F6_SW words of the warp's shared
-// memory; emit(v, r, c, sum) is called by one lane per output v at (r, c).  NC:
-// the limb rows and gb come from an earlier launch (read-only cache loads).
-constexpr int F6_SY = FX_CHUNK * 18, F6_SW = FX_CHUNK * 26;
+// two 64-bit integers and an FP32 number per output (DIAG: and gb as a fourth
+// column); the eight lane groups' totals meet in shared memory, and a lane per
+// output adds them to its FP64 sum.
+// Camera block (k, l), sm: F6_WORDS of the warp's shared memory; emit(v, r, c,
+// sum) is called by one lane per output v at (r, c).  SOLO: an observation's
+// limbs and third pieces are one row, and they and gb come from an earlier
+// launch (read-only cache loads); else limbs and third pieces are apart.
+constexpr int F6_L = 18, F6_F = 6, F6_G = 4;  // int2 words an entry: limbs, third pieces, gb (three limbs, third pieces)
+constexpr int F6_WORDS = FX_CHUNK * (2 * (F6_L + F6_F) + F6_G);
 
-template <bool DIAG, bool NC, typename Emit>
-__device__ void fx6_unit(const FxArgs &g, const SchurUnit u, int k, int l, int2 *sy, int2 *sw, Emit &&emit)
+template <bool DIAG, bool SOLO, typename Emit>
+__device__ void fx6_unit(const FxArgs &g, const SchurUnit u, int k, int l, int2 *sm, Emit &&emit)
 {
-    constexpr int CNP = 6, TC = DIAG ? 4 : 3, CP = 2 * TC;  // columns: 6, or 6 + gb + a pad
-    constexpr int SY = 18, SW = DIAG ? 26 : 18;             // words from entry to entry: no bank conflicts
+    constexpr int CNP = 6, TC = DIAG ? 4 : 3, CP = 2 * TC;  // totals of a row: 6, or 6 and each half's gb column
     constexpr int NV = n_out<CNP, DIAG>(), PER = (NV + 31) / 32;
-    const int lane = threadIdx.x & 31, q = lane & 3, r0 = 3 * (q >> 1), c0 = TC * (q & 1);
-    long long *st = reinterpret_cast<long long *>(sy);  // the totals, over the rows that are read
-    static_assert(8 * 6 * CP <= FX_CHUNK * SY, "the totals fit");
+    constexpr size_t ROW_L = SOLO ? F6_L + F6_F : F6_L, ROW_F = SOLO ? F6_L + F6_F : F6_F;
+    int2 *yl = sm, *wl = yl + FX_CHUNK * F6_L, *yf = wl + FX_CHUNK * F6_L, *wf = yf + FX_CHUNK * F6_F,
+         *sg = wf + FX_CHUNK * F6_F;
+    const int lane = threadIdx.x & 31, q = lane & 3, rg = q >> 1, cg = q & 1;
+    // the totals, over the rows that are read
+    long long *sH = reinterpret_cast<long long *>(yl);
+    unsigned *sL = reinterpret_cast<unsigned *>(sH + 8 * 6 * CP);
+    static_assert(8 * 6 * CP * 12 <= FX_CHUNK * F6_L * 8, "the totals fit");
     double acc[PER];
     int at[PER], we[PER];
 #pragma unroll
@@ -150,19 +154,21 @@ __device__ void fx6_unit(const FxArgs &g, const SchurUnit u, int k, int l, int2 
         bn = DIAG ? an : __ldg(pb + t);
     };
     auto exponents = [&](int &y, int &w, int &i) {
-        const int2 x = NC ? __ldg(g.ex + an) : g.ex[an];
+        const int2 x = SOLO ? __ldg(g.ex + an) : g.ex[an];
         y = x.x;
-        w = DIAG ? x.y : NC ? __ldg(&g.ex[bn].y) : g.ex[bn].y;
+        w = DIAG ? x.y : SOLO ? __ldg(&g.ex[bn].y) : g.ex[bn].y;
         if (DIAG) i = __ldg(g.obs_pt + an);
     };
     auto rows = [&]() {
 #pragma unroll
-        for (int m = 0; m < 9; ++m) {  // piece p of 9 x 32: row p / 9, 16 bytes p % 9
-            const int p = lane + 32 * m, r = p / 9, part = p - 9 * r;
+        for (int m = 0; m < 12; ++m) {  // piece p of 12 x 32: row p / 12, 16 bytes p % 12
+            const int p = lane + 32 * m, r = p / 12, part = p - 12 * r;
             const int ra = __shfl_sync(0xffffffffu, an, r), rb = __shfl_sync(0xffffffffu, bn, r);
-            const int wd = DIAG ? (part / 3) * CP + 2 * (part % 3) : 2 * part;
-            cp_async16(sy + r * SY + 2 * part, g.Yq + 18 * (size_t)ra + 2 * part);
-            cp_async16(sw + r * SW + wd, g.Wq + 18 * (size_t)rb + 2 * part);
+            const bool lim = part < 9;
+            const int d = lim ? r * F6_L + 2 * part : 2 * FX_CHUNK * F6_L + r * F6_F + 2 * (part - 9);
+            const int dw = d + (lim ? FX_CHUNK * F6_L : FX_CHUNK * F6_F);
+            cp_async16(sm + d, lim ? g.Yq + ROW_L * ra + 2 * part : g.Yl + ROW_F * ra + 2 * (part - 9));
+            cp_async16(sm + dw, lim ? g.Wq + ROW_L * rb + 2 * part : g.Wl + ROW_F * rb + 2 * (part - 9));
         }
     };
     indices(0);
@@ -182,7 +188,7 @@ __device__ void fx6_unit(const FxArgs &g, const SchurUnit u, int k, int l, int2 
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
                 const double *gj = g.gb + 3 * (size_t)pt + j;
-                gv[j] = NC ? __ldg(gj) : *gj;
+                gv[j] = SOLO ? __ldg(gj) : *gj;
                 eg = max(eg, fx_exp(gv[j]));
                 nf |= fx_nonfinite(gv[j]);
             }
@@ -197,45 +203,84 @@ __device__ void fx6_unit(const FxArgs &g, const SchurUnit u, int k, int l, int2 
             // entry lane's W row, d bits down
             if (lane < n) {
                 const int d = E - e;
-                int4 *row = reinterpret_cast<int4 *>(sw + lane * SW);
+                int4 *row = reinterpret_cast<int4 *>(wl + lane * F6_L), *low = reinterpret_cast<int4 *>(wf + lane * F6_F);
 #pragma unroll
-                for (int m = 0; m < 9; ++m) {
-                    int4 &x = row[DIAG ? (m / 3) * (CP / 2) + m % 3 : m];
-                    const int2 s0 = fx_shift(make_int2(x.x, x.y), d), s1 = fx_shift(make_int2(x.z, x.w), d);
-                    x = make_int4(s0.x, s0.y, s1.x, s1.y);
-                }
-                if (DIAG)
+                for (int j = 0; j < 3; ++j) {
+                    const int4 f = low[j];
+                    Fx3 s[6];
 #pragma unroll
-                    for (int j = 0; j < 3; ++j) {
-                        const int2 s = fx_limbs(gv[j], Eg - eyt - fx_exp(gv[j]));
-                        row[j * (CP / 2) + 3] = make_int4(s.x, s.y, 0, 0);
+                    for (int m = 0; m < 3; ++m) {
+                        const int4 x = row[3 * j + m];
+                        const unsigned f0 = m == 0 ? f.x & 0xffff : m == 1 ? f.y & 0xffff : (unsigned)f.z >> 16;
+                        const unsigned f1 = m == 0 ? (unsigned)f.x >> 16 : m == 1 ? f.z & 0xffff : f.w & 0xffff;
+                        s[2 * m] = fx_shift(make_int2(x.x, x.y), f0, d);
+                        s[2 * m + 1] = fx_shift(make_int2(x.z, x.w), f1, d);
+                        row[3 * j + m] = make_int4(s[2 * m].v.x, s[2 * m].v.y, s[2 * m + 1].v.x, s[2 * m + 1].v.y);
                     }
+                    low[j] = make_int4(s[0].f | s[1].f << 16, s[2].f, s[3].f | s[4].f << 16, s[5].f);
+                }
+                if (DIAG) {
+                    Fx3 s[3];
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) s[j] = fx_limbs3(gv[j], Eg - eyt - fx_exp(gv[j]));
+                    int4 *gr = reinterpret_cast<int4 *>(sg + lane * F6_G);
+                    gr[0] = make_int4(s[0].v.x, s[0].v.y, s[1].v.x, s[1].v.y);
+                    gr[1] = make_int4(s[2].v.x, s[2].v.y, s[0].f | s[1].f << 16, s[2].f);
+                }
             }
             __syncwarp();
             long long hh[3][TC], hl[3][TC];
+            float cr[3][TC];
 #pragma unroll
             for (int i = 0; i < 3; ++i)
 #pragma unroll
-                for (int j = 0; j < TC; ++j) hh[i][j] = hl[i][j] = 0;
-#pragma unroll
+                for (int j = 0; j < TC; ++j) {
+                    hh[i][j] = hl[i][j] = 0;
+                    cr[i][j] = 0.0f;
+                }
+#pragma unroll 1
             for (int m = 0; m < FX_CHUNK / 8; ++m) {
                 const int t = (lane >> 2) + 8 * m;
-                if (t < n) fx_tile<3, TC, 6, CP>(sy + t * SY + r0, sw + t * SW + c0, hh, hl);
+                if (t >= n) break;
+                float fg[3];
+                if (DIAG) ld_lows<3>(sg + t * F6_G + 3, fg);
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    int2 a[3], b[TC];
+                    float fa[3], fb[TC], fw[3];
+                    ld_limbs<3>(yl + t * F6_L + 6 * j + 3 * rg, a);
+                    ld_limbs<3>(wl + t * F6_L + 6 * j + 3 * cg, b);
+                    ld_lows<3>(yf + t * F6_F + 2 * j + rg, fa);
+                    ld_lows<3>(wf + t * F6_F + 2 * j + cg, fw);
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) fb[c] = fw[c];
+                    if (DIAG) {
+                        b[TC - 1] = sg[t * F6_G + j];
+                        fb[TC - 1] = fg[j];
+                    }
+                    fx_products<3, TC>(a, fa, b, fb, hh, hl, cr);
+                }
             }
             __syncwarp();  // the rows are read
 #pragma unroll
             for (int i = 0; i < 3; ++i)
 #pragma unroll
-                for (int j = 0; j < TC; ++j)
-                    st[(lane >> 2) * 6 * CP + (r0 + i) * CP + c0 + j] = fx_total(hh[i][j], hl[i][j]);
+                for (int j = 0; j < TC; ++j) {
+                    const int to = (lane >> 2) * 6 * CP + (3 * rg + i) * CP + (j < 3 ? 3 * cg + j : 6 + cg);
+                    fx_carry(hh[i][j], hl[i][j], cr[i][j], sH[to], sL[to]);
+                }
             __syncwarp();
 #pragma unroll
             for (int p = 0; p < PER; ++p) {
                 if (at[p] < 0) continue;
-                long long T = 0;
+                long long H = 0;
+                unsigned L = 0;
 #pragma unroll
-                for (int s = 0; s < 8; ++s) T += st[s * 6 * CP + at[p]];
-                acc[p] = fx_add(acc[p], T, we[p] + (DIAG && at[p] % CP == CNP ? Eg : E));
+                for (int s = 0; s < 8; ++s) {
+                    H += sH[s * 6 * CP + at[p]];
+                    L += sL[s * 6 * CP + at[p]];
+                }
+                acc[p] = fx_add(acc[p], H, L, we[p] + (DIAG && at[p] % CP == CNP ? Eg : E));
             }
         } else {
 #pragma unroll

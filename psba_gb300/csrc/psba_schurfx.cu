@@ -3,12 +3,12 @@
 // sums Y gb (compute_S.cl:39-77, compute_ea.cl:21-36).
 //
 // k_limb_rows forms Y = W V^-1 (compute_Yblks.cl:26-37) and cuts each
-// observation's Y and W rows into limbs, relative to the observation's own
-// largest value after the camera's row weights (fx_weight).  The sums then
-// need one more shift per pair entry, of its W row, to the largest
-// eY + eW among the 32 entries taken together: a point close to one camera has a W
-// row there 10^4 times the others' and Y rows as much smaller, and only what
-// lies 57 bits below the largest product is lost.  Cutting both rows at every
+// observation's Y and W rows into limbs and third pieces (psba_fixed.h),
+// relative to the observation's own largest value after the camera's row
+// weights (fx_weight).  The sums then need one more shift per pair entry, of
+// its W row, to the largest eY + eW among the 32 entries taken together: a point
+// close to one camera has a W row there 10^4 times the others' and Y rows as
+// much smaller, and only what lies 73 bits below the largest product is lost.  Cutting both rows at every
 // use instead (a point is in about six pairs per observation) cost 1,560
 // instructions per warp and 32 entries, twice the products' own.
 #include "psba_fixed_schur.h"
@@ -36,7 +36,8 @@ __global__ void __launch_bounds__(LR_THREADS) k_limb_rows(int no, const int *__r
                                                           const double *__restrict__ U, int2 *__restrict__ Yq,
                                                           int2 *__restrict__ Wq, int2 *__restrict__ ex)
 {
-    constexpr int RP = fx_rows(CNP), TPO = CNP == 6 ? 2 : 4, TR = RP / TPO, OB = LR_THREADS / TPO, WORDS = 3 * RP;
+    constexpr int RP = fx_rows(CNP), TPO = CNP == 6 ? 2 : 4, TR = RP / TPO, OB = LR_THREADS / TPO, WORDS = fx_words(CNP);
+    static_assert(TR == fx_group(CNP), "a thread's rows are a group of third pieces");
     __shared__ __align__(16) double sw[OB * 3 * CNP];
     __shared__ __align__(16) int2 sq[2][OB * WORDS];
     const int o0 = blockIdx.x * OB, n = min(OB, no - o0), tid = threadIdx.x;
@@ -84,13 +85,21 @@ __global__ void __launch_bounds__(LR_THREADS) k_limb_rows(int no, const int *__r
         by |= __shfl_xor_sync(0xffffffffu, by, x);
     }
 #pragma unroll
-    for (int a = 0; a < TR; ++a)
+    for (int j = 0; j < 3; ++j) {
+        unsigned fy[4] = {}, fw[4] = {};
 #pragma unroll
-        for (int j = 0; j < 3; ++j) {
+        for (int a = 0; a < TR; ++a) {
             const int at = t * WORDS + j * RP + q * TR + a;
-            sq[0][at] = fx_limbs(y[a][j], ey + rho[a] - fx_exp(y[a][j]));
-            sq[1][at] = fx_limbs(w[a][j], ew + rho[a] - fx_exp(w[a][j]));
+            const Fx3 vy = fx_limbs3(y[a][j], ey + rho[a] - fx_exp(y[a][j])), vw = fx_limbs3(w[a][j], ew + rho[a] - fx_exp(w[a][j]));
+            sq[0][at] = vy.v;
+            sq[1][at] = vw.v;
+            fy[a] = vy.f;
+            fw[a] = vw.f;
         }
+        const int at = t * WORDS + fx_limb_words(CNP) + j * TPO + q;
+        sq[0][at] = make_int2(fy[0] | fy[1] << 16, fy[2] | fy[3] << 16);
+        sq[1][at] = make_int2(fw[0] | fw[1] << 16, fw[2] | fw[3] << 16);
+    }
     if (q == 0 && t < n) ex[o] = make_int2(by ? FX_NAN : ey, bw ? FX_NAN : ew);
     __syncthreads();
     int4 *yd = reinterpret_cast<int4 *>(Yq + WORDS * (size_t)o0), *wd = reinterpret_cast<int4 *>(Wq + WORDS * (size_t)o0);
@@ -101,26 +110,28 @@ __global__ void __launch_bounds__(LR_THREADS) k_limb_rows(int no, const int *__r
     }
 }
 
-constexpr int F6_WARPS = 4, F6_CTAS = 4;  // resident CTAs per SM: 188 / 173 / 185 us with 3 / 4 / 5 at 88 cameras
+constexpr int F6_WARPS = 4, F6_CTAS = 4;  // resident CTAs per SM: 287 / 283 us with 3 / 4 at 88 cameras
+constexpr int F6_SMEM = F6_WARPS * F6_WORDS * (int)sizeof(int2);  // dynamic: 52 KB
 
 // The diagonal units' blocks first (more work per entry), then the pairs'.
 __global__ void __launch_bounds__(32 * F6_WARPS, F6_CTAS) k_schur_fx6(FxArgs g, int n_diag, const SchurUnit *__restrict__ diag,
                                                              int n_off, const SchurUnit *__restrict__ off)
 {
-    __shared__ __align__(16) int2 sy[F6_WARPS][F6_SY], sw[F6_WARPS][F6_SW];
+    extern __shared__ __align__(16) int2 fx_sm[];
     const int warp = threadIdx.x >> 5, diag_ctas = (n_diag + F6_WARPS - 1) / F6_WARPS;
+    int2 *sm = fx_sm + warp * F6_WORDS;
     if ((int)blockIdx.x < diag_ctas) {
         const int uid = blockIdx.x * F6_WARPS + warp;
         if (uid < n_diag) {
             const SchurUnit u = diag[uid];
-            fx6_unit<true, true>(g, u, u.slot, u.slot, sy[warp], sw[warp],
+            fx6_unit<true, true>(g, u, u.slot, u.slot, sm,
                            [&](int v, int, int, double x) { g.diag_partial[(size_t)u.out * 27 + v] = x; });
         }
     } else {
         const int uid = (blockIdx.x - diag_ctas) * F6_WARPS + warp;
         if (uid < n_off) {
             const SchurUnit u = off[uid];
-            fx6_unit<false, true>(g, u, __ldg(g.pair_kl + 2 * u.slot), __ldg(g.pair_kl + 2 * u.slot + 1), sy[warp], sw[warp],
+            fx6_unit<false, true>(g, u, __ldg(g.pair_kl + 2 * u.slot), __ldg(g.pair_kl + 2 * u.slot + 1), sm,
                             [&](int v, int, int, double x) { g.off_partial[(size_t)u.out * 36 + v] = x; });
         }
     }
@@ -128,25 +139,40 @@ __global__ void __launch_bounds__(32 * F6_WARPS, F6_CTAS) k_schur_fx6(FxArgs g, 
 
 // ---------------------------------------------------------------------------
 // 11- and 16-parameter cameras: a CTA of four warps per unit, the same steps;
-// half-warps take the entries in turn, 4 x 4 threads with a TR x TC tile each.
+// half-warps take the entries in turn, 4 x 4 threads with a TR x TR tile each
+// (diagonal blocks: and gb, as the 12th column's pad, or as a fifth column).
 constexpr int FV_THREADS = 128;
 
+// Shared memory of a CTA in int2 words: per entry limbs (two words of padding)
+// and third pieces of Y and of W and gb's three limbs and third pieces, then the warps' totals.
 template <int CNP, bool DIAG>
-__global__ void __launch_bounds__(FV_THREADS) k_schur_fxv(FxArgs g, const SchurUnit *__restrict__ units)
+struct FvShape {
+    static constexpr int RP = fx_rows(CNP), TR = RP / 4, NL = fx_limb_words(CNP), NF = fx_low_words(CNP), NW = FV_THREADS / 32;
+    static constexpr int XG = DIAG && CNP == RP ? 1 : 0;  // gb is a column more
+    static constexpr int TC = TR + XG, CP = RP + 4 * XG;
+    static constexpr int SL = NL + 2, ENTRY = 2 * (SL + NF) + 4 * XG;
+    static constexpr int ROWS = FX_CHUNK * ENTRY, TOTALS = NW * RP * CP;
+    static constexpr int BYTES = ROWS * 8 + TOTALS * 12;
+    // CTAs an SM: as many as the tile's registers leave (without the bound the 16-parameter
+    // diagonal blocks take 242 registers, with it 166: 21 cameras 154 -> 142 us both launches)
+    static constexpr int CTAS = CNP == 11 ? 4 : 3;
+};
+
+template <int CNP, bool DIAG>
+__global__ void __launch_bounds__(FV_THREADS, FvShape<CNP, DIAG>::CTAS)
+    k_schur_fxv(FxArgs g, const SchurUnit *__restrict__ units)
 {
-    constexpr int RP = fx_rows(CNP), TR = RP / 4, TC = DIAG && CNP == 16 ? 5 : TR, CP = 4 * TC;
-    constexpr int SY = 3 * RP + 2, SW = 3 * CP + 2, NW = FV_THREADS / 32;
+    using F = FvShape<CNP, DIAG>;
+    constexpr int RP = F::RP, TR = F::TR, TC = F::TC, CP = F::CP, SL = F::SL, NF = F::NF, NW = F::NW, G = fx_group(CNP);
     constexpr int NV = n_out<CNP, DIAG>(), PER = (NV + FV_THREADS - 1) / FV_THREADS;
-    constexpr int PIECES = 3 * RP / 2;  // 16-byte pieces of a row
-    // this chunk's rows and, where 48 KB hold them (CNP 11), the next one's, which
-    // are then under way while this one is summed; else they are fetched after it
-    constexpr int NB = 2 * 8 * FX_CHUNK * (SY + SW) + 8 * NW * RP * CP <= 48 * 1024 ? 2 : 1;
-    __shared__ __align__(16) int2 sys[NB][FX_CHUNK * SY], sws[NB][FX_CHUNK * SW];
-    __shared__ long long st[NW][RP * CP];
+    constexpr int LIMBS = F::NL / 2, PIECES = LIMBS + NF / 2;  // 16-byte pieces of a row
+    static_assert(TR == G, "a thread's rows are a group of third pieces");
+    extern __shared__ __align__(16) int2 fx_sm[];
+    long long *sH = reinterpret_cast<long long *>(fx_sm + F::ROWS);
+    unsigned *sL = reinterpret_cast<unsigned *>(sH + F::TOTALS);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const SchurUnit u = units[blockIdx.x];
     const int *pa = DIAG ? g.cam_obs + u.begin : g.pa + u.begin, *pb = DIAG ? pa : g.pb + u.begin;
-    for (int e = tid; e < NB * FX_CHUNK * SW; e += FV_THREADS) sws[0][e] = make_int2(0, 0);  // the padding columns
     double acc[PER];
     int at[PER], we[PER];
 #pragma unroll
@@ -171,17 +197,20 @@ __global__ void __launch_bounds__(FV_THREADS) k_schur_fxv(FxArgs g, const SchurU
         an = __ldg(pa + t);
         bn = DIAG ? an : __ldg(pb + t);
     };
+    // (a second buffer for the next chunk's rows, 58 KB a CTA, left too few CTAs: 52
+    // cameras, 11 parameters, 642 us for both launches instead of 580)
+    int2 *yl = fx_sm, *wl = yl + FX_CHUNK * SL, *yf = wl + FX_CHUNK * SL, *wf = yf + FX_CHUNK * NF, *sg = wf + FX_CHUNK * NF;
     auto fetch = [&](int t0) {
         const int n = min(FX_CHUNK, u.count - t0);
-        int2 *sy = sys[(t0 / FX_CHUNK) & (NB - 1)], *sw = sws[(t0 / FX_CHUNK) & (NB - 1)];
 #pragma unroll
         for (int m = 0; m < (FX_CHUNK * PIECES + FV_THREADS - 1) / FV_THREADS; ++m) {
             const int p = tid + FV_THREADS * m, t = p / PIECES, part = p % PIECES;
             const int ia = __shfl_sync(0xffffffffu, an, t & 31), ib = DIAG ? ia : __shfl_sync(0xffffffffu, bn, t & 31);
             if (t >= n) continue;
-            const int wd = (part / (RP / 2)) * CP + 2 * (part % (RP / 2));
-            cp_async16(sy + t * SY + 2 * part, g.Yq + 3 * RP * (size_t)ia + 2 * part);
-            cp_async16(sw + t * SW + wd, g.Wq + 3 * RP * (size_t)ib + 2 * part);
+            const bool lim = part < LIMBS;
+            const int to = lim ? t * SL + 2 * part : t * NF + 2 * (part - LIMBS);
+            cp_async16((lim ? yl : yf) + to, g.Yq + fx_words(CNP) * (size_t)ia + 2 * part);
+            cp_async16((lim ? wl : wf) + to, g.Wq + fx_words(CNP) * (size_t)ib + 2 * part);
         }
         en = -(1 << 20);
         if (lane < n) {
@@ -193,11 +222,9 @@ __global__ void __launch_bounds__(FV_THREADS) k_schur_fxv(FxArgs g, const SchurU
         if (t0 + FX_CHUNK < u.count) indices(t0 + FX_CHUNK);
     };
     indices(0);
-    __syncthreads();
     fetch(0);
     for (int t0 = 0; t0 < u.count; t0 += FX_CHUNK) {
         const int n = min(FX_CHUNK, u.count - t0), e = en, ey = eyn, pt = ptn;
-        int2 *sy = sys[(t0 / FX_CHUNK) & (NB - 1)], *sw = sws[(t0 / FX_CHUNK) & (NB - 1)];
         const int E = __reduce_max_sync(0xffffffffu, e);
         const int d = E - e;
         bool bad = E >= FX_NAN / 2;  // the same in every warp
@@ -217,47 +244,95 @@ __global__ void __launch_bounds__(FV_THREADS) k_schur_fxv(FxArgs g, const SchurU
         }
         cp_async_wait();
         __syncthreads();
-        if (NB == 2 && t0 + FX_CHUNK < u.count) fetch(t0 + FX_CHUNK);
         if (!bad) {
             if (lane < n) {
-                // entry lane's W row, d bits down; the warps share out the row
+                // entry lane's W row, d bits down; the warps share out its groups
 #pragma unroll
-                for (int m = 0; m < (PIECES + NW - 1) / NW; ++m) {
-                    const int part = warp + NW * m;
-                    if (part < PIECES) {
-                        int4 &x = *reinterpret_cast<int4 *>(sw + lane * SW + (part / (RP / 2)) * CP + 2 * (part % (RP / 2)));
-                        const int2 s0 = fx_shift(make_int2(x.x, x.y), d), s1 = fx_shift(make_int2(x.z, x.w), d);
-                        x = make_int4(s0.x, s0.y, s1.x, s1.y);
+                for (int m = 0; m < NF / NW; ++m) {
+                    const int gr = warp + NW * m;  // column gr / 4, rows of group gr % 4
+                    int2 *v = wl + lane * SL + (gr / 4) * RP + (gr % 4) * G;
+                    int2 &f = wf[lane * NF + gr];
+                    const int2 f0 = f;
+                    Fx3 x[4] = {};
+#pragma unroll
+                    for (int k = 0; k < G; ++k) {
+                        const unsigned w = k < 2 ? f0.x : f0.y;
+                        x[k] = fx_shift(v[k], k & 1 ? w >> 16 : w & 0xffff, d);
+                        v[k] = x[k].v;
                     }
+                    if (DIAG && F::XG == 0 && gr % 4 == 3) {
+                        // the group of the padding row, whose place gb takes
+                        const double gj = gr / 4 == 0 ? gv[0] : gr / 4 == 1 ? gv[1] : gv[2];
+                        x[CNP % G] = fx_limbs3(gj, Eg - ey - fx_exp(gj));
+                        v[CNP % G] = x[CNP % G].v;
+                    }
+                    f = make_int2(x[0].f | x[1].f << 16, x[2].f | x[3].f << 16);
                 }
-            }
-            if (DIAG) {
-                if (CNP < RP) __syncthreads();  // gb takes the place of the padding column that the shift has rewritten
-                if (lane < n && warp < 3)
-                    sw[lane * SW + warp * CP + CNP] = fx_limbs(gv[warp], Eg - ey - fx_exp(gv[warp]));
+                if (F::XG && warp == 0) {
+                    Fx3 x[3];
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) {
+                        x[j] = fx_limbs3(gv[j], Eg - ey - fx_exp(gv[j]));
+                        sg[lane * 4 + j] = x[j].v;
+                    }
+                    sg[lane * 4 + 3] = make_int2(x[0].f | x[1].f << 16, x[2].f);
+                }
             }
         }
         __syncthreads();
         if (!bad) {
-            const int l = tid & 15, r0 = (l >> 2) * TR, c0 = (l & 3) * TC;
+            const int l = tid & 15, rg = l >> 2, cg = l & 3;
             long long hh[TR][TC], hl[TR][TC];
-#pragma unroll
-            for (int i = 0; i < TR; ++i)
-#pragma unroll
-                for (int j = 0; j < TC; ++j) hh[i][j] = hl[i][j] = 0;
-            for (int t = tid >> 4; t < n; t += FV_THREADS / 16)
-                fx_tile<TR, TC, RP, CP>(sy + t * SY + r0, sw + t * SW + c0, hh, hl);
+            float cr[TR][TC];
 #pragma unroll
             for (int i = 0; i < TR; ++i)
 #pragma unroll
                 for (int j = 0; j < TC; ++j) {
-                    long long T = fx_total(hh[i][j], hl[i][j]);
-                    T += __shfl_xor_sync(0xffffffffu, T, 16);
-                    if (lane < 16) st[warp][(r0 + i) * CP + c0 + j] = T;
+                    hh[i][j] = hl[i][j] = 0;
+                    cr[i][j] = 0.0f;
+                }
+#pragma unroll 1
+            for (int t = tid >> 4; t < n; t += FV_THREADS / 16) {
+                float fg[3] = {};
+                if (F::XG) ld_lows<3>(sg + t * 4 + 3, fg);
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    int2 a[TR], b[TC], bw[TR];
+                    float fa[TR], fb[TC], fw[TR];
+                    ld_limbs<TR>(yl + t * SL + j * RP + rg * TR, a);
+                    ld_limbs<TR>(wl + t * SL + j * RP + cg * TR, bw);
+                    ld_lows<TR>(yf + t * NF + 4 * j + rg, fa);
+                    ld_lows<TR>(wf + t * NF + 4 * j + cg, fw);
+#pragma unroll
+                    for (int c = 0; c < TR; ++c) {
+                        b[c] = bw[c];
+                        fb[c] = fw[c];
+                    }
+                    if (F::XG) {
+                        b[TC - 1] = sg[t * 4 + j];
+                        fb[TC - 1] = fg[j];
+                    }
+                    fx_products<TR, TC>(a, fa, b, fb, hh, hl, cr);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < TR; ++i)
+#pragma unroll
+                for (int j = 0; j < TC; ++j) {
+                    long long H;
+                    unsigned L;
+                    fx_carry(hh[i][j], hl[i][j], cr[i][j], H, L);
+                    H += __shfl_xor_sync(0xffffffffu, H, 16);
+                    L += __shfl_xor_sync(0xffffffffu, L, 16);
+                    if (lane < 16) {
+                        const int to = (warp * RP + rg * TR + i) * CP + (j < TR ? cg * TR + j : RP + cg);
+                        sH[to] = H;
+                        sL[to] = L;
+                    }
                 }
         }
         __syncthreads();
-        if (NB == 1 && t0 + FX_CHUNK < u.count) fetch(t0 + FX_CHUNK);
+        if (t0 + FX_CHUNK < u.count) fetch(t0 + FX_CHUNK);
 #pragma unroll
         for (int p = 0; p < PER; ++p) {
             if (at[p] < 0) continue;
@@ -266,10 +341,14 @@ __global__ void __launch_bounds__(FV_THREADS) k_schur_fxv(FxArgs g, const SchurU
                 acc[p] = fx_plain<CNP>(g, pa + t0, pb + t0, n, r, c, acc[p]);
                 continue;
             }
-            long long T = 0;
+            long long H = 0;
+            unsigned L = 0;
 #pragma unroll
-            for (int w = 0; w < NW; ++w) T += st[w][at[p]];
-            acc[p] = fx_add(acc[p], T, we[p] + (DIAG && c == CNP ? Eg : E));
+            for (int w = 0; w < NW; ++w) {
+                H += sH[w * RP * CP + at[p]];
+                L += sL[w * RP * CP + at[p]];
+            }
+            acc[p] = fx_add(acc[p], H, L, we[p] + (DIAG && c == CNP ? Eg : E));
         }
     }
     double *out = (DIAG ? g.diag_partial : g.off_partial) + (size_t)u.out * NV;
@@ -295,11 +374,14 @@ __global__ void __launch_bounds__(FV_THREADS) k_camera_fx(const CamUnit *__restr
     constexpr int ST = 2 * CP + 2;  // words from observation to observation
     constexpr int NU = CNP * (CNP + 1) / 2, NV = NU + CNP, PER = (NV + FV_THREADS - 1) / FV_THREADS;
     __shared__ __align__(16) long long sa[FX_CHUNK * ST];
-    __shared__ long long st[NW][RP * CP];
+    __shared__ float sf[FX_CHUNK * 2 * CP];  // third pieces
+    __shared__ long long sH[NW][RP * CP];
+    __shared__ unsigned sL[NW][RP * CP];
     __shared__ int s_E[CP];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const CamUnit u = units[blockIdx.x];
     for (int e = tid; e < FX_CHUNK * ST; e += FV_THREADS) sa[e] = 0;  // the padding columns
+    for (int e = tid; e < FX_CHUNK * 2 * CP; e += FV_THREADS) sf[e] = 0.0f;
     double acc[PER];
     int at[PER];
 #pragma unroll
@@ -386,36 +468,65 @@ __global__ void __launch_bounds__(FV_THREADS) k_camera_fx(const CamUnit *__restr
             const int c = warp + NW * q;
             if (c < NC && lane < n)
 #pragma unroll
-                for (int i = 0; i < 2; ++i)
-                    *reinterpret_cast<int2 *>(sa + lane * ST + i * CP + c) = fx_limbs(x[q][i], E[q] - fx_exp(x[q][i]));
+                for (int i = 0; i < 2; ++i) {
+                    const Fx3 v = fx_limbs3(x[q][i], E[q] - fx_exp(x[q][i]));
+                    *reinterpret_cast<int2 *>(sa + lane * ST + i * CP + c) = v.v;
+                    sf[lane * 2 * CP + i * CP + c] = (float)v.f;
+                }
         }
         __syncthreads();
         const int l = tid & 15, r0 = (l >> 2) * TR, c0 = (l & 3) * TC;
         long long hh[TR][TC], hl[TR][TC];
+        float cr[TR][TC];
 #pragma unroll
         for (int i = 0; i < TR; ++i)
 #pragma unroll
-            for (int j = 0; j < TC; ++j) hh[i][j] = hl[i][j] = 0;
+            for (int j = 0; j < TC; ++j) {
+                hh[i][j] = hl[i][j] = 0;
+                cr[i][j] = 0.0f;
+            }
         for (int t = tid >> 4; t < n; t += FV_THREADS / 16) {
             const int2 *row = reinterpret_cast<const int2 *>(sa) + t * ST;
-            fx_tile<TR, TC, CP, CP, 2>(row + r0, row + c0, hh, hl);
+            const float *low = sf + t * 2 * CP;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                int2 a[TR], b[TC];
+                float fa[TR], fb[TC];
+                ld_limbs<TR>(row + i * CP + r0, a);
+                ld_limbs<TC>(row + i * CP + c0, b);
+#pragma unroll
+                for (int k = 0; k < TR; ++k) fa[k] = low[i * CP + r0 + k];
+#pragma unroll
+                for (int k = 0; k < TC; ++k) fb[k] = low[i * CP + c0 + k];
+                fx_products<TR, TC>(a, fa, b, fb, hh, hl, cr);
+            }
         }
 #pragma unroll
         for (int i = 0; i < TR; ++i)
 #pragma unroll
             for (int j = 0; j < TC; ++j) {
-                long long T = fx_total(hh[i][j], hl[i][j]);
-                T += __shfl_xor_sync(0xffffffffu, T, 16);
-                if (lane < 16) st[warp][(r0 + i) * CP + c0 + j] = T;
+                long long H;
+                unsigned L;
+                fx_carry(hh[i][j], hl[i][j], cr[i][j], H, L);
+                H += __shfl_xor_sync(0xffffffffu, H, 16);
+                L += __shfl_xor_sync(0xffffffffu, L, 16);
+                if (lane < 16) {
+                    sH[warp][(r0 + i) * CP + c0 + j] = H;
+                    sL[warp][(r0 + i) * CP + c0 + j] = L;
+                }
             }
         __syncthreads();
 #pragma unroll
         for (int p = 0; p < PER; ++p) {
             if (at[p] < 0) continue;
-            long long T = 0;
+            long long H = 0;
+            unsigned L = 0;
 #pragma unroll
-            for (int w = 0; w < NW; ++w) T += st[w][at[p]];
-            acc[p] = fx_add(acc[p], T, s_E[at[p] / CP] + s_E[at[p] % CP]);
+            for (int w = 0; w < NW; ++w) {
+                H += sH[w][at[p]];
+                L += sL[w][at[p]];
+            }
+            acc[p] = fx_add(acc[p], H, L, s_E[at[p] / CP] + s_E[at[p] % CP]);
         }
     }
 #pragma unroll
@@ -429,6 +540,17 @@ void limb_rows_t(const DeviceProblem &d, cudaStream_t s)
     constexpr int OB = LR_THREADS / (CNP == 6 ? 2 : 4);
     k_limb_rows<CNP><<<ceil_div(d.no, OB), LR_THREADS, 0, s>>>(d.no, d.obs_pt, d.obs_cam, d.W, d.Vinv, d.U,
                                                                reinterpret_cast<int2 *>(d.Y), d.Wq, d.fx_ex);
+}
+
+template <int CNP, bool DIAG>
+void schur_fxv_t(const FxArgs &g, int n, const SchurUnit *units, cudaStream_t s)
+{
+    constexpr int bytes = FvShape<CNP, DIAG>::BYTES;
+    if (n == 0) return;
+    if (bytes > 40 * 1024)  // above the default limit (as for k_schur_fx6)
+        cudaFuncSetAttribute(k_schur_fxv<CNP, DIAG>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    k_schur_fxv<CNP, DIAG><<<n, FV_THREADS, bytes, s>>>(g, units);
+    note_launch(1);
 }
 
 }  // namespace
@@ -452,24 +574,25 @@ void launch_camera_fx(const DeviceProblem &d, cudaStream_t s)
 
 void launch_schur_fx(const DeviceProblem &d, double *diag_partial, cudaStream_t s)
 {
-    FxArgs g{d.pair_a, d.pair_b, d.cam_obs, d.obs_pt, reinterpret_cast<const int2 *>(d.Y), d.Wq, d.fx_ex, d.W, d.Vinv,
+    const int2 *Yq = reinterpret_cast<const int2 *>(d.Y);
+    const int low = fx_limb_words(d.cnp);
+    FxArgs g{d.pair_a, d.pair_b, d.cam_obs, d.obs_pt, Yq, d.Wq, Yq + low, d.Wq + low, d.fx_ex, d.W, d.Vinv,
              d.U, d.g + d.N, d.pair_kl, d.schur_partial, diag_partial};
     if (d.cnp == 6) {
         const int ctas = ceil_div(d.n_fx_diag_units, F6_WARPS) + ceil_div(d.n_off_units, F6_WARPS);
         if (ctas == 0) return;
-        k_schur_fx6<<<ctas, 32 * F6_WARPS, 0, s>>>(g, d.n_fx_diag_units, d.fx_diag_units, d.n_off_units, d.off_units);
+        // above the default limit (an attribute of the kernel on this device; the same value always)
+        cudaFuncSetAttribute(k_schur_fx6, cudaFuncAttributeMaxDynamicSharedMemorySize, F6_SMEM);
+        k_schur_fx6<<<ctas, 32 * F6_WARPS, F6_SMEM, s>>>(g, d.n_fx_diag_units, d.fx_diag_units, d.n_off_units, d.off_units);
         note_launch(1);
         return;
     }
-    if (d.n_diag_units > 0) {
-        if (d.cnp == 11) k_schur_fxv<11, true><<<d.n_diag_units, FV_THREADS, 0, s>>>(g, d.diag_units);
-        else k_schur_fxv<16, true><<<d.n_diag_units, FV_THREADS, 0, s>>>(g, d.diag_units);
-        note_launch(1);
-    }
-    if (d.n_off_units > 0) {
-        if (d.cnp == 11) k_schur_fxv<11, false><<<d.n_off_units, FV_THREADS, 0, s>>>(g, d.off_units);
-        else k_schur_fxv<16, false><<<d.n_off_units, FV_THREADS, 0, s>>>(g, d.off_units);
-        note_launch(1);
+    if (d.cnp == 11) {
+        schur_fxv_t<11, true>(g, d.n_diag_units, d.diag_units, s);
+        schur_fxv_t<11, false>(g, d.n_off_units, d.off_units, s);
+    } else {
+        schur_fxv_t<16, true>(g, d.n_diag_units, d.diag_units, s);
+        schur_fxv_t<16, false>(g, d.n_off_units, d.off_units, s);
     }
 }
 
