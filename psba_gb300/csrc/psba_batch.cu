@@ -24,6 +24,7 @@
 #include <cmath>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -1688,12 +1689,17 @@ struct HostBatch {
     size_t bytes = 0;
     cudaGraphExec_t graph = nullptr;  // captured [queue reset, persistent launch]
     int graph_key = -1;               // precision * 1024 + threads of the captured graph
-    // Reading every problem's parameters one by one took two small copies and
-    // a wait each (22 us; 6.8 ms for 304 problems).  The second read since the
-    // parameters last changed brings all of them over in one copy; a caller
-    // that wants one problem's does not pay for the others.
-    std::mutex read_mu;  // reads may come from several threads
-    int reads = 0;       // since the parameters last changed
+    // Reading every problem's parameters one by one takes two small copies and
+    // a wait each (22 us; 6.8 ms for 304 problems).  Once a 16th of the problems,
+    // at least two, have been read since the parameters last changed, the next
+    // read brings all of them over in one copy (that costs about as much as the
+    // single reads before it), so a caller that wants a few does not pay for the
+    // others.  The copy is good until a solve or a reset begins and is not made,
+    // nor used, while one runs, whichever thread reads; its memory, the size of the
+    // parameters, is the batch's until psba_batch_destroy.
+    std::mutex read_mu;
+    int reads = 0;         // since the parameters last changed
+    bool changing = false;  // a solve or a reset is under way
     bool mirrored = false;
     std::vector<double> mirror;
     std::vector<long long> mirror_off;
@@ -1744,11 +1750,16 @@ namespace {
 // Every problem's parameters into h.mirror; on an error the mirror stays unused.
 bool read_all(HostBatch &h)
 {
-    h.mirror_off.resize(h.n);
     long long total = 0;
-    for (int q = 0; q < h.n; ++q) {
-        h.mirror_off[q] = total;
-        total += 6LL * h.probs[q].nc + 3LL * h.probs[q].np;
+    try {
+        h.mirror_off.resize(h.n);
+        for (int q = 0; q < h.n; ++q) {
+            h.mirror_off[q] = total;
+            total += 6LL * h.probs[q].nc + 3LL * h.probs[q].np;
+        }
+        h.mirror.resize((size_t)total);
+    } catch (const std::bad_alloc &) {
+        return false;
     }
     double *d_out = nullptr;
     long long *d_off = nullptr;
@@ -1759,7 +1770,9 @@ bool read_all(HostBatch &h)
     if (e == cudaSuccess) {
         k_batch_pack<<<h.n, 256, 0, h.stream>>>(h.d_probs, d_off, h.d_arena, d_out);
         note_launch(1);
-        h.mirror.resize((size_t)total);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) {
         e = cudaMemcpyAsync(h.mirror.data(), d_out, sizeof(double) * total, cudaMemcpyDeviceToHost, h.stream);
     }
     if (d_out) cudaFreeAsync(d_out, h.stream);
@@ -1770,12 +1783,20 @@ bool read_all(HostBatch &h)
     return e == cudaSuccess;
 }
 
-void params_changed(HostBatch &h)
-{
-    std::lock_guard<std::mutex> lk(h.read_mu);
-    h.reads = 0;
-    h.mirrored = false;
-}
+// Held while a call changes the parameters: the copy that reads are served from
+// is dropped before and after.
+struct Changing {
+    HostBatch &h;
+    explicit Changing(HostBatch &hb) : h(hb) { mark(true); }
+    ~Changing() { mark(false); }
+    void mark(bool on)
+    {
+        std::lock_guard<std::mutex> lk(h.read_mu);
+        h.reads = 0;
+        h.mirrored = false;
+        h.changing = on;
+    }
+};
 
 }  // namespace
 
@@ -1865,10 +1886,11 @@ int psba_batch_reset_params(psba_batch *b)
 {
     if (!b) return set_error("null batch"), PSBA_ERR_ARG;
     HostBatch &h = b->hb;
-    params_changed(h);
+    const Changing guard(h);
     k_batch_reset<<<h.n, 256, 0, h.stream>>>(h.d_probs, h.d_arena);
     note_launch(1);
-    const cudaError_t e = cudaStreamSynchronize(h.stream);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h.stream);
     return e == cudaSuccess ? PSBA_OK : cuda_fail(e, "psba_batch_reset_params");
 }
 
@@ -1877,7 +1899,7 @@ int psba_batch_levmar(psba_batch *b, const psba_opts *opts, psba_batch_result *r
     if (!b || !opts) return set_error("null argument"), PSBA_ERR_ARG;
     if (opts->refine != 0) return set_error("psba_batch_levmar: refine is for the per-handle solver"), PSBA_ERR_ARG;
     HostBatch &h = b->hb;
-    params_changed(h);
+    const Changing guard(h);
     BatchOpts o;
     o.tau = opts->tau;
     o.stop_thresh = opts->stop_thresh;
@@ -1951,7 +1973,8 @@ int psba_batch_get_params(psba_batch *b, int q, double *cams, double *pts)
     const BatchProblem &p = h.probs[q];
     {
         std::lock_guard<std::mutex> lk(h.read_mu);
-        if (!h.mirrored && h.n > 2 && ++h.reads == 2) h.mirrored = read_all(h);
+        const int few = std::max(2, h.n / 16);
+        if (!h.changing && !h.mirrored && h.n > few && ++h.reads == few + 1) h.mirrored = read_all(h);
         if (h.mirrored) {
             const double *m = h.mirror.data() + h.mirror_off[q];
             std::memcpy(cams, m, sizeof(double) * 6 * p.nc);
