@@ -445,7 +445,7 @@ __device__ void stage_schur(const BatchProblem &p, const Arenas<double> &ar, dou
 // along, then L^T x = y.  Returns 0, or 1 on a non-positive / non-finite pivot
 // (the reference's status, SPD_inv.cl:66-107).
 //
-// By panels of chol_width(N) columns in shared memory (P, chol_smem(N) bytes):
+// By panels of chol_width(N) columns in shared memory (P, chol_panel(N) bytes):
 // the panel's columns are eliminated there, one barrier per column (rhs is the
 // row below; thread 0, whose entry is the next pivot, takes its reciprocal
 // root), and the rest of S takes the panel's product from shared memory in
@@ -461,10 +461,14 @@ __device__ void stage_schur(const BatchProblem &p, const Arenas<double> &ar, dou
 // panel where the FP64 pipe would take sixteen.
 // The width depends on N alone, so a result does not depend on the batch.
 __host__ __device__ inline int chol_width(int N) { return N <= 384 ? 16 : N <= 768 ? 8 : N <= 1536 ? 4 : N <= 3072 ? 2 : 1; }
-__host__ __device__ inline size_t chol_smem(int N)
+__host__ __device__ inline size_t chol_panel(int N)  // bytes
 {
     return sizeof(double) * (size_t)(N + 1) * (size_t)(chol_width(N) + 1) + sizeof(int) * (size_t)(N + 2);
 }
+// Above CHOL_SHARED_N the panel, one column by then, is a piece of the problem's
+// arena: it grows without a bound, and shared memory has one (N ~ 11,000).  What
+// a pass costs there is S itself, which it reads and writes once per column.
+constexpr int CHOL_SHARED_N = 3072;
 constexpr int CHOL_NB = 16;  // the widest panel
 
 template <bool FX>
@@ -1308,7 +1312,7 @@ __device__ void solve_problem(const BatchProblem &p, const Arenas<R> &ar, const 
             }
             __syncthreads();
             double *S = ar.d + p.d_S, *rhs = ar.d + p.d_rhs, *x = ar.d + p.d_x;
-            const int st = stage_cholesky_solve<!MX>(S, N, rhs, x, sh, dyn);
+            const int st = stage_cholesky_solve<!MX>(S, N, rhs, x, sh, N > CHOL_SHARED_N ? ar.d + p.d_panel : dyn);
             if (threadIdx.x == 0) shi[4]++;
             int decided = 0;  // 0: retry with larger mu, 1: accepted, 2: stop
             if (st == 0) {
@@ -1559,6 +1563,7 @@ bool build_problem_layout(const psba_problem_desc &p, ProblemLayout &L, std::str
     bp.d_tab2 = dres((size_t)CAMTAB * nc);
     bp.d_rhs = dres((size_t)N);
     bp.d_x = dres((size_t)N);
+    bp.d_panel = dres(N > CHOL_SHARED_N ? (chol_panel(N) + sizeof(double) - 1) / sizeof(double) : 0);
     // one LM iteration: per-observation work plus the in-CTA FP64 Cholesky
     L.work = (double)no + 0.02 * std::pow((double)N, 3) / 64.0;
     return true;
@@ -1568,7 +1573,7 @@ void rebase_problem(BatchProblem &bp, long long db, long long ib, long long rb)
 {
     for (long long *f : {&bp.d_K, &bp.d_q0, &bp.d_cams, &bp.d_pts, &bp.d_cams0, &bp.d_pts0, &bp.d_meas, &bp.d_V,
                          &bp.d_Vinv, &bp.d_U, &bp.d_g, &bp.d_uvdiag, &bp.d_dp, &bp.d_S, &bp.d_tab,
-                         &bp.d_tab2, &bp.d_rhs, &bp.d_x})
+                         &bp.d_tab2, &bp.d_rhs, &bp.d_x, &bp.d_panel})
         *f += db;
     for (long long *f : {&bp.i_obs_pt, &bp.i_obs_cam, &bp.i_pt_start, &bp.i_cam_start, &bp.i_cam_obs,
                          &bp.i_pair_start, &bp.i_pair_kl, &bp.i_pair_a, &bp.i_pair_b})
@@ -1591,9 +1596,9 @@ size_t pool_bytes(const ProblemLayout &L, int precision)
 static size_t batch_smem(int precision, int threads, int max_N)
 {
     // the width steps down as N grows, so a smaller N can need more
-    size_t b = chol_smem(max_N);
-    for (int step : {384, 768, 1536, 3072})
-        if (max_N > step) b = std::max(b, chol_smem(step));
+    size_t b = chol_panel(std::min(max_N, CHOL_SHARED_N));
+    for (int step : {384, 768, 1536})
+        if (max_N > step) b = std::max(b, chol_panel(step));
     if (precision != PSBA_PREC_MIXED) b = std::max(b, sizeof(int2) * F6_WORDS * (size_t)(threads / 32));
     return b;
 }
@@ -1926,9 +1931,10 @@ int psba_batch_levmar(psba_batch *b, const psba_opts *opts, psba_batch_result *r
         cudaMemsetAsync(h.d_queue, 0, sizeof(int), h.stream);
         cudaMemsetAsync(h.d_res, 0, sizeof(BatchResult) * h.n, h.stream);  // every problem starts afresh
         const int grid = std::min(h.n, batch_blocks_per_sm(opts->precision, h.threads, h.max_N) * sms);
-        launch_batch_lm(opts->precision, grid, h.threads, h.max_N, h.stream, h.d_probs, h.d_order, h.n, h.d_queue,
-                        h.d_arena, h.i_arena, h.r_arena, h.d_opts, h.d_res);
-        e = cudaStreamEndCapture(h.stream, &g);
+        e = launch_batch_lm(opts->precision, grid, h.threads, h.max_N, h.stream, h.d_probs, h.d_order, h.n, h.d_queue,
+                            h.d_arena, h.i_arena, h.r_arena, h.d_opts, h.d_res);
+        const cudaError_t ended = cudaStreamEndCapture(h.stream, &g);
+        if (e == cudaSuccess) e = ended;
         if (e == cudaSuccess) e = cudaGraphInstantiate(&h.graph, g, 0);
         if (g) cudaGraphDestroy(g);
         if (e != cudaSuccess) return cuda_fail(e, "psba_batch_levmar graph");

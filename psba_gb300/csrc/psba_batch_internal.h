@@ -25,7 +25,7 @@ struct BatchProblem {
     // camera step, and gb rounded to FP32
     long long r_tab32, r_tab2f, r_tab2f2, r_meas2f, r_pts2f, r_x2f, r_vinv2f, r_dpa2f, r_gb32;
     long long r_fx;  // R arena, FP64 form: the limb rows' third pieces, in the place of the mixed form's copies
-    long long d_V, d_Vinv, d_U, d_g, d_uvdiag, d_dp, d_S, d_tab, d_tab2, d_rhs, d_x;  // double arena
+    long long d_V, d_Vinv, d_U, d_g, d_uvdiag, d_dp, d_S, d_tab, d_tab2, d_rhs, d_x, d_panel;  // double arena
 };
 
 // A problem's LM state between launches (and its result at the end): the
