@@ -445,7 +445,7 @@ __device__ void stage_schur(const BatchProblem &p, const Arenas<double> &ar, dou
 // along, then L^T x = y.  Returns 0, or 1 on a non-positive / non-finite pivot
 // (the reference's status, SPD_inv.cl:66-107).
 //
-// By panels of chol_width(N) columns in shared memory (P, chol_panel(N) bytes):
+// By panels of chol_width(N) columns (P, chol_panel(N) bytes, in shared memory if it fits):
 // the panel's columns are eliminated there, one barrier per column (rhs is the
 // row below; thread 0, whose entry is the next pivot, takes its reciprocal
 // root), and the rest of S takes the panel's product from shared memory in
@@ -460,15 +460,22 @@ __device__ void stage_schur(const BatchProblem &p, const Arenas<double> &ar, dou
 // cut is 2^-57 of the row's own scale), one FP64 instruction per entry and
 // panel where the FP64 pipe would take sixteen.
 // The width depends on N alone, so a result does not depend on the batch.
-__host__ __device__ inline int chol_width(int N) { return N <= 384 ? 16 : N <= 768 ? 8 : N <= 1536 ? 4 : N <= 3072 ? 2 : 1; }
+//
+// Up to CHOL_SHARED_N the panel is in shared memory, as wide as leaves room for
+// two CTAs an SM; above it is a piece of the problem's arena, sixteen columns
+// wide, and a problem of any size has one: narrower panels in shared memory
+// pass over S too often there (one iteration, FP64 / mixed: 257 cameras 588 /
+// 299 ms with two columns in shared memory, 184 / 188 so; 513 cameras, FP64, 8.7 s
+// with one, 1.3 s so; 129 cameras, mixed, 26.5 with four in shared memory, 29.0 so).
+constexpr int CHOL_SHARED_N = 1536;
+__host__ __device__ inline int chol_width(int N)
+{
+    return N <= 384 || N > CHOL_SHARED_N ? 16 : N <= 768 ? 8 : 4;
+}
 __host__ __device__ inline size_t chol_panel(int N)  // bytes
 {
     return sizeof(double) * (size_t)(N + 1) * (size_t)(chol_width(N) + 1) + sizeof(int) * (size_t)(N + 2);
 }
-// Above CHOL_SHARED_N the panel, one column by then, is a piece of the problem's
-// arena: it grows without a bound, and shared memory has one (N ~ 11,000).  What
-// a pass costs there is S itself, which it reads and writes once per column.
-constexpr int CHOL_SHARED_N = 3072;
 constexpr int CHOL_NB = 16;  // the widest panel
 
 template <bool FX>
@@ -1228,7 +1235,9 @@ __device__ double stage_cost_mx(const BatchProblem &p, const Arenas<float> &ar, 
 
 // ---------------------------------------------------------------- one problem
 
-template <typename R>
+// FAR: some problem of the launch has its panel in global memory (apart from the
+// rest, because accesses to shared memory then go by generic addresses)
+template <typename R, bool FAR>
 __device__ void solve_problem(const BatchProblem &p, const Arenas<R> &ar, const BatchOpts &o, BatchResult *res,
                               double *sh, int *shi, double *shd, double *dyn)
 {
@@ -1312,7 +1321,7 @@ __device__ void solve_problem(const BatchProblem &p, const Arenas<R> &ar, const 
             }
             __syncthreads();
             double *S = ar.d + p.d_S, *rhs = ar.d + p.d_rhs, *x = ar.d + p.d_x;
-            const int st = stage_cholesky_solve<!MX>(S, N, rhs, x, sh, N > CHOL_SHARED_N ? ar.d + p.d_panel : dyn);
+            const int st = stage_cholesky_solve<!MX>(S, N, rhs, x, sh, FAR && N > CHOL_SHARED_N ? ar.d + p.d_panel : dyn);
             if (threadIdx.x == 0) shi[4]++;
             int decided = 0;  // 0: retry with larger mu, 1: accepted, 2: stop
             if (st == 0) {
@@ -1397,7 +1406,7 @@ __device__ void solve_problem(const BatchProblem &p, const Arenas<R> &ar, const 
     __syncthreads();
 }
 
-template <typename R>
+template <typename R, bool FAR>
 __global__ void __launch_bounds__(MAX_THREADS) k_batch_lm(const BatchProblem *__restrict__ probs,
                                                            const int *__restrict__ order, int n,
                                                            int *__restrict__ queue, Arenas<R> ar,
@@ -1418,7 +1427,7 @@ __global__ void __launch_bounds__(MAX_THREADS) k_batch_lm(const BatchProblem *__
         if (q >= n) break;
         const int pi = order[q];
         const BatchProblem p = probs[pi];
-        solve_problem<R>(p, ar, o, res + pi, sh, shi, shd, dyn);
+        solve_problem<R, FAR>(p, ar, o, res + pi, sh, shi, shd, dyn);
     }
 }
 
@@ -1597,7 +1606,7 @@ static size_t batch_smem(int precision, int threads, int max_N)
 {
     // the width steps down as N grows, so a smaller N can need more
     size_t b = chol_panel(std::min(max_N, CHOL_SHARED_N));
-    for (int step : {384, 768, 1536})
+    for (int step : {384, 768})
         if (max_N > step) b = std::max(b, chol_panel(step));
     if (precision != PSBA_PREC_MIXED) b = std::max(b, sizeof(int2) * F6_WORDS * (size_t)(threads / 32));
     return b;
@@ -1614,15 +1623,16 @@ static cudaError_t batch_attributes()
     std::lock_guard<std::mutex> lk(mu);
     if (done[dev]) return cudaSuccess;
     e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    cudaFuncAttributes fa;
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_batch_lm<float>);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_batch_lm<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 most - (int)fa.sharedSizeBytes);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_batch_lm<double>);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_batch_lm<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 most - (int)fa.sharedSizeBytes);
+    auto opt_in = [&](auto *kernel) {
+        cudaFuncAttributes fa;
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, kernel);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fa.sharedSizeBytes);
+    };
+    opt_in(k_batch_lm<float, false>);
+    opt_in(k_batch_lm<float, true>);
+    opt_in(k_batch_lm<double, false>);
+    opt_in(k_batch_lm<double, true>);
     done[dev] = e == cudaSuccess;
     return e;
 }
@@ -1636,10 +1646,12 @@ cudaError_t launch_batch_lm(int precision, int grid, int threads, int max_N, cud
     const size_t smem = batch_smem(precision, threads, max_N);
     if (precision == PSBA_PREC_MIXED) {
         Arenas<float> ar{darena, iarena, (float *)rarena};
-        k_batch_lm<float><<<grid, threads, smem, s>>>(probs, order, n, queue, ar, opts, res);
+        const auto kernel = max_N > CHOL_SHARED_N ? k_batch_lm<float, true> : k_batch_lm<float, false>;
+        kernel<<<grid, threads, smem, s>>>(probs, order, n, queue, ar, opts, res);
     } else {
         Arenas<double> ar{darena, iarena, (double *)rarena};
-        k_batch_lm<double><<<grid, threads, smem, s>>>(probs, order, n, queue, ar, opts, res);
+        const auto kernel = max_N > CHOL_SHARED_N ? k_batch_lm<double, true> : k_batch_lm<double, false>;
+        kernel<<<grid, threads, smem, s>>>(probs, order, n, queue, ar, opts, res);
     }
     return cudaGetLastError();  // the caller counts the launch (it may be inside a graph capture)
 }
@@ -1650,9 +1662,9 @@ int batch_blocks_per_sm(int precision, int threads, int max_N)
     if (batch_attributes() != cudaSuccess) return 1;
     const size_t smem = batch_smem(precision, threads, max_N);
     if (precision == PSBA_PREC_MIXED)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_lm<float>, threads, smem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_lm<float, false>, threads, smem);
     else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_lm<double>, threads, smem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_lm<double, false>, threads, smem);
     return per_sm > 0 ? per_sm : 1;
 }
 
