@@ -188,7 +188,8 @@ int psba_levmar_resume(psba_handle *h, const psba_opts *opts, double mu, int nu,
                        psba_result *res);
 
 /* Bound of the handle's device-side waits: the dense factor's waits on its
- * tile flags and hand-offs, in polls (0: the default, 2^22, a second or two).  A wait that runs out ends its kernel
+ * tile flags and hand-offs and the triangular solves' waits for one another's
+ * blocks, in polls (0: the default, 2^22, a second or two).  A wait that runs out ends its kernel
  * with a status the driver reads; the solve then returns PSBA_ERR_STATE and
  * the handle stays usable.  No reference counterpart: the reference's
  * device-side enqueue chain has no waits of its own (CL_files/SPD_inv.cl:165-179). */

@@ -981,7 +981,8 @@ __global__ void __launch_bounds__(TS_THREADS) k_tri_solve(int refine, int Np, in
 // N = 528 takes 28 us, with a barrier of the cluster a step 56.
 constexpr int TC_CTAS = 8, TC_THREADS = 256, TC_OWNERS = TC_CTAS - 1;
 constexpr int TC_NEAR = 3;           // blocks up to p + TC_NEAR - 1 take x_p in CTA 0
-constexpr int TC_POLLS = 1 << 20;    // polls per wait (~1 s)
+constexpr int TC_SPIN = 1 << 12;     // polls without a pause (~60 us, longer than any wait of a solve that runs)
+constexpr int TC_DRAIN = 1 << 20;    // polls for what is still under way to a CTA that gave up
 
 __device__ __forceinline__ unsigned smem_at(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 
@@ -1000,21 +1001,32 @@ __device__ __forceinline__ void mb_arrive(unsigned long long *b)
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_at(b)) : "memory");
 }
 
-// Waits for the barrier's first phase; *dead is set, and nothing waited for any
-// more, when the polls run out.
-__device__ __forceinline__ void mb_wait(unsigned long long *b, bool *dead)
+// Waits for the barrier's first phase, `limit` polls at most; false if they ran
+// out.  (test_wait: try_wait suspends the thread for as long as the device likes,
+// a hint of 100 ns notwithstanding, so its polls bound nothing.)
+__device__ __forceinline__ bool mb_poll(unsigned long long *b, long long limit)
 {
-    if (*dead) return;
-    for (int it = 0; it < TC_POLLS; ++it) {
+    for (long long it = 0; it < limit; ++it) {
         int ok;
-        asm volatile("{ .reg .pred q; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 q, [%1], 0; selp.s32 %0, 1, 0, q; }"
+        asm volatile("{ .reg .pred q; mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 q, [%1], 0; selp.s32 %0, 1, 0, q; }"
                      : "=r"(ok)
                      : "r"(smem_at(b))
                      : "memory");
-        if (ok) return;
+        if (ok) return true;
+        if (it >= TC_SPIN) __nanosleep(200);
     }
-    *dead = true;
+    return false;
 }
+
+// The waits of a thread: after one that ran out, nothing is waited for any more
+struct TriWait {
+    long long limit;
+    bool dead;
+    __device__ __forceinline__ void operator()(unsigned long long *b)
+    {
+        if (!dead) dead = !mb_poll(b, limit);
+    }
+};
 
 // The address of p's place in the shared memory of CTA `rank`
 __device__ __forceinline__ unsigned peer_at(const void *p, int rank)
@@ -1085,7 +1097,7 @@ struct TriView {
 // CTA, far (Np) is CTA 0's inbox and the others' blocks, bars 2 nb barriers.
 template <bool FWD>
 __device__ __forceinline__ void tri_pass(const TriView<FWD> &m, int rank, const double *base, double *xs, double *far,
-                                         unsigned long long *bars, double (*yb)[T], double (*near2)[T], bool *dead)
+                                         unsigned long long *bars, double (*yb)[T], double (*near2)[T], TriWait &wait)
 {
     const int tid = threadIdx.x, lane = tid & 31, g = tid & 3, nb = m.nb;
     if (rank == 0) {
@@ -1150,9 +1162,9 @@ __device__ __forceinline__ void tri_pass(const TriView<FWD> &m, int rank, const 
             if (nb > 3) m.coef(cp += cs, cn);
             for (int p = 2; p < nb; ++p) {
                 if (p + 2 < nb) m.coef(cp += cs, cm);
-                if (p >= TC_NEAR) mb_wait(bfar + p, dead);
+                if (p >= TC_NEAR) wait(bfar + p);
                 const double b = (p >= TC_NEAR ? far : base)[m.block(p) * T + c];
-                mb_wait(bx + p - 2, dead);
+                wait(bx + p - 2);
                 const double v = b - dot4(cf, xs + m.block(p - 2) * T + 4 * g);
                 if (g == 0) near2[p & 1][c] = v;
                 // a barrier per parity: the next but one, p + 2, needs an x_p that
@@ -1183,7 +1195,7 @@ __device__ __forceinline__ void tri_pass(const TriView<FWD> &m, int rank, const 
             int p = next(q + TC_NEAR);
             const int pn = next(q + 2 + TC_NEAR);
             if (pn < nb) coef(q + 2, pn, cm);
-            mb_wait(bars + q, dead);
+            wait(bars + q);
             const double *xq = xs + m.block(q) * T + 4 * g;
             if (p < nb) {
                 const double s = dot4(cf, xq);
@@ -1230,7 +1242,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tri_cluster(int refine, int N
                                                             const double *__restrict__ Linv,
                                                             const double *__restrict__ rhs,
                                                             double *__restrict__ x, float2 *__restrict__ x2,
-                                                            int *__restrict__ status)
+                                                            int *__restrict__ status, long long spin_limit)
 {
     static_assert(T == 16 && TC_CTAS == 8, "two sends a lane reach the other CTAs");
     extern __shared__ double tri_sm[];  // per pass: x, inbox; then the barriers
@@ -1246,20 +1258,23 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tri_cluster(int refine, int N
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     cl_sync();
-    bool dead = false;
+    TriWait wait{spin_limit, false};
     double *xs = tri_sm, *far = tri_sm + (size_t)passes * Np;
     if (refine) {
-        tri_pass(TriView<true>{S, Linv, Np, nb}, rank, rhs, xs, far, bars, yb, near2, &dead);
+        tri_pass(TriView<true>{S, Linv, Np, nb}, rank, rhs, xs, far, bars, yb, near2, wait);
         __syncthreads();
-        tri_pass(TriView<false>{S, Linv, Np, nb}, rank, xs, xs + Np, far + Np, bars + 2 * nb, yb, near2, &dead);
+        tri_pass(TriView<false>{S, Linv, Np, nb}, rank, xs, xs + Np, far + Np, bars + 2 * nb, yb, near2, wait);
         xs += Np;
     } else {
-        tri_pass(TriView<false>{S, Linv, Np, nb}, rank, rhs, xs, far, bars, yb, near2, &dead);
+        tri_pass(TriView<false>{S, Linv, Np, nb}, rank, rhs, xs, far, bars, yb, near2, wait);
     }
-    if (dead) atomicCAS(status, 0, 2);
-    __syncthreads();
-    // every block sent to a CTA has been waited for there; a CTA that gave up
-    // stays until all have sent
+    if (wait.dead) atomicCAS(status, 0, 2);
+    // Every block sent to a CTA has been waited for there, or (all are sent, if
+    // late, whoever gave up) is waited for now: a store under way must not outlive
+    // the CTA whose shared memory it goes to.
+    if (__syncthreads_or(wait.dead))
+        for (int i = tid; i < passes * nb; i += TC_THREADS)
+            if (rank != 0 || i % nb >= TC_NEAR) mb_poll(bars + (i >= nb ? nb + i : i), TC_DRAIN);
     cl_sync();
     if (rank == 0)
         for (int i = tid; i < Np; i += TC_THREADS) {
@@ -1293,7 +1308,7 @@ void launch_tri(const DeviceProblem &d, int refine, double *x, cudaStream_t s)
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const double *S = d.S, *Linv = d.Linv, *rhs = d.rhs;
-    cudaLaunchKernelEx(&cfg, k_tri_cluster, refine, Np, nb, S, Linv, rhs, x, x2, d.status);
+    cudaLaunchKernelEx(&cfg, k_tri_cluster, refine, Np, nb, S, Linv, rhs, x, x2, d.status, d.wait_limit);
 #else
     k_tri_solve<<<1, TS_THREADS, sizeof(double) * Np, s>>>(refine, Np, nb, d.S, d.Linv, d.rhs, x, x2, d.status);
 #endif

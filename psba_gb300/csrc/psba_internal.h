@@ -272,7 +272,7 @@ struct DeviceProblem {
     int2 *chol_tasks = nullptr;   // helper tasks of the dense factor, in dependency order
     int chol_n_tasks = 0;
     int chol_grid_cap = 0;        // CTAs of the dense factor at most (0: one per SM)
-    long long wait_limit = DEFAULT_WAIT_LIMIT;  // polls per device-side wait (dense factor flags and mail)
+    long long wait_limit = DEFAULT_WAIT_LIMIT;  // polls per device-side wait (dense factor and triangular solves)
     ulonglong2 *chol_mail = nullptr;  // hand-offs of the dense factor's chain: CHOL_MAIL packets (value, epoch) per block column
     int *chol_flags = nullptr;    // one flag per tile (value = epoch when done)
     int chol_n_flags = 0;
