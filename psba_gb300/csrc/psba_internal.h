@@ -250,8 +250,8 @@ struct DeviceProblem {
     float *Vinv2f = nullptr;      // 12 per point: V^-1 as FP32 pairs hi + lo (the mixed form's Y)
     float *gb32 = nullptr;        // 3 per point: gb rounded to FP32 (the mixed form's ea sums)
     float *camtab32 = nullptr;    // CAMTAB32 per camera: the table's M, D, fx, sk, fy in FP32 (mixed J)
-    double *Y = nullptr;          // 18 per obs; FP64 form: Y's limb rows (fx_words per obs), Y after psba_eval_reduced
-    int2 *Wq = nullptr;           // FP64 form: W's limb rows (fx_words per obs)
+    double *Y = nullptr;          // 18 per obs (FP64 form: after psba_eval_reduced)
+    int2 *Yq = nullptr, *Wq = nullptr;  // FP64 form, from its first solve on: Y's and W's limb rows (fx_words per obs)
     int2 *fx_ex = nullptr;        // FP64 form: per obs, the exponents of its Y and W limb rows
     double *schur_partial = nullptr;  // off-diagonal slots (off_partial_slots), then the diagonal units'
     double *S = nullptr;          // Np x Np (lower)

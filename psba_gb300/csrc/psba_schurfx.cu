@@ -539,7 +539,7 @@ void limb_rows_t(const DeviceProblem &d, cudaStream_t s)
 {
     constexpr int OB = LR_THREADS / (CNP == 6 ? 2 : 4);
     k_limb_rows<CNP><<<ceil_div(d.no, OB), LR_THREADS, 0, s>>>(d.no, d.obs_pt, d.obs_cam, d.W, d.Vinv, d.U,
-                                                               reinterpret_cast<int2 *>(d.Y), d.Wq, d.fx_ex);
+                                                               d.Yq, d.Wq, d.fx_ex);
 }
 
 template <int CNP, bool DIAG>
@@ -574,9 +574,8 @@ void launch_camera_fx(const DeviceProblem &d, cudaStream_t s)
 
 void launch_schur_fx(const DeviceProblem &d, double *diag_partial, cudaStream_t s)
 {
-    const int2 *Yq = reinterpret_cast<const int2 *>(d.Y);
     const int low = fx_limb_words(d.cnp);
-    FxArgs g{d.pair_a, d.pair_b, d.cam_obs, d.obs_pt, Yq, d.Wq, Yq + low, d.Wq + low, d.fx_ex, d.W, d.Vinv,
+    FxArgs g{d.pair_a, d.pair_b, d.cam_obs, d.obs_pt, d.Yq, d.Wq, d.Yq + low, d.Wq + low, d.fx_ex, d.W, d.Vinv,
              d.U, d.g + d.N, d.pair_kl, d.schur_partial, diag_partial};
     if (d.cnp == 6) {
         const int ctas = ceil_div(d.n_fx_diag_units, F6_WARPS) + ceil_div(d.n_off_units, F6_WARPS);

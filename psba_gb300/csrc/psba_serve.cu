@@ -345,7 +345,7 @@ size_t large_bytes(const psba_problem_desc &p, int cnp)
     const size_t N = c * nc, Np = (N + TILE - 1) / TILE * TILE;
     // Schur units of at least 32 entries or observations, and one more per pair and camera
     const size_t off_units = entries / 32 + nc * (nc - 1) / 2, diag_units = no / 32 + nc;
-    const size_t per_obs = 2 + 2 * c + 6 + 3 * c + 2 * (size_t)fx_words(cnp) + 1 + 3 * 2 + 3 + 4;
+    const size_t per_obs = 2 + 2 * c + 6 + 2 * 3 * c + 2 * (size_t)fx_words(cnp) + 1 + 3 * 2 + 3 + 4;
     const size_t per_pt = 3 * 3 + 6 * 2 + 9 + 3 * 6;
     const size_t doubles = no * per_obs + np * per_pt + N * 8 + nc * (c * c + 2 * CAMTAB) + 3 * Np * Np +
                            Np * TILE + Np / TILE * CHOL_MAIL * 2 + (off_units + nc * 8) * c * c + diag_units * (c * (c + 1) / 2 + c);

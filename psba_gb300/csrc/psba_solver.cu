@@ -331,10 +331,23 @@ void enqueue_linearize(psba_handle *h, double coeff, bool tables = false)
     }
 }
 
-// Reduced system for damping mu: V^-1, Y, S, ea (rhs).
-void enqueue_reduced(psba_handle *h, double mu)
+// The FP64 form's limb rows, as long as the handle lives from its first FP64 solve
+// on: 392 bytes an observation at six parameters that the mixed form has no use for.
+int have_limb_rows(psba_handle *h)
 {
     DeviceProblem &d = h->d;
+    if (d.prec != PSBA_PREC_FP64 || d.fx_ex) return PSBA_OK;
+    const size_t words = (size_t)fx_words(d.cnp) * (size_t)d.no;
+    if (!d.Yq) TRY(dalloc(h, &d.Yq, words));
+    if (!d.Wq) TRY(dalloc(h, &d.Wq, words));
+    return dalloc(h, &d.fx_ex, (size_t)d.no);
+}
+
+// Reduced system for damping mu: V^-1, Y, S, ea (rhs).
+int enqueue_reduced(psba_handle *h, double mu)
+{
+    DeviceProblem &d = h->d;
+    TRY(have_limb_rows(h));
     {
         StageScope sc(h, ST_VINV);
         launch_vinv(d, mu, h->stream);
@@ -356,6 +369,7 @@ void enqueue_reduced(psba_handle *h, double mu)
         StageScope sc(h, ST_SCHUR_REDUCE);
         launch_schur_reduce(d, mu, h->stream);
     }
+    return PSBA_OK;
 }
 
 // Cholesky + solves -> dpa into dp[0..N), then eb, dpb, scalars.
@@ -452,7 +466,7 @@ int levmar_impl(psba_handle *h, const psba_opts *o, int *itno, psba_result *res,
             nu = 2;
         }
         while (true) {
-            enqueue_reduced(h, mu);
+            TRY(enqueue_reduced(h, mu));
             enqueue_step(h, mu);
             enqueue_cost_trial(h, d.dp, true);
             TRY(check_launch());
@@ -542,7 +556,7 @@ int compute_pb(psba_handle *h, double *lambda, int *solved)
 {
     DeviceProblem &d = h->d;
     const long long nt = d.N + 3LL * d.np;
-    enqueue_reduced(h, *lambda);
+    TRY(enqueue_reduced(h, *lambda));
     if (d.Nm3 == d.Np)
         PSBA_CUDA_TRY(cudaMemcpyAsync(d.Ssave, d.S, sizeof(double) * (size_t)d.Np * d.Np,
                                       cudaMemcpyDeviceToDevice, h->stream));
@@ -1048,9 +1062,7 @@ int create_impl(const psba_problem_desc *p, psba_handle *h)
     TRY(dalloc(h, &d.Vinv, 6 * (size_t)np));
     TRY(dalloc(h, &d.Vinv2f, 12 * (size_t)np));
     TRY(dalloc(h, &d.gb32, 3 * (size_t)np));
-    TRY(dalloc(h, &d.Y, (size_t)fx_words(d.cnp) * (size_t)no));
-    TRY(dalloc(h, &d.Wq, (size_t)fx_words(d.cnp) * (size_t)no));
-    TRY(dalloc(h, &d.fx_ex, (size_t)no));
+    TRY(dalloc(h, &d.Y, 3 * cnp * (size_t)no));
     TRY(dalloc(h, &d.schur_partial,
                cnp * cnp * off_partial_slots(d) + diag_nv * std::max(diag_units.size(), fx_diag_units.size())));
     TRY(dalloc(h, &d.S, (size_t)d.Np * d.Np));
@@ -1429,11 +1441,11 @@ int psba_eval_reduced(psba_handle *h, double mu, double *Vinv, double *Y, double
     if (!h) return set_error("null handle"), PSBA_ERR_ARG;
     if (!h->linearized) return set_error("psba_eval_reduced needs a linearization first"), PSBA_ERR_STATE;
     DeviceProblem &d = h->d;
-    enqueue_reduced(h, mu);
+    TRY(enqueue_reduced(h, mu));
     h->last_mu = mu;
     TRY(check_launch());
     const size_t no = (size_t)d.no, np = (size_t)d.np;
-    if (Y && d.prec == PSBA_PREC_FP64) {  // in the place of its limb rows
+    if (Y && d.prec == PSBA_PREC_FP64) {  // the solves take it in limbs
         launch_yblocks(d, h->stream);
         TRY(check_launch());
     }
