@@ -10,9 +10,8 @@
 // inverses, in a fixed dependency order; waits are bounded spins on per-tile
 // flags in global memory (acquire/release) or on the values themselves, sent
 // with the launch's epoch (mail).  After the factor, the back
-// solve L^T x = y runs on a thread-block cluster (k_tri_cluster; k_tri_solve,
-// one CTA, when PSBA_TRI_CLUSTER is 0).  On request one step of iterative
-// refinement follows: r = b - S x in FP64 against a copy of S taken before
+// solve L^T x = y runs on a thread-block cluster (k_tri_cluster).  On request
+// one step of iterative refinement follows: r = b - S x in FP64 against a copy of S taken before
 // the factor (k_refine_residual), then both triangular solves of r with the
 // factor, added into x (the same kernels with their forward part on).
 //
@@ -42,9 +41,6 @@ constexpr int TT = TILE * TILE;
 #endif
 #ifndef PSBA_CHOL_BJ
 #define PSBA_CHOL_BJ 8
-#endif
-#ifndef PSBA_TRI_CLUSTER
-#define PSBA_TRI_CLUSTER 1  // triangular solves on a cluster of CTAs (else one CTA)
 #endif
 #ifndef PSBA_CHOL_PER_SM
 #define PSBA_CHOL_PER_SM 1  // the panel's FP64 chain runs alone on its SM
@@ -410,139 +406,29 @@ __device__ __forceinline__ bool panel_finish(const double (*X)[T + 1], const int
     return bad;
 }
 
-// The single-CTA back solve over the factor (S lower = L, Linv = diagonal
-// tile inverses) with the right-hand side in shared memory.  A block step is
-// the 16 x 16 product with the diagonal inverse, then the update of the other
-// blocks, one column of it per thread, reading one row panel of L with
-// independent loads; it is bound by the SM's FP64 rate (N^2 / 2
-// multiply-adds on one SM).  The diagonal product is spread over 256 threads
-// (one product each, summed by a fixed shuffle tree over 16 lanes), and the
-// values a thread needs for the next block step (its Linv entry, its 16
-// panel values) are loaded while the current one runs.
-
-// One lane of the 16 x 16 diagonal product: 16 lanes hold the products of one
-// output, summed in a fixed order.
-__device__ __forceinline__ double half_warp_sum(double p)
-{
-#pragma unroll
-    for (int off = T / 2; off > 0; off >>= 1) p += __shfl_xor_sync(0xffffffffu, p, off);
-    return p;
-}
-
-// forward: b <- L^-1 b (right-looking: y_K = Linv_K b_K, then b_I -= L_IK y_K)
-__device__ void cta_forward(int Np, int nb, const double *__restrict__ S, const double *__restrict__ Linv,
-                            double *bs, double *tmp)
-{
-    const int tid = threadIdx.x;
-    for (int K = 0; K < nb; ++K) {
-        if (tid < T) {
-            const double *Li = Linv + (size_t)K * TT + tid * T;
-            double y = 0.0;
-#pragma unroll
-            for (int k = 0; k < T; ++k) y = fma(k <= tid ? __ldcg(Li + k) : 0.0, bs[K * T + k], y);
-            tmp[tid] = y;
-        }
-        __syncthreads();
-        if (tid < T) bs[K * T + tid] = tmp[tid];
-        for (int i = (K + 1) * T + tid; i < Np; i += blockDim.x) {
-            const double2 *row = reinterpret_cast<const double2 *>(S + (size_t)i * Np + K * T);
-            double s = 0.0;
-#pragma unroll
-            for (int c = 0; c < T / 2; ++c) {
-                const double2 v = __ldcg(row + c);
-                s = fma(v.x, tmp[2 * c], s);
-                s = fma(v.y, tmp[2 * c + 1], s);
-            }
-            bs[i] -= s;
-        }
-        __syncthreads();
-    }
-}
-
-// back: x <- L^-T y (right-looking over the columns of L^T: x_K = Linv_K^T y_K,
-// then y_I -= L_KI^T x_K for I < K, reading rows K*T..K*T+T-1 of L); acc: x
-// += the solution instead.
-__device__ void cta_back(int Np, int nb, const double *__restrict__ S, const double *__restrict__ Linv,
-                         double *ys, double *xs, double *__restrict__ x, bool acc, float2 *__restrict__ x2)
-{
-    const int tid = threadIdx.x, nthr = blockDim.x;
-    const int dc = tid / T, dk = tid % T;  // diagonal product: output column, term
-    auto load_diag = [&](int K) {
-        return (tid < TT && dk >= dc) ? __ldcg(Linv + (size_t)K * TT + dk * T + dc) : 0.0;
-    };
-    auto load_panel = [&](int K, double (&v)[T]) {
-        if (tid < K * T) {
-            const double *base = S + (size_t)(K * T) * Np + tid;
-#pragma unroll
-            for (int c = 0; c < T; ++c) v[c] = __ldcg(base + (size_t)c * Np);
-        }
-    };
-    double curL = load_diag(nb - 1), curS[T] = {}, nxtS[T] = {};
-    load_panel(nb - 1, curS);
-    for (int K = nb - 1; K >= 0; --K) {
-        double nxtL = 0.0;
-        if (K > 0) {
-            nxtL = load_diag(K - 1);
-            load_panel(K - 1, nxtS);
-        }
-        if (tid < TT) {
-            const double v = half_warp_sum(curL * ys[K * T + dk]);
-            if (dk == 0) {
-                xs[dc] = v;
-                const double xv = acc ? x[K * T + dc] + v : v;
-                x[K * T + dc] = xv;
-                if (x2) x2[K * T + dc] = split2f(xv);
-            }
-        }
-        __syncthreads();
-        if (tid < K * T) {
-            double s = 0.0;
-#pragma unroll
-            for (int c = 0; c < T; ++c) s = fma(curS[c], xs[c], s);
-            ys[tid] -= s;
-        }
-        for (int col = tid + nthr; col < K * T; col += nthr) {  // columns beyond the prefetched one
-            const double *base = S + (size_t)(K * T) * Np + col;
-            double v[T];
-#pragma unroll
-            for (int c = 0; c < T; ++c) v[c] = __ldcg(base + (size_t)c * Np);
-            double s = 0.0;
-#pragma unroll
-            for (int c = 0; c < T; ++c) s = fma(v[c], xs[c], s);
-            ys[col] -= s;
-        }
-        __syncthreads();
-        curL = nxtL;
-#pragma unroll
-        for (int c = 0; c < T; ++c) curS[c] = nxtS[c];
-    }
-}
-
 // Dealt-out tile products.  A tile operation costs the largest number of
 // FP64 instructions any thread of a warp runs, so the products below are
 // spread evenly over the CTA.
 
-// a[r][c] -= sum_k L[r][k] L[c][k] for c <= r and, when WITH_B,
+// a[r][c] -= sum_k L[r][k] L[c][k] for c <= r and
 // b[r] -= sum_k L[r][k] y[k]: the NE x T products (element, k) are cut into
 // consecutive runs of PER, one per thread; a run spans at most NACC
 // elements, whose partial sums go to part[NACC t ...].  Each element then
 // subtracts its partial sums in k order.  The accumulator and operands of a
 // product are picked by selects, so a warp issues one FMA per product.
-template <bool WITH_B>
 struct LowerUpdate {
     static constexpr int NT = CF_THREADS;
     static constexpr int NTRI = T * (T + 1) / 2;
-    static constexpr int NE = NTRI + (WITH_B ? T : 0);
+    static constexpr int NE = NTRI + T;
     static constexpr int PER = (NE * T + NT - 1) / NT;
     static constexpr int NACC = (T - 1 + PER + T - 1) / T;  // elements one run can touch
     static constexpr int PART = NACC * NT;                  // doubles of partial sums
 };
 
-template <bool WITH_B>
 __device__ void update_lower(double (*a)[T + 1], const double (*L)[T + 1], double *b, const double *y, double *part)
 {
     constexpr int NT = CF_THREADS;
-    using U = LowerUpdate<WITH_B>;
+    using U = LowerUpdate;
     constexpr int NTRI = U::NTRI, NE = U::NE, PER = U::PER, NACC = U::NACC;
     auto sync = [] { __syncthreads(); };
     const int tid = threadIdx.x;
@@ -659,7 +545,7 @@ __global__ void __launch_bounds__(CF_THREADS, 1) k_chol_dataflow(int Np, int nb,
                                                               int *__restrict__ flags, int epoch,
                                                               int *__restrict__ status, long long spin_limit)
 {
-    static_assert(LowerUpdate<true>::PART <= BJ * T * (T + 1), "update_lower's partial sums fit in the staging area");
+    static_assert(LowerUpdate::PART <= BJ * T * (T + 1), "update_lower's partial sums fit in the staging area");
     __shared__ double a[T][T + 1], linv[T][T + 1];
     __shared__ double bi[BJ][T][T + 1], bk[BJ][T][T + 1], by[BJ][T];
     __shared__ double bvec[T];
@@ -814,7 +700,7 @@ __global__ void __launch_bounds__(CF_THREADS, 1) k_chol_dataflow(int Np, int nb,
             __syncthreads();
             if (kind == 0) {
                 // the partial sums use bk, which the diagonal accumulation leaves free
-                for (int q = 0; q < n; ++q) update_lower<true>(a, bi[q], bvec, by[q], part);
+                for (int q = 0; q < n; ++q) update_lower(a, bi[q], bvec, by[q], part);
             } else {
                 for (int q = 0; q < n; ++q)
                     for (int e2 = tid; e2 < TT; e2 += CF_THREADS) {
@@ -865,7 +751,7 @@ __global__ void __launch_bounds__(CF_THREADS, 1) k_chol_dataflow(int Np, int nb,
             __syncthreads();
             const int r = tid / T, c = tid % T;
             if (kind == 0) {
-                update_lower<true>(a, bi[0], bvec, by[0], part);
+                update_lower(a, bi[0], bvec, by[0], part);
                 ulonglong2 *to = mail + (size_t)I * ML_COLUMN + ML_PD;
                 if (c <= r) mail_put(to + tri_at(r, c), a[r][c], epoch);
                 if (tid < T) mail_put(to + TRI + tid, bvec[tid], epoch);
@@ -938,26 +824,6 @@ int chol_grid(int n_tasks, int grid_cap)
     if (grid_cap > 0 && grid_cap < cap) cap = grid_cap;
     if (cap < 2) cap = 2;  // the panel and at least one helper
     return n_tasks < cap ? n_tasks : cap;
-}
-
-// The back solve L^T x = rhs in one CTA of TS_THREADS threads with the
-// right-hand side in shared memory (the factor's diagonal tasks already
-// applied L^-1 to rhs); refine = 1: both solves of rhs, added into x.  A
-// failed factor (status != 0) leaves x untouched.
-constexpr int TS_THREADS = 512;
-
-__global__ void __launch_bounds__(TS_THREADS) k_tri_solve(int refine, int Np, int nb, const double *__restrict__ S,
-                                                           const double *__restrict__ Linv,
-                                                           const double *__restrict__ rhs, double *__restrict__ x,
-                                                           float2 *__restrict__ x2, const int *__restrict__ status)
-{
-    extern __shared__ double vec[];  // Np
-    __shared__ double tmp[T];
-    if (*status != 0) return;
-    for (int i = threadIdx.x; i < Np; i += blockDim.x) vec[i] = rhs[i];
-    __syncthreads();
-    if (refine) cta_forward(Np, nb, S, Linv, vec, tmp);
-    cta_back(Np, nb, S, Linv, vec, tmp, x, refine != 0, x2);
 }
 
 // ---------------------------------------------------------------------------
@@ -1292,7 +1158,6 @@ void launch_tri(const DeviceProblem &d, int refine, double *x, cudaStream_t s)
     // the solution also as FP32 pairs for the mixed form's eb sums (x is dpa
     // on every path that reaches them)
     float2 *x2 = d.prec == PSBA_PREC_MIXED && d.cnp == 6 ? d.dpa2f : nullptr;
-#if PSBA_TRI_CLUSTER
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(TC_CTAS);
     cfg.blockDim = dim3(TC_THREADS);
@@ -1309,9 +1174,6 @@ void launch_tri(const DeviceProblem &d, int refine, double *x, cudaStream_t s)
     cfg.numAttrs = 1;
     const double *S = d.S, *Linv = d.Linv, *rhs = d.rhs;
     cudaLaunchKernelEx(&cfg, k_tri_cluster, refine, Np, nb, S, Linv, rhs, x, x2, d.status, d.wait_limit);
-#else
-    k_tri_solve<<<1, TS_THREADS, sizeof(double) * Np, s>>>(refine, Np, nb, d.S, d.Linv, d.rhs, x, x2, d.status);
-#endif
     note_launch(1);
 }
 

@@ -584,20 +584,23 @@ int residual_stage_nc(const DeviceProblem &d)
     return (size_t)d.nc * RES_TAB * sizeof(double) <= 48 * 1024 ? d.nc : 0;
 }
 
-// k_residual's grid: four blocks of 256 per SM at most (its loop takes the rest)
-int residual_blocks(const DeviceProblem &d)
+// SMs of the current device, asked for once per device
+static int sm_count()
 {
     static std::mutex mu;
     static int sms_dev[MAX_DEVICES] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= MAX_DEVICES) dev = 0;
-    int sms = 0;
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        if (sms_dev[dev] == 0) cudaDeviceGetAttribute(&sms_dev[dev], cudaDevAttrMultiProcessorCount, dev);
-        sms = std::max(1, sms_dev[dev]);
-    }
+    std::lock_guard<std::mutex> lk(mu);
+    if (sms_dev[dev] == 0) cudaDeviceGetAttribute(&sms_dev[dev], cudaDevAttrMultiProcessorCount, dev);
+    return std::max(1, sms_dev[dev]);
+}
+
+// k_residual's grid: four blocks of 256 per SM at most (its loop takes the rest)
+int residual_blocks(const DeviceProblem &d)
+{
+    const int sms = sm_count();
     return std::max(1, std::min(ceil_div(d.no > 0 ? d.no : 1, 256), 4 * sms));
 }
 
@@ -1049,9 +1052,10 @@ void launch_camera_blocks(const DeviceProblem &d, double coeff, cudaStream_t s)
 {
     if (d.cnp != 6) return launch_camera_blocks_v(d, coeff, s);
     if (d.n_cam_units > 0) {
-        if (d.prec == PSBA_PREC_FP64 && d.n_cam_units <= 2 * 152 / 9)  // up to two CTAs per SM
+        const int sms = sm_count();
+        if (d.prec == PSBA_PREC_FP64 && d.n_cam_units <= 2 * sms / 9)  // up to two CTAs per SM
             k_camera_part<9><<<dim3(d.n_cam_units, 9), CAM_THREADS, 0, s>>>(d.cam_units, d.cam_obs, d.A, d.ex, d.cam_partial);
-        else if (d.prec == PSBA_PREC_FP64 && d.n_cam_units <= 152)
+        else if (d.prec == PSBA_PREC_FP64 && d.n_cam_units <= sms)
             k_camera_part<3><<<dim3(d.n_cam_units, 3), CAM_THREADS, 0, s>>>(d.cam_units, d.cam_obs, d.A, d.ex, d.cam_partial);
         else if (d.prec == PSBA_PREC_FP64)
             k_camera_partial<double><<<d.n_cam_units, CAM_THREADS, 0, s>>>(d.cam_units, d.cam_obs, d.A, d.ex,
@@ -1599,7 +1603,7 @@ void launch_schur_diag(const DeviceProblem &d, cudaStream_t s)
 void launch_schur_reduce(const DeviceProblem &d, double mu, cudaStream_t s)
 {
     if (d.Np > d.N) {
-        k_clear_padded<<<std::min(ceil_div((long long)d.Np * d.Np / 2, 256), 152 * 8), 256, 0, s>>>(d.N, d.Np, d.S, d.rhs);
+        k_clear_padded<<<std::min(ceil_div((long long)d.Np * d.Np / 2, 256), sm_count() * 8), 256, 0, s>>>(d.N, d.Np, d.S, d.rhs);
         note_launch(1);
     } else {
         cudaMemsetAsync(d.S, 0, sizeof(double) * (size_t)d.Np * d.Np, s);
@@ -1843,9 +1847,6 @@ __global__ void __launch_bounds__(256) k_eb_dpb(int np, int ncp, const int2 *__r
     }
 }
 
-// k_eb_dpb blocks: EB_WARPS warps of the schedule each, at least np / EB_PPB
-// (the variable-intrinsics version uses one thread per point, and its
-// surplus blocks write zero partials)
 // 11/16-parameter cameras: eb = gb - sum_j W_ij^T dpa_j from the
 // observations' sums, dpb = V^-1 eb and the trial's step scalars, a thread per point.
 __global__ void __launch_bounds__(256) k_eb_finish(int np, int ncp, const int *__restrict__ pt_start,
@@ -1911,6 +1912,7 @@ __global__ void __launch_bounds__(256) k_eb_finish(int np, int ncp, const int *_
     }
 }
 
+// k_eb_dpb's blocks: EB_WARPS warps of the schedule each
 int eb_blocks(const DeviceProblem &d) { return d.n_eb_warps / EB_WARPS; }
 
 void launch_eb_dpb(const DeviceProblem &d, double mu, cudaStream_t s)
