@@ -73,7 +73,7 @@ UNIT = "iterations/s"
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per launch, from
 # one ncu capture of this workload's kernels.
-SCHUR_TRAFFIC = 275.4e6  # k_schur_fx6: 248.9 MB read + 26.5 MB written
+SCHUR_TRAFFIC = 363.6e6  # k_schur_fx6: 323.0 MB read + 40.6 MB written
 INT_MADS = 27.7  # 32 x 32 + 64-bit integer multiply-adds per clock and SM, measured
 CHOL_TRAFFIC = 1.6e6  # S (2.2 MB) stays in L2 between the Schur stage and the factor
 SCHUR_F32_TRAFFIC = 83.1e6  # k_schur_f32, mixed form: 79.8 MB read + 3.3 MB written

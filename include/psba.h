@@ -243,15 +243,17 @@ int psba_eval_cholmod(int n, double *S, double *E);
  * by the caller: S row-major, lower triangle read, 1 <= n <= 4096; x = S^-1 b.
  * *status is 0 when S was factored, 1 when a pivot was not positive, finite
  * and normal (the reference's failure test, SPD_inv.cl:66-107; subnormal
- * pivots count as failures here), 2 when a device-side wait ran out.
+ * pivots count as failures here, and so do four in a row below 2^-60 of what
+ * their diagonal entries were before a tile's last update), 2 when a device-side wait ran out.
  * Replaces SPDinv + matVec_mul (PSBA/cl_spdinv.cpp:18-40,
  * PSBA/cl_linearalg.cpp:19-55) for parity checks at any size. */
 int psba_eval_dense_solve(int n, const double *S, const double *b, double *x, int *status);
 
-/* The dense factor's pivot reciprocal (the hardware's approximate reciprocal
- * refined by one order-3 Householder step) applied to n values on the
- * device, for accuracy checks against the correctly rounded 1.0 / x.  No
- * reference counterpart: the reference divides (SPD_inv.cl:60-111). */
+/* The reciprocal of the projections' 1 / depth and of V^-1's determinant (the
+ * hardware's approximate reciprocal refined by one order-3 Householder step)
+ * applied to n values on the device, for accuracy checks against the correctly
+ * rounded 1.0 / x.  (The dense factor, after whose pivots the entry point is
+ * named, divides by none.)  No reference counterpart: the reference divides. */
 int psba_eval_pivot_reciprocal(int n, const double *x, double *y);
 
 /* ---- measurement (no reference counterpart: the reference only keeps

@@ -383,7 +383,7 @@ def dense_solve(S, b):
 
 
 def pivot_reciprocal(x):
-    """The dense factor's pivot reciprocal, evaluated on the device."""
+    """The projections' reciprocal (1 / depth), evaluated on the device."""
     x = _f64(x).ravel()
     y = np.empty_like(x)
     _check(lib().psba_eval_pivot_reciprocal(x.size, _d(x), _d(y)))

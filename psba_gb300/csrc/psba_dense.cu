@@ -1553,7 +1553,7 @@ void launch_cholmod(double *S, int n, int ld, double *E, double *work, cudaStrea
 
 // ---------------------------------------------------------------------------
 // Diagnostic entry points for the parity tests: the dense solve on a caller
-// matrix, and the pivot chain's reciprocal.
+// matrix, and the projections' reciprocal.
 namespace psba {
 
 __global__ void k_pivot_reciprocal(int n, const double *__restrict__ x, double *__restrict__ y)

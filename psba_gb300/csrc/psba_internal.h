@@ -16,8 +16,8 @@ namespace psba {
 // 1 / x: the hardware's approximate reciprocal (rcp.approx.ftz.f64, ~2^-20
 // relative error) and one step of the order-3 Householder iteration for
 // f(y) = 1/y - x: with e = 1 - x y, y <- y (1 + e + e^2), cubing the
-// relative error.  Within 1 ulp of 1.0 / x for x in [2^-80, 2^80] (the dense
-// factor's pivot chain; the projections' 1 / depth), in ~200 cycles and four
+// relative error.  Within 1 ulp of 1.0 / x for x in [2^-80, 2^80] (the
+// projections' 1 / depth, V^-1's determinant), in ~200 cycles and four
 // FP64 instructions against ~330 cycles for the division.
 #ifdef __CUDACC__
 __device__ __forceinline__ double rcp_fast(double x)

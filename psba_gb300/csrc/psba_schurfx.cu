@@ -24,8 +24,8 @@ inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 // Y and the limb rows.  A CTA takes LR_THREADS / TPO consecutive observations
 // (their W rows are contiguous), TPO threads each, TR rows a thread; rows go
 // through shared memory so that global loads and stores are coalesced.
-// Bound by the FP64 pipe (9 multiply-adds a row) and the ~25 integer
-// instructions that cut a value.
+// Bound by the FP64 pipe (9 multiply-adds a row) and the ~35 integer
+// instructions that cut a value (88 cameras: 51 us).
 constexpr int LR_THREADS = 128;
 
 template <int CNP>
@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(FV_THREADS) k_camera_fx(const CamUnit *__restr
     }
     // the thread's LD values of a chunk: the next chunk's are on their way while
     // this one is summed, and their observations' indices one chunk before that
-    // (52 cameras: 99.4 -> 81.9 us)
+    // (52 cameras, two limbs a factor: 99.4 -> 81.9 us; with the third piece 109)
     constexpr int LD = (FX_CHUNK * 2 * NC + FV_THREADS - 1) / FV_THREADS;
     int oi[LD];
     double v[LD];
